@@ -25,7 +25,8 @@ OUT_DIR = PKG / "lib"
 OUT = OUT_DIR / "libsocu_b200.so"
 STAMP = OUT_DIR / ".build_stamp"
 
-SOURCES = ["capi.cu", "peak.cu", "tc_selftest.cu"]
+SOURCES = ["capi.cu", "node_rows_f32.cu", "node_rows_f64.cu", "peak.cu", "ragged_f32.cu", "ragged_f64.cu",
+           "ragged_mixed.cu", "sweeps_f32.cu", "sweeps_f64.cu", "tc_selftest.cu"]
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 
 

@@ -14,6 +14,7 @@
 
 #include "../../include/socu_b200.h"
 #include "grad.cuh"
+#include "node_rows.cuh"
 #include "ragged.cuh"
 #include "tc_node.cuh"
 #include "tc_update.cuh"
@@ -117,56 +118,11 @@ cudaError_t prepare(K kernel, size_t smem) {
   return e;
 }
 
-// Threads per CTA for a node launch: 128 instead of 256 when the narrower
-// CTAs (twice as many resident per SM) finish the level in fewer waves, as on
-// the wide bottom level of the float factor (measured: 80 -> 70 us for 512
-// n = 64 nodes; the Schur-update launches lose more per CTA than the waves
-// save and keep 256).  Occupancies are cached per kernel, device,
-// shared-memory size and thread count.
-struct OccSlot {
-  const void* fn;
-  int dev;
-  size_t smem;
-  int threads, blocks;
-};
-std::mutex g_occ_mu;
-OccSlot g_occ[kCacheSlots];
-int g_n_occ = 0;
-
-template <typename K>
-int occupancy(K kernel, int dev, int threads, size_t smem) {
-  const void* fn = reinterpret_cast<const void*>(kernel);
-  std::lock_guard<std::mutex> g(g_occ_mu);
-  for (int i = 0; i < g_n_occ; ++i)
-    if (g_occ[i].fn == fn && g_occ[i].dev == dev && g_occ[i].smem == smem && g_occ[i].threads == threads)
-      return g_occ[i].blocks;
-  int v = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&v, kernel, threads, smem) != cudaSuccess) {
-    v = 0;
-    (void)cudaGetLastError();   // the fallback path handles it; do not leave the error pending
-  }
-  if (g_n_occ < kCacheSlots) g_occ[g_n_occ++] = OccSlot{fn, dev, smem, threads, v};
-  return v;
-}
-
 int sm_count() {
   int dev = 0, sms = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
     return 0;
   return sms;
-}
-
-template <typename K, class Smem>
-int level_threads(K kernel, int nth, long long blocks, Smem smem) {
-  if (nth != 256 || blocks <= 0) return nth;
-  int dev = 0;
-  const int sms = sm_count();
-  if (sms <= 0 || cudaGetDevice(&dev) != cudaSuccess) return nth;
-  const int o256 = occupancy(kernel, dev, 256, smem(256)), o128 = occupancy(kernel, dev, 128, smem(128));
-  if (o256 <= 0 || o128 <= 0) return nth;
-  const long long w256 = (blocks + (long long)sms * o256 - 1) / ((long long)sms * o256);
-  const long long w128 = (blocks + (long long)sms * o128 - 1) / ((long long)sms * o128);
-  return w128 < w256 ? 128 : 256;
 }
 
 // ---------------------------------------------------------------------------
@@ -590,21 +546,14 @@ int enqueue(socu_op op, const Problem<T>& p, cudaStream_t st, long long* count, 
   const int K = lv.K;
   for (int l = 0; l < K; ++l) lv.lv[l].tile = tile;
   const bool withY = op == SOCU_OP_FACTOR_AND_SOLVE;
-  // node shared memory by CTA size (the register-resident chain's buffers only where it runs)
-  auto node_smem = [&](int threads) {
-    return (size_t)smem_node_launch_elems(n, withY ? p.m : 0, sizeof(T), threads) * sizeof(T);
-  };
-  const size_t sd = node_smem(256);   // the largest
   const size_t su = smem_update_launch_elems(n, sizeof(T), tile) * sizeof(T);
   const int mm = p.m > 0 ? p.m : 1;
   const bool res = (long long)smem_sweep_res_elems(n, mm) * (long long)sizeof(T) <= (long long)max_smem_optin();
   const size_t ss = (res ? smem_sweep_res_elems(n, mm) : smem_sweep_elems(n, mm)) * sizeof(T);
   inv = inv && res && n <= 64;
-  auto node_kernel = withY ? (inv ? k_node<T, true, true> : k_node<T, true, false>)
-                           : (inv ? k_node<T, false, true> : k_node<T, false, false>);
-  auto fwd_kernel = res ? (inv ? k_fwd<T, true, false, true> : k_fwd<T, true>) : k_fwd<T, false>;
-  auto pull_kernel = res ? k_fwd<T, true, true> : k_fwd<T, false, true>;
-  auto bwd_kernel = res ? (inv ? k_bwd<T, true, true> : k_bwd<T, true>) : k_bwd<T, false>;
+  const SweepFn<T> fwd_kernel = sweep_kernel<T>(kSweepForward, res, inv);
+  const SweepFn<T> pull_kernel = sweep_kernel<T>(kSweepPull, res, inv);
+  const SweepFn<T> bwd_kernel = sweep_kernel<T>(kSweepBackward, res, inv);
   // Schur updates of float factors on the tcgen05 tensor cores (3xTF32), on
   // request: the FP64-pipe updates (exact products of the float operands,
   // FP64 sums) keep the float factor accurate enough for the reference's
@@ -629,6 +578,8 @@ int enqueue(socu_op op, const Problem<T>& p, cudaStream_t st, long long* count, 
                        smem_node_tm_bytes(n, m_node) <= (long long)max_smem_optin();
   const size_t sd_tm = (size_t)smem_node_tm_bytes(n, m_node);
   auto node_tm_kernel = withY ? k_node_tm<true> : k_node_tm<false>;
+  const size_t sd_rows = (size_t)smem_rows_bytes(n);
+  const NodeRowsFn<T> rows_kernel = node_rows_kernel<T>(n);
   long long launches = 0;
   const bool run = count == nullptr;
   const int sms = run ? sm_count() : 0;
@@ -638,7 +589,7 @@ int enqueue(socu_op op, const Problem<T>& p, cudaStream_t st, long long* count, 
   if (run) {
     cudaError_t e = cudaSuccess;
     if (op == SOCU_OP_FACTOR || op == SOCU_OP_FACTOR_AND_SOLVE) {
-      e = prepare(node_kernel, sd);
+      e = prepare(rows_kernel, sd_rows);
       if (e == cudaSuccess) e = update_uses_big(n) ? prepare(k_update_big<T>, su) : prepare(k_update<T>, su);
       if (e == cudaSuccess && upd_tc) e = prepare(k_update_tc, su_tc);
       if (e == cudaSuccess && node_tc_any) e = prepare(node_tc_kernel, sd_tc);
@@ -681,9 +632,27 @@ int enqueue(socu_op op, const Problem<T>& p, cudaStream_t st, long long* count, 
   SweepMaps maps;
   std::memset(&maps, 0, sizeof maps);
   if (run && res) maps = sweep_maps(p);
-  auto node_threads = [&](long long blocks) {
-    if (cfg.node_threads) return cfg.node_threads;
-    return run ? level_threads(node_kernel, nth, blocks, node_smem) : nth;
+  // Level nodes: k_node_rows.  On levels with fewer nodes than
+  // SMs a cluster of up to 8 blocks shares each node's row tiles (as many as
+  // there are blocks' worth of row tiles outside L_i, while every block still
+  // gets an SM of its own).
+  auto go_rows = [&](long long nodes, const Level& L) {
+    if (nodes <= 0) return;
+    ++launches;
+    if (!run) return;
+    const int nta = ceil_div(n, 8), warps = rows_warps(rows_nt(n));
+    const int tiles = 3 * nta + (withY ? ceil_div(p.m, 8) : 0);
+    int splits = 1;
+    while (splits < 8 && splits * 4 < tiles && nodes * splits * 2 <= sms) splits *= 2;
+    const bool pdl = !first && g_prof == nullptr;
+    first = false;
+    prof_begin(st, SOCU_KIND_NODE);
+    const unsigned blocks = (unsigned)(nodes * splits), threads = 32u * (unsigned)warps;
+    if (splits > 1)
+      launch_cluster(rows_kernel, blocks, threads, sd_rows, st, pdl, splits, p, L, splits, (int)withY, (int)inv);
+    else
+      launch(rows_kernel, blocks, threads, sd_rows, st, pdl, p, L, splits, (int)withY, (int)inv);
+    prof_end(st);
   };
   const bool forked = run && fork != nullptr && fork->ok();
 
@@ -697,7 +666,7 @@ int enqueue(socu_op op, const Problem<T>& p, cudaStream_t st, long long* count, 
   const bool want_fwd = op == SOCU_OP_FORWARD_SUBSTITUTION || op == SOCU_OP_SOLVE;
   const bool want_bwd =
       op == SOCU_OP_BACKWARD_SUBSTITUTION || op == SOCU_OP_SOLVE || op == SOCU_OP_FACTOR_AND_SOLVE;
-  auto top_kernel = inv ? k_top<T, true> : k_top<T, false>;
+  const TopFn<T> top_kernel = top_sweep_kernel<T>(inv);
   TopLevels top;
   std::memset(&top, 0, sizeof top);
   int top_cluster = 0;
@@ -762,32 +731,14 @@ int enqueue(socu_op op, const Problem<T>& p, cudaStream_t st, long long* count, 
       const long long node_blocks = (long long)p.B * L.d;
       if constexpr (sizeof(T) == 4) {
         const bool node_tc = node_tc_any && (!node_tc_wide_only || node_blocks >= 4LL * sms);
-        // inverse-first nodes on levels that fit one wave of CTAs with the W^T
-        // buffer: the chain also writes W^T and the products run from it
-        auto node_wt_kernel = withY ? (inv ? k_node<float, true, true, true> : k_node<float, true, false, true>)
-                                    : (inv ? k_node<float, false, true, true> : k_node<float, false, false, true>);
-        const size_t sd_wt = (size_t)smem_node_gemm_elems(n, withY ? p.m : 0, 4, true) * 4;
-        const int nthr = node_threads(node_blocks);
-        bool node_wt = false;
-        if (run && !node_tm && !node_tc && node_uses_gemm(n) && reg_chain_ok(n, nthr) &&
-            sd_wt <= (size_t)max_smem_optin() && sms > 0 && prepare(node_wt_kernel, sd_wt) == cudaSuccess) {
-          int dev = 0;
-          cudaGetDevice(&dev);
-          node_wt = (long long)occupancy(node_wt_kernel, dev, nthr, sd_wt) * sms >= node_blocks;
-        }
         if (node_tm)
           go_on(st, node_tm_kernel, SOCU_KIND_NODE, node_blocks, sd_tm, L, 256);
         else if (node_tc)
           go_on(st, node_tc_kernel, SOCU_KIND_NODE, node_blocks, sd_tc, L, 256);
-        else if (node_wt)
-          go_on(st, node_wt_kernel, SOCU_KIND_NODE, node_blocks, sd_wt, L, nthr);
         else
-          go_on(st, node_kernel, SOCU_KIND_NODE, node_blocks, node_smem(nthr), L, nthr);
+          go_rows(node_blocks, L);
       } else {
-        {
-          const int nthr = node_threads(node_blocks);
-          go_on(st, node_kernel, SOCU_KIND_NODE, node_blocks, node_smem(nthr), L, nthr);
-        }
+        go_rows(node_blocks, L);
       }
       if (l + 1 < K) {
         // fused forward: apply this level's updates to every target vector
@@ -1328,7 +1279,7 @@ void rg_free(socu_ragged_s* r) {
 
 template <typename T, int MODE>
 int rg_prepare_kernel(socu_ragged_s* r) {
-  auto kern = k_ragged<T, MODE>;
+  auto kern = ragged_kernel<T, MODE>();
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)r->smem);
   int per_sm = 0, sms = 0;
   if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kRgThreads, r->smem);
@@ -1373,7 +1324,7 @@ int rg_create(socu_ragged_s* r, const int64_t* horizon, const int64_t* n, const 
   // shared memory: the largest body at the largest block size (n <= 64: the
   // inverse-first node body)
   r->vc = maxnv;
-  size_t smem = (size_t)smem_node_gemm_elems(maxn, maxm, es, false, false) * es;   // ragged nodes: shared-memory chain (measured faster there)
+  size_t smem = (size_t)smem_node_gemm_elems(maxn, maxm, es) * es;
   smem = std::max(smem, (size_t)smem_update_full_elems(maxn, es) * es);
   smem = std::max(smem, (size_t)smem_sweep_res_elems(maxn, maxm) * es);
   if (r->refine) smem = std::max(smem, (size_t)smem_residual_rows_elems(maxn) * sizeof(double));
@@ -1434,7 +1385,7 @@ int rg_launch(socu_ragged_s* r, RgArgs<T> a, cudaStream_t st) {
   const int sb = (int)std::min<long long>((work + 255) / 256, 1024);
   prof_begin(st, SOCU_KIND_RAGGED);
   k_rg_start<T, MODE><<<sb, 256, 0, st>>>(a);
-  k_ragged<T, MODE><<<r->grid, kRgThreads, r->smem, st>>>(a);
+  ragged_kernel<T, MODE>()<<<r->grid, kRgThreads, r->smem, st>>>(a);
   prof_end(st);
   return cuda_status(cudaGetLastError());
 }
@@ -1636,7 +1587,7 @@ int64_t socu_max_block_size(socu_dtype dtype, int64_t n_rhs) {
   const long long limit = max_smem_optin();
   int64_t best = 0;
   for (int n = 1; n <= 512; ++n) {
-    long long need = smem_node_elems(n, (int)es);
+    long long need = smem_rows_bytes(n) / (long long)es;
     const long long u = smem_update_elems(n, (int)es), s = smem_sweep_elems(n, m > 0 ? m : 1);
     if (u > need) need = u;
     if (s > need) need = s;
@@ -2025,6 +1976,11 @@ int socu_tc_error(int* flag, int reset) {
     const int zero = 0;
     e = cudaMemcpyToSymbol(g_tc_error, &zero, sizeof(int));
   }
+  int sweep = 0;
+  if (e == cudaSuccess) e = sweep_wait_error<float>(&sweep, reset != 0);
+  if (e == cudaSuccess && *flag == 0) *flag = sweep;
+  if (e == cudaSuccess) e = sweep_wait_error<double>(&sweep, reset != 0);
+  if (e == cudaSuccess && *flag == 0) *flag = sweep;
   return cuda_status(e);
 }
 

@@ -1,0 +1,502 @@
+// Level node as rows of 8x8 tiles held in registers (n <= 128), one thread
+// block per node (or a thread-block cluster of `splits` blocks on levels with
+// fewer nodes than SMs).
+//
+// The node's Cholesky factor C and everything multiplied by C^{-T} are one
+// matrix of row tiles over the same 8-column steps:
+//     X = [ L_i ; R ; Lf^T ; y^T ; I ],      X <- X C^{-T}
+// whose rows end as C, F = R C^{-T}, G^T = Lf^T C^{-T}, (C^{-1} y)^T and
+// W^T = C^{-T}: exactly the blocks the factor stores.  A warp owns a whole row
+// tile (8 x n) as FP64 tensor-core accumulators (mma.m8n8k4 .f64, fragment
+// {c0, c1} = C[g][2t + {0, 1}], g = lane / 4, t = lane % 4), read from global
+// memory straight into registers.  Step k:
+//   1. the warp of row k factors its diagonal tile with shuffles
+//      (warp_chol8) and publishes Inv_k = C_kk^{-1} in shared memory;
+//   2. every later row multiplies its tile k by Inv_k^T: the final tile P,
+//      stored to global memory at once and, for rows of L_i, to shared memory;
+//   3. every later row subtracts P P_j^T from its tiles j > k.
+// The accumulator fragment is the A operand of the next product without any
+// shuffle: the contraction index is enumerated as 2t, 2t + 1 (one MMA each),
+// and the B operand (a row of Inv_k or of P_j) is then one 16-byte load.
+//
+// Rows of L_i go through the steps together (phase 1, two barriers per step;
+// the warp of row k + 1 has one tile left to update, so it reaches its factor
+// while the other warps still update).  The other rows only read what phase 1
+// left in shared memory, so each warp takes them one row tile at a time with
+// no barrier (phase 2); the first one is loaded when the warp leaves phase 1.
+//
+// Bound by the latency of phase 1: per step one tile factor (770 cycles FP64,
+// 556 float) and two dependent MMA pairs, about 1200 / 950 cycles.  The blocks
+// of a cluster repeat phase 1 and share out phase 2; the cluster barrier keeps
+// one block from overwriting L_i before the others have read it.  Measured,
+// all level nodes of one factor_and_solve (event-timed launches), against the
+// blocked solve in shared memory that it replaces: N=1024, n=64, m=8 FP64
+// 409 -> 214 us, float 373 -> 212 us; N=2048, n=128, m=32 FP64 3308 -> 995 us.
+#pragma once
+
+#include "nd_kernels.cuh"
+
+namespace socu {
+
+constexpr int kRowsMaxN = 128;
+__host__ __device__ inline bool node_uses_rows(int n) { return n <= kRowsMaxN; }
+// 8-column tiles: exact up to 64, then even counts (fewer instantiations)
+__host__ __device__ inline int rows_nt(int n) {
+  const int t = (n + 7) / 8;
+  return t <= 8 ? t : ((t + 1) & ~1);
+}
+// row stride of the shared factor: 8 (mod 16) doubles, so the 16-byte operand
+// loads of a quarter warp (two rows of 64 bytes) cover all banks
+__host__ __device__ inline int rows_ld(int nt) { return (nt & 1) ? 8 * nt : 8 * nt + 8; }
+__host__ __device__ inline int rows_warps(int nt) { return nt < 4 ? 4 : nt; }
+__host__ __device__ inline long long smem_rows_bytes(int n) {
+  const int nt = rows_nt(n);
+  return 8LL * (8LL * nt * rows_ld(nt) + 128LL * nt);
+}
+
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;\n" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;\n" ::: "memory"); }
+
+// Accumulate one MMA.  Not volatile: the compiler may interleave independent ones.
+__device__ __forceinline__ void mma_acc(double& c0, double& c1, double a, double b) {
+  asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
+      : "+d"(c0), "+d"(c1)
+      : "d"(a), "d"(b));
+}
+
+// named barriers: producers arrive, consumers wait
+__device__ __forceinline__ void bar_arrive(int id, int threads) {
+  asm volatile("bar.arrive %0, %1;\n" ::"r"(id), "r"(threads) : "memory");
+}
+__device__ __forceinline__ void bar_wait(int id, int threads) {
+  asm volatile("bar.sync %0, %1;\n" ::"r"(id), "r"(threads) : "memory");
+}
+
+// 1 / sqrt(d) without a branch: the approximate instruction, then one step of
+// Householder's third-order iteration y (1 + e/2 + 3 e^2 / 8), e = 1 - d y^2.
+// For normal d; a subnormal one (flushed by the instruction) gives NaN, and the
+// caller starts over with the library function.
+template <typename T, bool FAST>
+__device__ __forceinline__ T pivot_rsqrt(T d) {
+  if constexpr (FAST && sizeof(T) == 8) {
+    double y;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(d));
+    const double e = fma(-(d * y), y, 1.0);
+    return fma(y * e, fma(e, 0.375, 0.5), y);
+  } else {
+    return rsqrt_t(d);
+  }
+}
+
+// Cholesky factor of the 8x8 tile in S (lower triangle, left in c) and its
+// inverse, written to Ivk (8 x 8, lane l the column l % 8).  Every lane of the
+// warp factors the whole tile: the chain is 8 times rsqrt -> multiply ->
+// subtract, about 70 cycles each in FP64, with no exchange between lanes.
+// Measured per tile: 770 cycles FP64, 556 float; spread over the lanes instead
+// (16 shuffles a column, which issue every 4.3 cycles) 1500 and 790.
+template <typename T, bool FAST>
+__device__ __forceinline__ void chol8_tile(const T* S, double* Ivk, T (&c)[8][8]) {
+  const int col = threadIdx.x & 7;
+  T y[8];
+#pragma unroll
+  for (int i = 0; i < 8; ++i)
+#pragma unroll
+    for (int j = 0; j <= i; j += 2) {
+      if constexpr (sizeof(T) == 8) {
+        const double2 v = *reinterpret_cast<const double2*>(S + 8 * i + j);
+        c[i][j] = v.x;
+        c[i][j + 1] = v.y;
+      } else {
+        const float2 v = *reinterpret_cast<const float2*>(S + 8 * i + j);
+        c[i][j] = v.x;
+        c[i][j + 1] = v.y;
+      }
+    }
+#pragma unroll
+  for (int i = 0; i < 8; ++i) y[i] = T(0);
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    const T r = pivot_rsqrt<T, FAST>(c[j][j]);
+#pragma unroll
+    for (int i = j; i < 8; ++i) c[i][j] *= r;
+#pragma unroll
+    for (int l = j + 1; l < 8; ++l)
+#pragma unroll
+      for (int i = l; i < 8; ++i) c[i][l] = fma(-c[i][j], c[l][j], c[i][l]);
+    y[j] = j == col ? r : y[j] * r;
+#pragma unroll
+    for (int i = j + 1; i < 8; ++i) y[i] = fma(-c[i][j], y[j], y[i]);
+    Ivk[8 * j + col] = (double)y[j];
+  }
+}
+
+template <typename T>
+__device__ __forceinline__ void chol8_keep(T* S, const T (&c)[8][8]) {
+#pragma unroll
+  for (int i = 0; i < 8; ++i)
+#pragma unroll
+    for (int j = 0; j <= i; ++j) S[8 * i + j] = c[i][j];   // every lane writes the same values
+}
+
+// the factor with the library's reciprocal square root (subnormal pivots)
+template <typename T>
+__device__ __noinline__ void chol8_redo(T* S, double* Ivk) {
+  T c[8][8];
+  chol8_tile<T, false>(S, Ivk, c);
+  __syncwarp();
+  chol8_keep(S, c);
+}
+
+// Factor the diagonal tile held as an accumulator fragment (d0, d1): its
+// inverse goes to Ivk, then publish() runs, then lower(C_kk) goes to S (8 x 8,
+// first the tile's scratch).  All lanes of the warp; the caller orders its reads
+// of S and Ivk with __syncwarp.
+template <typename T, class Publish>
+__device__ __forceinline__ void rows_factor_tile(double d0, double d1, T* S, double* Ivk, Publish publish) {
+  const int lane = threadIdx.x & 31;
+  if constexpr (sizeof(T) == 8)
+    *reinterpret_cast<double2*>(S + 2 * lane) = make_double2(d0, d1);
+  else
+    *reinterpret_cast<float2*>(S + 2 * lane) = make_float2((float)d0, (float)d1);
+  __syncwarp();
+  T c[8][8];
+  chol8_tile<T, true>(S, Ivk, c);
+  // a NaN reaches the last pivot from any earlier one
+  const bool redo = sizeof(T) == 8 && c[7][7] != c[7][7];
+  if (redo) chol8_redo<T>(S, Ivk);
+  publish();
+  if (!redo) chol8_keep(S, c);
+}
+
+// two consecutive elements, widened; `vec`: the pair is aligned and inside
+template <typename T>
+__device__ __forceinline__ void load_pair(const T* p, bool vec, bool v0, bool v1, double& x0, double& x1) {
+  if (vec) {
+    if constexpr (sizeof(T) == 8) {
+      const double2 v = *reinterpret_cast<const double2*>(p);
+      x0 = v.x;
+      x1 = v.y;
+    } else {
+      const float2 v = *reinterpret_cast<const float2*>(p);
+      x0 = (double)v.x;
+      x1 = (double)v.y;
+    }
+  } else {
+    x0 = v0 ? (double)p[0] : 0.0;
+    x1 = v1 ? (double)p[1] : 0.0;
+  }
+}
+template <typename T>
+__device__ __forceinline__ void store_pair(T* p, bool vec, bool v0, bool v1, double x0, double x1) {
+  if (vec) {
+    if constexpr (sizeof(T) == 8)
+      *reinterpret_cast<double2*>(p) = make_double2(x0, x1);
+    else
+      *reinterpret_cast<float2*>(p) = make_float2((float)x0, (float)x1);
+  } else {
+    if (v0) p[0] = (T)x0;
+    if (v1) p[1] = (T)x1;
+  }
+}
+
+// A row tile outside L_i: element (r, c) of X, r < lim, at base[r * rs + c * cs].
+// kind 0: a row-major block (cs = 1, rs = n); 1: a transposed block (rs = 1);
+// 2: rows of the identity (W^T), 3: zeros of the upper triangle of L_i.
+template <typename T>
+struct RowSrc {
+  int kind;
+  T* base;      // first element of the row tile
+  int ld;       // kind 0: rs; kind 1: cs
+  int lim;      // valid rows in the tile
+  int k0;       // first step
+};
+
+// X tile row: P = X_k Inv_k^T
+__device__ __forceinline__ void rows_panel(double& p0, double& p1, double x0, double x1, double2 iv) {
+  p0 = p1 = 0.0;
+  mma_acc(p0, p1, x0, iv.x);
+  mma_acc(p0, p1, x1, iv.y);
+}
+
+// (identity rows start at their own step: tile k0 is the identity, later tiles zero)
+template <typename T, int NT>
+__device__ __forceinline__ void rows_load(double (&acc)[NT][2], const RowSrc<T>& s, int n, bool vec) {
+  const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  const bool rv = g < s.lim;
+  if (s.kind == 0) {
+#pragma unroll
+    for (int j = 0; j < NT; ++j) {
+      const int c = 8 * j + 2 * t;
+      load_pair(s.base + (long long)g * s.ld + c, vec && 8 * j < n, rv && c < n, rv && c + 1 < n, acc[j][0], acc[j][1]);
+    }
+  } else if (s.kind == 1) {
+#pragma unroll
+    for (int j = 0; j < NT; ++j)
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        const int c = 8 * j + 2 * t + e;
+        acc[j][e] = (rv && c < n) ? (double)s.base[(long long)c * s.ld + g] : 0.0;
+      }
+  } else {
+#pragma unroll
+    for (int j = 0; j < NT; ++j)
+#pragma unroll
+      for (int e = 0; e < 2; ++e) acc[j][e] = (j == s.k0 && g == 2 * t + e) ? 1.0 : 0.0;
+  }
+}
+
+template <typename T, int NT>
+__device__ __forceinline__ void rows_store(const double (&acc)[NT][2], const RowSrc<T>& s, int n, bool vec) {
+  const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  const bool rv = g < s.lim;
+  if (s.kind == 1) {
+#pragma unroll
+    for (int j = 0; j < NT; ++j)
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        const int c = 8 * j + 2 * t + e;
+        if (rv && c < n) s.base[(long long)c * s.ld + g] = (T)acc[j][e];
+      }
+  } else {
+    // (rows of the identity: tiles right of the diagonal one, which is written with C_kk)
+    const int j0 = s.kind == 2 ? s.k0 + 1 : 0;
+#pragma unroll
+    for (int j = 0; j < NT; ++j) {
+      const int c = 8 * j + 2 * t;
+      if (j >= j0)
+        store_pair(s.base + (long long)g * s.ld + c, vec && 8 * j < n, rv && c < n, rv && c + 1 < n, acc[j][0], acc[j][1]);
+    }
+  }
+}
+
+// tiles j0 .. j0 + CH - 1 (below NT) of one row tile -= P P_j^T
+template <int NT, int CH>
+__device__ __forceinline__ void rows_update(double (&acc)[NT][2], int j0, double p0, double p1, const double* Ck,
+                                            int ld) {
+  double2 bv[CH];
+#pragma unroll
+  for (int h = 0; h < CH; ++h)
+    if (j0 + h < NT) bv[h] = *reinterpret_cast<const double2*>(Ck + 8 * (j0 + h) * ld);
+#pragma unroll
+  for (int h = 0; h < CH; ++h)
+    if (j0 + h < NT) mma_acc(acc[j0 + h][0], acc[j0 + h][1], -p0, bv[h].x);
+#pragma unroll
+  for (int h = 0; h < CH; ++h)
+    if (j0 + h < NT) mma_acc(acc[j0 + h][0], acc[j0 + h][1], -p1, bv[h].y);
+}
+
+// All steps of one row tile against the finished factor (FROM0: k0 is 0, and no
+// branch separates the steps; the tile that the next step starts from comes first).
+template <int NT, bool FROM0>
+__device__ __forceinline__ void rows_solve(double (&acc)[NT][2], int k0, int nta, const double* Cs, const double* Iv) {
+  constexpr int ld = (NT & 1) ? 8 * NT : 8 * NT + 8;
+  const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+#pragma unroll
+  for (int k = 0; k < NT; ++k) {
+    if ((FROM0 || k >= k0) && (NT <= 8 || k < nta)) {   // (NT is exact up to 8)
+      const double2 iv = *reinterpret_cast<const double2*>(Iv + 64 * k + 2 * lane);
+      const double* Ck = Cs + g * ld + 8 * k + 2 * t;
+      double p0, p1;
+      rows_panel(p0, p1, acc[k][0], acc[k][1], iv);
+      rows_update<NT, 1>(acc, k + 1, p0, p1, Ck, ld);
+#pragma unroll
+      for (int j = k + 2; j < NT; j += 4) rows_update<NT, 4>(acc, j, p0, p1, Ck, ld);
+      acc[k][0] = p0;
+      acc[k][1] = p1;
+    }
+  }
+}
+
+// One node.  q, splits: this block's share of the row tiles outside L_i (every
+// block of a cluster runs phase 1).  Warp w < n / 8 owns row tile w of L_i.
+template <typename T, int NT>
+__device__ __forceinline__ void node_rows_body(const Problem<T>& p, const Level& lv, int b, int t,
+                                               unsigned char* smem_raw, int q, int splits, bool with_y, bool inv) {
+  constexpr int ld = (NT & 1) ? 8 * NT : 8 * NT + 8;
+  const int lane = threadIdx.x & 31, row = threadIdx.x >> 5, W = blockDim.x >> 5;
+  const int g = lane >> 2, tq = lane & 3;
+  const int n = p.n, s = lv.s, i = s - 1 + 2 * s * t;
+  const int nta = (n + 7) >> 3;
+  const bool right = i + s < p.N, left = t >= 1;
+  double* Cs = reinterpret_cast<double*>(smem_raw);   // rows of C, 8 NT x ld
+  double* Iv = Cs + 8 * NT * ld;                      // Inv_k, 8 x 8 each
+  T* Ct = reinterpret_cast<T*>(Iv + 64 * NT);         // C_kk, 8 x 8 each
+  T* Li = p.Lb(b, i);
+  T* R = right ? p.Eb(b, lv.oc + 2 * t) : nullptr;
+  T* Lf = left ? p.Eb(b, lv.oc + 2 * t - 1) : nullptr;
+  T* yi = with_y ? p.Xb(b, i) : nullptr;
+  // paired accesses: whole tiles, and every row of a block on a pair boundary
+  const bool vec = n == 8 * nta && ((reinterpret_cast<uintptr_t>(p.L) | reinterpret_cast<uintptr_t>(p.E)) &
+                                    (2 * sizeof(T) - 1)) == 0;
+  const int vr = right ? nta : 0, vl = left ? nta : 0, vy = with_y ? (p.m + 7) >> 3 : 0;
+  const int vtot = vr + vl + vy + nta;
+  auto source = [&](int v) {
+    RowSrc<T> o;
+    o.ld = n;
+    o.k0 = 0;
+    if (v < vr) {
+      o.kind = 0;
+      o.base = R + (long long)8 * v * n;
+      o.lim = n - 8 * v;
+    } else if (v < vr + vl) {
+      const int c = v - vr;
+      o.kind = 1;
+      o.base = Lf + 8 * c;
+      o.lim = n - 8 * c;
+    } else if (v < vr + vl + vy) {
+      const int c = v - vr - vl;
+      o.kind = 1;
+      o.base = yi + 8 * c;
+      o.ld = p.m;
+      o.lim = p.m - 8 * c;
+    } else {
+      const int c = v - vr - vl - vy;
+      o.kind = inv ? 2 : 3;
+      o.base = Li + (long long)8 * c * n;
+      o.lim = n - 8 * c;
+      o.k0 = c;
+    }
+    return o;
+  };
+
+  // this warp's row tile of L_i (lower tiles; the padding of the last tile is an identity)
+  const int gr = 8 * row + g;
+  double acc[NT][2];
+#pragma unroll
+  for (int j = 0; j < NT; ++j) {
+    acc[j][0] = acc[j][1] = 0.0;
+    if (row < nta && j <= row) {
+      const int c = 8 * j + 2 * tq;
+      load_pair(Li + (long long)gr * n + c, vec, gr < n && c < n, gr < n && c + 1 < n, acc[j][0], acc[j][1]);
+      if (!vec && gr >= n) {
+        if (c == gr) acc[j][0] = 1.0;
+        if (c + 1 == gr) acc[j][1] = 1.0;
+      }
+    }
+  }
+  const int v_first = q + splits * row;
+  if (splits > 1) cluster_arrive();   // L_i is in this thread's registers
+
+  // Phase 1.  Barrier 1, step k: Inv_k is published (its warp arrives, later
+  // rows wait); barrier 2: the step's panel is published (row k + 1 arrives, as
+  // its own tile needs nothing else, later rows wait).  Warps past their row
+  // leave the steps and meet the others at the end.
+  if (row < nta) {
+    double d0 = acc[0][0], d1 = acc[0][1];
+#pragma unroll
+    for (int k = 0; k < NT - 1; ++k) {
+      if (k < row) {
+        const int after = nta - 1 - k;   // rows after k
+        bar_wait(1, 32 * (after + 1));
+        const double2 iv = *reinterpret_cast<const double2*>(Iv + 64 * k + 2 * lane);
+        double p0, p1;
+        rows_panel(p0, p1, acc[k][0], acc[k][1], iv);
+        *reinterpret_cast<double2*>(Cs + gr * ld + 8 * k + 2 * tq) = make_double2(p0, p1);
+        if (row == k + 1) {
+          if (after > 1) bar_arrive(2, 32 * after);
+          d0 = acc[k + 1][0];
+          d1 = acc[k + 1][1];
+          mma_acc(d0, d1, -p0, p0);
+          mma_acc(d0, d1, -p1, p1);
+        } else {
+          bar_wait(2, 32 * after);
+#pragma unroll
+          for (int j = k + 1; j < NT; j += 4)
+            if (j <= row) rows_update<NT, 4>(acc, j, p0, p1, Cs + g * ld + 8 * k + 2 * tq, ld);
+        }
+      }
+    }
+    rows_factor_tile<T>(d0, d1, Ct + 64 * row, Iv + 64 * row, [&] {
+      if (row + 1 < nta) bar_arrive(1, 32 * (nta - row));
+    });
+    if (splits > 1) cluster_wait();   // every block of the cluster has read L_i
+    if (q == 0) {
+      __syncwarp();
+      for (int j = 0; j < row; ++j) {
+        const double2 v = *reinterpret_cast<const double2*>(Cs + gr * ld + 8 * j + 2 * tq);
+        const int c = 8 * j + 2 * tq;
+        store_pair(Li + (long long)gr * n + c, vec, gr < n && c < n, gr < n && c + 1 < n, v.x, v.y);
+      }
+      // diagonal tile: C_kk and, above the diagonal, W^T (or zeros)
+      const double* Ik = Iv + 64 * row;
+      const double c0 = (double)Ct[64 * row + 2 * lane], c1 = (double)Ct[64 * row + 2 * lane + 1];
+      const int c = 8 * row + 2 * tq;
+      const double u0 = inv ? Ik[8 * (2 * tq) + g] : 0.0, u1 = inv ? Ik[8 * (2 * tq + 1) + g] : 0.0;
+      store_pair(Li + (long long)gr * n + c, vec, gr < n && c < n, gr < n && c + 1 < n, 2 * tq <= g ? c0 : u0,
+                 2 * tq + 1 <= g ? c1 : u1);
+      if (p.info != nullptr) {
+        const double dg = (g & 1) ? c1 : c0;   // lanes with t = g / 2 hold the diagonal
+        const bool bad = (g >> 1) == tq && gr < n && (!(dg > 0.0) || isinf(dg));
+        if (__any_sync(kFull, bad) && lane == 0) record_failure(p.info + b, i);
+      }
+    }
+  } else if (splits > 1) {
+    cluster_wait();
+  }
+  // (the first row tile arrives while later rows finish phase 1)
+  double av[NT][2];
+  if (v_first < vtot) rows_load<T, NT>(av, source(v_first), n, vec);
+  __syncthreads();   // the factor is complete in shared memory
+
+  // phase 2
+  for (int v = v_first; v < vtot; v += splits * W) {
+    const RowSrc<T> src = source(v);
+    if (src.kind == 3) {   // no inverse kept: zeros right of the diagonal tile
+      for (int k = src.k0 + 1; k < nta; ++k) {
+        const int c = 8 * k + 2 * tq;
+        store_pair(src.base + (long long)g * n + c, vec, g < src.lim && c < n, g < src.lim && c + 1 < n, 0.0, 0.0);
+      }
+      continue;
+    }
+    if (v != v_first) rows_load<T, NT>(av, src, n, vec);
+    if (src.kind == 2)
+      rows_solve<NT, false>(av, src.k0, nta, Cs, Iv);
+    else
+      rows_solve<NT, true>(av, 0, nta, Cs, Iv);
+    rows_store<T, NT>(av, src, n, vec);
+  }
+}
+
+template <typename T, int NT>
+__global__ void __launch_bounds__(32 * (NT < 4 ? 4 : NT), NT <= 4 ? 4 : (NT <= 8 ? 2 : 1))
+    k_node_rows(Problem<T> p, Level lv, int splits, int with_y, int inv) {
+  const int node = blockIdx.x / splits, q = blockIdx.x - node * splits;
+  const int b = node / lv.d, t = node - b * lv.d;
+  pdl_wait();
+  pdl_trigger();
+  if (!p.active(b)) return;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  node_rows_body<T, NT>(p, lv, b, t, smem_raw, q, splits, with_y != 0, inv != 0);
+}
+
+template <typename T>
+using NodeRowsFn = void (*)(Problem<T>, Level, int, int, int);
+
+// the kernel for block size n (node_rows_f32.cu, node_rows_f64.cu: one
+// translation unit per type, so the instantiations compile in parallel)
+template <typename T>
+NodeRowsFn<T> node_rows_kernel(int n);
+
+#define SOCU_NODE_ROWS_KERNELS(T)                      \
+  template <>                                          \
+  NodeRowsFn<T> node_rows_kernel<T>(int n) {           \
+    switch (rows_nt(n)) {                              \
+      case 1: return k_node_rows<T, 1>;                \
+      case 2: return k_node_rows<T, 2>;                \
+      case 3: return k_node_rows<T, 3>;                \
+      case 4: return k_node_rows<T, 4>;                \
+      case 5: return k_node_rows<T, 5>;                \
+      case 6: return k_node_rows<T, 6>;                \
+      case 7: return k_node_rows<T, 7>;                \
+      case 8: return k_node_rows<T, 8>;                \
+      case 10: return k_node_rows<T, 10>;              \
+      case 12: return k_node_rows<T, 12>;              \
+      case 14: return k_node_rows<T, 14>;              \
+      default: return k_node_rows<T, 16>;              \
+    }                                                  \
+  }
+
+template <> NodeRowsFn<float> node_rows_kernel<float>(int n);
+template <> NodeRowsFn<double> node_rows_kernel<double>(int n);
+
+}  // namespace socu

@@ -311,7 +311,7 @@ __device__ void rg_run(const RgArgs<T>& a, int ii, int ph, int chunk, unsigned c
     switch (P.kind) {
       case kRgNode: {
         const Problem<T> p = rg_problem(a, I, I.m);
-        node_gemm_body<T, true, true, false>(p, lv, 0, u, smem);
+        node_gemm_body<T, true, true>(p, lv, 0, u, smem);
         break;
       }
       case kRgUpd: {
@@ -469,5 +469,12 @@ __global__ void __launch_bounds__(kRgThreads, sizeof(T) == 8 ? 3 : 4) k_ragged(R
     __syncthreads();
   }
 }
+
+// the kernel (ragged_f64.cu, ragged_f32.cu, ragged_mixed.cu: one translation unit each)
+template <typename T, int MODE>
+void (*ragged_kernel())(RgArgs<T>);
+template <> void (*ragged_kernel<double, kRgPlain>())(RgArgs<double>);
+template <> void (*ragged_kernel<float, kRgPlain>())(RgArgs<float>);
+template <> void (*ragged_kernel<float, kRgRefine>())(RgArgs<float>);
 
 }  // namespace socu

@@ -63,7 +63,7 @@ __device__ __forceinline__ double block_max(double v, double* red) {
 }
 
 // Per-instance state reset (before k_ref_init accumulates into it).
-__global__ void k_ref_reset(RefineArgs a) {
+static __global__ void k_ref_reset(RefineArgs a) {
   pdl_wait();
   pdl_trigger();
   for (int bi = blockIdx.x * blockDim.x + threadIdx.x; bi < a.B; bi += gridDim.x * blockDim.x) {
@@ -131,7 +131,7 @@ __device__ __forceinline__ void ref_init_body(const RefineArgs& a, int bi, int i
   }
 }
 
-__global__ void __launch_bounds__(256) k_ref_init(RefineArgs a) {
+static __global__ void __launch_bounds__(256) k_ref_init(RefineArgs a) {
   pdl_wait();
   pdl_trigger();
   const int per = a.N > a.S ? a.N : a.S;
@@ -155,7 +155,7 @@ __host__ __device__ inline long long smem_residual_elems(int n) {
 // REFINE: write R32 = float(r), accumulate norms, skip inactive instances.
 // Otherwise write r (double) to a.rout for every instance.
 // x += delta (R32) for active instances; grid-stride over the whole batch.
-__global__ void __launch_bounds__(256) k_ref_update(RefineArgs a) {
+static __global__ void __launch_bounds__(256) k_ref_update(RefineArgs a) {
   pdl_wait();
   pdl_trigger();
   const long long per = (long long)a.N * a.n * a.m;
@@ -541,7 +541,7 @@ __device__ __forceinline__ void ref_init_rows_body(const RefineArgs& a, int bi, 
   }
 }
 
-__global__ void __launch_bounds__(256) k_ref_init_rows(RefineArgs a) {
+static __global__ void __launch_bounds__(256) k_ref_init_rows(RefineArgs a) {
   pdl_wait();
   pdl_trigger();
   const int per = a.N > a.S ? a.N : a.S;
@@ -567,7 +567,7 @@ struct FallbackArgs {
   uint8_t* used;   // caller output (B,): 1 where x comes from the FP64 path
 };
 
-__global__ void k_fb_select(RefineArgs a, FallbackArgs f) {
+static __global__ void k_fb_select(RefineArgs a, FallbackArgs f) {
   for (int bi = blockIdx.x * blockDim.x + threadIdx.x; bi < a.B; bi += gridDim.x * blockDim.x) {
     const bool on = a.mask == nullptr || a.mask[bi] != 0;
     const bool fail = on && !(a.eta[bi] <= a.tol);
@@ -578,7 +578,7 @@ __global__ void k_fb_select(RefineArgs a, FallbackArgs f) {
 }
 
 // IF-node condition: run the FP64 stage when some instance needs it.
-__global__ void k_fb_decide(cudaGraphConditionalHandle h, int* any) {
+static __global__ void k_fb_decide(cudaGraphConditionalHandle h, int* any) {
   const int v = *any;
   *any = 0;
   cudaGraphSetConditional(h, v ? 1u : 0u);
@@ -586,7 +586,7 @@ __global__ void k_fb_decide(cudaGraphConditionalHandle h, int* any) {
 
 // One CTA per (instance, block index i < max(N, S)) of the selected
 // instances: FP64 copies of L_i and slot i (zero for slots >= N-1), x_i = b_i.
-__global__ void __launch_bounds__(256) k_fb_copy(RefineArgs a, FallbackArgs f) {
+static __global__ void __launch_bounds__(256) k_fb_copy(RefineArgs a, FallbackArgs f) {
   const int per = a.N > a.S ? a.N : a.S;
   const int bi = blockIdx.x / per;
   const int i = blockIdx.x - bi * per;
@@ -610,7 +610,7 @@ __global__ void __launch_bounds__(256) k_fb_copy(RefineArgs a, FallbackArgs f) {
 
 // Backward error of the FP64 solution (norms accumulated by the residual
 // kernel with fb as its instance mask).
-__global__ void k_fb_eta(RefineArgs a, FallbackArgs f) {
+static __global__ void k_fb_eta(RefineArgs a, FallbackArgs f) {
   for (int bi = blockIdx.x * blockDim.x + threadIdx.x; bi < a.B; bi += gridDim.x * blockDim.x) {
     if (!f.fb[bi]) continue;
     RefineState& s = a.st[bi];
@@ -627,7 +627,7 @@ __global__ void k_fb_eta(RefineArgs a, FallbackArgs f) {
 
 // Loop control for a graph WHILE node: keep iterating while some instance
 // is still active, and clear the flag for the next round.
-__global__ void k_ref_decide(cudaGraphConditionalHandle h, int* any_active) {
+static __global__ void k_ref_decide(cudaGraphConditionalHandle h, int* any_active) {
   const int v = *any_active;
   *any_active = 0;
   cudaGraphSetConditional(h, v ? 1u : 0u);

@@ -1,0 +1,6 @@
+// float instantiations of the sweep kernels.
+#include "top_sweep.cuh"
+
+namespace socu {
+SOCU_SWEEP_KERNELS(float)
+}  // namespace socu

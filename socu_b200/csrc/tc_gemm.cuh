@@ -34,7 +34,7 @@ __device__ __forceinline__ uint32_t saddr(const void* p) {
 
 // Error word of the asynchronous units on one device: 1 a tensor-core wait
 // ran out, 2 a TMA copy wait ran out (that kernel skipped its result).
-__device__ int g_tc_error;
+static __device__ int g_tc_error;   // one per translation unit; socu_tc_error reads them all
 
 // ---- instruction / shared-memory descriptors --------------------------------
 // kind::tf32 instruction descriptor: D F32 (bits 4-5 = 1), A and B TF32

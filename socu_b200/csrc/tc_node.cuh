@@ -4,7 +4,7 @@
 //
 // socu: potrf K2 fused with trsm_rltn / trsm_llnn (K3/K4) and the forward
 // step, socu/block_tridiag_solver.py:197-279, :108-110.  Same results layout
-// as node_body (nd_kernels.cuh): lower(L_i) = C_i, zero strict upper triangle,
+// as k_node_rows (node_rows.cuh): lower(L_i) = C_i, zero strict upper triangle,
 // R <- R C^{-T}, Lf <- C^{-1} Lf, y <- C^{-1} y.
 //
 // State, one TMEM lane per block row r (M = 128; rows n..127 unused):
@@ -163,7 +163,7 @@ __device__ __forceinline__ void node_tm_body(const Problem<float>& p, const Leve
     tc::fence_after_sync();
 
     // b. panel chain: C11 = chol(A11), Vc <- C11^{-1} Vc
-    cta_chol_solve<float, true>(A11, lda, pw, Vc, ldc, ncat);
+    cta_chol_solve<float>(A11, lda, pw, Vc, ldc, ncat);
     if (p.info != nullptr) {
       bool bad = false;
       for (int r = threadIdx.x; r < pw; r += blockDim.x) {

@@ -296,7 +296,7 @@ __device__ __forceinline__ void node_tc_body(const Problem<float>& p, const Leve
   }
   cp_async_wait_all();
   __syncthreads();
-  cta_chol_solve<float, true, true>(S1, ld, n, W, ld, n);
+  cta_chol_solve<float, true>(S1, ld, n, W, ld, n);
   check_factor(p, b, i, S1, ld);
   for (int e = threadIdx.x; e < n * n; e += blockDim.x) {
     const int r = e / n, c = e - r * n;

@@ -328,4 +328,46 @@ __global__ void __launch_bounds__(256) k_top(Problem<T> p, const __grid_constant
     for (int k = consumed; k < issued; ++k) tc::mbar_wait(bar + k % stages, (unsigned)(k / stages) & 1u, kTmaWaitNs);
 }
 
+// Sweep kernels by op, residency and inverse-carrying factors (sweeps_f32.cu,
+// sweeps_f64.cu: one translation unit per type).
+enum SweepKind { kSweepForward, kSweepPull, kSweepBackward };
+template <typename T>
+using SweepFn = void (*)(Problem<T>, Level, SweepMaps);
+template <typename T>
+using TopFn = void (*)(Problem<T>, TopLevels, SweepMaps);
+template <typename T>
+SweepFn<T> sweep_kernel(SweepKind kind, bool resident, bool inv);
+template <typename T>
+TopFn<T> top_sweep_kernel(bool inv);
+// the wait-error word of that translation unit's kernels
+template <typename T>
+cudaError_t sweep_wait_error(int* flag, bool reset);
+
+#define SOCU_SWEEP_KERNELS(T)                                                                       \
+  template <>                                                                                       \
+  SweepFn<T> sweep_kernel<T>(SweepKind kind, bool resident, bool inv) {                             \
+    if (kind == kSweepPull) return resident ? k_fwd<T, true, true> : k_fwd<T, false, true>;         \
+    if (kind == kSweepForward)                                                                      \
+      return resident ? (inv ? k_fwd<T, true, false, true> : k_fwd<T, true>) : k_fwd<T, false>;     \
+    return resident ? (inv ? k_bwd<T, true, true> : k_bwd<T, true>) : k_bwd<T, false>;              \
+  }                                                                                                 \
+  template <>                                                                                       \
+  TopFn<T> top_sweep_kernel<T>(bool inv) {                                                          \
+    return inv ? k_top<T, true> : k_top<T, false>;                                                  \
+  }                                                                                                 \
+  template <>                                                                                       \
+  cudaError_t sweep_wait_error<T>(int* flag, bool reset) {                                          \
+    const int zero = 0;                                                                             \
+    cudaError_t e = cudaMemcpyFromSymbol(flag, tc::g_tc_error, sizeof(int));                        \
+    if (e == cudaSuccess && reset) e = cudaMemcpyToSymbol(tc::g_tc_error, &zero, sizeof(int));      \
+    return e;                                                                                       \
+  }
+
+template <> SweepFn<float> sweep_kernel<float>(SweepKind, bool, bool);
+template <> SweepFn<double> sweep_kernel<double>(SweepKind, bool, bool);
+template <> TopFn<float> top_sweep_kernel<float>(bool);
+template <> TopFn<double> top_sweep_kernel<double>(bool);
+template <> cudaError_t sweep_wait_error<float>(int*, bool);
+template <> cudaError_t sweep_wait_error<double>(int*, bool);
+
 }  // namespace socu
