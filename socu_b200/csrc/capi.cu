@@ -19,6 +19,7 @@
 #include "tc_node.cuh"
 #include "tc_update.cuh"
 #include "top_sweep.cuh"
+#include "update_rows.cuh"
 
 namespace socu {
 namespace {
@@ -56,7 +57,6 @@ void schedule(int N, Schedule* out) {
     lv.on = nxt;
     lv.op = prev;
     lv.tc = 0;
-    lv.tile = kTile;
     lv.pre = 0;
     s *= 2;
     prev = curr;
@@ -486,28 +486,6 @@ bool use_inverse(int n, int m) {
                         (long long)max_smem_optin();
 }
 
-// Second stream and two events for graph capture: inside factor_and_solve,
-// each level's forward pull runs on a parallel branch beside the Schur update
-// (both only depend on the level's node kernel).
-struct Fork {
-  cudaStream_t aux = nullptr;
-  cudaEvent_t split = nullptr, join = nullptr;
-  bool ok() const { return aux && split && join; }
-  int create() {
-    cudaError_t e = cudaStreamCreateWithFlags(&aux, cudaStreamNonBlocking);
-    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&split, cudaEventDisableTiming);
-    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&join, cudaEventDisableTiming);
-    return cuda_status(e);
-  }
-  void destroy() {
-    if (aux) cudaStreamDestroy(aux);
-    if (split) cudaEventDestroy(split);
-    if (join) cudaEventDestroy(join);
-    aux = nullptr;
-    split = join = nullptr;
-  }
-};
-
 // Block-row FP64 residual (n <= 128): 1, 2 or 4 eight-column groups of
 // right-hand sides per pass over the matrix blocks, by n_rhs.
 template <bool REFINE>
@@ -532,21 +510,19 @@ cudaError_t launch_residual_rows(const RefineArgs& a, cudaStream_t st, bool pdl)
 // Enqueue (or count, when st == nullptr and count != nullptr) the kernels of one op.
 // inv: the factor carries (FACTOR, FACTOR_AND_SOLVE) or has (SOLVE) its
 // diagonal inverses; only for internal factors or within factor_and_solve.
-// fork (graph capture only): run the forward pulls on a parallel branch.
 // over: per-launch settings (block_dim / block_size), on top of the tuned table.
 template <typename T>
 int enqueue(socu_op op, const Problem<T>& p, cudaStream_t st, long long* count, bool inv = false,
-            const Fork* fork = nullptr, const socu_tuning* over = nullptr) {
+            const socu_tuning* over = nullptr) {
   const int n = p.n, nth = threads_for(n);
   socu_tuning cfg = tuning_lookup(sizeof(T) == 8 ? SOCU_FLOAT64 : SOCU_FLOAT32, n, p.m);
   if (over) tuning_merge(&cfg, *over);
-  const int tile = cfg.update_tile ? cfg.update_tile : kTile;
   Schedule lv;
   schedule(p.N, &lv);
   const int K = lv.K;
-  for (int l = 0; l < K; ++l) lv.lv[l].tile = tile;
   const bool withY = op == SOCU_OP_FACTOR_AND_SOLVE;
-  const size_t su = smem_update_launch_elems(n, sizeof(T), tile) * sizeof(T);
+  const size_t su = (size_t)smem_update_rows_bytes(n, sizeof(T));
+  const UpdateRowsFn<T> update_kernel = update_rows_kernel<T>(n);
   const int mm = p.m > 0 ? p.m : 1;
   const bool res = (long long)smem_sweep_res_elems(n, mm) * (long long)sizeof(T) <= (long long)max_smem_optin();
   const size_t ss = (res ? smem_sweep_res_elems(n, mm) : smem_sweep_elems(n, mm)) * sizeof(T);
@@ -583,14 +559,13 @@ int enqueue(socu_op op, const Problem<T>& p, cudaStream_t st, long long* count, 
   long long launches = 0;
   const bool run = count == nullptr;
   const int sms = run ? sm_count() : 0;
-  const int upd_thr = cfg.update_threads ? cfg.update_threads : nth;
   const int swp_thr = cfg.sweep_threads ? cfg.sweep_threads : nth;
 
   if (run) {
     cudaError_t e = cudaSuccess;
     if (op == SOCU_OP_FACTOR || op == SOCU_OP_FACTOR_AND_SOLVE) {
       e = prepare(rows_kernel, sd_rows);
-      if (e == cudaSuccess) e = update_uses_big(n) ? prepare(k_update_big<T>, su) : prepare(k_update<T>, su);
+      if (e == cudaSuccess) e = prepare(update_kernel, su);
       if (e == cudaSuccess && upd_tc) e = prepare(k_update_tc, su_tc);
       if (e == cudaSuccess && node_tc_any) e = prepare(node_tc_kernel, sd_tc);
       if (e == cudaSuccess && node_tm) e = prepare(node_tm_kernel, sd_tm);
@@ -615,14 +590,14 @@ int enqueue(socu_op op, const Problem<T>& p, cudaStream_t st, long long* count, 
     return o;
   };
   // programmatic launches inside the op's chain on its own stream (not the
-  // first kernel, not the forked branch, not while profiling with events)
+  // first kernel, not while profiling with events)
   bool first = true;
   auto go_on = [&](cudaStream_t s, auto kernel, int kind, long long blocks, size_t smem, const Level& L,
                    int threads, auto... extra) {
     if (blocks <= 0) return;
     ++launches;
     if (!run) return;
-    const bool pdl = !first && s == st && g_prof == nullptr;
+    const bool pdl = !first && g_prof == nullptr;
     first = false;
     prof_begin(s, kind);
     launch(kernel, (unsigned)blocks, (unsigned)threads, smem, s, pdl, p, L, extra...);
@@ -654,7 +629,6 @@ int enqueue(socu_op op, const Problem<T>& p, cudaStream_t st, long long* count, 
       launch(rows_kernel, blocks, threads, sd_rows, st, pdl, p, L, splits, (int)withY, (int)inv);
     prof_end(st);
   };
-  const bool forked = run && fork != nullptr && fork->ok();
 
   // On request (SOCU_TOP_SWEEP=1), the top levels of the sweeps in one
   // cluster-resident kernel (k_top): the forward levels with at most `cluster`
@@ -741,34 +715,27 @@ int enqueue(socu_op op, const Problem<T>& p, cudaStream_t st, long long* count, 
         go_rows(node_blocks, L);
       }
       if (l + 1 < K) {
-        // fused forward: apply this level's updates to every target vector
+        // Fused forward: apply this level's updates to every target vector.  It
+        // only depends on the node, as the Schur update does, so the update is
+        // launched behind it without waiting for it (k_update_rows, `behind`).
         const long long pull_blocks = withY ? (long long)p.B * (p.N / lv[l + 1].s) : 0;
-        const Level PL = sweep_level(lv[l + 1], pull_blocks, false);
-        if (forked && pull_blocks > 0) {
-          cudaEventRecord(fork->split, st);
-          cudaStreamWaitEvent(fork->aux, fork->split, 0);
-          go_on(fork->aux, pull_kernel, SOCU_KIND_PULL, pull_blocks, ss, PL, swp_thr, maps);
-          cudaEventRecord(fork->join, fork->aux);
-        }
-        const long long upd_blocks = (long long)p.B * update_launch_tasks(n, p.N, L);
+        go_on(st, pull_kernel, SOCU_KIND_PULL, pull_blocks, ss, sweep_level(lv[l + 1], pull_blocks, false), swp_thr,
+              maps);
+        const long long upd_blocks = (long long)p.B * update_blocks(p.N, L);
         bool tc_done = false;
         if constexpr (sizeof(T) == 4) {
           if (upd_tc) {
-            go_on(st, k_update_tc, SOCU_KIND_UPDATE, (long long)p.B * update_blocks(p.N, L), su_tc, L, 256);
+            go_on(st, k_update_tc, SOCU_KIND_UPDATE, upd_blocks, su_tc, L, 256);
             tc_done = true;
           }
         }
         if (!tc_done) {
-          if (update_uses_big(n))
-            go_on(st, k_update_big<T>, SOCU_KIND_UPDATE, upd_blocks, su, L, 256);
-          else
-            go_on(st, k_update<T>, SOCU_KIND_UPDATE, upd_blocks, su, L, upd_thr);
+          // narrow levels: several blocks per output block (k_update_rows)
+          int splits = 1;
+          while (splits < 8 && splits * 2 <= ceil_div(n, 8) && upd_blocks * splits * 2 <= sms) splits *= 2;
+          go_on(st, update_kernel, SOCU_KIND_UPDATE, upd_blocks * splits, su, L, 32 * update_rows_warps(n, splits),
+                splits, (int)(pull_blocks > 0));
         }
-        if (forked && pull_blocks > 0) {
-          cudaStreamWaitEvent(st, fork->join, 0);
-          first = true;   // the next node waits for the forked branch in full
-        } else
-          go_on(st, pull_kernel, SOCU_KIND_PULL, pull_blocks, ss, PL, swp_thr, maps);
       }
     }
   }
@@ -841,7 +808,7 @@ int validate(socu_op op, socu_dtype dtype, const void* L, const void* E, const v
 
 int dispatch(socu_op op, socu_dtype dtype, void* L, void* E, void* x, const uint8_t* mask,
              int64_t batch, int64_t horizon, int64_t n, int64_t n_rhs, cudaStream_t st,
-             long long* count, const Fork* fork = nullptr, const socu_tuning* over = nullptr,
+             long long* count, const socu_tuning* over = nullptr,
              int32_t* info = nullptr) {
   Dims d;
   const int v = validate(op, dtype, L, E, x, batch, horizon, n, n_rhs, &d);
@@ -863,11 +830,11 @@ int dispatch(socu_op op, socu_dtype dtype, void* L, void* E, void* x, const uint
   if (dtype == SOCU_FLOAT64) {
     Problem<double> p = make_problem<double>(L, E, x, mask, d);
     p.info = info;
-    return enqueue<double>(op, p, st, count, inv, fork, over);
+    return enqueue<double>(op, p, st, count, inv, over);
   }
   Problem<float> p = make_problem<float>(L, E, x, mask, d);
   p.info = info;
-  return enqueue<float>(op, p, st, count, inv, fork, over);
+  return enqueue<float>(op, p, st, count, inv, over);
 }
 
 
@@ -978,7 +945,7 @@ int refine_finish_round(const RefineArgs& a, cudaStream_t st, long long* count) 
 // Mixed solve, part 1: state reset, float copies, norms, then the first
 // round fused into the float factor: factor_and_solve on R32 = b gives
 // delta = x_1, followed by x += delta, the FP64 residual and the test.
-int refine_prologue(const RefineArgs& a, cudaStream_t st, long long* count, const Fork* fork = nullptr) {
+int refine_prologue(const RefineArgs& a, cudaStream_t st, long long* count) {
   const bool run = count == nullptr;
   Dims d{a.B, a.N, a.n, a.m, a.S};
   Problem<float> pf = make_problem<float>(a.L32, a.E32, a.R32, a.active, d);
@@ -1009,8 +976,7 @@ int refine_prologue(const RefineArgs& a, cudaStream_t st, long long* count, cons
   socu_tuning mixed{};
   if (a.n > 64 && update_tc_ok(a.n) && tuning_lookup(SOCU_FLOAT32, a.n, a.m).update_tensor_cores == 0)
     mixed.update_tensor_cores = 1;
-  int s = enqueue<float>(SOCU_OP_FACTOR_AND_SOLVE, pf, st, run ? nullptr : &c, use_inverse<float>(a.n, a.m), fork,
-                         &mixed);
+  int s = enqueue<float>(SOCU_OP_FACTOR_AND_SOLVE, pf, st, run ? nullptr : &c, use_inverse<float>(a.n, a.m), &mixed);
   if (s != SOCU_OK) return s;
   s = refine_finish_round(a, st, run ? nullptr : &cr);
   if (count) *count = 2 + c + cr;
@@ -1112,9 +1078,7 @@ int capture_refine_while(const RefineArgs& a, cudaGraph_t* out, const FallbackAr
     st = cuda_status(e);
     capturing = st == SOCU_OK;
   }
-  Fork fork;
-  if (st == SOCU_OK) st = fork.create();
-  if (st == SOCU_OK) st = refine_prologue(a, cap, nullptr, &fork);
+  if (st == SOCU_OK) st = refine_prologue(a, cap, nullptr);
   cudaGraph_t g = nullptr;
   cudaGraphConditionalHandle hnd = 0;
   cudaGraphNode_t node = nullptr;
@@ -1164,7 +1128,6 @@ int capture_refine_while(const RefineArgs& a, cudaGraph_t* out, const FallbackAr
   }
   if (cap) cudaStreamDestroy(cap);
   if (body) cudaStreamDestroy(body);
-  fork.destroy();
   if (st != SOCU_OK) {
     if (fin) cudaGraphDestroy(fin);
     return st;
@@ -1443,8 +1406,8 @@ int rg_refine_solve(socu_ragged_s* r, const double* L, const double* E, const do
   return rg_launch<float, kRgRefine>(r, a, st);
 }
 
-// enqueue one run of a launch object on `st` (fork: graph capture only)
-int launch_enqueue(socu_launch_s* h, cudaStream_t st, const Fork* fork = nullptr) {
+// enqueue one run of a launch object on `st`
+int launch_enqueue(socu_launch_s* h, cudaStream_t st) {
   if (h->rg) {
     if (h->rg->refine)
       return rg_refine_solve(h->rg, static_cast<const double*>(h->L), static_cast<const double*>(h->E), h->b,
@@ -1458,7 +1421,7 @@ int launch_enqueue(socu_launch_s* h, cudaStream_t st, const Fork* fork = nullptr
     return refine_enqueue(h->ra, st, nullptr);
   }
   return dispatch(h->op, h->dtype, h->L, h->E, h->x, h->mask, h->batch, h->horizon, h->n, h->n_rhs, st, nullptr,
-                  fork, &h->over, h->info);
+                  &h->over, h->info);
 }
 
 // Capture one run into a CUDA graph on a private stream (the legacy default
@@ -1474,11 +1437,9 @@ int capture(socu_launch_s* h) {
   cudaStream_t cap = nullptr;
   cudaError_t e = cudaStreamCreateWithFlags(&cap, cudaStreamNonBlocking);
   int st = SOCU_OK;
-  Fork fork;
-  if (e == cudaSuccess && fork.create() != SOCU_OK) e = static_cast<cudaError_t>(g_last_cuda_error);
   if (e == cudaSuccess) e = cudaStreamBeginCapture(cap, cudaStreamCaptureModeThreadLocal);
   if (e == cudaSuccess) {
-    st = launch_enqueue(h, cap, &fork);
+    st = launch_enqueue(h, cap);
     cudaGraph_t g = nullptr;
     const cudaError_t e2 = cudaStreamEndCapture(cap, &g);
     if (st == SOCU_OK && e2 != cudaSuccess) st = cuda_status(e2);
@@ -1488,7 +1449,6 @@ int capture(socu_launch_s* h) {
     st = cuda_status(e);
   }
   if (cap) cudaStreamDestroy(cap);
-  fork.destroy();
   if (st != SOCU_OK) {
     if (h->exec) cudaGraphExecDestroy(h->exec);
     if (h->graph) cudaGraphDestroy(h->graph);
@@ -1588,7 +1548,7 @@ int64_t socu_max_block_size(socu_dtype dtype, int64_t n_rhs) {
   int64_t best = 0;
   for (int n = 1; n <= 512; ++n) {
     long long need = smem_rows_bytes(n) / (long long)es;
-    const long long u = smem_update_elems(n, (int)es), s = smem_sweep_elems(n, m > 0 ? m : 1);
+    const long long u = smem_update_rows_bytes(n, (int)es) / (long long)es, s = smem_sweep_elems(n, m > 0 ? m : 1);
     if (u > need) need = u;
     if (s > need) need = s;
     if (need * (long long)es <= limit && n <= 128) best = n;
@@ -1641,7 +1601,7 @@ int socu_cholesky_run_info(socu_op op, socu_dtype dtype, void* L, void* E, void*
   if (info == nullptr && batch > 0) return SOCU_ERR_INVALID_ARGUMENT;
   if (bop != SOCU_OP_FACTOR && bop != SOCU_OP_FACTOR_AND_SOLVE) return SOCU_ERR_INVALID_ARGUMENT;
   return dispatch(op, dtype, L, E, x, mask, batch, horizon, n, n_rhs, static_cast<cudaStream_t>(stream), nullptr,
-                  nullptr, nullptr, info);
+                  nullptr, info);
 }
 
 int socu_launch_create(socu_launch_t* out, socu_op op, socu_dtype dtype, void* L, void* E, void* x,
@@ -1668,7 +1628,7 @@ int socu_launch_create_ex(socu_launch_t* out, socu_op op, socu_dtype dtype, void
   const socu_op bop = base_op(op, &inv_op);
   if (info != nullptr && bop != SOCU_OP_FACTOR && bop != SOCU_OP_FACTOR_AND_SOLVE) return SOCU_ERR_INVALID_ARGUMENT;
   long long kernels = 0;
-  int st = dispatch(op, dtype, L, E, x, mask, batch, horizon, n, n_rhs, nullptr, &kernels, nullptr, settings, info);
+  int st = dispatch(op, dtype, L, E, x, mask, batch, horizon, n, n_rhs, nullptr, &kernels, settings, info);
   if (st != SOCU_OK) return st;
   socu_launch_s* h = new (std::nothrow) socu_launch_s();
   if (!h) return SOCU_ERR_UNSUPPORTED;

@@ -8,7 +8,7 @@
 //               rows of the right slot     -> F = E[o_l+i/s] C_i^{-T}   (K3 trsm_rltn, :219-248)
 //               columns of the left slot   -> G = C_i^{-1} E[o_l+(i-s)/s] (K4 trsm_llnn, :251-279)
 //               columns of y_i (factor_and_solve) -> y_i <- C_i^{-1} y_i (:108-110)
-//   k_update  one CTA per 32x32 output tile:
+//   update    (k_update_rows, update_rows.cuh)
 //             target j = 2 s u - 1 (owner computes; the reference uses
 //             atomics here, K5/K6 :282-342)
 //                 L_j -= F_{j-s} F_{j-s}^T + G_{j+s}^T G_{j+s}
@@ -37,12 +37,6 @@ __host__ __device__ inline int min_i(int a, int b) { return a < b ? a : b; }
 // shared-memory sizes (elements) ------------------------------------------------
 __host__ __device__ inline int gemm_ld(int n, int es) { return es == 8 ? ((n + 15) / 16) * 16 + 4 : n + 1; }
 __host__ __device__ inline int update_ld(int k, int es) { return gemm_ld(k, es); }
-// blocked Schur update (n > 64) with tile x tile output tiles
-__host__ __device__ inline long long smem_update_elems(int n, int es, int tile = kTile) {
-  const long long a = 2LL * tile * update_ld(2 * n, es);
-  const long long f = (long long)tile * update_ld(n, es) + (long long)n * update_ld(tile, es);
-  return a > f ? a : f;
-}
 // streamed (non-resident) sweeps: Y, Z1, Z2 (n x sweep_ldy) and the chunk buffer
 // Cc (n x sweep_ldc >= kTile x (n + 1) for the triangular panels), dv (kTile)
 __host__ __device__ inline int sweep_ldy(int mc) { return mc + 4; }
@@ -147,85 +141,6 @@ static __global__ void k_info_reset(int* info, int B) {
 // ---------------------------------------------------------------------------
 // k_update
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ void lower_tile_index(int lt, int& ta, int& tc) {
-  int a = 0;
-  while ((a + 1) * (a + 2) / 2 <= lt) ++a;
-  ta = a;
-  tc = lt - a * (a + 1) / 2;
-}
-
-// Number of output tiles of one update level per instance: U targets with
-// nlt lower tiles each, then d-1 fill-in blocks with nt*nt tiles each.
-__host__ __device__ inline int update_tiles(int n, int N, const Level& lv) {
-  const int nt = ceil_div(n, lv.tile);
-  return (N / (2 * lv.s)) * (nt * (nt + 1) / 2) + (lv.d - 1) * nt * nt;
-}
-
-// Body of one output tile `task` in [0, update_tiles) of instance b.
-template <typename T>
-__device__ __forceinline__ void update_body(const Problem<T>& p, const Level& lv, int b, int task,
-                                            unsigned char* smem_raw) {
-  constexpr int es = sizeof(T);
-  const int n = p.n, N = p.N, s = lv.s;
-  const int tile = lv.tile;
-  const int nt = ceil_div(n, tile);
-  const int nlt = nt * (nt + 1) / 2;
-  const int U = N / (2 * s);
-  T* Ab = reinterpret_cast<T*>(smem_raw);
-
-  if (task < U * nlt) {
-    const int u = task / nlt + 1;
-    int ta, tc;
-    lower_tile_index(task - (u - 1) * nlt, ta, tc);
-    const int j = 2 * s * u - 1;
-    const T* F = p.Eb(b, lv.oc + 2 * (u - 1));
-    const bool hasG = j + s < N;
-    const T* G = hasG ? p.Eb(b, lv.oc + 2 * u - 1) : nullptr;
-    const int r0 = ta * tile, wa = min_i(tile, n - r0);
-    const int c0 = tc * tile, wc = min_i(tile, n - c0);
-    const bool diag = ta == tc;
-    const int K = hasG ? 2 * n : n;
-    const int lda = update_ld(K, es);       // rows of [F | G^T]
-    T* Bb = Ab + tile * lda;
-    T* Bop = diag ? Ab : Bb;
-    // Ab[r][k] = F[r0+r][k], Ab[r][n+k] = G[k][r0+r]   (k < n)
-    async_load(Ab, lda, F + (long long)r0 * n, wa, n, n);
-    if (hasG) async_load_t(Ab + n, lda, G + r0, n, wa, n);
-    if (!diag) {
-      async_load(Bb, lda, F + (long long)c0 * n, wc, n, n);
-      if (hasG) async_load_t(Bb + n, lda, G + c0, n, wc, n);
-    }
-    cp_async_wait_all();
-    __syncthreads();
-    T* Lj = p.Lb(b, j);
-    auto out = [&](int r, int c, T v) { Lj[(long long)(r0 + r) * n + c0 + c] -= v; };
-    if (diag)
-      cta_gemm<T, false, true, true>(wa, wc, K, Ab, lda, Bop, lda, out);
-    else
-      cta_gemm<T, false, true, false>(wa, wc, K, Ab, lda, Bop, lda, out);
-  } else {
-    const int f = task - U * nlt;
-    const int t = f / (nt * nt) + 1;
-    const int tt = f - (t - 1) * nt * nt;
-    const int ta = tt / nt, tc = tt - ta * nt;
-    const int i = s - 1 + 2 * s * t;
-    if (i + s >= N) return;
-    const T* F = p.Eb(b, lv.oc + 2 * t);
-    const T* G = p.Eb(b, lv.oc + 2 * t - 1);
-    T* X = p.Eb(b, lv.on + t - 1);
-    const int r0 = ta * tile, wa = min_i(tile, n - r0);
-    const int c0 = tc * tile, wc = min_i(tile, n - c0);
-    const int lda = update_ld(n, es), ldg = update_ld(tile, es);
-    T* Bb = Ab + tile * lda;
-    async_load(Ab, lda, F + (long long)r0 * n, wa, n, n);   // F rows
-    async_load(Bb, ldg, G + c0, n, wc, n);                    // G columns, n x wc
-    cp_async_wait_all();
-    __syncthreads();
-    cta_gemm<T, false, false>(wa, wc, n, Ab, lda, Bb, ldg,
-                              [&](int r, int c, T v) { X[(long long)(r0 + r) * n + c0 + c] -= v; });
-  }
-}
-
 // Whole-block update for n <= kNodeGemmMaxN: task u-1 < U updates target
 // j = 2su-1 completely (all lower tiles, K = 2n), task U + t-1 forms the whole
 // fill-in block of node t.  One CTA per block keeps every warp busy.
@@ -283,200 +198,6 @@ __device__ __forceinline__ void update_full_body(const Problem<T>& p, const Leve
       *o = (T)((double)*o - v);
     });
   }
-}
-
-// ---------------------------------------------------------------------------
-// Whole-block update for 64 < n <= 128 (same tasks as update_full_body): one
-// CTA of 256 threads per target / fill-in block, K streamed through shared
-// memory in kBigKC-column chunks (target: A = [F | G^T], B = A; fill-in:
-// A = F, B(c, k) = G[k][c]), and each warp keeping the accumulators of up to
-// kBigTiles 16 x 32 DMMA tiles of the n x n output (lower tiles only for a
-// target) in registers across the chunks; float operands are widened (exact
-// products, FP64 sums, one rounding per entry).
-// ---------------------------------------------------------------------------
-constexpr int kBigMaxN = 128;
-constexpr int kBigKC = 32;
-constexpr int kBigLd = kBigKC + 4;   // 4 (mod 16) doubles: conflict-free fragments
-constexpr int kBigTiles = 4;         // (128/16) x (128/32) = 32 tiles over 8 warps
-// two chunk buffers (A and B each): the next chunk's copies overlap this chunk's products
-__host__ __device__ inline long long smem_update_big_elems(int n) { return 4LL * n * kBigLd; }
-__host__ __device__ inline bool update_uses_big(int n) { return n > kNodeGemmMaxN && n <= kBigMaxN; }
-
-template <typename T>
-__device__ __forceinline__ void update_big_body(const Problem<T>& p, const Level& lv, int b, int task,
-                                                unsigned char* smem_raw) {
-  const int n = p.n, N = p.N, s = lv.s;
-  const int U = N / (2 * s);
-  T* buf = reinterpret_cast<T*>(smem_raw);   // [2][A | B], each n x kBigLd
-  const bool target = task < U;
-  const T *F, *G;
-  T* Out;
-  int K;
-  if (target) {
-    const int u = task + 1, j = 2 * s * u - 1;
-    F = p.Eb(b, lv.oc + 2 * (u - 1));
-    G = j + s < N ? p.Eb(b, lv.oc + 2 * u - 1) : nullptr;
-    Out = p.Lb(b, j);
-    K = G ? 2 * n : n;
-  } else {
-    const int t = task - U + 1, i = s - 1 + 2 * s * t;
-    if (i + s >= N) return;
-    F = p.Eb(b, lv.oc + 2 * t);
-    G = p.Eb(b, lv.oc + 2 * t - 1);
-    Out = p.Eb(b, lv.on + t - 1);
-    K = n;
-  }
-  // asynchronous copies of chunk c (columns [32c, 32c + 32) of A and B) into
-  // buffer c & 1; columns past K are zero-filled with plain stores
-  auto stage = [&](int c) {
-    T* As = buf + (c & 1) * 2 * n * kBigLd;
-    T* Bs = As + n * kBigLd;
-    const int k0 = c * kBigKC, kw = min_i(kBigKC, K - k0);
-    if (k0 + kw <= n) {
-      // A(r, kk) = F[r][k0 + kk]: rows of F
-      for (int e = threadIdx.x; e < n * kw; e += blockDim.x) {
-        const int r = e / kw, kk = e - r * kw;
-        cp_async_elem(As + r * kBigLd + kk, F + (long long)r * n + k0 + kk);
-      }
-    } else if (k0 >= n) {
-      // A(r, kk) = G[k0 + kk - n][r]: rows of G, transposed
-      for (int e = threadIdx.x; e < n * kw; e += blockDim.x) {
-        const int kk = e / n, r = e - kk * n;
-        cp_async_elem(As + r * kBigLd + kk, G + (long long)(k0 + kk - n) * n + r);
-      }
-    } else {
-      for (int e = threadIdx.x; e < n * kw; e += blockDim.x) {
-        const int r = e / kw, kk = e - r * kw, k = k0 + kk;
-        cp_async_elem(As + r * kBigLd + kk, k < n ? F + (long long)r * n + k : G + (long long)(k - n) * n + r);
-      }
-    }
-    if (!target)   // B(c, kk) = G[k0 + kk][c]
-      for (int e = threadIdx.x; e < n * kw; e += blockDim.x) {
-        const int kk = e / n, cc = e - kk * n;
-        cp_async_elem(Bs + cc * kBigLd + kk, G + (long long)(k0 + kk) * n + cc);
-      }
-    if (kw < kBigKC)
-      for (int e = threadIdx.x; e < n * (kBigKC - kw); e += blockDim.x) {
-        const int r = e / (kBigKC - kw), kk = kw + e - r * (kBigKC - kw);
-        As[r * kBigLd + kk] = T(0);
-        if (!target) Bs[r * kBigLd + kk] = T(0);
-      }
-    cp_async_commit();
-  };
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  const int g = lane >> 2, tq = lane & 3;
-  const int tm = (n + 15) / 16, tn = (n + 31) / 32;
-  // this warp's tiles: the warp-th, (warp + nw)-th, ... tile of the (lower) tile list
-  int tr[kBigTiles], tc[kBigTiles];
-  int nt = 0;
-  {
-    int idx = 0;
-    for (int i = 0; i < tm; ++i)
-      for (int j = 0; j < tn; ++j) {
-        if (target && 32 * j > 16 * i + 15) continue;
-        if (idx % nw == warp && nt < kBigTiles) {
-          tr[nt] = i * 16;
-          tc[nt] = j * 32;
-          ++nt;
-        }
-        ++idx;
-      }
-  }
-  double acc[kBigTiles][2][4][2];
-#pragma unroll
-  for (int q = 0; q < kBigTiles; ++q)
-#pragma unroll
-    for (int i = 0; i < 2; ++i)
-#pragma unroll
-      for (int j = 0; j < 4; ++j) acc[q][i][j][0] = acc[q][i][j][1] = 0.0;
-  const int chunks = (K + kBigKC - 1) / kBigKC;
-  stage(0);
-  for (int c = 0; c < chunks; ++c) {
-    if (c + 1 < chunks) stage(c + 1);
-    else cp_async_commit();       // empty group: wait_group 1 then covers chunk c
-    cp_async_wait_one();
-    __syncthreads();
-    const T* As = buf + (c & 1) * 2 * n * kBigLd;
-    const T* Bsrc = target ? As : As + n * kBigLd;
-#pragma unroll
-    for (int q = 0; q < kBigTiles; ++q) {
-      if (q >= nt) break;
-      int ra[2], cb[4];
-#pragma unroll
-      for (int i = 0; i < 2; ++i) ra[i] = min_i(tr[q] + 8 * i + g, n - 1);
-#pragma unroll
-      for (int j = 0; j < 4; ++j) cb[j] = min_i(tc[q] + 8 * j + g, n - 1);
-#pragma unroll 2
-      for (int kq = 0; kq < kBigKC; kq += 4) {
-        const int kk = kq + tq;
-        double a[2], bb[4];
-#pragma unroll
-        for (int i = 0; i < 2; ++i) a[i] = (double)As[ra[i] * kBigLd + kk];
-#pragma unroll
-        for (int j = 0; j < 4; ++j) bb[j] = (double)Bsrc[cb[j] * kBigLd + kk];
-#pragma unroll
-        for (int i = 0; i < 2; ++i)
-#pragma unroll
-          for (int j = 0; j < 4; ++j) dmma_8x8x4(acc[q][i][j][0], acc[q][i][j][1], a[i], bb[j]);
-      }
-    }
-    __syncthreads();   // buffer c & 1 is restaged for chunk c + 2
-  }
-  // epilogue: Out -= D (lower triangle for a target)
-#pragma unroll
-  for (int q = 0; q < kBigTiles; ++q) {
-    if (q >= nt) break;
-#pragma unroll
-    for (int i = 0; i < 2; ++i)
-#pragma unroll
-      for (int j = 0; j < 4; ++j)
-#pragma unroll
-        for (int e = 0; e < 2; ++e) {
-          const int r = tr[q] + 8 * i + g, c = tc[q] + 8 * j + 2 * tq + e;
-          if (r < n && c < n && (!target || c <= r)) {
-            T* o = Out + (long long)r * n + c;
-            *o = (T)((double)*o - acc[q][i][j][e]);
-          }
-        }
-  }
-}
-
-__host__ __device__ inline bool update_uses_full(int n) { return n <= kNodeGemmMaxN; }
-__host__ __device__ inline int update_launch_tasks(int n, int N, const Level& lv) {
-  return (update_uses_full(n) || update_uses_big(n)) ? update_blocks(N, lv) : update_tiles(n, N, lv);
-}
-__host__ __device__ inline long long smem_update_launch_elems(int n, int es, int tile = kTile) {
-  if (update_uses_big(n)) return smem_update_big_elems(n);
-  return update_uses_full(n) ? smem_update_full_elems(n, es) : smem_update_elems(n, es, tile);
-}
-
-template <typename T>
-__global__ void __launch_bounds__(256) k_update(Problem<T> p, Level lv) {
-  const int per_b = update_launch_tasks(p.n, p.N, lv);
-  const int b = blockIdx.x / per_b;
-  const int task = blockIdx.x - b * per_b;
-  pdl_wait();
-  pdl_trigger();
-  if (!p.active(b)) return;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  if (update_uses_full(p.n))
-    update_full_body<T>(p, lv, b, task, smem_raw);
-  else
-    update_body<T>(p, lv, b, task, smem_raw);
-}
-
-// 64 < n <= 128: whole-block update (its own kernel: its register-held
-// accumulators would lower the occupancy of the small-block update)
-template <typename T>
-__global__ void __launch_bounds__(256, 1) k_update_big(Problem<T> p, Level lv) {
-  const int per_b = update_blocks(p.N, lv);
-  const int b = blockIdx.x / per_b;
-  const int task = blockIdx.x - b * per_b;
-  pdl_wait();
-  pdl_trigger();
-  if (!p.active(b)) return;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  update_big_body<T>(p, lv, b, task, smem_raw);
 }
 
 // ---------------------------------------------------------------------------

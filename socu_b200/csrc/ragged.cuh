@@ -83,7 +83,6 @@ __host__ __device__ inline Level rg_level(int N, int l) {
   lv.on = nxt;
   lv.op = prev;
   lv.tc = 0;       // persistent CTAs: SIMT sweep products (lower latency per node)
-  lv.tile = 32;    // unused (n <= 64: whole-block updates)
   lv.pre = 0;      // no programmatic launches in the persistent kernel
   return lv;
 }

@@ -1,0 +1,6 @@
+// float instantiations of the Schur update.
+#include "update_rows.cuh"
+
+namespace socu {
+SOCU_UPDATE_ROWS_KERNELS(float)
+}  // namespace socu
