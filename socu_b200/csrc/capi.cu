@@ -1,6 +1,5 @@
 // C ABI of socu_b200: argument validation, level scheduling, kernel enqueue,
 // and launch objects with optional CUDA-graph capture.
-#include <cuda.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -64,8 +63,6 @@ void schedule(int N, Schedule* out) {
     nxt += N / s - 1;
   }
 }
-
-int threads_for(int n) { return n <= 16 ? 64 : (n <= 32 ? 128 : 256); }
 
 int max_smem_optin() {
   static int cached = -1;
@@ -362,82 +359,6 @@ bool top_sweep_enabled() {
   return on != 0;
 }
 
-// ---------------------------------------------------------------------------
-// TMA tensor maps of the resident sweeps.  cuTensorMapEncodeTiled is a
-// driver-API call; it is resolved through the runtime's entry-point query, so
-// the library does not link against libcuda.  SOCU_TMA=0 keeps the sweeps on
-// per-thread cp.async copies.
-// ---------------------------------------------------------------------------
-using TmaEncodeFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
-                                 const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
-                                 CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
-TmaEncodeFn tma_encoder() {
-  static const TmaEncodeFn fn = [] {
-    void* f = nullptr;
-    cudaDriverEntryPointQueryResult q = cudaDriverEntryPointSymbolNotFound;
-    if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &f, 12000, cudaEnableDefault, &q) !=
-            cudaSuccess ||
-        q != cudaDriverEntryPointSuccess || f == nullptr) {
-      (void)cudaGetLastError();
-      return static_cast<TmaEncodeFn>(nullptr);
-    }
-    return reinterpret_cast<TmaEncodeFn>(f);
-  }();
-  return fn;
-}
-
-bool tma_enabled() {
-  static const int on = [] {
-    const char* v = std::getenv("SOCU_TMA");
-    return (v != nullptr && v[0] == '0') ? 0 : 1;
-  }();
-  return on != 0;
-}
-
-// 4-D map {cols, rows, count, batch} of an array of row-major rows x cols
-// tiles (batch entries batch_stride elements apart), box {box_cols, rows, 1, 1}.
-// false when an alignment rule of the TMA unit is not met (the caller then
-// copies with cp.async): base, row, tile and batch strides on 16 bytes, box
-// rows of a multiple of 16 bytes, box extents <= 256.
-bool encode_tiles(CUtensorMap* map, const void* base, int es, int cols, int rows, long long count, int batch,
-                  long long batch_stride, int box_cols) {
-  const TmaEncodeFn enc = tma_encoder();
-  if (enc == nullptr || base == nullptr || cols < 1 || rows < 1 || count < 1 || batch < 1) return false;
-  const unsigned long long row_b = (unsigned long long)cols * es, tile_b = row_b * (unsigned long long)rows;
-  const unsigned long long batch_b =
-      (unsigned long long)(batch > 1 ? batch_stride : count * rows * (long long)cols) * (unsigned long long)es;
-  if ((reinterpret_cast<uintptr_t>(base) & 15u) != 0 || (row_b & 15u) != 0 || (tile_b & 15u) != 0 ||
-      (batch_b & 15u) != 0 || batch_b == 0)
-    return false;
-  if (box_cols < 1 || box_cols > 256 || rows > 256 || ((long long)box_cols * es) % 16 != 0) return false;
-  const cuuint64_t dims[4] = {(cuuint64_t)cols, (cuuint64_t)rows, (cuuint64_t)count, (cuuint64_t)batch};
-  const cuuint64_t strides[3] = {row_b, tile_b, batch_b};
-  const cuuint32_t box[4] = {(cuuint32_t)box_cols, (cuuint32_t)rows, 1u, 1u};
-  const cuuint32_t estr[4] = {1u, 1u, 1u, 1u};
-  return enc(map, es == 8 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT64 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4,
-             const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-             CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
-}
-
-// Maps of one op's resident sweeps: factor / coupling blocks with the padded
-// block row (res_ldm), vector chunks with the padded vector row (res_ldy).
-template <typename T>
-SweepMaps sweep_maps(const Problem<T>& p) {
-  SweepMaps m;
-  std::memset(&m, 0, sizeof m);
-  // (the sweeps wait for their block copies in the first vector chunk)
-  if (!tma_enabled() || p.m <= 0 || p.X == nullptr) return m;
-  constexpr int es = sizeof(T);
-  const int ldm = res_ldm(p.n);
-  m.blocks = encode_tiles(&m.L, p.L, es, p.n, p.n, p.N, p.B, p.sL, ldm) &&
-             (p.S == 0 || encode_tiles(&m.E, p.E, es, p.n, p.n, p.S, p.B, p.sE, ldm));
-  m.vecs = p.X != nullptr && p.m > 0 &&
-           encode_tiles(&m.X, p.X, es, p.m, p.n, p.N, p.B, p.sX, res_ldy(std::min(p.m, kMC)));
-  return m;
-}
-
 // The library links the CUDA runtime statically, so its notion of the
 // current device is separate from the caller's: follow the device that owns
 // the data.
@@ -478,13 +399,8 @@ Problem<T> make_problem(void* L, void* E, void* x, const uint8_t* mask, const Di
   return p;
 }
 
-// Whether a factor may carry its diagonal inverses (k_node<INV>) for
-// matvec-based sweeps: small blocks whose sweeps run resident.
-template <typename T>
-bool use_inverse(int n, int m) {
-  return n <= 64 && (long long)smem_sweep_res_elems(n, m > 0 ? m : 1) * (long long)sizeof(T) <=
-                        (long long)max_smem_optin();
-}
+// Whether a factor may carry its diagonal inverses for sweeps by products.
+inline bool use_inverse(int n) { return n <= 64; }
 
 // Block-row FP64 residual (n <= 128): 1, 2 or 4 eight-column groups of
 // right-hand sides per pass over the matrix blocks, by n_rhs.
@@ -514,7 +430,7 @@ cudaError_t launch_residual_rows(const RefineArgs& a, cudaStream_t st, bool pdl)
 template <typename T>
 int enqueue(socu_op op, const Problem<T>& p, cudaStream_t st, long long* count, bool inv = false,
             const socu_tuning* over = nullptr) {
-  const int n = p.n, nth = threads_for(n);
+  const int n = p.n;
   socu_tuning cfg = tuning_lookup(sizeof(T) == 8 ? SOCU_FLOAT64 : SOCU_FLOAT32, n, p.m);
   if (over) tuning_merge(&cfg, *over);
   Schedule lv;
@@ -523,13 +439,12 @@ int enqueue(socu_op op, const Problem<T>& p, cudaStream_t st, long long* count, 
   const bool withY = op == SOCU_OP_FACTOR_AND_SOLVE;
   const size_t su = (size_t)smem_update_rows_bytes(n, sizeof(T));
   const UpdateRowsFn<T> update_kernel = update_rows_kernel<T>(n);
-  const int mm = p.m > 0 ? p.m : 1;
-  const bool res = (long long)smem_sweep_res_elems(n, mm) * (long long)sizeof(T) <= (long long)max_smem_optin();
-  const size_t ss = (res ? smem_sweep_res_elems(n, mm) : smem_sweep_elems(n, mm)) * sizeof(T);
-  inv = inv && res && n <= 64;
-  const SweepFn<T> fwd_kernel = sweep_kernel<T>(kSweepForward, res, inv);
-  const SweepFn<T> pull_kernel = sweep_kernel<T>(kSweepPull, res, inv);
-  const SweepFn<T> bwd_kernel = sweep_kernel<T>(kSweepBackward, res, inv);
+  inv = inv && use_inverse(n);
+  const SweepFn<T> fwd_kernel = sweep_kernel<T>(kModeForward, n, inv);
+  const SweepFn<T> pull_kernel = sweep_kernel<T>(kModePull, n, inv);
+  const SweepFn<T> bwd_kernel = sweep_kernel<T>(kModeBackward, n, inv);
+  const size_t ss = (size_t)smem_sweep_rows_bytes(n, inv), ss_pull = (size_t)smem_sweep_rows_bytes(n, true);
+  const int swp_thr = 32 * rows_nt(n);
   // Schur updates of float factors on the tcgen05 tensor cores (3xTF32), on
   // request: the FP64-pipe updates (exact products of the float operands,
   // FP64 sums) keep the float factor accurate enough for the reference's
@@ -559,7 +474,6 @@ int enqueue(socu_op op, const Problem<T>& p, cudaStream_t st, long long* count, 
   long long launches = 0;
   const bool run = count == nullptr;
   const int sms = run ? sm_count() : 0;
-  const int swp_thr = cfg.sweep_threads ? cfg.sweep_threads : nth;
 
   if (run) {
     cudaError_t e = cudaSuccess;
@@ -571,24 +485,11 @@ int enqueue(socu_op op, const Problem<T>& p, cudaStream_t st, long long* count, 
       if (e == cudaSuccess && node_tm) e = prepare(node_tm_kernel, sd_tm);
     }
     if (e == cudaSuccess) e = prepare(fwd_kernel, ss);
-    if (e == cudaSuccess) e = prepare(pull_kernel, ss);
+    if (e == cudaSuccess) e = prepare(pull_kernel, ss_pull);
     if (e == cudaSuccess) e = prepare(bwd_kernel, ss);
     if (e != cudaSuccess) return cuda_status(e);
   }
 
-  // sweep products on inverse-carrying float factors: tensor cores when the
-  // launch is wider than the resident sweep CTAs (3 per SM), or as tuned
-  // pre: the level's factor blocks were final before the previous kernel
-  // started (any sweep over a stored factor, and every backward level of
-  // factor_and_solve but the first), so they may be loaded before the wait
-  auto sweep_level = [&](const Level& L, long long blocks, bool pre) {
-    Level o = L;
-    if (cfg.sweep_tensor_cores == 1) o.tc = 1;
-    else if (cfg.sweep_tensor_cores == 2) o.tc = 0;
-    else o.tc = sms > 0 && blocks > 3LL * sms;
-    o.pre = pre ? 1 : 0;
-    return o;
-  };
   // programmatic launches inside the op's chain on its own stream (not the
   // first kernel, not while profiling with events)
   bool first = true;
@@ -603,10 +504,6 @@ int enqueue(socu_op op, const Problem<T>& p, cudaStream_t st, long long* count, 
     launch(kernel, (unsigned)blocks, (unsigned)threads, smem, s, pdl, p, L, extra...);
     prof_end(s);
   };
-  // TMA maps of the resident sweeps (zeros: cp.async copies)
-  SweepMaps maps;
-  std::memset(&maps, 0, sizeof maps);
-  if (run && res) maps = sweep_maps(p);
   // Level nodes: k_node_rows.  On levels with fewer nodes than
   // SMs a cluster of up to 8 blocks shares each node's row tiles (as many as
   // there are blocks' worth of row tiles outside L_i, while every block still
@@ -640,29 +537,22 @@ int enqueue(socu_op op, const Problem<T>& p, cudaStream_t st, long long* count, 
   const bool want_fwd = op == SOCU_OP_FORWARD_SUBSTITUTION || op == SOCU_OP_SOLVE;
   const bool want_bwd =
       op == SOCU_OP_BACKWARD_SUBSTITUTION || op == SOCU_OP_SOLVE || op == SOCU_OP_FACTOR_AND_SOLVE;
-  const TopFn<T> top_kernel = top_sweep_kernel<T>(inv);
+  const TopFn<T> top_kernel = top_sweep_kernel<T>(n, inv);
   TopLevels top;
   std::memset(&top, 0, sizeof top);
   int top_cluster = 0;
-  size_t top_smem = 0;
-  const int top_thr = swp_thr;
-  if (res && p.m > 0 && top_sweep_enabled() && (want_fwd || want_bwd)) {
-    for (int stages = 2; stages >= 1 && top_smem == 0; --stages) {
-      const size_t bytes = (size_t)smem_top_elems(n, p.m, stages) * sizeof(T);
-      if (bytes <= (size_t)max_smem_optin()) {
-        top_smem = bytes;
-        top.stages = stages;
-      }
-    }
-    for (int cl = 16; top_smem > 0 && cl >= 4 && top_cluster == 0; cl /= 2) {
+  const size_t top_smem = (size_t)smem_top_bytes(n, inv);
+  const int top_thr = 32 * top_nt(n);
+  if (n <= 64 && p.m > 0 && top_sweep_enabled() && (want_fwd || want_bwd)) {
+    for (int cl = 16; cl >= 4 && top_cluster == 0; cl /= 2) {
       int flo = K, blo = K;
       if (want_fwd)
-        while (flo > 0 && K - flo < kTopMaxLevels && fwd_tasks(p.N, lv[flo - 1]) <= cl) --flo;
+        while (flo > 0 && K - flo < kTopMaxLevels && sweep_tasks<kModeForward>(p.N, lv[flo - 1]) <= cl) --flo;
       if (want_bwd)
         while (blo > 0 && K - blo < kTopMaxLevels && lv[blo - 1].d <= cl) --blo;
       if ((K - flo) + (K - blo) < 2) break;
       int widest = 1;
-      for (int l = flo; l < K; ++l) widest = std::max(widest, fwd_tasks(p.N, lv[l]));
+      for (int l = flo; l < K; ++l) widest = std::max(widest, sweep_tasks<kModeForward>(p.N, lv[l]));
       for (int l = blo; l < K; ++l) widest = std::max(widest, lv[l].d);
       int c = 1;
       while (c < widest) c *= 2;
@@ -672,10 +562,8 @@ int enqueue(socu_op op, const Problem<T>& p, cudaStream_t st, long long* count, 
       top.fwd_n = K - flo;
       top.bwd_lo = blo;
       top.bwd_n = K - blo;
-      top.pre = op != SOCU_OP_FACTOR_AND_SOLVE ? 1 : 0;
-      for (int l = flo; l < K; ++l)
-        top.fl[l - flo] = sweep_level(lv[l], (long long)p.B * fwd_tasks(p.N, lv[l]), true);
-      for (int l = blo; l < K; ++l) top.bl[l - blo] = sweep_level(lv[l], (long long)p.B * lv[l].d, true);
+      for (int l = flo; l < K; ++l) top.fl[l - flo] = lv[l];
+      for (int l = blo; l < K; ++l) top.bl[l - blo] = lv[l];
     }
   }
   auto go_top = [&]() {
@@ -685,7 +573,7 @@ int enqueue(socu_op op, const Problem<T>& p, cudaStream_t st, long long* count, 
     first = false;
     prof_begin(st, top.bwd_n > 0 ? SOCU_KIND_BACKWARD : SOCU_KIND_FORWARD);
     launch_cluster(top_kernel, (unsigned)((long long)p.B * top_cluster), (unsigned)top_thr, top_smem, st, pdl,
-                   top_cluster, p, top, maps);
+                   top_cluster, p, top);
     prof_end(st);
   };
 
@@ -715,12 +603,6 @@ int enqueue(socu_op op, const Problem<T>& p, cudaStream_t st, long long* count, 
         go_rows(node_blocks, L);
       }
       if (l + 1 < K) {
-        // Fused forward: apply this level's updates to every target vector.  It
-        // only depends on the node, as the Schur update does, so the update is
-        // launched behind it without waiting for it (k_update_rows, `behind`).
-        const long long pull_blocks = withY ? (long long)p.B * (p.N / lv[l + 1].s) : 0;
-        go_on(st, pull_kernel, SOCU_KIND_PULL, pull_blocks, ss, sweep_level(lv[l + 1], pull_blocks, false), swp_thr,
-              maps);
         const long long upd_blocks = (long long)p.B * update_blocks(p.N, L);
         bool tc_done = false;
         if constexpr (sizeof(T) == 4) {
@@ -734,23 +616,30 @@ int enqueue(socu_op op, const Problem<T>& p, cudaStream_t st, long long* count, 
           int splits = 1;
           while (splits < 8 && splits * 2 <= ceil_div(n, 8) && upd_blocks * splits * 2 <= sms) splits *= 2;
           go_on(st, update_kernel, SOCU_KIND_UPDATE, upd_blocks * splits, su, L, 32 * update_rows_warps(n, splits),
-                splits, (int)(pull_blocks > 0));
+                splits);
         }
+        // Fused forward: apply this level's updates to every target vector.  It
+        // only depends on the node, as the update does, and runs beside it.
+        const long long pull_blocks = withY ? (long long)p.B * (p.N / lv[l + 1].s) : 0;
+        go_on(st, pull_kernel, SOCU_KIND_PULL, pull_blocks, ss_pull, lv[l + 1], swp_thr, (int)kWaitEnd);
       }
     }
   }
+  // the blocks of a sweep over a stored factor, and of every backward level of
+  // factor_and_solve but the first, were complete before the previous kernel
+  // started: they are loaded before the wait for it
   if (op == SOCU_OP_FORWARD_SUBSTITUTION || op == SOCU_OP_SOLVE) {
     for (int l = 0; l < (top_cluster ? top.fwd_lo : K); ++l) {
-      const long long blocks = (long long)p.B * (l == 0 ? lv[l].d : p.N / lv[l].s);
-      go_on(st, fwd_kernel, SOCU_KIND_FORWARD, blocks, ss, sweep_level(lv[l], blocks, true), swp_thr, maps);
+      const long long blocks = (long long)p.B * sweep_tasks<kModeForward>(p.N, lv[l]);
+      go_on(st, fwd_kernel, SOCU_KIND_FORWARD, blocks, ss, lv[l], swp_thr, (int)kWaitVectors);
     }
   }
   if (top_cluster) go_top();
   if (op == SOCU_OP_BACKWARD_SUBSTITUTION || op == SOCU_OP_SOLVE || op == SOCU_OP_FACTOR_AND_SOLVE) {
     for (int l = (top_cluster ? top.bwd_lo : K) - 1; l >= 0; --l) {
       const long long blocks = (long long)p.B * lv[l].d;
-      go_on(st, bwd_kernel, SOCU_KIND_BACKWARD, blocks, ss,
-            sweep_level(lv[l], blocks, op != SOCU_OP_FACTOR_AND_SOLVE || l != K - 1), swp_thr, maps);
+      go_on(st, bwd_kernel, SOCU_KIND_BACKWARD, blocks, ss, lv[l], swp_thr,
+            (int)(op != SOCU_OP_FACTOR_AND_SOLVE || l != K - 1 ? kWaitVectors : kWaitFirst));
     }
   }
   if (count) *count = launches;
@@ -789,9 +678,7 @@ int validate(socu_op op, socu_dtype dtype, const void* L, const void* E, const v
   }
   if ((int64_t)n > socu_max_block_size(dtype, needs_x ? n_rhs : 0)) return SOCU_ERR_UNSUPPORTED;
   if (inv_op) {
-    const int mm = needs_x ? (int)n_rhs : 1;
-    const bool ok = dtype == SOCU_FLOAT64 ? use_inverse<double>((int)n, mm) : use_inverse<float>((int)n, mm);
-    if (!ok) return SOCU_ERR_UNSUPPORTED;
+    if (!use_inverse((int)n)) return SOCU_ERR_UNSUPPORTED;
   }
   d->B = (int)batch;
   d->N = (int)horizon;
@@ -976,7 +863,7 @@ int refine_prologue(const RefineArgs& a, cudaStream_t st, long long* count) {
   socu_tuning mixed{};
   if (a.n > 64 && update_tc_ok(a.n) && tuning_lookup(SOCU_FLOAT32, a.n, a.m).update_tensor_cores == 0)
     mixed.update_tensor_cores = 1;
-  int s = enqueue<float>(SOCU_OP_FACTOR_AND_SOLVE, pf, st, run ? nullptr : &c, use_inverse<float>(a.n, a.m), &mixed);
+  int s = enqueue<float>(SOCU_OP_FACTOR_AND_SOLVE, pf, st, run ? nullptr : &c, use_inverse(a.n), &mixed);
   if (s != SOCU_OK) return s;
   s = refine_finish_round(a, st, run ? nullptr : &cr);
   if (count) *count = 2 + c + cr;
@@ -990,7 +877,7 @@ int refine_iteration(const RefineArgs& a, cudaStream_t st, long long* count) {
   Dims d{a.B, a.N, a.n, a.m, a.S};
   Problem<float> pf = make_problem<float>(a.L32, a.E32, a.R32, a.active, d);
   long long c = 0, cr = 0;
-  int s = enqueue<float>(SOCU_OP_SOLVE, pf, st, run ? nullptr : &c, use_inverse<float>(a.n, a.m));
+  int s = enqueue<float>(SOCU_OP_SOLVE, pf, st, run ? nullptr : &c, use_inverse(a.n));
   if (s != SOCU_OK) return s;
   s = refine_finish_round(a, st, run ? nullptr : &cr);
   if (count) *count = c + cr;
@@ -1543,12 +1430,11 @@ int64_t socu_off_diag_storage_len(int64_t horizon) {
 
 int64_t socu_max_block_size(socu_dtype dtype, int64_t n_rhs) {
   const size_t es = dtype == SOCU_FLOAT64 ? sizeof(double) : sizeof(float);
-  const int m = n_rhs > 0 ? (int)(n_rhs < kMC ? n_rhs : kMC) : 0;
   const long long limit = max_smem_optin();
   int64_t best = 0;
   for (int n = 1; n <= 512; ++n) {
     long long need = smem_rows_bytes(n) / (long long)es;
-    const long long u = smem_update_rows_bytes(n, (int)es) / (long long)es, s = smem_sweep_elems(n, m > 0 ? m : 1);
+    const long long u = smem_update_rows_bytes(n, (int)es) / (long long)es, s = smem_sweep_rows_bytes(n, false) / (long long)es;
     if (u > need) need = u;
     if (s > need) need = s;
     if (need * (long long)es <= limit && n <= 128) best = n;
@@ -1936,11 +1822,6 @@ int socu_tc_error(int* flag, int reset) {
     const int zero = 0;
     e = cudaMemcpyToSymbol(g_tc_error, &zero, sizeof(int));
   }
-  int sweep = 0;
-  if (e == cudaSuccess) e = sweep_wait_error<float>(&sweep, reset != 0);
-  if (e == cudaSuccess && *flag == 0) *flag = sweep;
-  if (e == cudaSuccess) e = sweep_wait_error<double>(&sweep, reset != 0);
-  if (e == cudaSuccess && *flag == 0) *flag = sweep;
   return cuda_status(e);
 }
 

@@ -817,16 +817,6 @@ __device__ __forceinline__ void fwd_body(const Problem<T>& p, const Level& lv, i
   }
 }
 
-template <typename T, bool RES, bool PULL_ONLY = false, bool INV = false>
-__global__ void __launch_bounds__(256) k_fwd(Problem<T> p, Level lv, const __grid_constant__ SweepMaps tm) {
-  const int per_b = fwd_tasks(p.N, lv);
-  const int b = blockIdx.x / per_b;
-  const int task = blockIdx.x - b * per_b;
-  if (!p.active(b)) return;
-  extern __shared__ __align__(128) unsigned char smem_raw[];
-  fwd_body<T, RES, PULL_ONLY, INV>(p, lv, b, task, smem_raw, &tm);
-}
-
 // ---------------------------------------------------------------------------
 // k_bwd (level l, descending): x_i -= F_i^T x_{i+s} + G_i x_{i-s};  x_i <- C_i^{-T} x_i
 // ---------------------------------------------------------------------------
@@ -922,15 +912,6 @@ __device__ __forceinline__ void bwd_body(const Problem<T>& p, const Level& lv, i
     }
     store_block(xi + c0, p.m, Y, ldy, n, mc);
   }
-}
-
-template <typename T, bool RES, bool INV = false>
-__global__ void __launch_bounds__(256) k_bwd(Problem<T> p, Level lv, const __grid_constant__ SweepMaps tm) {
-  const int b = blockIdx.x / lv.d;
-  const int t = blockIdx.x - b * lv.d;
-  if (!p.active(b)) return;
-  extern __shared__ __align__(128) unsigned char smem_raw[];
-  bwd_body<T, RES, INV>(p, lv, b, t, smem_raw, &tm);
 }
 
 }  // namespace socu

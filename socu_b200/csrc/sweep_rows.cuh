@@ -1,0 +1,396 @@
+// Substitution sweeps (n <= 128): one thread block per vector, one warp per
+// 8-row tile of it, products on FP64 tensor cores (mma.m8n8k4 .f64; float
+// factors and vectors are widened, one rounding per result).
+//
+//   forward (level l >= 1):  y_j -= F y_{j-s/2} + G^T y_{j+s/2}, then at the
+//                            level's own nodes  y_j <- C_j^{-1} y_j
+//   forward (level 0):       y_i <- C_i^{-1} y_i
+//   backward:                x_i -= F^T x_{i+s} + G x_{i-s};  x_i <- C_i^{-T} x_i
+//   pull:                    the coupling part of a forward level alone
+// (socu/block_tridiag_solver.py:425-736)
+//
+// A sweep reads every block once and no element of a block is needed by two
+// warps, so the blocks are not staged: each lane loads its MMA operands from
+// global memory straight into registers (row-major blocks as pairs along the
+// contraction, transposed ones down it; both fill whole 32-byte sectors) and,
+// up to n = 64, holds a whole row tile of all three blocks before the vectors
+// of the previous level are needed.  Only the vectors go through shared memory.
+//
+// On a factor that carries W = C^{-1} (INV) the solve is one more product.
+// Otherwise it is a substitution by 8-row tiles: each warp inverts its diagonal
+// tile ahead of the vectors, the warps take turns.
+#pragma once
+
+#include "node_rows.cuh"
+
+namespace socu {
+
+enum SweepMode { kModeForward = 0, kModeBackward = 1, kModePull = 2 };
+// how the kernel meets the one before it (programmatic dependent launch)
+enum SweepWait {
+  kWaitNone = 0,    // called inside another kernel
+  kWaitFirst = 1,   // the blocks themselves come from the previous kernel
+  kWaitVectors = 2, // the blocks were complete before: only the vectors are waited for
+  kWaitEnd = 3      // nothing comes from the previous kernel, see below
+};
+// kWaitEnd: the pull of factor_and_solve needs a level's nodes and is launched
+// behind their Schur update, which gives it nothing.  The update's blocks let
+// their successor start only after their own wait for the nodes, so the nodes'
+// results are complete when the pull runs: it works beside the update and waits
+// for it at its end, so that whatever waits for the pull has waited for both.
+
+// columns per pass: 8 up to n = 64, where the blocks stay in registers between passes, else 32
+__host__ __device__ constexpr int sweep_cols(int nt) { return nt <= 8 ? 8 : 32; }
+// stride of a staged vector row: 2 (mod 8) doubles, so the two rows of an operand pair and the
+// next three pairs of a half warp are on distinct banks
+__host__ __device__ constexpr int sweep_ldz(int nt) { return sweep_cols(nt) + 2; }
+__host__ __device__ inline long long smem_sweep_rows_bytes(int n, bool inv) {
+  const int nt = rows_nt(n);
+  return 8LL * (3LL * 8 * nt * sweep_ldz(nt) + (inv ? 0 : 64LL * nt));
+}
+
+// two consecutive elements through L2 (another block may have written them in this kernel's lifetime)
+template <typename T>
+__device__ __forceinline__ void ldcg_pair(const T* p, bool vec, bool v0, bool v1, double& x0, double& x1) {
+  if (vec) {
+    if constexpr (sizeof(T) == 8) {
+      const double2 v = __ldcg(reinterpret_cast<const double2*>(p));
+      x0 = v.x;
+      x1 = v.y;
+    } else {
+      const float2 v = __ldcg(reinterpret_cast<const float2*>(p));
+      x0 = (double)v.x;
+      x1 = (double)v.y;
+    }
+  } else {
+    x0 = v0 ? (double)__ldcg(p) : 0.0;
+    x1 = v1 ? (double)__ldcg(p + 1) : 0.0;
+  }
+}
+
+// MMA operand of an n x n block, row tile i, column tile kk: elements (r, c), (r, c + 1) with
+// r = 8i + g, c = 8kk + 2t; TR: of the block's transpose.  raw: as stored (widened later).
+template <typename T, bool TR>
+__device__ __forceinline__ void block_frag(const T* M, int n, int i, int kk, bool vec, T& a0, T& a1) {
+  const int lane = threadIdx.x & 31, r = 8 * i + (lane >> 2), c = 8 * kk + 2 * (lane & 3);
+  if (TR) {
+    a0 = (r < n && c < n) ? M[(long long)c * n + r] : T(0);
+    a1 = (r < n && c + 1 < n) ? M[(long long)(c + 1) * n + r] : T(0);
+  } else if (vec) {
+    if constexpr (sizeof(T) == 8) {
+      const double2 v = *reinterpret_cast<const double2*>(M + (long long)r * n + c);
+      a0 = v.x;
+      a1 = v.y;
+    } else {
+      const float2 v = *reinterpret_cast<const float2*>(M + (long long)r * n + c);
+      a0 = v.x;
+      a1 = v.y;
+    }
+  } else {
+    a0 = (r < n && c < n) ? M[(long long)r * n + c] : T(0);
+    a1 = (r < n && c + 1 < n) ? M[(long long)r * n + c + 1] : T(0);
+  }
+}
+
+// Operand of the solve, row tile i, column tile kk (0 outside its triangle).
+//   INV forward: W (strictly upper L transposed), backward: W^T; the diagonal is 1 / C[r][r].
+//   Else forward: C left of the diagonal tile, backward: C^T right of it.
+template <typename T, bool BWD, bool INV>
+__device__ __forceinline__ void solve_frag(const T* L, int n, int i, int kk, bool vec, T& a0, T& a1) {
+  a0 = a1 = T(0);
+  if (BWD ? kk < i : kk > i) return;
+  if (kk != i) {
+    block_frag<T, INV != BWD>(L, n, i, kk, vec, a0, a1);
+    return;
+  }
+  if (!INV) return;
+  const int lane = threadIdx.x & 31, r = 8 * i + (lane >> 2), c = 8 * i + 2 * (lane & 3);
+  T a[2];
+#pragma unroll
+  for (int e = 0; e < 2; ++e) {
+    const int k = c + e;
+    const bool in = r < n && k < n;
+    const bool off = BWD ? k > r : k < r;
+    const T v = in && (off || k == r) ? (BWD ? L[(long long)r * n + k] : L[(long long)k * n + r]) : T(0);
+    a[e] = in && k == r ? T(1) / v : (off ? v : T(0));
+  }
+  a0 = a[0];
+  a1 = a[1];
+}
+
+// One vector.  ONE: the block has a warp per row tile (else the warps loop over them and the
+// blocks are read as they are used).
+template <typename T, int NT, int MODE, bool INV, bool ONE>
+__device__ __forceinline__ void sweep_rows_body(const Problem<T>& p, const Level& lv, int b, int task,
+                                                unsigned char* smem_raw, int wait) {
+  constexpr bool BWD = MODE == kModeBackward, KEEP = ONE && NT <= 8;
+  constexpr int XC = sweep_cols(NT), CG = XC / 8, ldz = sweep_ldz(NT), NK = KEEP ? NT : 1;
+  static_assert(INV || ONE, "the substitution needs a warp per row tile");
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, W = blockDim.x >> 5;
+  const int g = lane >> 2, t = lane & 3;
+  const int n = p.n, m = p.m, N = p.N, s = lv.s, nta = (n + 7) >> 3;
+  // the vector, the row-major block P with its vector and the transposed block Q with its
+  int j, jp = 0, jq = 0;
+  bool solve = MODE != kModePull;
+  const T *P = nullptr, *Q = nullptr;
+  if (BWD) {
+    j = s - 1 + 2 * s * task;
+    jp = j - s;
+    jq = j + s;
+    if (j >= s) P = p.Eb(b, lv.oc + 2 * task - 1);
+    if (j + s < N) Q = p.Eb(b, lv.oc + 2 * task);
+  } else if (s == 1) {
+    j = 2 * task;
+  } else {
+    const int u = task + 1, h = s / 2;
+    j = s * u - 1;
+    jp = j - h;
+    jq = j + h;
+    P = p.Eb(b, lv.op + 2 * u - 2);
+    if (jq < N) Q = p.Eb(b, lv.op + 2 * u - 1);
+    solve = MODE == kModeForward && (u & 1) != 0;
+  }
+  const T* L = p.Lb(b, j);
+  T* yj = p.Xb(b, j);
+  const bool vec = n == 8 * nta && ((reinterpret_cast<uintptr_t>(p.L) | reinterpret_cast<uintptr_t>(p.E)) &
+                                    (2 * sizeof(T) - 1)) == 0;
+  const bool vecx = (m & 1) == 0 && (reinterpret_cast<uintptr_t>(p.X) & (2 * sizeof(T) - 1)) == 0;
+  double* Zp = reinterpret_cast<double*>(smem_raw);
+  double* Zq = Zp + 8 * NT * ldz;
+  double* Rs = Zq + 8 * NT * ldz;
+  double* Iv = Rs + 8 * NT * ldz;
+
+  if (wait == kWaitFirst) pdl_wait();
+  if (wait == kWaitEnd) {
+    __threadfence();
+    pdl_trigger();
+  }
+  T fp[NK][2], fq[NK][2], fs[ONE ? NT : 1][2];
+  if (KEEP && warp < nta) {
+#pragma unroll
+    for (int kk = 0; kk < NT; ++kk) {
+      if (P) block_frag<T, false>(P, n, warp, kk, vec && kk < nta, fp[KEEP ? kk : 0][0], fp[KEEP ? kk : 0][1]);
+      if (Q) block_frag<T, true>(Q, n, warp, kk, false, fq[KEEP ? kk : 0][0], fq[KEEP ? kk : 0][1]);
+    }
+    if (solve)
+#pragma unroll
+      for (int kk = 0; kk < NT; ++kk) solve_frag<T, BWD, INV>(L, n, warp, kk, vec && kk < nta, fs[ONE ? kk : 0][0], fs[ONE ? kk : 0][1]);
+  }
+  double i0 = 0.0, i1 = 0.0;   // inverse of the diagonal tile (transposed for the backward sweep)
+  if (!INV && solve && warp < nta) {
+    // every lane: column lane % 8 of C_kk^{-1}, from the tile in shared memory
+    double* D = Iv + 64 * warp;
+    {
+      T d0, d1;
+      block_frag<T, false>(L, n, warp, warp, vec, d0, d1);
+      const int r = 8 * warp + g, c = 8 * warp + 2 * t;   // padding: an identity
+      D[2 * lane] = r >= n && r == c ? 1.0 : (double)d0;
+      D[2 * lane + 1] = r >= n && r == c + 1 ? 1.0 : (double)d1;
+    }
+    __syncwarp();
+    double y[8], rd[8];
+#pragma unroll
+    for (int a = 0; a < 8; ++a) rd[a] = 1.0 / D[9 * a];
+#pragma unroll
+    for (int a = 0; a < 8; ++a) {
+      double v = a == (lane & 7) ? 1.0 : 0.0;
+#pragma unroll
+      for (int c = 0; c < a; ++c) v = fma(-D[8 * a + c], y[c], v);
+      y[a] = v * rd[a];
+    }
+    __syncwarp();
+#pragma unroll
+    for (int a = 0; a < 8; ++a) D[8 * a + (lane & 7)] = y[a];
+    __syncwarp();
+    i0 = BWD ? D[8 * (2 * t) + g] : D[8 * g + 2 * t];
+    i1 = BWD ? D[8 * (2 * t + 1) + g] : D[8 * g + 2 * t + 1];
+  }
+  if (wait == kWaitVectors) pdl_wait();
+  if (wait == kWaitFirst || wait == kWaitVectors) pdl_trigger();
+
+  for (int c0 = 0; c0 < m; c0 += XC) {
+    const int mc = min_i(XC, m - c0), groups = (mc + 7) >> 3;
+    if (c0 > 0) __syncthreads();
+    // neighbours' vectors, zeros outside
+    if (P || Q) {
+      for (int e = threadIdx.x; e < 8 * nta * 8 * groups; e += blockDim.x) {
+        const int k = e / (8 * groups), c = e - k * (8 * groups);
+        const bool in = k < n && c < mc;
+        const long long o = (long long)k * m + c0 + c;
+        if (P) Zp[k * ldz + c] = in ? (double)__ldcg(p.Xb(b, jp) + o) : 0.0;
+        if (Q) Zq[k * ldz + c] = in ? (double)__ldcg(p.Xb(b, jq) + o) : 0.0;
+      }
+    }
+    double ys[ONE ? CG : 1][2];
+    if (ONE && CG == 1 && warp < nta) {   // (with four column groups the registers are short: after the products)
+      const int r = 8 * warp + g, c = c0 + 2 * t;
+      ldcg_pair(yj + (long long)r * m + c, vecx && r < n && c < m, r < n && c < m, r < n && c + 1 < m, ys[0][0], ys[0][1]);
+    }
+    __syncthreads();
+    for (int i = warp; i < nta; i += ONE ? 8 * NT : W) {
+      // one column group: a chain of MMAs per block; four groups are four chains as they are
+      double ap[CG][2], aq[1][2] = {{0.0, 0.0}};
+#pragma unroll
+      for (int q = 0; q < CG; ++q) ap[q][0] = ap[q][1] = 0.0;
+      if (P || Q) {
+#pragma unroll(KEEP ? NT : 4)
+        for (int kk = 0; kk < (KEEP ? NT : nta); ++kk) {
+          {
+            T f0 = T(0), f1 = T(0), h0 = T(0), h1 = T(0);
+            if (KEEP) {
+              f0 = fp[KEEP ? kk : 0][0];
+              f1 = fp[KEEP ? kk : 0][1];
+              h0 = fq[KEEP ? kk : 0][0];
+              h1 = fq[KEEP ? kk : 0][1];
+            } else {
+              if (P) block_frag<T, false>(P, n, i, kk, vec, f0, f1);
+              if (Q) block_frag<T, true>(Q, n, i, kk, false, h0, h1);
+            }
+            const int zo = (8 * kk + 2 * t) * ldz + g;
+#pragma unroll
+            for (int q = 0; q < CG; ++q) {
+              if (CG == 1 || q < groups) {
+                if (P) {
+                  mma_acc(ap[q][0], ap[q][1], (double)f0, Zp[zo + 8 * q]);
+                  mma_acc(ap[q][0], ap[q][1], (double)f1, Zp[zo + ldz + 8 * q]);
+                }
+                if (Q) {
+                  double(&ac)[2] = CG == 1 ? aq[0] : ap[q];
+                  mma_acc(ac[0], ac[1], (double)h0, Zq[zo + 8 * q]);
+                  mma_acc(ac[0], ac[1], (double)h1, Zq[zo + ldz + 8 * q]);
+                }
+              }
+            }
+          }
+        }
+      }
+#pragma unroll
+      for (int q = 0; q < CG; ++q) {
+        if (CG > 1 && q >= groups) break;
+        const int r = 8 * i + g, c = c0 + 8 * q + 2 * t;
+        const bool ok0 = r < n && c < m, ok1 = r < n && c + 1 < m;
+        double y0, y1;
+        if (ONE && CG == 1) {
+          y0 = ys[0][0];
+          y1 = ys[0][1];
+        } else {
+          ldcg_pair(yj + (long long)r * m + c, vecx && ok0, ok0, ok1, y0, y1);
+        }
+        y0 -= ap[q][0] + (CG == 1 ? aq[0][0] : 0.0);
+        y1 -= ap[q][1] + (CG == 1 ? aq[0][1] : 0.0);
+        if (!solve) {
+          store_pair(yj + (long long)r * m + c, vecx && ok0, ok0, ok1, y0, y1);
+        } else {
+          if (ONE) {
+            ys[ONE ? q : 0][0] = y0;
+            ys[ONE ? q : 0][1] = y1;
+          }
+          if (INV) {
+            Rs[r * ldz + 8 * q + 2 * t] = y0;
+            Rs[r * ldz + 8 * q + 2 * t + 1] = y1;
+          }
+        }
+      }
+    }
+    if (!solve) continue;
+    if (ONE && !KEEP && warp < nta) {
+#pragma unroll
+      for (int kk = 0; kk < NT; ++kk) solve_frag<T, BWD, INV>(L, n, warp, kk, vec && kk < nta, fs[ONE ? kk : 0][0], fs[ONE ? kk : 0][1]);
+    }
+    if (INV) {
+      __syncthreads();
+      for (int i = warp; i < nta; i += ONE ? 8 * NT : W) {
+        double ax[CG][2], ay[CG][2];
+#pragma unroll
+        for (int q = 0; q < CG; ++q) ax[q][0] = ax[q][1] = ay[q][0] = ay[q][1] = 0.0;
+#pragma unroll
+        for (int kk = 0; kk < NT; ++kk) {
+          if (ONE ? kk < nta : (BWD ? kk >= i && kk < nta : kk <= i)) {
+            T f0, f1;
+            if (ONE) {
+              f0 = fs[ONE ? kk : 0][0];
+              f1 = fs[ONE ? kk : 0][1];
+            } else {
+              solve_frag<T, BWD, INV>(L, n, i, kk, vec, f0, f1);
+            }
+            const int zo = (8 * kk + 2 * t) * ldz + g;
+#pragma unroll
+            for (int q = 0; q < CG; ++q)
+              if (CG == 1 || q < groups) {
+                mma_acc(ax[q][0], ax[q][1], (double)f0, Rs[zo + 8 * q]);
+                mma_acc(ay[q][0], ay[q][1], (double)f1, Rs[zo + ldz + 8 * q]);
+              }
+          }
+        }
+#pragma unroll
+        for (int q = 0; q < CG; ++q) {
+          if (CG > 1 && q >= groups) break;
+          const int r = 8 * i + g, c = c0 + 8 * q + 2 * t;
+          store_pair(yj + (long long)r * m + c, vecx && r < n && c < m, r < n && c < m, r < n && c + 1 < m,
+                     ax[q][0] + ay[q][0], ax[q][1] + ay[q][1]);
+        }
+      }
+    } else {
+#pragma unroll
+      for (int st = 0; st < NT; ++st) {
+        const int kk = BWD ? NT - 1 - st : st;
+        if (kk < nta) {
+          if (warp == kk) {
+#pragma unroll
+            for (int q = 0; q < CG; ++q) {
+              Rs[(8 * kk + g) * ldz + 8 * q + 2 * t] = ys[ONE ? q : 0][0];
+              Rs[(8 * kk + g) * ldz + 8 * q + 2 * t + 1] = ys[ONE ? q : 0][1];
+            }
+            __syncwarp();
+            double xr[CG][2];
+#pragma unroll
+            for (int q = 0; q < CG; ++q) {
+              xr[q][0] = xr[q][1] = 0.0;
+              const int zo = (8 * kk + 2 * t) * ldz + 8 * q + g;
+              mma_acc(xr[q][0], xr[q][1], i0, Rs[zo]);
+              mma_acc(xr[q][0], xr[q][1], i1, Rs[zo + ldz]);
+            }
+            __syncwarp();
+#pragma unroll
+            for (int q = 0; q < CG; ++q) {
+              if (CG > 1 && q >= groups) break;
+              const int r = 8 * kk + g, c = c0 + 8 * q + 2 * t;
+              Rs[r * ldz + 8 * q + 2 * t] = xr[q][0];
+              Rs[r * ldz + 8 * q + 2 * t + 1] = xr[q][1];
+              store_pair(yj + (long long)r * m + c, vecx && r < n && c < m, r < n && c < m, r < n && c + 1 < m, xr[q][0],
+                         xr[q][1]);
+            }
+          }
+          __syncthreads();
+          if ((BWD ? warp < kk : warp > kk) && warp < nta) {
+#pragma unroll
+            for (int q = 0; q < CG; ++q) {
+              if (CG > 1 && q >= groups) break;
+              const int zo = (8 * kk + 2 * t) * ldz + 8 * q + g;
+              mma_acc(ys[ONE ? q : 0][0], ys[ONE ? q : 0][1], -(double)fs[ONE ? kk : 0][0], Rs[zo]);
+              mma_acc(ys[ONE ? q : 0][0], ys[ONE ? q : 0][1], -(double)fs[ONE ? kk : 0][1], Rs[zo + ldz]);
+            }
+          }
+        }
+      }
+    }
+  }
+  if (wait == kWaitEnd) pdl_wait();
+}
+
+// vectors of one level per instance
+template <int MODE>
+__host__ __device__ inline int sweep_tasks(int N, const Level& lv) {
+  return MODE == kModeBackward || lv.s == 1 ? lv.d : N / lv.s;
+}
+
+template <typename T, int NT, int MODE, bool INV>
+__global__ void __launch_bounds__(32 * NT, NT <= 8 ? 16 / NT : 1) k_sweep_rows(Problem<T> p, Level lv, int wait) {
+  const int per_b = sweep_tasks<MODE>(p.N, lv);
+  const int b = blockIdx.x / per_b;
+  if (!p.active(b)) return;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  sweep_rows_body<T, NT, MODE, INV, true>(p, lv, b, blockIdx.x - b * per_b, smem_raw, wait);
+}
+
+}  // namespace socu

@@ -235,35 +235,24 @@ __device__ __forceinline__ void update_rows_body(const Problem<T>& p, const Leve
   }
 }
 
-// behind: the kernel launched before this one (programmatically) is the
-// forward pull, which needs nothing from the update and gives it nothing.  Its
-// blocks let their successor start only after their own wait for the level's
-// nodes, so the nodes' blocks are complete when this kernel runs: it works
-// beside the pull and waits for it at the end, so that whatever waits for the
-// update has waited for the pull too.
 template <typename T, int NT>
 __global__ void __launch_bounds__(NT <= 8 ? 256 : 512, NT <= 8 ? 2 : 1)
-    k_update_rows(Problem<T> p, Level lv, int splits, int behind) {
+    k_update_rows(Problem<T> p, Level lv, int splits) {
   const int block = blockIdx.x / splits, q = blockIdx.x - block * splits;
   const int per_b = update_blocks(p.N, lv);
   const int b = block / per_b, task = block - b * per_b;
-  if (behind)
-    __threadfence();
-  else
-    pdl_wait();
+  pdl_wait();
   pdl_trigger();
-  if (p.active(b)) {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    if (splits > 1)
-      update_rows_body<T, NT, true>(p, lv, b, task, smem_raw, q, splits);
-    else
-      update_rows_body<T, NT, false>(p, lv, b, task, smem_raw, 0, 1);
-  }
-  if (behind) pdl_wait();
+  if (!p.active(b)) return;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  if (splits > 1)
+    update_rows_body<T, NT, true>(p, lv, b, task, smem_raw, q, splits);
+  else
+    update_rows_body<T, NT, false>(p, lv, b, task, smem_raw, 0, 1);
 }
 
 template <typename T>
-using UpdateRowsFn = void (*)(Problem<T>, Level, int, int);
+using UpdateRowsFn = void (*)(Problem<T>, Level, int);
 
 template <typename T>
 UpdateRowsFn<T> update_rows_kernel(int n);
