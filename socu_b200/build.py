@@ -25,9 +25,9 @@ OUT_DIR = PKG / "lib"
 OUT = OUT_DIR / "libsocu_b200.so"
 STAMP = OUT_DIR / ".build_stamp"
 
-SOURCES = ["capi.cu", "node_rows_f32.cu", "node_rows_f64.cu", "peak.cu", "ragged_f32.cu", "ragged_f64.cu",
-           "ragged_mixed.cu", "sweeps_f32.cu", "sweeps_f64.cu", "tc_selftest.cu",
-           "update_rows_f32.cu", "update_rows_f64.cu"]
+SOURCES = ["capi.cu", "node_rows_f32.cu", "node_rows_f64.cu", "peak.cu", "ragged_f32.cu", "ragged_f32_blocks.cu",
+           "ragged_f64.cu", "ragged_f64_blocks.cu", "ragged_mixed.cu", "ragged_mixed_blocks.cu", "sweeps_f32.cu",
+           "sweeps_f64.cu", "tc_selftest.cu", "update_rows_f32.cu", "update_rows_f64.cu"]
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 
 

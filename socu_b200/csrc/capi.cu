@@ -55,8 +55,6 @@ void schedule(int N, Schedule* out) {
     lv.oc = curr;
     lv.on = nxt;
     lv.op = prev;
-    lv.tc = 0;
-    lv.pre = 0;
     s *= 2;
     prev = curr;
     curr = nxt;
@@ -245,14 +243,14 @@ bool pdl_enabled() {
 }
 
 template <typename... KArgs, typename... Args>
-void launch(void (*kernel)(KArgs...), unsigned blocks, unsigned threads, size_t smem, cudaStream_t s, bool pdl,
+void launch(void (*kernel)(KArgs...), dim3 blocks, unsigned threads, size_t smem, cudaStream_t s, bool pdl,
             Args... args) {
   if (!pdl || !pdl_enabled()) {
     kernel<<<blocks, threads, smem, s>>>(args...);
     return;
   }
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(blocks);
+  cfg.gridDim = blocks;
   cfg.blockDim = dim3(threads);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = s;
@@ -437,12 +435,14 @@ int enqueue(socu_op op, const Problem<T>& p, cudaStream_t st, long long* count, 
   schedule(p.N, &lv);
   const int K = lv.K;
   const bool withY = op == SOCU_OP_FACTOR_AND_SOLVE;
+  // whole tiles: kernels with the block size built in
+  const bool full = 8 * rows_nt(n) == n && pairs_ok(p, n);
   const size_t su = (size_t)smem_update_rows_bytes(n, sizeof(T));
-  const UpdateRowsFn<T> update_kernel = update_rows_kernel<T>(n);
+  const UpdateRowsFn<T> update_kernel = update_rows_kernel<T>(n, full);
   inv = inv && use_inverse(n);
-  const SweepFn<T> fwd_kernel = sweep_kernel<T>(kModeForward, n, inv);
-  const SweepFn<T> pull_kernel = sweep_kernel<T>(kModePull, n, inv);
-  const SweepFn<T> bwd_kernel = sweep_kernel<T>(kModeBackward, n, inv);
+  const SweepFn<T> fwd_kernel = sweep_kernel<T>(kModeForward, n, full, inv);
+  const SweepFn<T> pull_kernel = sweep_kernel<T>(kModePull, n, full, inv);
+  const SweepFn<T> bwd_kernel = sweep_kernel<T>(kModeBackward, n, full, inv);
   const size_t ss = (size_t)smem_sweep_rows_bytes(n, inv), ss_pull = (size_t)smem_sweep_rows_bytes(n, true);
   const int swp_thr = 32 * rows_nt(n);
   // Schur updates of float factors on the tcgen05 tensor cores (3xTF32), on
@@ -470,7 +470,7 @@ int enqueue(socu_op op, const Problem<T>& p, cudaStream_t st, long long* count, 
   const size_t sd_tm = (size_t)smem_node_tm_bytes(n, m_node);
   auto node_tm_kernel = withY ? k_node_tm<true> : k_node_tm<false>;
   const size_t sd_rows = (size_t)smem_rows_bytes(n);
-  const NodeRowsFn<T> rows_kernel = node_rows_kernel<T>(n);
+  const NodeRowsFn<T> rows_kernel = node_rows_kernel<T>(n, full);
   long long launches = 0;
   const bool run = count == nullptr;
   const int sms = run ? sm_count() : 0;
@@ -503,6 +503,22 @@ int enqueue(socu_op op, const Problem<T>& p, cudaStream_t st, long long* count, 
     prof_begin(s, kind);
     launch(kernel, (unsigned)blocks, (unsigned)threads, smem, s, pdl, p, L, extra...);
     prof_end(s);
+  };
+  // One sweep level over `vecs` vectors.  Where they leave SMs idle, blocks of
+  // 8, 16, ... right-hand sides share a vector (each reads the vector's blocks,
+  // from L2; the products, which bound the block, are shared out).
+  auto go_sweep = [&](SweepFn<T> kernel, int kind, long long vecs, size_t smem, const Level& L, SweepWait wait) {
+    int cols = 8 * ceil_div(p.m, 8);
+    while (cols > 8 && vecs * ceil_div(p.m, 8 * ceil_div(cols, 16)) <= sms) cols = 8 * ceil_div(cols, 16);
+    if (vecs <= 0) return;
+    ++launches;
+    if (!run) return;
+    const bool pdl = !first && g_prof == nullptr;
+    first = false;
+    prof_begin(st, kind);
+    launch(kernel, dim3((unsigned)vecs, (unsigned)ceil_div(p.m, cols)), (unsigned)swp_thr, smem, st, pdl, p, L,
+           (int)wait, cols);
+    prof_end(st);
   };
   // Level nodes: k_node_rows.  On levels with fewer nodes than
   // SMs a cluster of up to 8 blocks shares each node's row tiles (as many as
@@ -621,7 +637,7 @@ int enqueue(socu_op op, const Problem<T>& p, cudaStream_t st, long long* count, 
         // Fused forward: apply this level's updates to every target vector.  It
         // only depends on the node, as the update does, and runs beside it.
         const long long pull_blocks = withY ? (long long)p.B * (p.N / lv[l + 1].s) : 0;
-        go_on(st, pull_kernel, SOCU_KIND_PULL, pull_blocks, ss_pull, lv[l + 1], swp_thr, (int)kWaitEnd);
+        go_sweep(pull_kernel, SOCU_KIND_PULL, pull_blocks, ss_pull, lv[l + 1], kWaitEnd);
       }
     }
   }
@@ -631,15 +647,15 @@ int enqueue(socu_op op, const Problem<T>& p, cudaStream_t st, long long* count, 
   if (op == SOCU_OP_FORWARD_SUBSTITUTION || op == SOCU_OP_SOLVE) {
     for (int l = 0; l < (top_cluster ? top.fwd_lo : K); ++l) {
       const long long blocks = (long long)p.B * sweep_tasks<kModeForward>(p.N, lv[l]);
-      go_on(st, fwd_kernel, SOCU_KIND_FORWARD, blocks, ss, lv[l], swp_thr, (int)kWaitVectors);
+      go_sweep(fwd_kernel, SOCU_KIND_FORWARD, blocks, ss, lv[l], kWaitVectors);
     }
   }
   if (top_cluster) go_top();
   if (op == SOCU_OP_BACKWARD_SUBSTITUTION || op == SOCU_OP_SOLVE || op == SOCU_OP_FACTOR_AND_SOLVE) {
     for (int l = (top_cluster ? top.bwd_lo : K) - 1; l >= 0; --l) {
       const long long blocks = (long long)p.B * lv[l].d;
-      go_on(st, bwd_kernel, SOCU_KIND_BACKWARD, blocks, ss, lv[l], swp_thr,
-            (int)(op != SOCU_OP_FACTOR_AND_SOLVE || l != K - 1 ? kWaitVectors : kWaitFirst));
+      go_sweep(bwd_kernel, SOCU_KIND_BACKWARD, blocks, ss, lv[l],
+               op != SOCU_OP_FACTOR_AND_SOLVE || l != K - 1 ? kWaitVectors : kWaitFirst);
     }
   }
   if (count) *count = launches;
@@ -1049,7 +1065,8 @@ struct socu_ragged_s {
   float* d_w32 = nullptr;         // refinement: L32 | E32 | R32
   size_t w_off[3] = {0, 0, 0};
   RefineState* d_state = nullptr;
-  int vc = 0, grid = 0;
+  int grid = 0, worker_bytes = 0;
+  bool blocks = false;            // thread blocks as workers (else warps)
   size_t smem = 0;
 };
 
@@ -1129,10 +1146,11 @@ void rg_free(socu_ragged_s* r) {
 
 template <typename T, int MODE>
 int rg_prepare_kernel(socu_ragged_s* r) {
-  auto kern = ragged_kernel<T, MODE>();
+  auto kern = r->blocks ? ragged_kernel<T, MODE, true>() : ragged_kernel<T, MODE, false>();
+  const int threads = rg_threads(r->blocks);
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)r->smem);
   int per_sm = 0, sms = 0;
-  if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kRgThreads, r->smem);
+  if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, threads, r->smem);
   if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, r->device);
   if (e != cudaSuccess) return cuda_status(e);
   if (per_sm < 1) return SOCU_ERR_UNSUPPORTED;
@@ -1146,17 +1164,12 @@ int rg_create(socu_ragged_s* r, const int64_t* horizon, const int64_t* n, const 
   r->count = (int)count;
   if (count == 0) return SOCU_OK;
   const int mode = r->refine ? kRgRefine : kRgPlain;
-  const int es = r->refine ? 4 : (r->dtype == SOCU_FLOAT64 ? 8 : 4);
   // queue capacity: every chunk of every phase (max_iter rounds when refining)
   long long cap = 0;
-  int maxn = 1, maxm = 1, maxnv = 1;
   for (const RgInst& I : r->inst) {
     const int phases = r->refine ? rg_refine_phases(I.K, r->max_iter) : rg_plain_phases(I.K);
     if (phases >= (1 << kRgPhaseBits)) return SOCU_ERR_UNSUPPORTED;
     for (int ph = 0; ph < phases; ++ph) cap += rg_chunks(rg_phase(I, mode, ph));
-    maxn = std::max(maxn, I.n);
-    maxm = std::max(maxm, I.m);
-    maxnv = std::max(maxnv, 3 * I.n + I.m);
   }
   // first-phase chunks, largest instances first
   std::vector<int> order(r->inst.size());
@@ -1171,13 +1184,16 @@ int rg_create(socu_ragged_s* r, const int64_t* horizon, const int64_t* n, const 
     const int c = rg_chunks(rg_phase(r->inst[i], mode, 0));
     for (int j = 0; j < c; ++j) init.push_back(rg_encode(i, 0, j));
   }
-  // shared memory: the largest body at the largest block size (n <= 64: the
-  // inverse-first node body)
-  r->vc = maxnv;
-  size_t smem = (size_t)smem_node_gemm_elems(maxn, maxm, es) * es;
-  smem = std::max(smem, (size_t)smem_update_full_elems(maxn, es) * es);
-  smem = std::max(smem, (size_t)smem_sweep_res_elems(maxn, maxm) * es);
-  if (r->refine) smem = std::max(smem, (size_t)smem_residual_rows_elems(maxn) * sizeof(double));
+  // Few nodes per warp worker: block workers (rg_use_blocks).
+  const int es = r->refine ? 4 : (r->dtype == SOCU_FLOAT64 ? 8 : 4);
+  long long nodes = 0;
+  for (const RgInst& I : r->inst) nodes += I.N;
+  r->blocks = rg_use_blocks(nodes, sm_count());
+  size_t smem = 0;
+  for (const RgInst& I : r->inst) {
+    smem = std::max(smem, (size_t)rg_block_bytes(I.n, es, r->refine, r->blocks));
+    r->worker_bytes = std::max(r->worker_bytes, (int)rg_unit_bytes(I.n, es, r->refine, r->blocks));
+  }
   if ((long long)smem > (long long)max_smem_optin()) return SOCU_ERR_UNSUPPORTED;
   r->smem = smem;
   cudaError_t e = cudaGetDevice(&r->device);
@@ -1186,7 +1202,7 @@ int rg_create(socu_ragged_s* r, const int64_t* horizon, const int64_t* n, const 
   else if (r->dtype == SOCU_FLOAT64) st = rg_prepare_kernel<double, kRgPlain>(r);
   else st = rg_prepare_kernel<float, kRgPlain>(r);
   if (st != SOCU_OK) return st;
-  cap += r->grid + 64;
+  cap += (long long)r->grid * kRgWorkers + 64;
   if (cap >= (1LL << 31)) return SOCU_ERR_UNSUPPORTED;
   r->capacity = (unsigned)cap;
   r->n_init = (unsigned)init.size();
@@ -1226,8 +1242,8 @@ int rg_launch(socu_ragged_s* r, RgArgs<T> a, cudaStream_t st) {
   a.q.init = r->d_init;
   a.q.n_init = r->n_init;
   a.q.capacity = r->capacity;
-  a.vc = r->vc;
   a.timeout_ns = r->timeout_ns > 0 ? r->timeout_ns : kRgTimeoutNs;
+  a.worker_bytes = r->worker_bytes;
   cudaError_t e = cudaMemsetAsync(r->d_slot + r->n_init, 0,
                                   sizeof(unsigned long long) * (r->capacity - r->n_init), st);
   if (e != cudaSuccess) return cuda_status(e);
@@ -1235,7 +1251,8 @@ int rg_launch(socu_ragged_s* r, RgArgs<T> a, cudaStream_t st) {
   const int sb = (int)std::min<long long>((work + 255) / 256, 1024);
   prof_begin(st, SOCU_KIND_RAGGED);
   k_rg_start<T, MODE><<<sb, 256, 0, st>>>(a);
-  ragged_kernel<T, MODE>()<<<r->grid, kRgThreads, r->smem, st>>>(a);
+  (r->blocks ? ragged_kernel<T, MODE, true>() : ragged_kernel<T, MODE, false>())<<<r->grid, rg_threads(r->blocks),
+                                                                               r->smem, st>>>(a);
   prof_end(st);
   return cuda_status(cudaGetLastError());
 }

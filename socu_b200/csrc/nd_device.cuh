@@ -23,7 +23,6 @@
 namespace socu {
 
 constexpr unsigned kFull = 0xffffffffu;
-constexpr int kBS = 32;  // row block of the blocked triangular solves
 
 template <typename T> __device__ __forceinline__ T rsqrt_t(T x);
 template <> __device__ __forceinline__ double rsqrt_t<double>(double x) { return rsqrt(x); }
@@ -92,9 +91,6 @@ struct Level {
   int oc;   // offset of this level's slots
   int on;   // offset of the next level's slots
   int op;   // offset of the previous level's slots (unused at level 0)
-  int tc;   // sweeps on inverse-carrying factors: 1 = FP64 tensor-core (DMMA) products, 0 = SIMT row dots
-  int pre;  // sweeps: the factor blocks were complete before the previous kernel started, so they may be
-            // loaded before the grid-dependency wait (programmatic dependent launch)
 };
 
 // Programmatic dependent launch (sm_90+).  A kernel launched with the
@@ -139,192 +135,49 @@ __device__ __forceinline__ int copy_width(const T* dst, int ld, const T* src, in
 }
 
 template <typename T, int BYTES>
-__device__ __forceinline__ void async_load_w(T* dst, int ld, const T* src, int rows, int cols, long long src_ld) {
+__device__ __forceinline__ void async_load_w(int tid, int threads, T* dst, int ld, const T* src, int rows, int cols,
+                                             long long src_ld) {
   constexpr int V = BYTES / sizeof(T);
   const int cv = cols / V;
-  const int total = rows * cv;
-  for (int e = threadIdx.x; e < total; e += blockDim.x) {
-    const int r = e / cv, c = (e - r * cv) * V;
-    cp_async_bytes<BYTES>(dst + r * ld + c, src + (long long)r * src_ld + c);
+  // element tid, tid + threads, ... of the rows x cv copies, without a division each
+  const int dr = threads / cv, dc = threads - dr * cv;
+  int r = tid / cv, c = tid - r * cv;
+#pragma unroll 2
+  while (r < rows) {
+    cp_async_bytes<BYTES>(dst + r * ld + c * V, src + (long long)r * src_ld + c * V);
+    r += dr;
+    c += dc;
+    if (c >= cv) {
+      c -= cv;
+      ++r;
+    }
   }
 }
 
-// dst[r*ld + c] = src[r*src_ld + c]; vectorised when alignment allows
+// dst[r*ld + c] = src[r*src_ld + c] by `threads` threads; vectorised when alignment allows
 template <typename T>
-__device__ __forceinline__ void async_load(T* dst, int ld, const T* src, int rows, int cols, long long src_ld) {
+__device__ __forceinline__ void async_load_by(int tid, int threads, T* dst, int ld, const T* src, int rows, int cols,
+                                              long long src_ld) {
   const int w = copy_width(dst, ld, src, cols, src_ld);
   if (w == 16)
-    async_load_w<T, 16>(dst, ld, src, rows, cols, src_ld);
+    async_load_w<T, 16>(tid, threads, dst, ld, src, rows, cols, src_ld);
   else if (w == 8)
-    async_load_w<T, 8>(dst, ld, src, rows, cols, src_ld);
+    async_load_w<T, 8>(tid, threads, dst, ld, src, rows, cols, src_ld);
   else
-    async_load_w<T, sizeof(T)>(dst, ld, src, rows, cols, src_ld);
+    async_load_w<T, sizeof(T)>(tid, threads, dst, ld, src, rows, cols, src_ld);
 }
-
-// dst[c*ld + r] = src[r*src_ld + c]   (global rows become shared columns)
 template <typename T>
-__device__ __forceinline__ void async_load_t(T* dst, int ld, const T* src, int rows, int cols, long long src_ld) {
-  const int total = rows * cols;
-  for (int e = threadIdx.x; e < total; e += blockDim.x) {
-    const int r = e / cols, c = e - r * cols;
-    cp_async_elem(dst + c * ld + r, src + (long long)r * src_ld + c);
-  }
+__device__ __forceinline__ void async_load(T* dst, int ld, const T* src, int rows, int cols, long long src_ld) {
+  async_load_by(threadIdx.x, blockDim.x, dst, ld, src, rows, cols, src_ld);
 }
 
-// even leading dimension (row starts 8/16-byte aligned) close to n
-__host__ __device__ inline int even_ld(int n) { return n + ((n & 1) ? 1 : 2); }
-
-template <typename T>
-__device__ __forceinline__ void store_block(T* dst, long long dst_ld, const T* src, int ld, int rows, int cols) {
-  const int total = rows * cols;
-  for (int e = threadIdx.x; e < total; e += blockDim.x) {
-    const int r = e / cols, c = e - r * cols;
-    dst[(long long)r * dst_ld + c] = src[r * ld + c];
-  }
-}
-
-// dst[r*dst_ld + c] = src[c*ld + r]
-template <typename T>
-__device__ __forceinline__ void store_block_t(T* dst, long long dst_ld, const T* src, int ld, int rows, int cols) {
-  const int total = rows * cols;
-  for (int e = threadIdx.x; e < total; e += blockDim.x) {
-    const int r = e / cols, c = e - r * cols;
-    dst[(long long)r * dst_ld + c] = src[c * ld + r];
-  }
-}
-
-// ---------------------------------------------------------------------------
-// Register-tiled CTA GEMM on shared-memory operands.
-//   acc(r,c) = sum_{k<K} opA(r,k) opB(k,c),  0<=r<M, 0<=c<N
-//   opA(r,k) = TA ? A[k*lda + r] : A[r*lda + k]
-//   opB(k,c) = TB ? B[c*ldb + k] : B[k*ldb + c]
-// then out(r, c, acc) for every valid entry (c <= r only if LOWER).
-// Threads own TM x TN micro-tiles; consecutive threads take consecutive
-// column tiles so row operands are broadcast inside a warp.  Out-of-range
-// rows/columns are clamped for loading and masked on output, so the k-loop
-// carries no branches.
-// ---------------------------------------------------------------------------
-template <typename T, int TM, int TN, bool TA, bool TB, bool LOWER = false, class Out>
-__device__ __forceinline__ void smem_gemm(int M, int N, int K, const T* __restrict__ A, int lda,
-                                          const T* __restrict__ B, int ldb, Out out) {
-  const int tm = (M + TM - 1) / TM;
-  const int tn = (N + TN - 1) / TN;
-  for (int t = threadIdx.x; t < tm * tn; t += blockDim.x) {
-    const int r0 = (t / tn) * TM;
-    const int c0 = (t % tn) * TN;
-    if (LOWER && c0 > r0 + TM - 1) continue;
-    int ra[TM], cb[TN];
-#pragma unroll
-    for (int i = 0; i < TM; ++i) ra[i] = min(r0 + i, M - 1);
-#pragma unroll
-    for (int j = 0; j < TN; ++j) cb[j] = min(c0 + j, N - 1);
-    T acc[TM][TN];
-#pragma unroll
-    for (int i = 0; i < TM; ++i)
-#pragma unroll
-      for (int j = 0; j < TN; ++j) acc[i][j] = T(0);
-#pragma unroll 4
-    for (int k = 0; k < K; ++k) {
-      T av[TM], bv[TN];
-#pragma unroll
-      for (int i = 0; i < TM; ++i) av[i] = TA ? A[k * lda + ra[i]] : A[ra[i] * lda + k];
-#pragma unroll
-      for (int j = 0; j < TN; ++j) bv[j] = TB ? B[cb[j] * ldb + k] : B[k * ldb + cb[j]];
-#pragma unroll
-      for (int i = 0; i < TM; ++i)
-#pragma unroll
-        for (int j = 0; j < TN; ++j) acc[i][j] = fma(av[i], bv[j], acc[i][j]);
-    }
-#pragma unroll
-    for (int i = 0; i < TM; ++i)
-#pragma unroll
-      for (int j = 0; j < TN; ++j) {
-        const int r = r0 + i, c = c0 + j;
-        if (r < M && c < N && (!LOWER || c <= r)) out(r, c, acc[i][j]);
-      }
-  }
-}
-
-// ---------------------------------------------------------------------------
-// FP64 tensor-core (DMMA, mma.sync m8n8k4 f64) warp GEMM on shared operands
-// of type T (float operands are widened to double in registers: exact
-// products, FP64 sums).
-//   acc(r,c) = sum_{k<K} opA(r,k) opB(k,c);  out(r, c, acc) per valid entry, acc a double.
-// Warp tiles of 16 x 32 (2 x 4 mma tiles).  Fragment layouts (PTX ISA,
-// mma.m8n8k4 .f64): A a0 = A[g][t], B b0 = B[t][g], C {c0,c1} = C[g][2t+{0,1}]
-// with g = lane/4, t = lane%4.  Leading dimensions of 4 (mod 16) doubles make
-// every fragment load conflict-free.
-// ---------------------------------------------------------------------------
+// FP64 tensor-core product of 8x8x4 (mma.m8n8k4 .f64).  Fragments (PTX ISA): A a0 = A[g][t],
+// B b0 = B[t][g], C {c0, c1} = C[g][2t + {0, 1}] with g = lane / 4, t = lane % 4.
 __device__ __forceinline__ void dmma_8x8x4(double& c0, double& c1, double a, double b) {
   asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
                : "+d"(c0), "+d"(c1)
                : "d"(a), "d"(b));
 }
-
-__host__ __device__ inline int ld_dmma(int n) { return ((n + 15) / 16) * 16 + 4; }
-
-template <typename T, bool TA, bool TB, bool LOWER = false, class Out>
-__device__ __forceinline__ void warp_gemm_dmma(int M, int N, int K, const T* __restrict__ A, int lda,
-                                               const T* __restrict__ B, int ldb, Out out) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  const int g = lane >> 2, t = lane & 3;
-  const int tm = (M + 15) / 16, tn = (N + 31) / 32;
-  for (int tile = warp; tile < tm * tn; tile += nw) {
-    const int r0 = (tile / tn) * 16, c0 = (tile % tn) * 32;
-    if (LOWER && c0 > r0 + 15) continue;
-    double acc[2][4][2];
-#pragma unroll
-    for (int i = 0; i < 2; ++i)
-#pragma unroll
-      for (int j = 0; j < 4; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
-    int ra[2], cb[4];
-#pragma unroll
-    for (int i = 0; i < 2; ++i) ra[i] = min(r0 + 8 * i + g, M - 1);
-#pragma unroll
-    for (int j = 0; j < 4; ++j) cb[j] = min(c0 + 8 * j + g, N - 1);
-#pragma unroll 2
-    for (int k0 = 0; k0 < K; k0 += 4) {
-      const int k = k0 + t;
-      const bool kv = k < K;
-      const int kc = kv ? k : K - 1;
-      double a[2], b[4];
-#pragma unroll
-      for (int i = 0; i < 2; ++i) {
-        const double v = (double)(TA ? A[kc * lda + ra[i]] : A[ra[i] * lda + kc]);
-        a[i] = kv ? v : 0.0;
-      }
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const double v = (double)(TB ? B[cb[j] * ldb + kc] : B[kc * ldb + cb[j]]);
-        b[j] = kv ? v : 0.0;
-      }
-#pragma unroll
-      for (int i = 0; i < 2; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) dmma_8x8x4(acc[i][j][0], acc[i][j][1], a[i], b[j]);
-    }
-#pragma unroll
-    for (int i = 0; i < 2; ++i)
-#pragma unroll
-      for (int j = 0; j < 4; ++j)
-#pragma unroll
-        for (int e = 0; e < 2; ++e) {
-          const int r = r0 + 8 * i + g, c = c0 + 8 * j + 2 * t + e;
-          if (r < M && c < N && (!LOWER || c <= r)) out(r, c, acc[i][j][e]);
-        }
-  }
-}
-
-// Type-dispatching CTA GEMM: DMMA for double, 4x4 SIMT micro-tiles for float.
-template <typename T, bool TA, bool TB, bool LOWER = false, class Out>
-__device__ __forceinline__ void cta_gemm(int M, int N, int K, const T* __restrict__ A, int lda,
-                                         const T* __restrict__ B, int ldb, Out out) {
-  if constexpr (sizeof(T) == 8)
-    warp_gemm_dmma<double, TA, TB, LOWER>(M, N, K, A, lda, B, ldb, out);
-  else
-    smem_gemm<T, 4, 4, TA, TB, LOWER>(M, N, K, A, lda, B, ldb, out);
-}
-
 
 // ---------------------------------------------------------------------------
 // Trailing update of one 8-column step of cta_chol_solve, both parts in one
@@ -337,69 +190,6 @@ __device__ __forceinline__ void cta_gemm(int M, int N, int K, const T* __restric
 // {c0, c1} = C[g][2t + {0, 1}], g = lane/4, t = lane%4).  FP32: 4 x 4 SIMT
 // micro-tiles per thread.
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ void rank_update_f64(double* A, int lda, double* V, int ldv, int n, int K, int kb,
-                                                int R0, int nv) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  const int g = lane >> 2, t = lane & 3;
-  const int M = n - R0;
-  const int tm = (M + 15) / 16;
-  const int tnA = (M + 31) / 32, tnV = (nv + 31) / 32;
-  const int nA = tm * tnA, total = nA + tm * tnV;
-  const double* P = A + R0 * lda + K;
-  for (int tile = warp; tile < total; tile += nw) {
-    const bool isA = tile < nA;
-    const int tt = isA ? tile : tile - nA;
-    const int tn = isA ? tnA : tnV;
-    const int r0 = (tt / tn) * 16, c0 = (tt % tn) * 32;
-    if (isA && c0 > r0 + 15) continue;
-    double* C = isA ? A + R0 * lda + R0 : V + R0 * ldv;
-    const int ldc = isA ? lda : ldv;
-    const int N = isA ? M : nv;
-    double acc[2][4][2];
-#pragma unroll
-    for (int i = 0; i < 2; ++i)
-#pragma unroll
-      for (int j = 0; j < 4; ++j)
-#pragma unroll
-        for (int e = 0; e < 2; ++e) {
-          const int r = r0 + 8 * i + g, c = c0 + 8 * j + 2 * t + e;
-          acc[i][j][e] = (r < M && c < N) ? C[r * ldc + c] : 0.0;
-        }
-    int ra[2], cb[4];
-#pragma unroll
-    for (int i = 0; i < 2; ++i) ra[i] = min(r0 + 8 * i + g, M - 1);
-#pragma unroll
-    for (int j = 0; j < 4; ++j) cb[j] = min(c0 + 8 * j + g, N - 1);
-#pragma unroll
-    for (int k0 = 0; k0 < 8; k0 += 4) {
-      const int k = k0 + t;
-      const bool kv = k < kb;
-      const int kc = kv ? k : 0;
-      double a[2], b[4];
-#pragma unroll
-      for (int i = 0; i < 2; ++i) a[i] = kv ? -P[ra[i] * lda + kc] : 0.0;
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const double v = isA ? P[cb[j] * lda + kc] : V[(K + kc) * ldv + cb[j]];
-        b[j] = kv ? v : 0.0;
-      }
-#pragma unroll
-      for (int i = 0; i < 2; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) dmma_8x8x4(acc[i][j][0], acc[i][j][1], a[i], b[j]);
-    }
-#pragma unroll
-    for (int i = 0; i < 2; ++i)
-#pragma unroll
-      for (int j = 0; j < 4; ++j)
-#pragma unroll
-        for (int e = 0; e < 2; ++e) {
-          const int r = r0 + 8 * i + g, c = c0 + 8 * j + 2 * t + e;
-          if (r < M && c < N && (!isA || c <= r)) C[r * ldc + c] = acc[i][j][e];
-        }
-  }
-}
-
 template <typename T>
 __device__ __forceinline__ void rank_update_simt(T* A, int lda, T* V, int ldv, int n, int K, int kb, int R0, int nv) {
   constexpr int BK = 8;
@@ -534,10 +324,7 @@ __device__ void cta_chol_solve(T* A, int lda, int n, T* V, int ldv, int nv) {
           if (i < kb) A[(K + i) * lda + K + j] = c[i][j];
     }
     if (R0 < n) {
-      if constexpr (sizeof(T) == 8)
-        rank_update_f64(A, lda, V, ldv, n, K, kb, R0, nv);
-      else
-        rank_update_simt<T>(A, lda, V, ldv, n, K, kb, R0, nv);
+      rank_update_simt<T>(A, lda, V, ldv, n, K, kb, R0, nv);
     }
     __syncthreads();
   }

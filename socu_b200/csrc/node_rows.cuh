@@ -168,6 +168,31 @@ __device__ __forceinline__ void rows_factor_tile(double d0, double d1, T* S, dou
   if (!redo) chol8_keep(S, c);
 }
 
+// The warps that work on one node, output block or vector: a whole thread
+// block, or some warps of one (ragged batches), with their barriers.
+struct BlockGroup {
+  __device__ __forceinline__ int tid() const { return threadIdx.x; }
+  __device__ __forceinline__ int threads() const { return blockDim.x; }
+  __device__ __forceinline__ int warp() const { return threadIdx.x >> 5; }
+  __device__ __forceinline__ int warps() const { return blockDim.x >> 5; }
+  __device__ __forceinline__ int bar(int k) const { return k; }
+  __device__ __forceinline__ void sync() const { __syncthreads(); }
+};
+struct WarpGroup {
+  int first, n, bar0;   // first warp, warps, barriers bar0 .. bar0 + 2
+  __device__ __forceinline__ int tid() const { return threadIdx.x - 32 * first; }
+  __device__ __forceinline__ int threads() const { return 32 * n; }
+  __device__ __forceinline__ int warp() const { return (threadIdx.x >> 5) - first; }
+  __device__ __forceinline__ int warps() const { return n; }
+  __device__ __forceinline__ int bar(int k) const { return bar0 + k; }
+  __device__ __forceinline__ void sync() const {
+    if (n == 1)
+      __syncwarp();
+    else
+      bar_wait(bar0, 32 * n);
+  }
+};
+
 // two consecutive elements, widened; `vec`: the pair is aligned and inside
 template <typename T>
 __device__ __forceinline__ void load_pair(const T* p, bool vec, bool v0, bool v1, double& x0, double& x1) {
@@ -199,6 +224,12 @@ __device__ __forceinline__ void store_pair(T* p, bool vec, bool v0, bool v1, dou
   }
 }
 
+// Whole 8x8 tiles, and every row of a block on a pair boundary.
+template <typename T>
+__host__ __device__ __forceinline__ bool pairs_ok(const Problem<T>& p, int n) {
+  return (n & 7) == 0 && ((reinterpret_cast<uintptr_t>(p.L) | reinterpret_cast<uintptr_t>(p.E)) & (2 * sizeof(T) - 1)) == 0;
+}
+
 // A row tile outside L_i: element (r, c) of X, r < lim, at base[r * rs + c * cs].
 // kind 0: a row-major block (cs = 1, rs = n); 1: a transposed block (rs = 1);
 // 2: rows of the identity (W^T), 3: zeros of the upper triangle of L_i.
@@ -209,6 +240,7 @@ struct RowSrc {
   int ld;       // kind 0: rs; kind 1: cs
   int lim;      // valid rows in the tile
   int k0;       // first step
+  bool full;    // whole tiles: no bounds to check (n == 8 nta; not the right-hand sides)
 };
 
 // X tile row: P = X_k Inv_k^T
@@ -227,7 +259,7 @@ __device__ __forceinline__ void rows_load(double (&acc)[NT][2], const RowSrc<T>&
 #pragma unroll
     for (int j = 0; j < NT; ++j) {
       const int c = 8 * j + 2 * t;
-      load_pair(s.base + (long long)g * s.ld + c, vec && 8 * j < n, rv && c < n, rv && c + 1 < n, acc[j][0], acc[j][1]);
+      load_pair(s.base + (g * s.ld + c), vec && 8 * j < n, rv && c < n, rv && c + 1 < n, acc[j][0], acc[j][1]);
     }
   } else if (s.kind == 1) {
 #pragma unroll
@@ -235,7 +267,8 @@ __device__ __forceinline__ void rows_load(double (&acc)[NT][2], const RowSrc<T>&
 #pragma unroll
       for (int e = 0; e < 2; ++e) {
         const int c = 8 * j + 2 * t + e;
-        acc[j][e] = (rv && c < n) ? (double)s.base[(long long)c * s.ld + g] : 0.0;
+        const bool in = s.full ? 8 * j < n : rv && c < n;
+        acc[j][e] = in ? (double)s.base[c * s.ld + g] : 0.0;
       }
   } else {
 #pragma unroll
@@ -255,7 +288,7 @@ __device__ __forceinline__ void rows_store(const double (&acc)[NT][2], const Row
 #pragma unroll
       for (int e = 0; e < 2; ++e) {
         const int c = 8 * j + 2 * t + e;
-        if (rv && c < n) s.base[(long long)c * s.ld + g] = (T)acc[j][e];
+        if (s.full ? 8 * j < n : rv && c < n) s.base[c * s.ld + g] = (T)acc[j][e];
       }
   } else {
     // (rows of the identity: tiles right of the diagonal one, which is written with C_kk)
@@ -264,7 +297,7 @@ __device__ __forceinline__ void rows_store(const double (&acc)[NT][2], const Row
     for (int j = 0; j < NT; ++j) {
       const int c = 8 * j + 2 * t;
       if (j >= j0)
-        store_pair(s.base + (long long)g * s.ld + c, vec && 8 * j < n, rv && c < n, rv && c + 1 < n, acc[j][0], acc[j][1]);
+        store_pair(s.base + (g * s.ld + c), vec && 8 * j < n, rv && c < n, rv && c + 1 < n, acc[j][0], acc[j][1]);
     }
   }
 }
@@ -286,14 +319,14 @@ __device__ __forceinline__ void rows_update(double (&acc)[NT][2], int j0, double
 }
 
 // All steps of one row tile against the finished factor (FROM0: k0 is 0, and no
-// branch separates the steps; the tile that the next step starts from comes first).
-template <int NT, bool FROM0>
+// branch separates the steps; the tile that the next step starts from comes first).  EXACT: nta is NT.
+template <int NT, bool FROM0, bool EXACT>
 __device__ __forceinline__ void rows_solve(double (&acc)[NT][2], int k0, int nta, const double* Cs, const double* Iv) {
   constexpr int ld = (NT & 1) ? 8 * NT : 8 * NT + 8;
   const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
 #pragma unroll
   for (int k = 0; k < NT; ++k) {
-    if ((FROM0 || k >= k0) && (NT <= 8 || k < nta)) {   // (NT is exact up to 8)
+    if ((FROM0 || k >= k0) && (EXACT || k < nta)) {
       const double2 iv = *reinterpret_cast<const double2*>(Iv + 64 * k + 2 * lane);
       const double* Ck = Cs + g * ld + 8 * k + 2 * t;
       double p0, p1;
@@ -308,14 +341,15 @@ __device__ __forceinline__ void rows_solve(double (&acc)[NT][2], int k0, int nta
 }
 
 // One node.  q, splits: this block's share of the row tiles outside L_i (every
-// block of a cluster runs phase 1).  Warp w < n / 8 owns row tile w of L_i.
-template <typename T, int NT>
-__device__ __forceinline__ void node_rows_body(const Problem<T>& p, const Level& lv, int b, int t,
+// block of a cluster runs phase 1).  Warp w < n / 8 of the group owns row tile w of L_i.
+// FULL: n is 8 NT and pairs are aligned, so sizes and offsets are constants.
+template <typename T, int NT, bool FULL, bool EXACT, class Group>
+__device__ __forceinline__ void node_rows_body(const Group& grp, const Problem<T>& p, const Level& lv, int b, int t,
                                                unsigned char* smem_raw, int q, int splits, bool with_y, bool inv) {
   constexpr int ld = (NT & 1) ? 8 * NT : 8 * NT + 8;
-  const int lane = threadIdx.x & 31, row = threadIdx.x >> 5, W = blockDim.x >> 5;
+  const int lane = threadIdx.x & 31, row = grp.warp(), W = grp.warps();
   const int g = lane >> 2, tq = lane & 3;
-  const int n = p.n, s = lv.s, i = s - 1 + 2 * s * t;
+  const int n = FULL ? 8 * NT : p.n, s = lv.s, i = s - 1 + 2 * s * t;
   const int nta = (n + 7) >> 3;
   const bool right = i + s < p.N, left = t >= 1;
   double* Cs = reinterpret_cast<double*>(smem_raw);   // rows of C, 8 NT x ld
@@ -326,14 +360,14 @@ __device__ __forceinline__ void node_rows_body(const Problem<T>& p, const Level&
   T* Lf = left ? p.Eb(b, lv.oc + 2 * t - 1) : nullptr;
   T* yi = with_y ? p.Xb(b, i) : nullptr;
   // paired accesses: whole tiles, and every row of a block on a pair boundary
-  const bool vec = n == 8 * nta && ((reinterpret_cast<uintptr_t>(p.L) | reinterpret_cast<uintptr_t>(p.E)) &
-                                    (2 * sizeof(T) - 1)) == 0;
+  const bool vec = FULL || pairs_ok(p, n);
   const int vr = right ? nta : 0, vl = left ? nta : 0, vy = with_y ? (p.m + 7) >> 3 : 0;
   const int vtot = vr + vl + vy + nta;
   auto source = [&](int v) {
     RowSrc<T> o;
     o.ld = n;
     o.k0 = 0;
+    o.full = vec;
     if (v < vr) {
       o.kind = 0;
       o.base = R + (long long)8 * v * n;
@@ -347,6 +381,7 @@ __device__ __forceinline__ void node_rows_body(const Problem<T>& p, const Level&
       const int c = v - vr - vl;
       o.kind = 1;
       o.base = yi + 8 * c;
+      o.full = false;
       o.ld = p.m;
       o.lim = p.m - 8 * c;
     } else {
@@ -387,19 +422,19 @@ __device__ __forceinline__ void node_rows_body(const Problem<T>& p, const Level&
     for (int k = 0; k < NT - 1; ++k) {
       if (k < row) {
         const int after = nta - 1 - k;   // rows after k
-        bar_wait(1, 32 * (after + 1));
+        bar_wait(grp.bar(1), 32 * (after + 1));
         const double2 iv = *reinterpret_cast<const double2*>(Iv + 64 * k + 2 * lane);
         double p0, p1;
         rows_panel(p0, p1, acc[k][0], acc[k][1], iv);
         *reinterpret_cast<double2*>(Cs + gr * ld + 8 * k + 2 * tq) = make_double2(p0, p1);
         if (row == k + 1) {
-          if (after > 1) bar_arrive(2, 32 * after);
+          if (after > 1) bar_arrive(grp.bar(2), 32 * after);
           d0 = acc[k + 1][0];
           d1 = acc[k + 1][1];
           mma_acc(d0, d1, -p0, p0);
           mma_acc(d0, d1, -p1, p1);
         } else {
-          bar_wait(2, 32 * after);
+          bar_wait(grp.bar(2), 32 * after);
 #pragma unroll
           for (int j = k + 1; j < NT; j += 4)
             if (j <= row) rows_update<NT, 4>(acc, j, p0, p1, Cs + g * ld + 8 * k + 2 * tq, ld);
@@ -407,7 +442,7 @@ __device__ __forceinline__ void node_rows_body(const Problem<T>& p, const Level&
       }
     }
     rows_factor_tile<T>(d0, d1, Ct + 64 * row, Iv + 64 * row, [&] {
-      if (row + 1 < nta) bar_arrive(1, 32 * (nta - row));
+      if (row + 1 < nta) bar_arrive(grp.bar(1), 32 * (nta - row));
     });
     if (splits > 1) cluster_wait();   // every block of the cluster has read L_i
     if (q == 0) {
@@ -436,7 +471,7 @@ __device__ __forceinline__ void node_rows_body(const Problem<T>& p, const Level&
   // (the first row tile arrives while later rows finish phase 1)
   double av[NT][2];
   if (v_first < vtot) rows_load<T, NT>(av, source(v_first), n, vec);
-  __syncthreads();   // the factor is complete in shared memory
+  grp.sync();   // the factor is complete in shared memory
 
   // phase 2
   for (int v = v_first; v < vtot; v += splits * W) {
@@ -450,14 +485,14 @@ __device__ __forceinline__ void node_rows_body(const Problem<T>& p, const Level&
     }
     if (v != v_first) rows_load<T, NT>(av, src, n, vec);
     if (src.kind == 2)
-      rows_solve<NT, false>(av, src.k0, nta, Cs, Iv);
+      rows_solve<NT, false, EXACT>(av, src.k0, nta, Cs, Iv);
     else
-      rows_solve<NT, true>(av, 0, nta, Cs, Iv);
+      rows_solve<NT, true, EXACT>(av, 0, nta, Cs, Iv);
     rows_store<T, NT>(av, src, n, vec);
   }
 }
 
-template <typename T, int NT>
+template <typename T, int NT, bool FULL>
 __global__ void __launch_bounds__(32 * (NT < 4 ? 4 : NT), NT <= 4 ? 4 : (NT <= 8 ? 2 : 1))
     k_node_rows(Problem<T> p, Level lv, int splits, int with_y, int inv) {
   const int node = blockIdx.x / splits, q = blockIdx.x - node * splits;
@@ -466,37 +501,37 @@ __global__ void __launch_bounds__(32 * (NT < 4 ? 4 : NT), NT <= 4 ? 4 : (NT <= 8
   pdl_trigger();
   if (!p.active(b)) return;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  node_rows_body<T, NT>(p, lv, b, t, smem_raw, q, splits, with_y != 0, inv != 0);
+  node_rows_body<T, NT, FULL, FULL || NT <= 8>(BlockGroup{}, p, lv, b, t, smem_raw, q, splits, with_y != 0, inv != 0);
 }
 
 template <typename T>
 using NodeRowsFn = void (*)(Problem<T>, Level, int, int, int);
 
-// the kernel for block size n (node_rows_f32.cu, node_rows_f64.cu: one
+// the kernel for block size n; full: n is a whole tile count and pairs_ok (node_rows_f32.cu, node_rows_f64.cu: one
 // translation unit per type, so the instantiations compile in parallel)
 template <typename T>
-NodeRowsFn<T> node_rows_kernel(int n);
+NodeRowsFn<T> node_rows_kernel(int n, bool full);
 
 #define SOCU_NODE_ROWS_KERNELS(T)                      \
   template <>                                          \
-  NodeRowsFn<T> node_rows_kernel<T>(int n) {           \
+  NodeRowsFn<T> node_rows_kernel<T>(int n, bool full) { \
     switch (rows_nt(n)) {                              \
-      case 1: return k_node_rows<T, 1>;                \
-      case 2: return k_node_rows<T, 2>;                \
-      case 3: return k_node_rows<T, 3>;                \
-      case 4: return k_node_rows<T, 4>;                \
-      case 5: return k_node_rows<T, 5>;                \
-      case 6: return k_node_rows<T, 6>;                \
-      case 7: return k_node_rows<T, 7>;                \
-      case 8: return k_node_rows<T, 8>;                \
-      case 10: return k_node_rows<T, 10>;              \
-      case 12: return k_node_rows<T, 12>;              \
-      case 14: return k_node_rows<T, 14>;              \
-      default: return k_node_rows<T, 16>;              \
+      case 1: return full ? k_node_rows<T, 1, true> : k_node_rows<T, 1, false>; \
+      case 2: return full ? k_node_rows<T, 2, true> : k_node_rows<T, 2, false>; \
+      case 3: return full ? k_node_rows<T, 3, true> : k_node_rows<T, 3, false>; \
+      case 4: return full ? k_node_rows<T, 4, true> : k_node_rows<T, 4, false>; \
+      case 5: return full ? k_node_rows<T, 5, true> : k_node_rows<T, 5, false>; \
+      case 6: return full ? k_node_rows<T, 6, true> : k_node_rows<T, 6, false>; \
+      case 7: return full ? k_node_rows<T, 7, true> : k_node_rows<T, 7, false>; \
+      case 8: return full ? k_node_rows<T, 8, true> : k_node_rows<T, 8, false>; \
+      case 10: return full ? k_node_rows<T, 10, true> : k_node_rows<T, 10, false>; \
+      case 12: return full ? k_node_rows<T, 12, true> : k_node_rows<T, 12, false>; \
+      case 14: return full ? k_node_rows<T, 14, true> : k_node_rows<T, 14, false>; \
+      default: return full ? k_node_rows<T, 16, true> : k_node_rows<T, 16, false>; \
     }                                                  \
   }
 
-template <> NodeRowsFn<float> node_rows_kernel<float>(int n);
-template <> NodeRowsFn<double> node_rows_kernel<double>(int n);
+template <> NodeRowsFn<float> node_rows_kernel<float>(int n, bool full);
+template <> NodeRowsFn<double> node_rows_kernel<double>(int n, bool full);
 
 }  // namespace socu

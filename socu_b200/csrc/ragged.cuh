@@ -16,25 +16,34 @@
 //     eta); every further round is FWD 0..K-1, BWD K-1..0, XUPD, RES, until
 //     eta <= tol, max_iter rounds, or a non-finite eta.
 //
-// NODE/UPD/FWD/BWD/RES run the same device bodies as the per-level kernels of
-// the uniform batch (nd_kernels.cuh, refine.cuh), so each output block has one
-// writer and the results do not depend on the task order.  UPD of the plain
+// NODE/UPD/FWD/BWD/INIT/RES run the same device bodies as the per-level kernels
+// of the uniform batch, or their one-warp forms (warp_rows.cuh, sweep_rows.cuh,
+// refine.cuh), so each output block has one writer and the results do not
+// depend on the task order.
+//
+// Workers.  In a large batch every warp is a worker of its own (twelve per SM):
+// with thousands of units ready, units in flight count and not the time of one.
+// In a small batch the levels of its largest systems, one after another, are
+// the time: there a thread block of eight warps is the worker, and a unit gets a
+// warp per 8-row tile (smaller blocks run side by side, rg_group_warps).  The
+// host chooses by the nodes per warp worker (rg_use_blocks).  UPD of the plain
 // path also applies the fused forward pull of the next level (the uniform
 // factor_and_solve launches it separately).
 //
-// Queue protocol (thread 0 of a CTA acts for the CTA):
+// Queue protocol (lane 0 of a worker acts for it):
 //   pop:      k = atomicAdd(head, 1); wait until slot[k] holds a task, or all
 //             instances are done (then exit); a wait that sees no queue
 //             progress for timeout_ns (%globaltimer) records an error and exits.
 //   complete: fence; if atomicSub(rem[inst], 1) == 1 the phase is over: fence,
 //             set rem for the next phase, push its chunks 1..c-1 and keep
-//             chunk 0 for this CTA (an instance's critical path never waits
+//             chunk 0 for this worker (an instance's critical path never waits
 //             in the queue).  The last phase increments `done`.
 // Tasks never wait on one another, only on the queue, so the protocol cannot
-// deadlock whether or not every CTA is resident.
+// deadlock whether or not every worker is resident.
 #pragma once
 
 #include "refine.cuh"
+#include "warp_rows.cuh"
 
 namespace socu {
 
@@ -82,8 +91,6 @@ __host__ __device__ inline Level rg_level(int N, int l) {
   lv.oc = curr;
   lv.on = nxt;
   lv.op = prev;
-  lv.tc = 0;       // persistent CTAs: SIMT sweep products (lower latency per node)
-  lv.pre = 0;      // no programmatic launches in the persistent kernel
   return lv;
 }
 
@@ -132,7 +139,7 @@ __host__ __device__ inline RgPhase rg_phase(const RgInst& I, int mode, int ph) {
   if (q < K) {
     r.kind = kRgFwd;
     r.level = q;
-    r.units = fwd_tasks(I.N, rg_level(I.N, q));
+    r.units = sweep_tasks<kModeForward>(I.N, rg_level(I.N, q));
   } else if (q < 2 * K) {
     r.kind = kRgBwd;
     r.level = 2 * K - 1 - q;
@@ -182,8 +189,8 @@ struct RgArgs {
   double tol;
   int max_iter;
   RgQueue q;
-  int vc;                     // unused (node vectors per pass of the blocked-solve body)
   long long timeout_ns;       // bound of one queue wait
+  int worker_bytes;           // shared memory of one warp worker
 };
 
 __device__ __forceinline__ unsigned long long rg_clock() {
@@ -204,7 +211,7 @@ __device__ __forceinline__ unsigned int rg_load_u32(const unsigned int* p) {
   return v;
 }
 
-// Thread 0: next task for this CTA, or kRgExit.
+// Lane 0: next task for this worker, or kRgExit.
 template <typename T>
 __device__ unsigned long long rg_pop(const RgArgs<T>& a) {
   const unsigned int k = atomicAdd(a.q.head, 1u);
@@ -286,8 +293,82 @@ __device__ __forceinline__ RefineArgs rg_refine_args(const RgArgs<T>& a, const R
   return r;
 }
 
-// Execute one chunk (all threads of the CTA).
-template <typename T, int MODE>
+// Tile counts the bodies are built for.
+__host__ __device__ inline int rg_nt(int n) { return n <= 8 ? 1 : (n <= 16 ? 2 : (n <= 32 ? 4 : (n <= 48 ? 6 : 8))); }
+// Block workers: warps per unit, one per 8-row tile, as a power of two.
+__host__ __device__ inline int rg_group_warps(int n) { return n <= 8 ? 1 : (n <= 16 ? 2 : (n <= 32 ? 4 : 8)); }
+// Shared memory of one unit (bytes) for blocks of size n.
+__host__ __device__ inline long long rg_unit_bytes(int n, int es, bool refine, bool blocks) {
+  const int nt = rg_nt(n);
+  long long v = blocks ? smem_rows_bytes(8 * nt) : smem_warp_node_bytes(nt);
+  const long long w = smem_sweep_rows_bytes(8 * nt, true), u = blocks ? smem_update_rows_bytes(8 * nt, es) : 0;
+  if (w > v) v = w;
+  if (u > v) v = u;
+  if (refine) {
+    const long long r = 8 * smem_residual_rows_elems(n), i = 8 * smem_ref_init_elems(n, blocks ? rg_group_warps(n) : 1);
+    if (r > v) v = r;
+    if (i > v) v = i;
+  }
+  return (v + 127) & ~127LL;
+}
+// Shared memory of a thread block: four warp workers, or one block worker's units.
+constexpr int kRgWorkers = 4, kRgBlockWarps = 8;
+__host__ __device__ inline long long rg_block_bytes(int n, int es, bool refine, bool blocks) {
+  const long long v = rg_unit_bytes(n, es, refine, blocks);
+  return v * (blocks ? kRgBlockWarps / rg_group_warps(n) : kRgWorkers);
+}
+// Block workers for batches with few nodes per warp worker (12 of those per SM).  Measured in
+// FP64 on N ~ U{8..256}, n in {8, 16, 32, 48}, m in {1, 4} (132 nodes a system), warp against
+// block workers: 16 systems 1.28 / 0.56 ms, 64 1.51 / 0.97, 128 2.07 / 1.82, 256 3.40 / 3.57,
+// 512 5.39 / 6.54, 1024 8.9 / 11.8 ms; the line lies at 175 such systems.
+__host__ __device__ inline bool rg_use_blocks(long long nodes, int sms) { return nodes < 13LL * 12 * sms; }
+
+// One unit of a level phase (one copy of each per tile count: the kernel calls them).
+template <typename T, int NT, bool FULL, bool BLOCKS>
+__device__ __noinline__ void rg_node_unit(const Problem<T>& p, const Level& lv, int u, unsigned char* smem,
+                                          WarpGroup grp) {
+  if constexpr (BLOCKS)
+    node_rows_body<T, NT, FULL, FULL>(grp, p, lv, 0, u, smem, 0, 1, true, true);
+  else
+    node_warp_body<T, NT, FULL>(p, lv, 0, u, smem);
+}
+template <typename T, int NT, bool FULL, bool BLOCKS>
+__device__ __noinline__ void rg_update_unit(const Problem<T>& p, const Level& lv, int task, unsigned char* smem,
+                                            WarpGroup grp) {
+  if constexpr (BLOCKS)
+    update_rows_body<T, NT, FULL, false>(grp, p, lv, 0, task, smem, 0, 1);
+  else
+    update_warp_body<T, NT, FULL>(p, lv, 0, task);
+}
+template <typename T, int NT, bool FULL, bool BLOCKS, int MODE>
+__device__ __noinline__ void rg_sweep_unit(const Problem<T>& p, const Level& lv, int u, unsigned char* smem,
+                                           WarpGroup grp) {
+  sweep_rows_body<T, NT, FULL, MODE, true, BLOCKS>(grp, p, lv, 0, u, smem, kWaitNone);
+}
+
+template <typename T, int MODE, int NT, bool FULL, bool BLOCKS>
+__device__ __forceinline__ void rg_level_unit(const Problem<T>& p, int kind, int level, const Level& lv, int u,
+                                              unsigned char* smem, const WarpGroup& grp) {
+  if (kind == kRgNode) {
+    rg_node_unit<T, NT, FULL, BLOCKS>(p, lv, u, smem, grp);
+  } else if (kind == kRgUpd) {
+    rg_update_unit<T, NT, FULL, BLOCKS>(p, lv, u, smem, grp);
+    if (u + 1 <= lv.d - 1) {   // fill-in block of node t = u + 1
+      grp.sync();
+      rg_update_unit<T, NT, FULL, BLOCKS>(p, lv, p.N / (2 * lv.s) + u, smem, grp);
+    }
+    // y_j -= F y_{j-s} + G^T y_{j+s} for target j = 2s(u+1) - 1
+    grp.sync();
+    rg_sweep_unit<T, NT, FULL, BLOCKS, kModePull>(p, rg_level(p.N, level + 1), u, smem, grp);
+  } else if (kind == kRgBwd) {
+    rg_sweep_unit<T, NT, FULL, BLOCKS, kModeBackward>(p, lv, u, smem, grp);
+  } else {
+    if constexpr (MODE != kRgPlain) rg_sweep_unit<T, NT, FULL, BLOCKS, kModeForward>(p, lv, u, smem, grp);
+  }
+}
+
+// Execute one chunk (all threads of the worker).
+template <typename T, int MODE, bool BLOCKS>
 __device__ void rg_run(const RgArgs<T>& a, int ii, int ph, int chunk, unsigned char* smem) {
   const RgInst I = a.inst[ii];
   const RgPhase P = rg_phase(I, MODE, ph);
@@ -301,60 +382,48 @@ __device__ void rg_run(const RgArgs<T>& a, int ii, int ph, int chunk, unsigned c
       const float* d = reinterpret_cast<const float*>(a.X) + I.oX + u0 * per;
       double* x = a.x64 + I.oX + u0 * per;
       const long long len = (long long)(u1 - u0) * per;
-      for (long long e = threadIdx.x; e < len; e += blockDim.x) x[e] += (double)d[e];
+      for (long long e = BLOCKS ? threadIdx.x : threadIdx.x & 31; e < len; e += BLOCKS ? blockDim.x : 32) x[e] += (double)d[e];
     }
     return;
   }
-  for (int u = u0; u < u1; ++u) {
-    if (u > u0) __syncthreads();
-    switch (P.kind) {
-      case kRgNode: {
-        const Problem<T> p = rg_problem(a, I, I.m);
-        node_gemm_body<T, true, true>(p, lv, 0, u, smem);
-        break;
-      }
-      case kRgUpd: {
-        const Problem<T> p = rg_problem(a, I, I.m);
-        const int U = I.N / (2 * lv.s);
-        update_full_body<T>(p, lv, 0, u, smem);
-        if (u + 1 <= lv.d - 1) {   // fill-in block of node t = u + 1
-          __syncthreads();
-          update_full_body<T>(p, lv, 0, U + u, smem);
-        }
-        // y_j -= F y_{j-s} + G^T y_{j+s} for target j = 2s(u+1) - 1
-        __syncthreads();
-        fwd_body<T, true, true, false>(p, rg_level(I.N, P.level + 1), 0, u, smem);
-        break;
-      }
-      case kRgBwd: {
-        const Problem<T> p = rg_problem(a, I, I.m);
-        bwd_body<T, true, true>(p, lv, 0, u, smem);
-        break;
-      }
-      case kRgFwd: {
-        if constexpr (!kPlain) {
-          const Problem<T> p = rg_problem(a, I, I.m);
-          fwd_body<T, true, false, true>(p, lv, 0, u, smem);
-        }
-        break;
-      }
-      case kRgInit: {
-        if constexpr (!kPlain) ref_init_rows_body(rg_refine_args(a, I, ii), 0, u, smem);
-        break;
-      }
-      case kRgRes: {
-        if constexpr (!kPlain) {
-          residual_rows_body<true, 1>(rg_refine_args(a, I, ii), 0, u, smem);
-        }
-        break;
-      }
-      default:
-        break;
+  // units side by side: one, or as many as the block's warps hold
+  const int gw = BLOCKS ? rg_group_warps(I.n) : 1, gi = BLOCKS ? (int)(threadIdx.x >> 5) / gw : 0;
+  const WarpGroup grp{BLOCKS ? gi * gw : (int)(threadIdx.x >> 5), gw, 1 + 3 * gi};
+  if (BLOCKS) smem += gi * rg_unit_bytes(I.n, (int)sizeof(T), !kPlain, true);
+  const Problem<T> p = rg_problem(a, I, I.m);
+  for (int u = u0 + gi; u < u1; u += BLOCKS ? kRgBlockWarps / gw : 1) {
+    grp.sync();
+    if (!kPlain && P.kind == kRgInit) {
+      if constexpr (!kPlain) ref_init_rows_body(grp, rg_refine_args(a, I, ii), 0, u, smem);
+      continue;
     }
+    if (!kPlain && P.kind == kRgRes) {
+      if constexpr (!kPlain) residual_rows_body<true, 1>(grp, rg_refine_args(a, I, ii), 0, u, smem);
+      continue;
+    }
+    const int nt = rg_nt(I.n);
+    const bool full = I.n == 8 * nt && pairs_ok(p, I.n);
+#define SOCU_RG_UNIT(NT)                                                                    \
+  if (full)                                                                                 \
+    rg_level_unit<T, MODE, NT, true, BLOCKS>(p, P.kind, P.level, lv, u, smem, grp);         \
+  else                                                                                      \
+    rg_level_unit<T, MODE, NT, false, BLOCKS>(p, P.kind, P.level, lv, u, smem, grp);
+    if (nt == 1) {
+      SOCU_RG_UNIT(1)
+    } else if (nt == 2) {
+      SOCU_RG_UNIT(2)
+    } else if (nt == 4) {
+      SOCU_RG_UNIT(4)
+    } else if (nt == 6) {
+      SOCU_RG_UNIT(6)
+    } else {
+      SOCU_RG_UNIT(8)
+    }
+#undef SOCU_RG_UNIT
   }
 }
 
-// Thread 0, after the CTA finished chunk `chunk` of phase `ph` of instance ii:
+// Lane 0, after the worker finished a chunk of phase `ph` of instance ii:
 // the continuation task (chunk 0 of the next phase) or 0.
 template <typename T, int MODE>
 __device__ unsigned long long rg_complete(const RgArgs<T>& a, int ii, int ph) {
@@ -440,40 +509,51 @@ __global__ void k_rg_start(RgArgs<T> a) {
   }
 }
 
-// The persistent solver: every CTA loops pop -> run -> complete.  128
-// threads, 3 CTAs per SM at n = 48 (shared-memory bound); registers capped at
-// 168 for FP64 (no spills: measured 66.9k -> 75.7k solves/s on the 4096-system
-// batch) and at 128 for float (the float path measured faster there).
-constexpr int kRgThreads = 128;
-template <typename T, int MODE>
-__global__ void __launch_bounds__(kRgThreads, sizeof(T) == 8 ? 3 : 4) k_ragged(RgArgs<T> a) {
+// The persistent solver: every worker loops pop -> run -> complete.  Warp
+// workers: three blocks of four per SM (168 registers, and the shared memory of
+// blocks up to n = 48); block workers: two per SM.
+__host__ __device__ constexpr int rg_threads(bool blocks) { return 32 * (blocks ? kRgBlockWarps : kRgWorkers); }
+template <typename T, int MODE, bool BLOCKS>
+__global__ void __launch_bounds__(rg_threads(BLOCKS), BLOCKS ? 2 : 3) k_ragged(const __grid_constant__ RgArgs<T> a) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ unsigned long long s_task;
+  unsigned char* smem = BLOCKS ? smem_raw : smem_raw + (threadIdx.x >> 5) * a.worker_bytes;
+  const bool lead = BLOCKS ? threadIdx.x == 0 : (threadIdx.x & 31) == 0;
+  auto share = [&](unsigned long long v) {   // the lead's value in every thread of the worker
+    if (!BLOCKS) return __shfl_sync(kFull, v, 0);
+    if (lead) s_task = v;
+    __syncthreads();
+    v = s_task;
+    __syncthreads();
+    return v;
+  };
   unsigned long long task = 0ull;
   while (true) {
     if (task == 0ull) {
-      if (threadIdx.x == 0) s_task = rg_pop(a);
-      __syncthreads();
-      task = s_task;
-      __syncthreads();
+      if (lead) task = rg_pop(a);
+      task = share(task);
       if (task == kRgExit) return;
     }
     int ii, ph, chunk;
     rg_decode(task, ii, ph, chunk);
-    rg_run<T, MODE>(a, ii, ph, chunk, smem_raw);
-    __syncthreads();
-    if (threadIdx.x == 0) s_task = rg_complete<T, MODE>(a, ii, ph);
-    __syncthreads();
-    task = s_task;
-    __syncthreads();
+    rg_run<T, MODE, BLOCKS>(a, ii, ph, chunk, smem);
+    if (BLOCKS)
+      __syncthreads();
+    else
+      __syncwarp();
+    if (lead) task = rg_complete<T, MODE>(a, ii, ph);
+    task = share(task);
   }
 }
 
-// the kernel (ragged_f64.cu, ragged_f32.cu, ragged_mixed.cu: one translation unit each)
-template <typename T, int MODE>
+// the kernels (ragged_*.cu: one translation unit each)
+template <typename T, int MODE, bool BLOCKS>
 void (*ragged_kernel())(RgArgs<T>);
-template <> void (*ragged_kernel<double, kRgPlain>())(RgArgs<double>);
-template <> void (*ragged_kernel<float, kRgPlain>())(RgArgs<float>);
-template <> void (*ragged_kernel<float, kRgRefine>())(RgArgs<float>);
+template <> void (*ragged_kernel<double, kRgPlain, false>())(RgArgs<double>);
+template <> void (*ragged_kernel<double, kRgPlain, true>())(RgArgs<double>);
+template <> void (*ragged_kernel<float, kRgPlain, false>())(RgArgs<float>);
+template <> void (*ragged_kernel<float, kRgPlain, true>())(RgArgs<float>);
+template <> void (*ragged_kernel<float, kRgRefine, false>())(RgArgs<float>);
+template <> void (*ragged_kernel<float, kRgRefine, true>())(RgArgs<float>);
 
 }  // namespace socu

@@ -10,7 +10,8 @@
 // `active` flags, which the solver kernels take as their batch mask.
 #pragma once
 
-#include "nd_kernels.cuh"
+#include "sweep_rows.cuh"
+#include "update_rows.cuh"
 
 namespace socu {
 
@@ -60,6 +61,24 @@ __device__ __forceinline__ double block_max(double v, double* red) {
     for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(kFull, v, o));
   }
   return v;  // valid in thread 0
+}
+
+// Maximum over a group's threads, valid in its first thread; red: one word per
+// warp of the block.
+template <class Group>
+__device__ __forceinline__ double group_max(const Group& grp, double v, double* red) {
+  for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(kFull, v, o));
+  if (grp.warps() == 1) return v;
+  const int lane = threadIdx.x & 31;
+  double* mine = red + (threadIdx.x >> 5) - grp.warp();
+  grp.sync();
+  if (lane == 0) mine[grp.warp()] = v;
+  grp.sync();
+  if (grp.warp() == 0) {
+    v = lane < grp.warps() ? mine[lane] : 0.0;
+    for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(kFull, v, o));
+  }
+  return v;
 }
 
 // Per-instance state reset (before k_ref_init accumulates into it).
@@ -317,8 +336,8 @@ __host__ __device__ inline long long smem_residual_x_elems(int n, int gr) { retu
 // shared memory the ragged kernel reserves for its residual / set-up phases
 // (doubles): the one-group residual's x staging, which exceeds the set-up's 17 n
 __host__ __device__ inline long long smem_residual_rows_elems(int n) { return smem_residual_x_elems(n, 1); }
-template <bool REFINE, int GR>
-__device__ __forceinline__ void residual_rows_body(const RefineArgs& a, int bi, int i, unsigned char* smem_raw) {
+template <bool REFINE, int GR, class Group>
+__device__ __forceinline__ void residual_rows_body(const Group& grp, const RefineArgs& a, int bi, int i, unsigned char* smem_raw) {
   constexpr int kResXC = 8 * GR, kResXld = kResXC + 4;
   __shared__ double red[32];
   double* const xs0 = reinterpret_cast<double*>(smem_raw);
@@ -331,20 +350,20 @@ __device__ __forceinline__ void residual_rows_body(const RefineArgs& a, int bi, 
   const double* Ep = a.E + ((long long)bi * a.S + (hasP ? i : 0)) * nn;
   const long long vi = ((long long)bi * N + i) * n * m;
   const double* x1 = a.x + vi;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  const int lane = threadIdx.x & 31, warp = grp.warp(), nw = grp.warps();
   const int g = lane >> 2, t = lane & 3;
   const int rts = (n + 7) >> 3;
   double rmax = 0.0, xmax = 0.0;
   for (int c0 = 0; c0 < m; c0 += kResXC) {
     const int mc = min(kResXC, m - c0);
     const int groups = (mc + 7) >> 3;
-    __syncthreads();
-    for (int e = threadIdx.x; e < 3 * n * kResXC; e += blockDim.x) {
+    grp.sync();
+    for (int e = grp.tid(); e < 3 * n * kResXC; e += grp.threads()) {
       const int j = e / (n * kResXC), rem = e - j * n * kResXC, k = rem / kResXC, c = rem - k * kResXC;
       const bool ok = c < mc && (j == 1 || (j == 0 ? hasM : hasP));
       xs0[j * xstride + k * kResXld + c] = ok ? x1[(long long)(j - 1) * n * m + (long long)k * m + c0 + c] : 0.0;
     }
-    __syncthreads();
+    grp.sync();
     for (int rt = warp; rt < rts; rt += nw) {
       const int r0 = rt * 8, ra = r0 + g;
       const bool rv = ra < n;
@@ -423,9 +442,9 @@ __device__ __forceinline__ void residual_rows_body(const RefineArgs& a, int bi, 
     }
   }
   if (REFINE) {
-    const double rm = block_max(rmax, red);
-    const double xm = block_max(xmax, red);
-    if (threadIdx.x == 0) {
+    const double rm = group_max(grp, rmax, red);
+    const double xm = group_max(grp, xmax, red);
+    if (grp.tid() == 0) {
       atomic_max_pos(&a.st[bi].rnorm, rm);
       atomic_max_pos(&a.st[bi].xnorm, xm);
     }
@@ -446,7 +465,7 @@ __global__ void __launch_bounds__(256, GR == 4 ? 2 : 3) k_residual_rows(RefineAr
   const int i = blockIdx.x - bi * a.N;
   if (REFINE && !a.active[bi]) return;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  residual_rows_body<REFINE, GR>(a, bi, i, smem_raw);
+  residual_rows_body<REFINE, GR>(BlockGroup{}, a, bi, i, smem_raw);
   if (REFINE) residual_arrive(a, bi, (unsigned)a.N);
 }
 
@@ -459,21 +478,22 @@ __global__ void __launch_bounds__(256, GR == 4 ? 2 : 3) k_residual_rows(RefineAr
 // keeps per-lane column partials for the transposed parts (strict lower(D)
 // columns, E_i columns).  The warps' column partials are added in warp order
 // in shared memory (smem_ref_init_elems doubles), so the sums are deterministic.
-__host__ __device__ inline long long smem_ref_init_elems(int n) { return 2LL * 8 * n + n; }
-__device__ __forceinline__ void ref_init_rows_body(const RefineArgs& a, int bi, int i, unsigned char* smem_raw) {
+__host__ __device__ inline long long smem_ref_init_elems(int n, int warps = 8) { return 2LL * warps * n + n; }
+template <class Group>
+__device__ __forceinline__ void ref_init_rows_body(const Group& grp, const RefineArgs& a, int bi, int i, unsigned char* smem_raw) {
   __shared__ double red[32];
   const int n = a.n, m = a.m, N = a.N;
   const long long nn = (long long)n * n;
   if (i >= N) {   // storage tail: zero slots only
     if (i < a.S) {
       float* E32 = a.E32 + ((long long)bi * a.S + i) * nn;
-      for (long long e = threadIdx.x; e < nn; e += blockDim.x) E32[e] = 0.0f;
+      for (long long e = grp.tid(); e < nn; e += grp.threads()) E32[e] = 0.0f;
     }
     return;
   }
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  const int lane = threadIdx.x & 31, warp = grp.warp(), nw = grp.warps();
   double* colp = reinterpret_cast<double*>(smem_raw);   // [warp][2][n] column partials
-  double* rs = colp + 2 * 8 * n;                         // [n] row parts
+  double* rs = colp + 2 * nw * n;                         // [n] row parts
   const bool hasM = i > 0, hasP = i < N - 1, hasS = i < a.S;
   const double* Lg = a.L + ((long long)bi * N + i) * nn;
   const double* Em = a.E + ((long long)bi * a.S + (hasM ? i - 1 : 0)) * nn;
@@ -482,7 +502,7 @@ __device__ __forceinline__ void ref_init_rows_body(const RefineArgs& a, int bi, 
   float* E32 = a.E32 + ((long long)bi * a.S + (hasS ? i : 0)) * nn;
   const long long vo = ((long long)bi * N + i) * n * m;
   double bmax = 0.0;
-  for (int e = threadIdx.x; e < n * m; e += blockDim.x) {
+  for (int e = grp.tid(); e < n * m; e += grp.threads()) {
     const double v = a.b[vo + e];
     a.R32[vo + e] = (float)v;
     a.x[vo + e] = 0.0;
@@ -526,16 +546,16 @@ __device__ __forceinline__ void ref_init_rows_body(const RefineArgs& a, int bi, 
       colp[(warp * 2 + 1) * n + c] = ce[h];
     }
   }
-  __syncthreads();
+  grp.sync();
   double rmax = 0.0;
-  for (int r = threadIdx.x; r < n; r += blockDim.x) {
+  for (int r = grp.tid(); r < n; r += grp.threads()) {
     double sum = rs[r];
     for (int w = 0; w < nw; ++w) sum += colp[(w * 2 + 0) * n + r] + colp[(w * 2 + 1) * n + r];
     rmax = fmax(rmax, sum);
   }
-  const double bm = block_max(bmax, red);
-  const double pm = block_max(rmax, red);
-  if (threadIdx.x == 0) {
+  const double bm = group_max(grp, bmax, red);
+  const double pm = group_max(grp, rmax, red);
+  if (grp.tid() == 0) {
     atomic_max_pos(&a.st[bi].bnorm, bm);
     atomic_max_pos(&a.st[bi].psi, pm);
   }
@@ -549,7 +569,7 @@ static __global__ void __launch_bounds__(256) k_ref_init_rows(RefineArgs a) {
   const int i = blockIdx.x - bi * per;
   if (a.mask != nullptr && a.mask[bi] == 0) return;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  ref_init_rows_body(a, bi, i, smem_raw);
+  ref_init_rows_body(BlockGroup{}, a, bi, i, smem_raw);
 }
 
 // ---------------------------------------------------------------------------

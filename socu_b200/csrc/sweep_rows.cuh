@@ -69,26 +69,27 @@ __device__ __forceinline__ void ldcg_pair(const T* p, bool vec, bool v0, bool v1
 }
 
 // MMA operand of an n x n block, row tile i, column tile kk: elements (r, c), (r, c + 1) with
-// r = 8i + g, c = 8kk + 2t; TR: of the block's transpose.  raw: as stored (widened later).
+// r = 8i + g, c = 8kk + 2t; TR: of the block's transpose.  vec: the tile is whole (and pairs are aligned).
 template <typename T, bool TR>
 __device__ __forceinline__ void block_frag(const T* M, int n, int i, int kk, bool vec, T& a0, T& a1) {
   const int lane = threadIdx.x & 31, r = 8 * i + (lane >> 2), c = 8 * kk + 2 * (lane & 3);
   if (TR) {
-    a0 = (r < n && c < n) ? M[(long long)c * n + r] : T(0);
-    a1 = (r < n && c + 1 < n) ? M[(long long)(c + 1) * n + r] : T(0);
+    const T* q = M + (c * n + r);   // (n <= 128: offsets inside a block fit 32 bits)
+    a0 = vec || (r < n && c < n) ? q[0] : T(0);
+    a1 = vec || (r < n && c + 1 < n) ? q[n] : T(0);
   } else if (vec) {
     if constexpr (sizeof(T) == 8) {
-      const double2 v = *reinterpret_cast<const double2*>(M + (long long)r * n + c);
+      const double2 v = *reinterpret_cast<const double2*>(M + (r * n + c));
       a0 = v.x;
       a1 = v.y;
     } else {
-      const float2 v = *reinterpret_cast<const float2*>(M + (long long)r * n + c);
+      const float2 v = *reinterpret_cast<const float2*>(M + (r * n + c));
       a0 = v.x;
       a1 = v.y;
     }
   } else {
-    a0 = (r < n && c < n) ? M[(long long)r * n + c] : T(0);
-    a1 = (r < n && c + 1 < n) ? M[(long long)r * n + c + 1] : T(0);
+    a0 = (r < n && c < n) ? M[r * n + c] : T(0);
+    a1 = (r < n && c + 1 < n) ? M[r * n + c + 1] : T(0);
   }
 }
 
@@ -118,17 +119,18 @@ __device__ __forceinline__ void solve_frag(const T* L, int n, int i, int kk, boo
   a1 = a[1];
 }
 
-// One vector.  ONE: the block has a warp per row tile (else the warps loop over them and the
+// One vector, its columns col0 .. col0 + cols (a multiple of 8).  ONE: the block has a warp per row tile (else the warps loop over them and the
 // blocks are read as they are used).
-template <typename T, int NT, int MODE, bool INV, bool ONE>
-__device__ __forceinline__ void sweep_rows_body(const Problem<T>& p, const Level& lv, int b, int task,
-                                                unsigned char* smem_raw, int wait) {
+template <typename T, int NT, bool FULL, int MODE, bool INV, bool ONE, class Group>
+__device__ __forceinline__ void sweep_rows_body(const Group& grp, const Problem<T>& p, const Level& lv, int b, int task,
+                                                unsigned char* smem_raw, int wait, int col0 = 0,
+                                                int cols = 1 << 30) {
   constexpr bool BWD = MODE == kModeBackward, KEEP = ONE && NT <= 8;
   constexpr int XC = sweep_cols(NT), CG = XC / 8, ldz = sweep_ldz(NT), NK = KEEP ? NT : 1;
   static_assert(INV || ONE, "the substitution needs a warp per row tile");
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, W = blockDim.x >> 5;
+  const int lane = threadIdx.x & 31, warp = grp.warp(), W = grp.warps();
   const int g = lane >> 2, t = lane & 3;
-  const int n = p.n, m = p.m, N = p.N, s = lv.s, nta = (n + 7) >> 3;
+  const int n = FULL ? 8 * NT : p.n, m = p.m, N = p.N, s = lv.s, nta = (n + 7) >> 3;
   // the vector, the row-major block P with its vector and the transposed block Q with its
   int j, jp = 0, jq = 0;
   bool solve = MODE != kModePull;
@@ -152,8 +154,7 @@ __device__ __forceinline__ void sweep_rows_body(const Problem<T>& p, const Level
   }
   const T* L = p.Lb(b, j);
   T* yj = p.Xb(b, j);
-  const bool vec = n == 8 * nta && ((reinterpret_cast<uintptr_t>(p.L) | reinterpret_cast<uintptr_t>(p.E)) &
-                                    (2 * sizeof(T) - 1)) == 0;
+  const bool vec = FULL || pairs_ok(p, n);
   const bool vecx = (m & 1) == 0 && (reinterpret_cast<uintptr_t>(p.X) & (2 * sizeof(T) - 1)) == 0;
   double* Zp = reinterpret_cast<double*>(smem_raw);
   double* Zq = Zp + 8 * NT * ldz;
@@ -165,17 +166,30 @@ __device__ __forceinline__ void sweep_rows_body(const Problem<T>& p, const Level
     __threadfence();
     pdl_trigger();
   }
-  T fp[NK][2], fq[NK][2], fs[ONE ? NT : 1][2];
+  // fs: the solve's operands, by column tile (INV) or by step of the substitution; larger
+  // blocks read them four steps at a time as they are used
+  T fp[NK][2], fq[NK][2], fs[KEEP ? NT : 4][2];
+  auto load_solve = [&](int e0) {
+#pragma unroll
+    for (int e = 0; e < (KEEP ? NT : 4); ++e) {
+      const int kk = INV || !BWD ? e0 + e : nta - 1 - e0 - e;
+      T f0 = T(0), f1 = T(0);
+      if (kk >= 0 && kk < nta) solve_frag<T, BWD, INV>(L, n, warp, kk, vec, f0, f1);
+      fs[e][0] = f0;
+      fs[e][1] = f1;
+    }
+  };
   if (KEEP && warp < nta) {
 #pragma unroll
     for (int kk = 0; kk < NT; ++kk) {
       if (P) block_frag<T, false>(P, n, warp, kk, vec && kk < nta, fp[KEEP ? kk : 0][0], fp[KEEP ? kk : 0][1]);
-      if (Q) block_frag<T, true>(Q, n, warp, kk, false, fq[KEEP ? kk : 0][0], fq[KEEP ? kk : 0][1]);
+      if (Q) block_frag<T, true>(Q, n, warp, kk, vec && kk < nta, fq[KEEP ? kk : 0][0], fq[KEEP ? kk : 0][1]);
     }
-    if (solve)
-#pragma unroll
-      for (int kk = 0; kk < NT; ++kk) solve_frag<T, BWD, INV>(L, n, warp, kk, vec && kk < nta, fs[ONE ? kk : 0][0], fs[ONE ? kk : 0][1]);
+    if (solve) load_solve(0);
   }
+  if (!KEEP && solve)   // the solve's block is read after the products: into L2 meanwhile
+    for (int e = grp.tid() * (128 / (int)sizeof(T)); e < n * n; e += grp.threads() * (128 / (int)sizeof(T)))
+      asm volatile("prefetch.global.L2 [%0];\n" ::"l"(L + e));
   double i0 = 0.0, i1 = 0.0;   // inverse of the diagonal tile (transposed for the backward sweep)
   if (!INV && solve && warp < nta) {
     // every lane: column lane % 8 of C_kk^{-1}, from the tile in shared memory
@@ -208,12 +222,13 @@ __device__ __forceinline__ void sweep_rows_body(const Problem<T>& p, const Level
   if (wait == kWaitVectors) pdl_wait();
   if (wait == kWaitFirst || wait == kWaitVectors) pdl_trigger();
 
-  for (int c0 = 0; c0 < m; c0 += XC) {
-    const int mc = min_i(XC, m - c0), groups = (mc + 7) >> 3;
-    if (c0 > 0) __syncthreads();
+  const int cend = cols < m - col0 ? col0 + cols : m;
+  for (int c0 = col0; c0 < cend; c0 += XC) {
+    const int mc = min_i(XC, cend - c0), groups = (mc + 7) >> 3;
+    if (c0 > col0) grp.sync();
     // neighbours' vectors, zeros outside
     if (P || Q) {
-      for (int e = threadIdx.x; e < 8 * nta * 8 * groups; e += blockDim.x) {
+      for (int e = grp.tid(); e < 8 * nta * 8 * groups; e += grp.threads()) {
         const int k = e / (8 * groups), c = e - k * (8 * groups);
         const bool in = k < n && c < mc;
         const long long o = (long long)k * m + c0 + c;
@@ -226,42 +241,59 @@ __device__ __forceinline__ void sweep_rows_body(const Problem<T>& p, const Level
       const int r = 8 * warp + g, c = c0 + 2 * t;
       ldcg_pair(yj + (long long)r * m + c, vecx && r < n && c < m, r < n && c < m, r < n && c + 1 < m, ys[0][0], ys[0][1]);
     }
-    __syncthreads();
+    grp.sync();
     for (int i = warp; i < nta; i += ONE ? 8 * NT : W) {
       // one column group: a chain of MMAs per block; four groups are four chains as they are
       double ap[CG][2], aq[1][2] = {{0.0, 0.0}};
 #pragma unroll
       for (int q = 0; q < CG; ++q) ap[q][0] = ap[q][1] = 0.0;
-      if (P || Q) {
-#pragma unroll(KEEP ? NT : 4)
-        for (int kk = 0; kk < (KEEP ? NT : nta); ++kk) {
-          {
-            T f0 = T(0), f1 = T(0), h0 = T(0), h1 = T(0);
-            if (KEEP) {
-              f0 = fp[KEEP ? kk : 0][0];
-              f1 = fp[KEEP ? kk : 0][1];
-              h0 = fq[KEEP ? kk : 0][0];
-              h1 = fq[KEEP ? kk : 0][1];
-            } else {
-              if (P) block_frag<T, false>(P, n, i, kk, vec, f0, f1);
-              if (Q) block_frag<T, true>(Q, n, i, kk, false, h0, h1);
-            }
-            const int zo = (8 * kk + 2 * t) * ldz + g;
+      auto products = [&](int kk, T f0, T f1, T h0, T h1) {
+        const int zo = (8 * kk + 2 * t) * ldz + g;
 #pragma unroll
-            for (int q = 0; q < CG; ++q) {
-              if (CG == 1 || q < groups) {
-                if (P) {
-                  mma_acc(ap[q][0], ap[q][1], (double)f0, Zp[zo + 8 * q]);
-                  mma_acc(ap[q][0], ap[q][1], (double)f1, Zp[zo + ldz + 8 * q]);
-                }
-                if (Q) {
-                  double(&ac)[2] = CG == 1 ? aq[0] : ap[q];
-                  mma_acc(ac[0], ac[1], (double)h0, Zq[zo + 8 * q]);
-                  mma_acc(ac[0], ac[1], (double)h1, Zq[zo + ldz + 8 * q]);
-                }
-              }
+        for (int q = 0; q < CG; ++q) {
+          if (CG == 1 || q < groups) {
+            if (P) {
+              mma_acc(ap[q][0], ap[q][1], (double)f0, Zp[zo + 8 * q]);
+              mma_acc(ap[q][0], ap[q][1], (double)f1, Zp[zo + ldz + 8 * q]);
+            }
+            if (Q) {
+              double(&ac)[2] = CG == 1 ? aq[0] : ap[q];
+              mma_acc(ac[0], ac[1], (double)h0, Zq[zo + 8 * q]);
+              mma_acc(ac[0], ac[1], (double)h1, Zq[zo + ldz + 8 * q]);
             }
           }
+        }
+      };
+      if (KEEP) {
+        if (P || Q)
+#pragma unroll
+          for (int kk = 0; kk < NT; ++kk)
+            products(kk, fp[KEEP ? kk : 0][0], fp[KEEP ? kk : 0][1], fq[KEEP ? kk : 0][0], fq[KEEP ? kk : 0][1]);
+      } else if (P || Q) {
+        // batches of operands, the next one requested before this one's products
+        constexpr int BK = 4;
+        T fb[BK][4];
+        auto fetch = [&](T (&f)[BK][4], int k0) {
+#pragma unroll
+          for (int h = 0; h < BK; ++h) {
+            f[h][0] = f[h][1] = f[h][2] = f[h][3] = T(0);
+            if (k0 + h < nta) {
+              if (P) block_frag<T, false>(P, n, i, k0 + h, vec, f[h][0], f[h][1]);
+              if (Q) block_frag<T, true>(Q, n, i, k0 + h, vec, f[h][2], f[h][3]);
+            }
+          }
+        };
+        fetch(fb, 0);
+        for (int k0 = 0; k0 < nta; k0 += BK) {
+          T cur[BK][4];
+#pragma unroll
+          for (int h = 0; h < BK; ++h)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) cur[h][e] = fb[h][e];
+          if (k0 + BK < nta) fetch(fb, k0 + BK);
+#pragma unroll
+          for (int h = 0; h < BK; ++h)
+            if (k0 + h < nta) products(k0 + h, cur[h][0], cur[h][1], cur[h][2], cur[h][3]);
         }
       }
 #pragma unroll
@@ -293,12 +325,8 @@ __device__ __forceinline__ void sweep_rows_body(const Problem<T>& p, const Level
       }
     }
     if (!solve) continue;
-    if (ONE && !KEEP && warp < nta) {
-#pragma unroll
-      for (int kk = 0; kk < NT; ++kk) solve_frag<T, BWD, INV>(L, n, warp, kk, vec && kk < nta, fs[ONE ? kk : 0][0], fs[ONE ? kk : 0][1]);
-    }
     if (INV) {
-      __syncthreads();
+      grp.sync();
       for (int i = warp; i < nta; i += ONE ? 8 * NT : W) {
         double ax[CG][2], ay[CG][2];
 #pragma unroll
@@ -308,8 +336,8 @@ __device__ __forceinline__ void sweep_rows_body(const Problem<T>& p, const Level
           if (ONE ? kk < nta : (BWD ? kk >= i && kk < nta : kk <= i)) {
             T f0, f1;
             if (ONE) {
-              f0 = fs[ONE ? kk : 0][0];
-              f1 = fs[ONE ? kk : 0][1];
+              f0 = fs[KEEP ? kk : 0][0];
+              f1 = fs[KEEP ? kk : 0][1];
             } else {
               solve_frag<T, BWD, INV>(L, n, i, kk, vec, f0, f1);
             }
@@ -331,46 +359,70 @@ __device__ __forceinline__ void sweep_rows_body(const Problem<T>& p, const Level
         }
       }
     } else {
+      // substitution: step st solves row tile kk, later row tiles subtract it.  Four steps are
+      // unrolled at a time, the next four's operands requested before them (all steps unrolled
+      // did not fit the instruction cache at n = 128: 3 us a step).
+      constexpr int U = KEEP ? NT : 4;
+      if (!KEEP && warp < nta) load_solve(0);
+#pragma unroll 1
+      for (int s0 = 0; s0 < nta; s0 += U) {
+        T cur[U][2];
 #pragma unroll
-      for (int st = 0; st < NT; ++st) {
-        const int kk = BWD ? NT - 1 - st : st;
-        if (kk < nta) {
-          if (warp == kk) {
+        for (int h = 0; h < U; ++h) {
+          cur[h][0] = fs[h][0];
+          cur[h][1] = fs[h][1];
+        }
+        if (!KEEP && s0 + U < nta && warp < nta) load_solve(s0 + U);
 #pragma unroll
-            for (int q = 0; q < CG; ++q) {
-              Rs[(8 * kk + g) * ldz + 8 * q + 2 * t] = ys[ONE ? q : 0][0];
-              Rs[(8 * kk + g) * ldz + 8 * q + 2 * t + 1] = ys[ONE ? q : 0][1];
+        for (int h = 0; h < U; ++h) {
+          const int st = s0 + h, kk = BWD ? nta - 1 - st : st;
+          if (st < nta) {
+            if (warp == kk) {
+#pragma unroll
+              for (int q = 0; q < CG; ++q) {
+                if (CG > 1 && q >= groups) break;
+                Rs[(8 * kk + g) * ldz + 8 * q + 2 * t] = ys[ONE ? q : 0][0];
+                Rs[(8 * kk + g) * ldz + 8 * q + 2 * t + 1] = ys[ONE ? q : 0][1];
+              }
+              __syncwarp();
+#pragma unroll
+              for (int q = 0; q < CG; ++q) {
+                if (CG > 1 && q >= groups) break;
+                double x0 = 0.0, x1 = 0.0;
+                const int zo = (8 * kk + 2 * t) * ldz + 8 * q + g;
+                mma_acc(x0, x1, i0, Rs[zo]);
+                mma_acc(x0, x1, i1, Rs[zo + ldz]);
+                ys[ONE ? q : 0][0] = x0;
+                ys[ONE ? q : 0][1] = x1;
+              }
+              __syncwarp();
+#pragma unroll
+              for (int q = 0; q < CG; ++q) {
+                if (CG > 1 && q >= groups) break;
+                Rs[(8 * kk + g) * ldz + 8 * q + 2 * t] = ys[ONE ? q : 0][0];
+                Rs[(8 * kk + g) * ldz + 8 * q + 2 * t + 1] = ys[ONE ? q : 0][1];
+              }
             }
-            __syncwarp();
-            double xr[CG][2];
+            grp.sync();
+            if ((BWD ? warp < kk : warp > kk) && warp < nta) {
 #pragma unroll
-            for (int q = 0; q < CG; ++q) {
-              xr[q][0] = xr[q][1] = 0.0;
-              const int zo = (8 * kk + 2 * t) * ldz + 8 * q + g;
-              mma_acc(xr[q][0], xr[q][1], i0, Rs[zo]);
-              mma_acc(xr[q][0], xr[q][1], i1, Rs[zo + ldz]);
-            }
-            __syncwarp();
-#pragma unroll
-            for (int q = 0; q < CG; ++q) {
-              if (CG > 1 && q >= groups) break;
-              const int r = 8 * kk + g, c = c0 + 8 * q + 2 * t;
-              Rs[r * ldz + 8 * q + 2 * t] = xr[q][0];
-              Rs[r * ldz + 8 * q + 2 * t + 1] = xr[q][1];
-              store_pair(yj + (long long)r * m + c, vecx && r < n && c < m, r < n && c < m, r < n && c + 1 < m, xr[q][0],
-                         xr[q][1]);
+              for (int q = 0; q < CG; ++q) {
+                if (CG > 1 && q >= groups) break;
+                const int zo = (8 * kk + 2 * t) * ldz + 8 * q + g;
+                mma_acc(ys[ONE ? q : 0][0], ys[ONE ? q : 0][1], -(double)cur[h][0], Rs[zo]);
+                mma_acc(ys[ONE ? q : 0][0], ys[ONE ? q : 0][1], -(double)cur[h][1], Rs[zo + ldz]);
+              }
             }
           }
-          __syncthreads();
-          if ((BWD ? warp < kk : warp > kk) && warp < nta) {
+        }
+      }
+      if (warp < nta) {
 #pragma unroll
-            for (int q = 0; q < CG; ++q) {
-              if (CG > 1 && q >= groups) break;
-              const int zo = (8 * kk + 2 * t) * ldz + 8 * q + g;
-              mma_acc(ys[ONE ? q : 0][0], ys[ONE ? q : 0][1], -(double)fs[ONE ? kk : 0][0], Rs[zo]);
-              mma_acc(ys[ONE ? q : 0][0], ys[ONE ? q : 0][1], -(double)fs[ONE ? kk : 0][1], Rs[zo + ldz]);
-            }
-          }
+        for (int q = 0; q < CG; ++q) {
+          if (CG > 1 && q >= groups) break;
+          const int r = 8 * warp + g, c = c0 + 8 * q + 2 * t;
+          store_pair(yj + (long long)r * m + c, vecx && r < n && c < m, r < n && c < m, r < n && c + 1 < m,
+                     ys[ONE ? q : 0][0], ys[ONE ? q : 0][1]);
         }
       }
     }
@@ -384,13 +436,15 @@ __host__ __device__ inline int sweep_tasks(int N, const Level& lv) {
   return MODE == kModeBackward || lv.s == 1 ? lv.d : N / lv.s;
 }
 
-template <typename T, int NT, int MODE, bool INV>
-__global__ void __launch_bounds__(32 * NT, NT <= 8 ? 16 / NT : 1) k_sweep_rows(Problem<T> p, Level lv, int wait) {
+// cols: columns per block; on narrow levels several blocks (along y) share a vector's right-hand sides
+template <typename T, int NT, bool FULL, int MODE, bool INV>
+__global__ void __launch_bounds__(32 * NT, NT <= 8 ? 16 / NT : 1)
+    k_sweep_rows(Problem<T> p, Level lv, int wait, int cols) {
   const int per_b = sweep_tasks<MODE>(p.N, lv);
   const int b = blockIdx.x / per_b;
   if (!p.active(b)) return;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  sweep_rows_body<T, NT, MODE, INV, true>(p, lv, b, blockIdx.x - b * per_b, smem_raw, wait);
+  sweep_rows_body<T, NT, FULL, MODE, INV, true>(BlockGroup{}, p, lv, b, blockIdx.x - b * per_b, smem_raw, wait, blockIdx.y * cols, cols);
 }
 
 }  // namespace socu

@@ -55,7 +55,7 @@ __global__ void __launch_bounds__(32 * NT) k_top(Problem<T> p, const __grid_cons
     const Level& L = tl.fl[li];
     for (int t = rank; t < sweep_tasks<kModeForward>(p.N, L); t += C) {
       __syncthreads();
-      sweep_rows_body<T, NT, kModeForward, INV, true>(p, L, b, t, smem_raw, kWaitNone);
+      sweep_rows_body<T, NT, false, kModeForward, INV, true>(BlockGroup{}, p, L, b, t, smem_raw, kWaitNone);
     }
     if (li + 1 < tl.fwd_n || tl.bwd_n > 0) {
       cluster_arrive();
@@ -66,7 +66,7 @@ __global__ void __launch_bounds__(32 * NT) k_top(Problem<T> p, const __grid_cons
     const Level& L = tl.bl[li];
     for (int t = rank; t < L.d; t += C) {
       __syncthreads();
-      sweep_rows_body<T, NT, kModeBackward, INV, true>(p, L, b, t, smem_raw, kWaitNone);
+      sweep_rows_body<T, NT, false, kModeBackward, INV, true>(BlockGroup{}, p, L, b, t, smem_raw, kWaitNone);
     }
     if (li > 0) {
       cluster_arrive();
@@ -82,43 +82,43 @@ __host__ __device__ inline long long smem_top_bytes(int n, bool inv) { return sm
 // Sweep kernels by op, block size and inverse-carrying factors (sweeps_f32.cu,
 // sweeps_f64.cu: one translation unit per type).
 template <typename T>
-using SweepFn = void (*)(Problem<T>, Level, int);
+using SweepFn = void (*)(Problem<T>, Level, int, int);
 template <typename T>
 using TopFn = void (*)(Problem<T>, TopLevels);
 template <typename T>
-SweepFn<T> sweep_kernel(SweepMode mode, int n, bool inv);
+SweepFn<T> sweep_kernel(SweepMode mode, int n, bool full, bool inv);
 template <typename T>
 TopFn<T> top_sweep_kernel(int n, bool inv);
 
-template <typename T, int NT>
+template <typename T, int NT, bool FULL>
 inline SweepFn<T> sweep_kernel_nt(SweepMode mode, bool inv) {
-  if (mode == kModePull) return k_sweep_rows<T, NT, kModePull, true>;
+  if (mode == kModePull) return k_sweep_rows<T, NT, FULL, kModePull, true>;
   if constexpr (NT <= 8) {   // factors carry inverses up to n = 64
     if (inv) {
-      if (mode == kModeForward) return k_sweep_rows<T, NT, kModeForward, true>;
-      return k_sweep_rows<T, NT, kModeBackward, true>;
+      if (mode == kModeForward) return k_sweep_rows<T, NT, FULL, kModeForward, true>;
+      return k_sweep_rows<T, NT, FULL, kModeBackward, true>;
     }
   }
-  if (mode == kModeForward) return k_sweep_rows<T, NT, kModeForward, false>;
-  return k_sweep_rows<T, NT, kModeBackward, false>;
+  if (mode == kModeForward) return k_sweep_rows<T, NT, FULL, kModeForward, false>;
+  return k_sweep_rows<T, NT, FULL, kModeBackward, false>;
 }
 
 #define SOCU_SWEEP_KERNELS(T)                                                              \
   template <>                                                                              \
-  SweepFn<T> sweep_kernel<T>(SweepMode mode, int n, bool inv) {                            \
+  SweepFn<T> sweep_kernel<T>(SweepMode mode, int n, bool full, bool inv) {                 \
     switch (rows_nt(n)) {                                                                  \
-      case 1: return sweep_kernel_nt<T, 1>(mode, inv);                                     \
-      case 2: return sweep_kernel_nt<T, 2>(mode, inv);                                     \
-      case 3: return sweep_kernel_nt<T, 3>(mode, inv);                                     \
-      case 4: return sweep_kernel_nt<T, 4>(mode, inv);                                     \
-      case 5: return sweep_kernel_nt<T, 5>(mode, inv);                                     \
-      case 6: return sweep_kernel_nt<T, 6>(mode, inv);                                     \
-      case 7: return sweep_kernel_nt<T, 7>(mode, inv);                                     \
-      case 8: return sweep_kernel_nt<T, 8>(mode, inv);                                     \
-      case 10: return sweep_kernel_nt<T, 10>(mode, inv);                                   \
-      case 12: return sweep_kernel_nt<T, 12>(mode, inv);                                   \
-      case 14: return sweep_kernel_nt<T, 14>(mode, inv);                                   \
-      default: return sweep_kernel_nt<T, 16>(mode, inv);                                   \
+      case 1: return full ? sweep_kernel_nt<T, 1, true>(mode, inv) : sweep_kernel_nt<T, 1, false>(mode, inv); \
+      case 2: return full ? sweep_kernel_nt<T, 2, true>(mode, inv) : sweep_kernel_nt<T, 2, false>(mode, inv); \
+      case 3: return full ? sweep_kernel_nt<T, 3, true>(mode, inv) : sweep_kernel_nt<T, 3, false>(mode, inv); \
+      case 4: return full ? sweep_kernel_nt<T, 4, true>(mode, inv) : sweep_kernel_nt<T, 4, false>(mode, inv); \
+      case 5: return full ? sweep_kernel_nt<T, 5, true>(mode, inv) : sweep_kernel_nt<T, 5, false>(mode, inv); \
+      case 6: return full ? sweep_kernel_nt<T, 6, true>(mode, inv) : sweep_kernel_nt<T, 6, false>(mode, inv); \
+      case 7: return full ? sweep_kernel_nt<T, 7, true>(mode, inv) : sweep_kernel_nt<T, 7, false>(mode, inv); \
+      case 8: return full ? sweep_kernel_nt<T, 8, true>(mode, inv) : sweep_kernel_nt<T, 8, false>(mode, inv); \
+      case 10: return full ? sweep_kernel_nt<T, 10, true>(mode, inv) : sweep_kernel_nt<T, 10, false>(mode, inv); \
+      case 12: return full ? sweep_kernel_nt<T, 12, true>(mode, inv) : sweep_kernel_nt<T, 12, false>(mode, inv); \
+      case 14: return full ? sweep_kernel_nt<T, 14, true>(mode, inv) : sweep_kernel_nt<T, 14, false>(mode, inv); \
+      default: return full ? sweep_kernel_nt<T, 16, true>(mode, inv) : sweep_kernel_nt<T, 16, false>(mode, inv); \
     }                                                                                      \
   }                                                                                        \
   template <>                                                                              \
@@ -130,8 +130,8 @@ inline SweepFn<T> sweep_kernel_nt(SweepMode mode, bool inv) {
     }                                                                                      \
   }
 
-template <> SweepFn<float> sweep_kernel<float>(SweepMode, int, bool);
-template <> SweepFn<double> sweep_kernel<double>(SweepMode, int, bool);
+template <> SweepFn<float> sweep_kernel<float>(SweepMode, int, bool, bool);
+template <> SweepFn<double> sweep_kernel<double>(SweepMode, int, bool, bool);
 template <> TopFn<float> top_sweep_kernel<float>(int, bool);
 template <> TopFn<double> top_sweep_kernel<double>(int, bool);
 

@@ -107,14 +107,14 @@ __device__ __forceinline__ void upd_step(double (&acc)[NT][2], const T* fk, cons
 }
 
 // One output block, `task` in [0, update_blocks).
-template <typename T, int NT, bool SPLIT>
-__device__ __forceinline__ void update_rows_body(const Problem<T>& p, const Level& lv, int b, int task,
+template <typename T, int NT, bool FULL, bool SPLIT, class Group>
+__device__ __forceinline__ void update_rows_body(const Group& grp, const Problem<T>& p, const Level& lv, int b, int task,
                                                  unsigned char* smem_raw, int q, int splits) {
   constexpr int es = sizeof(T), ldg = upd_ldg(NT, es);
   constexpr bool kAhead = NT <= 8;   // (registers: larger blocks read the output block at the end)
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, W = blockDim.x >> 5;
+  const int lane = threadIdx.x & 31, warp = grp.warp(), W = grp.warps();
   const int g = lane >> 2, t = lane & 3;
-  const int n = p.n, N = p.N, s = lv.s, nta = (n + 7) >> 3;
+  const int n = FULL ? 8 * NT : p.n, N = p.N, s = lv.s, nta = (n + 7) >> 3;
   const int U = N / (2 * s);
   const bool target = task < U;
   const T *F, *G;
@@ -131,8 +131,7 @@ __device__ __forceinline__ void update_rows_body(const Problem<T>& p, const Leve
     G = p.Eb(b, lv.oc + 2 * f - 1);
     Out = p.Eb(b, lv.on + f - 1);
   }
-  const bool vec = n == 8 * nta && ((reinterpret_cast<uintptr_t>(p.L) | reinterpret_cast<uintptr_t>(p.E)) &
-                                    (2 * sizeof(T) - 1)) == 0;
+  const bool vec = FULL || pairs_ok(p, n);
   const int part = warp % splits, step = splits * (W / splits);
   const int first = q + splits * (warp / splits);       // this warp's first row tile
   const int last = q + splits * ((nta - 1 - q) / splits);  // the block's last row tile
@@ -145,24 +144,23 @@ __device__ __forceinline__ void update_rows_body(const Problem<T>& p, const Leve
     T* Gs = Fs + 8 * NT * kUpdLdF;
     const int k0 = c * kUpdKC, kw = min_i(kUpdKC, n - k0);
     if (target || splits == 1) {
-      async_load(Fs, kUpdLdF, F + k0, lim, kw, n);
+      async_load_by(grp.tid(), grp.threads(), Fs, kUpdLdF, F + k0, lim, kw, n);
     } else {
       for (int i = q; i < nta; i += splits)
-        async_load(Fs + 8 * i * kUpdLdF, kUpdLdF, F + (long long)8 * i * n + k0, min_i(8, n - 8 * i), kw, n);
+        async_load_by(grp.tid(), grp.threads(), Fs + 8 * i * kUpdLdF, kUpdLdF, F + (long long)8 * i * n + k0, min_i(8, n - 8 * i), kw, n);
     }
-    if (G) async_load(Gs, ldg, G + (long long)k0 * n, kw, lim, n);
+    if (G) async_load_by(grp.tid(), grp.threads(), Gs, ldg, G + (long long)k0 * n, kw, lim, n);
     const int kp = (kw + 7) & ~7;   // zeros up to a whole k-step
     if (kp > kw) {
-      for (int e = threadIdx.x; e < 8 * nta * (kp - kw); e += blockDim.x)
+      for (int e = grp.tid(); e < 8 * nta * (kp - kw); e += grp.threads())
         Fs[(e / (kp - kw)) * kUpdLdF + kw + e % (kp - kw)] = T(0);
       if (G)
-        for (int e = threadIdx.x; e < 8 * nta * (kp - kw); e += blockDim.x)
+        for (int e = grp.tid(); e < 8 * nta * (kp - kw); e += grp.threads())
           Gs[(kw + e / (8 * nta)) * ldg + e % (8 * nta)] = T(0);
     }
     cp_async_commit();
   };
-  stage(0);
-  if (chunks > 1) stage(1);
+  int requested = 0;   // chunks
   bool staged = false;   // all chunks have arrived (n <= 64: later rows need no barrier)
   for (int i = first; i < nta || !staged; i += step) {
     const bool on = i < nta;
@@ -179,11 +177,17 @@ __device__ __forceinline__ void update_rows_body(const Problem<T>& p, const Leve
     }
     for (int c = 0; c < chunks; ++c) {
       if (!staged) {
+        // two chunks ahead (one call: the staging code is large, and the steps
+        // around it should stay in the instruction cache)
+        while (requested < chunks && requested < c + 2) {
+          if (requested > 1) grp.sync();   // its buffer is free again
+          stage(requested++);
+        }
         if (c + 1 < chunks)
           cp_async_wait_one();
         else
           cp_async_wait_all();
-        __syncthreads();
+        grp.sync();
       }
       if (on) {
         const T* Fs = buf + (c & 1) * upd_stage_elems(NT, es);
@@ -206,10 +210,6 @@ __device__ __forceinline__ void update_rows_body(const Problem<T>& p, const Leve
           else
             upd_step<T, NT, SPLIT, true, false>(acc, fk, gk, part, splits, jmax, a0, a1, h0, h1);
         }
-      }
-      if (!staged && c + 2 < chunks) {
-        __syncthreads();   // buffer c & 1 is free again
-        stage(c + 2);
       }
     }
     staged = true;
@@ -235,7 +235,7 @@ __device__ __forceinline__ void update_rows_body(const Problem<T>& p, const Leve
   }
 }
 
-template <typename T, int NT>
+template <typename T, int NT, bool FULL>
 __global__ void __launch_bounds__(NT <= 8 ? 256 : 512, NT <= 8 ? 2 : 1)
     k_update_rows(Problem<T> p, Level lv, int splits) {
   const int block = blockIdx.x / splits, q = blockIdx.x - block * splits;
@@ -246,37 +246,37 @@ __global__ void __launch_bounds__(NT <= 8 ? 256 : 512, NT <= 8 ? 2 : 1)
   if (!p.active(b)) return;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   if (splits > 1)
-    update_rows_body<T, NT, true>(p, lv, b, task, smem_raw, q, splits);
+    update_rows_body<T, NT, FULL, true>(BlockGroup{}, p, lv, b, task, smem_raw, q, splits);
   else
-    update_rows_body<T, NT, false>(p, lv, b, task, smem_raw, 0, 1);
+    update_rows_body<T, NT, FULL, false>(BlockGroup{}, p, lv, b, task, smem_raw, 0, 1);
 }
 
 template <typename T>
 using UpdateRowsFn = void (*)(Problem<T>, Level, int);
 
 template <typename T>
-UpdateRowsFn<T> update_rows_kernel(int n);
+UpdateRowsFn<T> update_rows_kernel(int n, bool full);
 
 #define SOCU_UPDATE_ROWS_KERNELS(T)                    \
   template <>                                          \
-  UpdateRowsFn<T> update_rows_kernel<T>(int n) {       \
+  UpdateRowsFn<T> update_rows_kernel<T>(int n, bool full) { \
     switch (rows_nt(n)) {                              \
-      case 1: return k_update_rows<T, 1>;              \
-      case 2: return k_update_rows<T, 2>;              \
-      case 3: return k_update_rows<T, 3>;              \
-      case 4: return k_update_rows<T, 4>;              \
-      case 5: return k_update_rows<T, 5>;              \
-      case 6: return k_update_rows<T, 6>;              \
-      case 7: return k_update_rows<T, 7>;              \
-      case 8: return k_update_rows<T, 8>;              \
-      case 10: return k_update_rows<T, 10>;            \
-      case 12: return k_update_rows<T, 12>;            \
-      case 14: return k_update_rows<T, 14>;            \
-      default: return k_update_rows<T, 16>;            \
+      case 1: return full ? k_update_rows<T, 1, true> : k_update_rows<T, 1, false>; \
+      case 2: return full ? k_update_rows<T, 2, true> : k_update_rows<T, 2, false>; \
+      case 3: return full ? k_update_rows<T, 3, true> : k_update_rows<T, 3, false>; \
+      case 4: return full ? k_update_rows<T, 4, true> : k_update_rows<T, 4, false>; \
+      case 5: return full ? k_update_rows<T, 5, true> : k_update_rows<T, 5, false>; \
+      case 6: return full ? k_update_rows<T, 6, true> : k_update_rows<T, 6, false>; \
+      case 7: return full ? k_update_rows<T, 7, true> : k_update_rows<T, 7, false>; \
+      case 8: return full ? k_update_rows<T, 8, true> : k_update_rows<T, 8, false>; \
+      case 10: return full ? k_update_rows<T, 10, true> : k_update_rows<T, 10, false>; \
+      case 12: return full ? k_update_rows<T, 12, true> : k_update_rows<T, 12, false>; \
+      case 14: return full ? k_update_rows<T, 14, true> : k_update_rows<T, 14, false>; \
+      default: return full ? k_update_rows<T, 16, true> : k_update_rows<T, 16, false>; \
     }                                                  \
   }
 
-template <> UpdateRowsFn<float> update_rows_kernel<float>(int n);
-template <> UpdateRowsFn<double> update_rows_kernel<double>(int n);
+template <> UpdateRowsFn<float> update_rows_kernel<float>(int n, bool full);
+template <> UpdateRowsFn<double> update_rows_kernel<double>(int n, bool full);
 
 }  // namespace socu
