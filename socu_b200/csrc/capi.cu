@@ -1171,11 +1171,14 @@ int rg_create(socu_ragged_s* r, const int64_t* horizon, const int64_t* n, const 
     if (phases >= (1 << kRgPhaseBits)) return SOCU_ERR_UNSUPPORTED;
     for (int ph = 0; ph < phases; ++ph) cap += rg_chunks(rg_phase(I, mode, ph));
   }
-  // first-phase chunks, largest instances first
+  // first-phase chunks: largest blocks first, so that the workers of an SM run
+  // the code of one block size at a time (it fits the instruction cache, several
+  // sizes' do not), and within a size the largest instances
   std::vector<int> order(r->inst.size());
   for (size_t i = 0; i < order.size(); ++i) order[i] = (int)i;
   std::stable_sort(order.begin(), order.end(), [&](int a, int b) {
     const RgInst &A = r->inst[a], &B = r->inst[b];
+    if (rg_nt(A.n) != rg_nt(B.n)) return rg_nt(A.n) > rg_nt(B.n);
     return (double)A.N * A.n * A.n * A.n > (double)B.N * B.n * B.n * B.n;
   });
   std::vector<unsigned long long>& init = r->init;

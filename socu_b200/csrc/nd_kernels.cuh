@@ -44,7 +44,15 @@ static __global__ void k_info_reset(int* info, int B) {
   for (int b = blockIdx.x * blockDim.x + threadIdx.x; b < B; b += gridDim.x * blockDim.x) info[b] = 0;
 }
 
-// Output blocks of one update level per instance: N / 2s targets, then the fill-in blocks.
-__host__ __device__ inline int update_blocks(int N, const Level& lv) { return N / (2 * lv.s) + lv.d - 1; }
+// Output blocks of one update level per instance: N / 2s targets (s is a power of two), then the
+// fill-in blocks.
+__host__ __device__ inline int update_targets(int N, const Level& lv) {
+#ifdef __CUDA_ARCH__
+  return N >> __ffs(lv.s);
+#else
+  return N / (2 * lv.s);
+#endif
+}
+__host__ __device__ inline int update_blocks(int N, const Level& lv) { return update_targets(N, lv) + lv.d - 1; }
 
 }  // namespace socu

@@ -78,16 +78,16 @@ __host__ __device__ inline void rg_decode(unsigned long long t, int& inst, int& 
 // Level l of the separator schedule of a horizon-N system
 // (socu/block_tridiag_solver.py:869-914).
 __host__ __device__ inline Level rg_level(int N, int l) {
-  int s = 1, prev = 0, curr = 0, nxt = N - 1;
-  for (int k = 0; k < l; ++k) {
-    s *= 2;
+  // (strides are powers of two: shifts, as every worker computes this for every chunk)
+  int prev = 0, curr = 0, nxt = N - 1;
+  for (int k = 1; k <= l; ++k) {
     prev = curr;
     curr = nxt;
-    nxt += N / s - 1;
+    nxt += (N >> k) - 1;
   }
   Level lv;
-  lv.s = s;
-  lv.d = (N + s) / (2 * s);
+  lv.s = 1 << l;
+  lv.d = (N + lv.s) >> (l + 1);
   lv.oc = curr;
   lv.on = nxt;
   lv.op = prev;
@@ -122,7 +122,7 @@ __host__ __device__ inline RgPhase rg_phase(const RgInst& I, int mode, int ph) {
       r.units = lv.d;
     } else {
       r.kind = kRgUpd;
-      r.units = I.N / (2 * lv.s);
+      r.units = I.N >> (r.level + 1);
     }
     return r;
   }
@@ -319,9 +319,10 @@ __host__ __device__ inline long long rg_block_bytes(int n, int es, bool refine, 
 }
 // Block workers for batches with few nodes per warp worker (12 of those per SM).  Measured in
 // FP64 on N ~ U{8..256}, n in {8, 16, 32, 48}, m in {1, 4} (132 nodes a system), warp against
-// block workers: 16 systems 1.28 / 0.56 ms, 64 1.51 / 0.97, 128 2.07 / 1.82, 256 3.40 / 3.57,
-// 512 5.39 / 6.54, 1024 8.9 / 11.8 ms; the line lies at 175 such systems.
-__host__ __device__ inline bool rg_use_blocks(long long nodes, int sms) { return nodes < 13LL * 12 * sms; }
+// block workers, ms: 16 systems 1.28 / 0.55, 64 1.51 / 0.95, 128 2.07 / 1.82, 512 4.56 / 6.54,
+// 1024 7.6 / 11.8; on either side of the line (240 such systems) 190 take 2.54 on blocks and 256
+// 2.88 on warps.
+__host__ __device__ inline bool rg_use_blocks(long long nodes, int sms) { return nodes < 18LL * 12 * sms; }
 
 // One unit of a level phase (one copy of each per tile count: the kernel calls them).
 template <typename T, int NT, bool FULL, bool BLOCKS>
@@ -355,7 +356,7 @@ __device__ __forceinline__ void rg_level_unit(const Problem<T>& p, int kind, int
     rg_update_unit<T, NT, FULL, BLOCKS>(p, lv, u, smem, grp);
     if (u + 1 <= lv.d - 1) {   // fill-in block of node t = u + 1
       grp.sync();
-      rg_update_unit<T, NT, FULL, BLOCKS>(p, lv, p.N / (2 * lv.s) + u, smem, grp);
+      rg_update_unit<T, NT, FULL, BLOCKS>(p, lv, update_targets(p.N, lv) + u, smem, grp);
     }
     // y_j -= F y_{j-s} + G^T y_{j+s} for target j = 2s(u+1) - 1
     grp.sync();

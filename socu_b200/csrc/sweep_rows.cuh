@@ -331,16 +331,20 @@ __device__ __forceinline__ void sweep_rows_body(const Group& grp, const Problem<
         double ax[CG][2], ay[CG][2];
 #pragma unroll
         for (int q = 0; q < CG; ++q) ax[q][0] = ax[q][1] = ay[q][0] = ay[q][1] = 0.0;
+        T fr[ONE ? 1 : NT][2];   // (all requested before the first is used)
+        if (!ONE)
+#pragma unroll
+          for (int kk = 0; kk < NT; ++kk) {
+            T f0 = T(0), f1 = T(0);
+            if (kk < nta) solve_frag<T, BWD, INV>(L, n, i, kk, vec, f0, f1);
+            fr[ONE ? 0 : kk][0] = f0;
+            fr[ONE ? 0 : kk][1] = f1;
+          }
 #pragma unroll
         for (int kk = 0; kk < NT; ++kk) {
           if (ONE ? kk < nta : (BWD ? kk >= i && kk < nta : kk <= i)) {
-            T f0, f1;
-            if (ONE) {
-              f0 = fs[KEEP ? kk : 0][0];
-              f1 = fs[KEEP ? kk : 0][1];
-            } else {
-              solve_frag<T, BWD, INV>(L, n, i, kk, vec, f0, f1);
-            }
+            const T f0 = ONE ? fs[KEEP ? kk : 0][0] : fr[ONE ? 0 : kk][0];
+            const T f1 = ONE ? fs[KEEP ? kk : 0][1] : fr[ONE ? 0 : kk][1];
             const int zo = (8 * kk + 2 * t) * ldz + g;
 #pragma unroll
             for (int q = 0; q < CG; ++q)
@@ -433,7 +437,11 @@ __device__ __forceinline__ void sweep_rows_body(const Group& grp, const Problem<
 // vectors of one level per instance
 template <int MODE>
 __host__ __device__ inline int sweep_tasks(int N, const Level& lv) {
+#ifdef __CUDA_ARCH__
+  return MODE == kModeBackward || lv.s == 1 ? lv.d : N >> (__ffs(lv.s) - 1);
+#else
   return MODE == kModeBackward || lv.s == 1 ? lv.d : N / lv.s;
+#endif
 }
 
 // cols: columns per block; on narrow levels several blocks (along y) share a vector's right-hand sides

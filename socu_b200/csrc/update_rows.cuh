@@ -115,7 +115,7 @@ __device__ __forceinline__ void update_rows_body(const Group& grp, const Problem
   const int lane = threadIdx.x & 31, warp = grp.warp(), W = grp.warps();
   const int g = lane >> 2, t = lane & 3;
   const int n = FULL ? 8 * NT : p.n, N = p.N, s = lv.s, nta = (n + 7) >> 3;
-  const int U = N / (2 * s);
+  const int U = update_targets(N, lv);
   const bool target = task < U;
   const T *F, *G;
   T* Out;

@@ -25,6 +25,14 @@ __device__ __forceinline__ void tile_put(double* tile, double x0, double x1) {
   *reinterpret_cast<double2*>(tile + 2 * (threadIdx.x & 31)) = make_double2(x0, x1);
 }
 
+// `count` elements from p into L2
+template <typename T>
+__device__ __forceinline__ void warp_prefetch(const T* p, int count) {
+  constexpr int line = 128 / (int)sizeof(T);
+  for (int e = (threadIdx.x & 31) * line; e < count; e += 32 * line)
+    asm volatile("prefetch.global.L2 [%0];\n" ::"l"(p + e));
+}
+
 // All steps of R row tiles against the finished factor: they share every operand load.
 template <int NT, int R>
 __device__ __forceinline__ void warp_rows_solve(double (&acc)[R][NT][2], int k0, int nta, const double* Ls,
@@ -69,24 +77,35 @@ __device__ __forceinline__ void node_warp_body(const Problem<T>& p, const Level&
   T* Ct = reinterpret_cast<T*>(Iv + 64 * NT);
   T* Li = p.Lb(b, i);
   const bool vec = FULL || pairs_ok(p, n);
-  // L_i's lower tiles (diagonal ones in the inverses' places; the padding is an identity)
-#pragma unroll 1
-  for (int r = 0; r < nta; ++r) {
-    const int gr = 8 * r + g;
-    double x[NT][2];
+  // the coupling blocks, needed after the factor: into L2 meanwhile
+  T* R = right ? p.Eb(b, lv.oc + 2 * t) : nullptr;
+  T* Lf = left ? p.Eb(b, lv.oc + 2 * t - 1) : nullptr;
+  if (right) warp_prefetch(R, n * n);
+  if (left) warp_prefetch(Lf, n * n);
+  // L_i's lower tiles (diagonal ones in the inverses' places; the padding is an identity),
+  // all requested before the first is used
+  {
+    T x[warp_node_tiles(NT)][2];
 #pragma unroll
-    for (int j = 0; j < NT; ++j)
-      if (j <= r) {
-        const int c = 8 * j + 2 * tq;
-        load_pair(Li + (long long)gr * n + c, vec, gr < n && c < n, gr < n && c + 1 < n, x[j][0], x[j][1]);
-        if (!vec && gr >= n) {
-          if (c == gr) x[j][0] = 1.0;
-          if (c + 1 == gr) x[j][1] = 1.0;
+    for (int r = 0; r < NT; ++r)
+#pragma unroll
+      for (int j = 0; j <= r; ++j) {
+        const int gr = 8 * r + g, c = 8 * j + 2 * tq, e = r * (r + 1) / 2 + j;
+        x[e][0] = x[e][1] = T(0);
+        if (r < nta) load_raw(Li + (gr * n + c), vec, gr < n && c < n, gr < n && c + 1 < n, x[e]);
+        if (!FULL && gr >= n) {
+          if (c == gr) x[e][0] = T(1);
+          if (c + 1 == gr) x[e][1] = T(1);
         }
       }
 #pragma unroll
-    for (int j = 0; j < NT; ++j)
-      if (j <= r) tile_put(j == r ? Iv + 64 * r : Ls + 64 * (r * (r - 1) / 2 + j), x[j][0], x[j][1]);
+    for (int r = 0; r < NT; ++r)
+#pragma unroll
+      for (int j = 0; j <= r; ++j)
+        if (r < nta) {
+          const int e = r * (r + 1) / 2 + j;
+          tile_put(j == r ? Iv + 64 * r : Ls + 64 * (r * (r - 1) / 2 + j), (double)x[e][0], (double)x[e][1]);
+        }
   }
   // (tiles are read as the fragments they were written as, each lane its own; only the
   // diagonal tiles, factored by the whole warp, need the warp in step)
@@ -133,8 +152,6 @@ __device__ __forceinline__ void node_warp_body(const Problem<T>& p, const Level&
   }
   // rows of the right slot, columns of the left slot and of y, two tiles at a time
   const int vr = right ? nta : 0, vl = left ? nta : 0, vy = (p.m + 7) >> 3;
-  T* R = right ? p.Eb(b, lv.oc + 2 * t) : nullptr;
-  T* Lf = left ? p.Eb(b, lv.oc + 2 * t - 1) : nullptr;
   T* yi = p.Xb(b, i);
   auto source = [&](int v) {
     RowSrc<T> o;
@@ -189,7 +206,7 @@ __device__ __forceinline__ void node_warp_body(const Problem<T>& p, const Level&
 template <typename T, int NT, bool FULL>
 __device__ __forceinline__ void update_warp_body(const Problem<T>& p, const Level& lv, int b, int task) {
   const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-  const int n = FULL ? 8 * NT : p.n, N = p.N, s = lv.s, nta = (n + 7) >> 3, U = N / (2 * s);
+  const int n = FULL ? 8 * NT : p.n, N = p.N, s = lv.s, nta = (n + 7) >> 3, U = update_targets(N, lv);
   const bool target = task < U;
   const T *F, *G;
   T* Out;
@@ -206,44 +223,44 @@ __device__ __forceinline__ void update_warp_body(const Problem<T>& p, const Leve
     Out = p.Eb(b, lv.on + f - 1);
   }
   const bool vec = FULL || pairs_ok(p, n);
+  warp_prefetch(Out, n * n);
 #pragma unroll 1
   for (int i = 0; i < nta; i += 2) {
     const int jmax = target ? min_i(i + 1, nta - 1) : nta - 1;   // last tile of the two rows
     double acc[2][NT][2];
 #pragma unroll
     for (int j = 0; j < NT; ++j) acc[0][j][0] = acc[0][j][1] = acc[1][j][0] = acc[1][j][1] = 0.0;
+    // steps: F's part of a target, then G's; a fill-in (F G) has one part.  (Requesting the next
+    // step's operands ahead made one size faster by 5 % and a mix of sizes slower by 12 %: code.)
+    const int p0 = target ? 0 : 1, parts = target && G != nullptr ? 2 : 1, steps = nta * parts;
 #pragma unroll 1
-    for (int kk = 0; kk < nta; ++kk) {
-      // F's part of a target, then G's; a fill-in is F G
-#pragma unroll 1
-      for (int part = 0; part < 2; ++part) {
-        if (part == 0 ? !target : (G == nullptr)) continue;
-        const bool tr = part == 1 && target;   // the row operand: G^T
-        T a[2][2], x[NT][2];
+    for (int it = 0; it < steps; ++it) {
+      const int kk = parts == 2 ? it >> 1 : it, part = parts == 2 ? it & 1 : p0;
+      const bool tr = part == 1 && target;   // the row operand: G^T
+      T a[2][2], x[NT][2];
 #pragma unroll
-        for (int r = 0; r < 2; ++r) {
-          if (tr)
-            block_frag<T, true>(G, n, i + r, kk, vec && i + r < nta, a[r][0], a[r][1]);
+      for (int r = 0; r < 2; ++r) {
+        if (tr)
+          block_frag<T, true>(G, n, i + r, kk, vec && i + r < nta, a[r][0], a[r][1]);
+        else
+          block_frag<T, false>(F, n, i + r, kk, vec && i + r < nta, a[r][0], a[r][1]);
+      }
+#pragma unroll
+      for (int j = 0; j < NT; ++j)
+        if (j <= jmax) {
+          if (part == 1)
+            block_frag<T, true>(G, n, j, kk, vec, x[j][0], x[j][1]);
           else
-            block_frag<T, false>(F, n, i + r, kk, vec && i + r < nta, a[r][0], a[r][1]);
+            block_frag<T, false>(F, n, j, kk, vec, x[j][0], x[j][1]);
         }
+#pragma unroll
+      for (int e = 0; e < 2; ++e)
 #pragma unroll
         for (int j = 0; j < NT; ++j)
           if (j <= jmax) {
-            if (part == 1)
-              block_frag<T, true>(G, n, j, kk, vec, x[j][0], x[j][1]);
-            else
-              block_frag<T, false>(F, n, j, kk, vec, x[j][0], x[j][1]);
+            mma_acc(acc[0][j][0], acc[0][j][1], (double)a[0][e], (double)x[j][e]);
+            mma_acc(acc[1][j][0], acc[1][j][1], (double)a[1][e], (double)x[j][e]);
           }
-#pragma unroll
-        for (int e = 0; e < 2; ++e)
-#pragma unroll
-          for (int j = 0; j < NT; ++j)
-            if (j <= jmax) {
-              mma_acc(acc[0][j][0], acc[0][j][1], (double)a[0][e], (double)x[j][e]);
-              mma_acc(acc[1][j][0], acc[1][j][1], (double)a[1][e], (double)x[j][e]);
-            }
-      }
     }
 #pragma unroll
     for (int r = 0; r < 2; ++r) {
