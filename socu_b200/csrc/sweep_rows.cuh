@@ -226,9 +226,10 @@ __device__ __forceinline__ void sweep_rows_body(const Group& grp, const Problem<
   for (int c0 = col0; c0 < cend; c0 += XC) {
     const int mc = min_i(XC, cend - c0), groups = (mc + 7) >> 3;
     if (c0 > col0) grp.sync();
-    // neighbours' vectors, zeros outside
+    // neighbours' vectors, zeros outside (KEEP's products run over all NT tiles: a zero operand
+    // does not cancel a NaN that an earlier kernel left in shared memory)
     if (P || Q) {
-      for (int e = grp.tid(); e < 8 * nta * 8 * groups; e += grp.threads()) {
+      for (int e = grp.tid(); e < 8 * (KEEP ? NT : nta) * 8 * groups; e += grp.threads()) {
         const int k = e / (8 * groups), c = e - k * (8 * groups);
         const bool in = k < n && c < mc;
         const long long o = (long long)k * m + c0 + c;
