@@ -403,22 +403,15 @@ inline bool use_inverse(int n) { return n <= 64; }
 // Block-row FP64 residual (n <= 128): 1, 2 or 4 eight-column groups of
 // right-hand sides per pass over the matrix blocks, by n_rhs.
 template <bool REFINE>
-cudaError_t launch_residual_rows(const RefineArgs& a, cudaStream_t st, bool pdl) {
+void launch_residual_rows(const RefineArgs& a, cudaStream_t st, bool pdl) {
   const int gr = residual_groups(a.m);
-  const size_t smem = smem_residual_x_elems(a.n, gr) * sizeof(double);
   const unsigned blocks = (unsigned)((long long)a.B * a.N), threads = (unsigned)residual_rows_threads(a.n, a.m);
-  cudaError_t e;
-  if (gr == 1) {
-    e = prepare(k_residual_rows<REFINE, 1>, smem);
-    if (e == cudaSuccess) launch(k_residual_rows<REFINE, 1>, blocks, threads, smem, st, pdl, a);
-  } else if (gr == 2) {
-    e = prepare(k_residual_rows<REFINE, 2>, smem);
-    if (e == cudaSuccess) launch(k_residual_rows<REFINE, 2>, blocks, threads, smem, st, pdl, a);
-  } else {
-    e = prepare(k_residual_rows<REFINE, 4>, smem);
-    if (e == cudaSuccess) launch(k_residual_rows<REFINE, 4>, blocks, threads, smem, st, pdl, a);
-  }
-  return e;
+  if (gr == 1)
+    launch(k_residual_rows<REFINE, 1>, blocks, threads, 0, st, pdl, a);
+  else if (gr == 2)
+    launch(k_residual_rows<REFINE, 2>, blocks, threads, 0, st, pdl, a);
+  else
+    launch(k_residual_rows<REFINE, 4>, blocks, threads, 0, st, pdl, a);
 }
 
 // Enqueue (or count, when st == nullptr and count != nullptr) the kernels of one op.
@@ -832,10 +825,9 @@ int refine_finish_round(const RefineArgs& a, cudaStream_t st, long long* count) 
     RefineArgs ac = a;
     ac.check_in_residual = 1;
     prof_begin(st, SOCU_KIND_RESIDUAL);
-    if (residual_uses_rows(a.n)) {
-      const cudaError_t e = launch_residual_rows<true>(ac, st, pdl);
-      if (e != cudaSuccess) return cuda_status(e);
-    } else
+    if (residual_uses_rows(a.n))
+      launch_residual_rows<true>(ac, st, pdl);
+    else
       launch(k_residual<true>, (unsigned)((long long)a.B * a.N * nrc), 256, smem_residual_elems(a.n) * sizeof(double),
              st, pdl, ac);
     prof_end(st);
@@ -863,8 +855,10 @@ int refine_prologue(const RefineArgs& a, cudaStream_t st, long long* count) {
     prof_end(st);
     const unsigned init_blocks = (unsigned)((long long)a.B * (a.N > a.S ? a.N : a.S));
     prof_begin(st, SOCU_KIND_REFINE_SETUP);
-    if (residual_uses_rows(a.n))
-      k_ref_init_rows<<<init_blocks, 256, sinit, st>>>(a);
+    if (a.n <= 64)
+      k_ref_init_rows<1><<<init_blocks, 256, sinit, st>>>(a);
+    else if (residual_uses_rows(a.n))
+      k_ref_init_rows<2><<<init_blocks, 256, sinit, st>>>(a);
     else
       k_ref_init<<<init_blocks, 256, 0, st>>>(a);
     prof_end(st);
@@ -1672,8 +1666,7 @@ int socu_block_tridiag_residual(const double* L, const double* E, const double* 
   a.B = d.B; a.N = d.N; a.n = d.n; a.m = d.m; a.S = d.S;
   const size_t sres = smem_residual_elems(d.n) * sizeof(double);
   if (residual_uses_rows(d.n)) {
-    e = launch_residual_rows<false>(a, static_cast<cudaStream_t>(stream), false);
-    if (e != cudaSuccess) return cuda_status(e);
+    launch_residual_rows<false>(a, static_cast<cudaStream_t>(stream), false);
   } else {
     e = prepare(k_residual<false>, sres);
     if (e != cudaSuccess) return cuda_status(e);

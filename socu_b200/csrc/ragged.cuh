@@ -305,8 +305,7 @@ __host__ __device__ inline long long rg_unit_bytes(int n, int es, bool refine, b
   if (w > v) v = w;
   if (u > v) v = u;
   if (refine) {
-    const long long r = 8 * smem_residual_rows_elems(n), i = 8 * smem_ref_init_elems(n, blocks ? rg_group_warps(n) : 1);
-    if (r > v) v = r;
+    const long long i = 8 * smem_ref_init_elems(n, blocks ? rg_group_warps(n) : 1);
     if (i > v) v = i;
   }
   return (v + 127) & ~127LL;
@@ -395,11 +394,11 @@ __device__ void rg_run(const RgArgs<T>& a, int ii, int ph, int chunk, unsigned c
   for (int u = u0 + gi; u < u1; u += BLOCKS ? kRgBlockWarps / gw : 1) {
     grp.sync();
     if (!kPlain && P.kind == kRgInit) {
-      if constexpr (!kPlain) ref_init_rows_body(grp, rg_refine_args(a, I, ii), 0, u, smem);
+      if constexpr (!kPlain) ref_init_rows_body<1>(grp, rg_refine_args(a, I, ii), 0, u, smem);
       continue;
     }
     if (!kPlain && P.kind == kRgRes) {
-      if constexpr (!kPlain) residual_rows_body<true, 1>(grp, rg_refine_args(a, I, ii), 0, u, smem);
+      if constexpr (!kPlain) residual_rows_body<true, 1>(grp, rg_refine_args(a, I, ii), 0, u);
       continue;
     }
     const int nt = rg_nt(I.n);

@@ -10,6 +10,8 @@
 // `active` flags, which the solver kernels take as their batch mask.
 #pragma once
 
+#include <type_traits>
+
 #include "sweep_rows.cuh"
 #include "update_rows.cuh"
 
@@ -316,32 +318,25 @@ constexpr int kResRowMaxN = 128;
 __host__ __device__ inline bool residual_uses_rows(int n) { return n <= kResRowMaxN; }
 
 // r_i = b_i - (D_i x_i + E_{i-1} x_{i-1} + E_i^T x_{i+1}) for the whole block
-// row, on FP64 tensor cores (mma.m8n8k4 .f64).  Per super-chunk of up to 32
-// right-hand sides the CTA stages x_{i-1}, x_i, x_{i+1} in shared memory
-// (stride 36: conflict-free B fragments; missing neighbours and columns as
-// zeros); the matrix fragments are read straight from global memory, each
-// element once per super-chunk, and multiplied into all (up to four) 8-column
-// groups of the chunk.  Warp task = one 8-row output tile: 3 blocks x
-// ceil(n/4) k-steps into independent accumulators (block x k parity x column
-// group).  Fragment layout: a0 = A[g][t], b0 = B[t][g], {c0, c1} = C[g][2t +
-// {0, 1}] (g = lane / 4, t = lane % 4).  D_i is symmetric from its lower
-// triangle: above the diagonal the transposed element is read.  Any
-// blockDim.x that is a multiple of 32 works.
-// Shared: 3 x n x kResXld doubles (smem_residual_x_elems).
-// GR = 8-column groups per super-chunk (1, 2 or 4, by the number of
-// right-hand sides): the super-chunk is 8 GR columns wide, staged with stride
-// 8 GR + 4 doubles (4 mod 16 for GR = 1 and 4; 20 for GR = 2).
+// row, on FP64 tensor cores (mma.m8n8k4 .f64), a warp per 8-row output tile.
+// The bound is latency: three blocks are read once and used m columns wide.  So every
+// operand goes straight from global memory into the registers that the products
+// take it from (column pairs as one 16-byte load: the two k-steps of eight columns
+// take the pair's first and second elements), whole tiles without bounds checks, at 64
+// registers, so that 32 warps' loads are in flight per SM; the vectors, which the
+// warps of a block share, come from L1.  Against vectors staged in shared memory and
+// bounds checked per element: refined solve of 1024 x (n = 64, m = 8) 540 -> 523 us, 512 ragged
+// systems 9.98 -> 8.87 ms (with the set-up below).  Two column tiles per step at 126
+// registers took 534 us, and requesting the blocks to L2 ahead of the vectors 526.
+// D_i is symmetric from its lower triangle: tiles right of the diagonal are read
+// transposed, the diagonal tile element by element.  Any blockDim.x that is a
+// multiple of 32 works.
+// GR = 8-column groups per pass over the blocks (1, 2 or 4, by the number of
+// right-hand sides).
 __host__ __device__ inline int residual_groups(int m) { return m <= 8 ? 1 : (m <= 16 ? 2 : 4); }
-__host__ __device__ inline long long smem_residual_x_elems(int n, int gr) { return 3LL * n * (8 * gr + 4); }
-// shared memory the ragged kernel reserves for its residual / set-up phases
-// (doubles): the one-group residual's x staging, which exceeds the set-up's 17 n
-__host__ __device__ inline long long smem_residual_rows_elems(int n) { return smem_residual_x_elems(n, 1); }
 template <bool REFINE, int GR, class Group>
-__device__ __forceinline__ void residual_rows_body(const Group& grp, const RefineArgs& a, int bi, int i, unsigned char* smem_raw) {
-  constexpr int kResXC = 8 * GR, kResXld = kResXC + 4;
+__device__ __forceinline__ void residual_rows_body(const Group& grp, const RefineArgs& a, int bi, int i) {
   __shared__ double red[32];
-  double* const xs0 = reinterpret_cast<double*>(smem_raw);
-  const int xstride = a.n * kResXld;   // x_{i-1}, x_i, x_{i+1} chunks back to back
   const int n = a.n, m = a.m, N = a.N;
   const long long nn = (long long)n * n;
   const double* D = a.L + ((long long)bi * N + i) * nn;
@@ -350,87 +345,108 @@ __device__ __forceinline__ void residual_rows_body(const Group& grp, const Refin
   const double* Ep = a.E + ((long long)bi * a.S + (hasP ? i : 0)) * nn;
   const long long vi = ((long long)bi * N + i) * n * m;
   const double* x1 = a.x + vi;
-  const int lane = threadIdx.x & 31, warp = grp.warp(), nw = grp.warps();
-  const int g = lane >> 2, t = lane & 3;
-  const int rts = (n + 7) >> 3;
+  const double* x0 = hasM ? x1 - n * m : x1;
+  const double* x2 = hasP ? x1 + n * m : x1;
+  const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  const int rts = (n + 7) >> 3, whole = n >> 3;
+  const bool pairs = (n & 1) == 0 && ((reinterpret_cast<unsigned long long>(D) | reinterpret_cast<unsigned long long>(Em)) & 15) == 0;
   double rmax = 0.0, xmax = 0.0;
-  for (int c0 = 0; c0 < m; c0 += kResXC) {
-    const int mc = min(kResXC, m - c0);
-    const int groups = (mc + 7) >> 3;
-    grp.sync();
-    for (int e = grp.tid(); e < 3 * n * kResXC; e += grp.threads()) {
-      const int j = e / (n * kResXC), rem = e - j * n * kResXC, k = rem / kResXC, c = rem - k * kResXC;
-      const bool ok = c < mc && (j == 1 || (j == 0 ? hasM : hasP));
-      xs0[j * xstride + k * kResXld + c] = ok ? x1[(long long)(j - 1) * n * m + (long long)k * m + c0 + c] : 0.0;
-    }
-    grp.sync();
-    for (int rt = warp; rt < rts; rt += nw) {
-      const int r0 = rt * 8, ra = r0 + g;
-      const bool rv = ra < n;
-      const int rr = rv ? ra : 0;
-      // accumulators per column group: block (D, E_{i-1}, E_i) x k-step parity
-      // (KP = 2 independent chains per block when there is one group; several
-      // groups already give the MMAs independent chains, and registers are short)
-      constexpr int KP = GR >= 2 ? 1 : 2;
-      double acc[GR][3 * KP][2];
+  for (int rt = grp.warp(); rt < rts; rt += grp.warps()) {
+    // rows past n repeat the last one and columns past m the last column: what they give is
+    // dropped.  Only the contraction's tail (k >= n) has to be zero.
+    const int r = 8 * rt + g, ra = min_i(r, n - 1);
+    const double *Dr = D + ra * n + 2 * t, *Dc = D + 2 * t * n + ra;   // rows; columns (D symmetric)
+    const double *Mr = Em + ra * n + 2 * t, *Pc = Ep + 2 * t * n + ra;
+    for (int c0 = 0; c0 < m; c0 += 8 * GR) {
+      const int groups = min_i(GR, (m - c0 + 7) >> 3);
+      int xo[GR];
+#pragma unroll
+      for (int q = 0; q < GR; ++q) xo[q] = 2 * t * m + min_i(c0 + 8 * q + g, m - 1);
+      // accumulators: column group x block (D, E_{i-1}, E_i)
+      double acc[GR][3][2];
 #pragma unroll
       for (int q = 0; q < GR; ++q)
 #pragma unroll
-        for (int u = 0; u < 3 * KP; ++u) acc[q][u][0] = acc[q][u][1] = 0.0;
-      // matrix fragments of one 8-column k-step (two m8n8k4 steps), loaded one
-      // k-step ahead of their products so the global loads overlap the MMAs
-      double fD[2], fM[2], fP[2];
-      auto load_step = [&](int k0) {
+        for (int u = 0; u < 3; ++u) acc[q][u][0] = acc[q][u][1] = 0.0;
+      auto products = [&](int kk, const double (&f)[3][2], bool ok0, bool ok1) {
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          const int k = k0 + 4 * h + t;
-          const bool kv = k < n;
-          const int kk = kv ? k : 0;
-          const bool av = rv && kv;
-          const double dv = kk <= rr ? D[rr * n + kk] : D[kk * n + rr];
-          fD[h] = av ? dv : 0.0;
-          fM[h] = (av && hasM) ? Em[rr * n + kk] : 0.0;
-          fP[h] = (av && hasP) ? Ep[kk * n + rr] : 0.0;
-        }
-      };
-      load_step(0);
-      for (int k0 = 0; k0 < n; k0 += 8) {
-        const double cD[2] = {fD[0], fD[1]}, cM[2] = {fM[0], fM[1]}, cP[2] = {fP[0], fP[1]};
-        if (k0 + 8 < n) load_step(k0 + 8);
+        for (int q = 0; q < GR; ++q) {
+          if (GR > 1 && q >= groups) break;
+          const int o = xo[q] + 8 * kk * m;
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          const int k = k0 + 4 * h + t;
-          const bool kv = k < n;
-          const int kk = kv ? k : 0;
-#pragma unroll
-          for (int q = 0; q < GR; ++q) {
-            if (q >= groups) break;
-            const int xo = kk * kResXld + 8 * q + g;
-            const double b1 = kv ? xs0[xstride + xo] : 0.0;
-            const double b0 = kv ? xs0[xo] : 0.0;
-            const double b2 = kv ? xs0[2 * xstride + xo] : 0.0;
-            const int u = KP == 2 ? h : 0;
-            dmma_8x8x4(acc[q][u][0], acc[q][u][1], cD[h], b1);
-            dmma_8x8x4(acc[q][KP + u][0], acc[q][KP + u][1], cM[h], b0);
-            dmma_8x8x4(acc[q][2 * KP + u][0], acc[q][2 * KP + u][1], cP[h], b2);
+          for (int e = 0; e < 2; ++e) {
+            const bool ok = e ? ok1 : ok0;
+            const double v1 = ok ? x1[o + e * m] : 0.0;
+            const double v0 = ok && hasM ? x0[o + e * m] : 0.0;
+            const double v2 = ok && hasP ? x2[o + e * m] : 0.0;
+            mma_acc(acc[q][0][0], acc[q][0][1], f[0][e], v1);
+            mma_acc(acc[q][1][0], acc[q][1][1], f[1][e], v0);
+            mma_acc(acc[q][2][0], acc[q][2][1], f[2][e], v2);
           }
         }
+      };
+      auto row_pair = [&](const double* q, double (&f)[2]) {
+        if (pairs) {
+          const double2 v = *reinterpret_cast<const double2*>(q);
+          f[0] = v.x;
+          f[1] = v.y;
+        } else {
+          f[0] = q[0];
+          f[1] = q[1];
+        }
+      };
+      // whole column tile kk; side < 0: left of the diagonal tile, > 0: right of it
+      auto step = [&](int kk, int side) {
+        double f[3][2] = {};
+        if (side < 0) {
+          row_pair(Dr + 8 * kk, f[0]);
+        } else if (side > 0) {
+          f[0][0] = Dc[8 * kk * n];
+          f[0][1] = Dc[8 * kk * n + n];
+        } else {
+#pragma unroll
+          for (int e = 0; e < 2; ++e) f[0][e] = 2 * t + e <= g ? Dr[8 * kk + e] : Dc[8 * kk * n + e * n];
+        }
+        if (hasM) row_pair(Mr + 8 * kk, f[1]);
+        if (hasP) {
+          f[2][0] = Pc[8 * kk * n];
+          f[2][1] = Pc[8 * kk * n + n];
+        }
+        products(kk, f, true, true);
+      };
+      const int left = min_i(rt, whole);
+#pragma unroll 1
+      for (int kk = 0; kk < left; ++kk) step(kk, -1);
+      if (rt < whole) step(rt, 0);
+#pragma unroll 1
+      for (int kk = rt + 1; kk < whole; ++kk) step(kk, 1);
+      if (whole < rts) {   // the tail, element by element
+        double f[3][2] = {};
+        bool ok[2];
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          const int k = 8 * whole + 2 * t + e;
+          ok[e] = k < n;
+          if (ok[e]) {
+            f[0][e] = k <= ra ? Dr[8 * whole + e] : Dc[8 * whole * n + e * n];
+            if (hasM) f[1][e] = Mr[8 * whole + e];
+            if (hasP) f[2][e] = Pc[8 * whole * n + e * n];
+          }
+        }
+        products(whole, f, ok[0], ok[1]);
       }
 #pragma unroll
       for (int q = 0; q < GR; ++q) {
         if (q >= groups) break;
 #pragma unroll
         for (int e = 0; e < 2; ++e) {
-          const int r = r0 + g, c = 8 * q + 2 * t + e;
-          if (r < n && c < mc) {
-            const long long o = vi + (long long)r * m + c0 + c;
-            double y = 0.0;
-#pragma unroll
-            for (int u = 0; u < 3 * KP; ++u) y += acc[q][u][e];
-            const double res = a.b[o] - y;
+          const int c = c0 + 8 * q + 2 * t + e;
+          if (r < n && c < m) {
+            const long long o = vi + (long long)r * m + c;
+            const double res = a.b[o] - (acc[q][0][e] + acc[q][1][e] + acc[q][2][e]);
             if (REFINE) {
               a.R32[o] = (float)res;
-              const double xv = xs0[xstride + r * kResXld + c];
+              const double xv = a.x[o];
               rmax = isfinite(res) ? fmax(rmax, fabs(res)) : __longlong_as_double(0x7ff0000000000000LL);
               xmax = isfinite(xv) ? fmax(xmax, fabs(xv)) : __longlong_as_double(0x7ff0000000000000LL);
             } else {
@@ -458,29 +474,31 @@ __host__ __device__ inline int residual_rows_threads(int n, int) {
 }
 
 template <bool REFINE, int GR>
-__global__ void __launch_bounds__(256, GR == 4 ? 2 : 3) k_residual_rows(RefineArgs a) {
-  pdl_wait();
-  pdl_trigger();
+__global__ void __launch_bounds__(256, GR == 1 ? 4 : 2) k_residual_rows(RefineArgs a) {
   const int bi = blockIdx.x / a.N;
   const int i = blockIdx.x - bi * a.N;
+  pdl_wait();
+  pdl_trigger();
   if (REFINE && !a.active[bi]) return;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  residual_rows_body<REFINE, GR>(BlockGroup{}, a, bi, i, smem_raw);
+  residual_rows_body<REFINE, GR>(BlockGroup{}, a, bi, i);
   if (REFINE) residual_arrive(a, bi, (unsigned)a.N);
 }
 
 // Refinement set-up for block row i (if i < N) and storage slot i (if i < S):
 // float copies of L_i and slot i, R32 = b_i, x_i = 0, ||b||_inf and the row
-// sums of |Psi| over block row i.  One streaming pass, no staging: warp w
-// takes rows w, w + nw, ... of L_i, E_{i-1} and E_i with coalesced loads
-// (lane owns columns lane, lane + 32, ...), writes the float copies, reduces
-// the row part of each row sum (lower(D) row, E_{i-1} row) with shuffles and
-// keeps per-lane column partials for the transposed parts (strict lower(D)
-// columns, E_i columns).  The warps' column partials are added in warp order
-// in shared memory (smem_ref_init_elems doubles), so the sums are deterministic.
+// sums of |Psi| over block row i.  One streaming pass, no staging: a row of
+// L_i, E_{i-1} and E_i goes to 2^ls lanes of a warp, a column pair each (and
+// the pair 64 further for n > 64: H = 2), the loads of 4 / H rows requested
+// together.  The bound is instructions (0.5 per cycle and scheduler): with bounds checked
+// per element 1024 x (n = 64) took 36 us, with whole pairs and rows as cases of their own
+// 30, of which 105 MB of HBM traffic would take 16.  The lanes write the float copies,
+// reduce the row part of each row sum (lower(D) row, E_{i-1} row) with shuffles and keep column partials for the transposed
+// parts (strict lower(D) columns, E_i columns), which are added in warp order
+// in shared memory (smem_ref_init_elems doubles): the sums are deterministic.
 __host__ __device__ inline long long smem_ref_init_elems(int n, int warps = 8) { return 2LL * warps * n + n; }
-template <class Group>
+template <int H, class Group>
 __device__ __forceinline__ void ref_init_rows_body(const Group& grp, const RefineArgs& a, int bi, int i, unsigned char* smem_raw) {
+  constexpr int R = 4 / H;
   __shared__ double red[32];
   const int n = a.n, m = a.m, N = a.N;
   const long long nn = (long long)n * n;
@@ -500,6 +518,10 @@ __device__ __forceinline__ void ref_init_rows_body(const Group& grp, const Refin
   const double* Ep = a.E + ((long long)bi * a.S + (hasP ? i : 0)) * nn;
   float* L32 = a.L32 + ((long long)bi * N + i) * nn;
   float* E32 = a.E32 + ((long long)bi * a.S + (hasS ? i : 0)) * nn;
+  const bool pairs = (n & 1) == 0 &&
+                     ((reinterpret_cast<unsigned long long>(Lg) | reinterpret_cast<unsigned long long>(Em) |
+                       reinterpret_cast<unsigned long long>(Ep)) & 15) == 0 &&
+                     ((reinterpret_cast<unsigned long long>(L32) | reinterpret_cast<unsigned long long>(E32)) & 7) == 0;
   const long long vo = ((long long)bi * N + i) * n * m;
   double bmax = 0.0;
   for (int e = grp.tid(); e < n * m; e += grp.threads()) {
@@ -508,44 +530,93 @@ __device__ __forceinline__ void ref_init_rows_body(const Group& grp, const Refin
     a.x[vo + e] = 0.0;
     bmax = fmax(bmax, fabs(v));
   }
-  constexpr int H = kResRowMaxN / 32;   // columns per lane
-  double cl[H], ce[H];
+  int ls = 5;
+  if (H == 1)
+    while (ls > 0 && (1 << ls) >= n) --ls;   // 2^ls column pairs cover a row: 2^(ls + 1) >= n
+  const int lpr = 1 << ls, sub = lane >> ls, step = nw * (32 >> ls), cb = 2 * (lane & (lpr - 1));
+  double cl[H][2], ce[H][2];
 #pragma unroll
-  for (int h = 0; h < H; ++h) cl[h] = ce[h] = 0.0;
-  for (int r = warp; r < n; r += nw) {
-    double vl[H], vm[H], vp[H];
+  for (int h = 0; h < H; ++h) cl[h][0] = cl[h][1] = ce[h][0] = ce[h][1] = 0.0;
+  // PAIRS: a row is whole pairs; ALL: and every lane has one
+  auto rows = [&](auto pairs_c, auto all_c) {
+    constexpr bool PAIRS = decltype(pairs_c)::value, ALL = decltype(all_c)::value;
+    auto load = [&](const double* M, int o, bool ok0, bool ok1) {
+      double2 v = make_double2(0.0, 0.0);
+      if (PAIRS) {
+        if (ok0) v = *reinterpret_cast<const double2*>(M + o);
+      } else {
+        if (ok0) v.x = M[o];
+        if (ok1) v.y = M[o + 1];
+      }
+      return v;
+    };
+    auto store = [&](float* M, int o, bool ok0, bool ok1, double2 v) {
+      if (PAIRS) {
+        if (ok0) *reinterpret_cast<float2*>(M + o) = make_float2((float)v.x, (float)v.y);
+      } else {
+        if (ok0) M[o] = (float)v.x;
+        if (ok1) M[o + 1] = (float)v.y;
+      }
+    };
+    // (the bound is the warp's: the shuffles need all lanes)
+#pragma unroll 1
+    for (int rb = warp * (32 >> ls); rb < n; rb += R * step) {
+      double2 vl[R][H], vm[R][H], vp[R][H];
 #pragma unroll
-    for (int h = 0; h < H; ++h) {
-      const int c = lane + 32 * h;
-      const bool ok = c < n;
-      const int o = r * n + (ok ? c : 0);
-      vl[h] = ok ? Lg[o] : 0.0;
-      vm[h] = (ok && hasM) ? Em[o] : 0.0;
-      vp[h] = (ok && hasP) ? Ep[o] : 0.0;
-    }
-    double part = 0.0;
+      for (int u = 0; u < R; ++u)
 #pragma unroll
-    for (int h = 0; h < H; ++h) {
-      const int c = lane + 32 * h;
-      if (c < n) {
-        L32[r * n + c] = (float)vl[h];
-        if (hasS) E32[r * n + c] = (float)vp[h];
-        part += (c <= r ? fabs(vl[h]) : 0.0) + fabs(vm[h]);
-        cl[h] += c < r ? fabs(vl[h]) : 0.0;   // D(c, r) = L[r][c] for r > c: row c's transposed part
-        ce[h] += fabs(vp[h]);                 // E_i^T couples row c to x_{i+1}: column sums of E_i
+        for (int h = 0; h < H; ++h) {
+          const int r = rb + u * step + sub, c = cb + 64 * h, o = r * n + c;
+          const bool ok0 = r < n && (ALL || c < n), ok1 = r < n && c + 1 < n;
+          vl[u][h] = load(Lg, o, ok0, ok1);
+          vm[u][h] = load(Em, o, ok0 && hasM, ok1 && hasM);
+          vp[u][h] = load(Ep, o, ok0 && hasP, ok1 && hasP);
+        }
+#pragma unroll
+      for (int u = 0; u < R; ++u) {
+        const int r = rb + u * step + sub;
+        double part = 0.0;
+#pragma unroll
+        for (int h = 0; h < H; ++h) {
+          const int c = cb + 64 * h, o = r * n + c;
+          const bool ok0 = r < n && (ALL || c < n), ok1 = r < n && c + 1 < n;
+          const double2 l = vl[u][h], e = vp[u][h];
+          store(L32, o, ok0, ok1, l);
+          store(E32, o, ok0 && hasS, ok1 && hasS, e);
+          // D(c, r) = L[r][c] for r > c: row c's transposed part.  E_i^T couples row c to x_{i+1}:
+          // column sums of E_i
+          const double l0 = c < r ? fabs(l.x) : 0.0, l1 = c + 1 < r ? fabs(l.y) : 0.0;
+          part += (c == r ? fabs(l.x) : l0) + (c + 1 == r ? fabs(l.y) : l1) + fabs(vm[u][h].x) + fabs(vm[u][h].y);
+          cl[h][0] += l0;
+          cl[h][1] += l1;
+          ce[h][0] += fabs(e.x);
+          ce[h][1] += fabs(e.y);
+        }
+        for (int o = lpr >> 1; o > 0; o >>= 1) part += __shfl_xor_sync(kFull, part, o);
+        if ((lane & (lpr - 1)) == 0 && r < n) rs[r] = part;
       }
     }
-    for (int o = 16; o > 0; o >>= 1) part += __shfl_xor_sync(kFull, part, o);
-    if (lane == 0) rs[r] = part;
-  }
+  };
+  if (pairs && n == 2 * H * lpr)
+    rows(std::true_type{}, std::true_type{});
+  else if (pairs)
+    rows(std::true_type{}, std::false_type{});
+  else
+    rows(std::false_type{}, std::false_type{});
 #pragma unroll
-  for (int h = 0; h < H; ++h) {
-    const int c = lane + 32 * h;
-    if (c < n) {
-      colp[(warp * 2 + 0) * n + c] = cl[h];
-      colp[(warp * 2 + 1) * n + c] = ce[h];
+  for (int h = 0; h < H; ++h)
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+      for (int o = lpr; o < 32; o <<= 1) {
+        cl[h][e] += __shfl_xor_sync(kFull, cl[h][e], o);
+        ce[h][e] += __shfl_xor_sync(kFull, ce[h][e], o);
+      }
+      const int c = cb + 64 * h + e;
+      if (sub == 0 && c < n) {
+        colp[(warp * 2 + 0) * n + c] = cl[h][e];
+        colp[(warp * 2 + 1) * n + c] = ce[h][e];
+      }
     }
-  }
   grp.sync();
   double rmax = 0.0;
   for (int r = grp.tid(); r < n; r += grp.threads()) {
@@ -561,7 +632,8 @@ __device__ __forceinline__ void ref_init_rows_body(const Group& grp, const Refin
   }
 }
 
-static __global__ void __launch_bounds__(256) k_ref_init_rows(RefineArgs a) {
+template <int H>
+__global__ void __launch_bounds__(256) k_ref_init_rows(RefineArgs a) {
   pdl_wait();
   pdl_trigger();
   const int per = a.N > a.S ? a.N : a.S;
@@ -569,7 +641,7 @@ static __global__ void __launch_bounds__(256) k_ref_init_rows(RefineArgs a) {
   const int i = blockIdx.x - bi * per;
   if (a.mask != nullptr && a.mask[bi] == 0) return;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  ref_init_rows_body(BlockGroup{}, a, bi, i, smem_raw);
+  ref_init_rows_body<H>(BlockGroup{}, a, bi, i, smem_raw);
 }
 
 // ---------------------------------------------------------------------------
