@@ -403,15 +403,14 @@ inline bool use_inverse(int n) { return n <= 64; }
 // Block-row FP64 residual (n <= 128): 1, 2 or 4 eight-column groups of
 // right-hand sides per pass over the matrix blocks, by n_rhs.
 template <bool REFINE>
-void launch_residual_rows(const RefineArgs& a, cudaStream_t st, bool pdl) {
+cudaError_t launch_residual_rows(const RefineArgs& a, cudaStream_t st, bool pdl) {
   const int gr = residual_groups(a.m);
+  const size_t smem = smem_residual_x_elems(a.n, gr) * sizeof(double);
   const unsigned blocks = (unsigned)((long long)a.B * a.N), threads = (unsigned)residual_rows_threads(a.n, a.m);
-  if (gr == 1)
-    launch(k_residual_rows<REFINE, 1>, blocks, threads, 0, st, pdl, a);
-  else if (gr == 2)
-    launch(k_residual_rows<REFINE, 2>, blocks, threads, 0, st, pdl, a);
-  else
-    launch(k_residual_rows<REFINE, 4>, blocks, threads, 0, st, pdl, a);
+  void (*k)(RefineArgs) = gr == 1 ? k_residual_rows<REFINE, 1> : (gr == 2 ? k_residual_rows<REFINE, 2> : k_residual_rows<REFINE, 4>);
+  const cudaError_t e = prepare(k, smem);
+  if (e == cudaSuccess) launch(k, blocks, threads, smem, st, pdl, a);
+  return e;
 }
 
 // Enqueue (or count, when st == nullptr and count != nullptr) the kernels of one op.
@@ -825,9 +824,10 @@ int refine_finish_round(const RefineArgs& a, cudaStream_t st, long long* count) 
     RefineArgs ac = a;
     ac.check_in_residual = 1;
     prof_begin(st, SOCU_KIND_RESIDUAL);
-    if (residual_uses_rows(a.n))
-      launch_residual_rows<true>(ac, st, pdl);
-    else
+    if (residual_uses_rows(a.n)) {
+      const cudaError_t e = launch_residual_rows<true>(ac, st, pdl);
+      if (e != cudaSuccess) return cuda_status(e);
+    } else
       launch(k_residual<true>, (unsigned)((long long)a.B * a.N * nrc), 256, smem_residual_elems(a.n) * sizeof(double),
              st, pdl, ac);
     prof_end(st);
@@ -866,14 +866,11 @@ int refine_prologue(const RefineArgs& a, cudaStream_t st, long long* count) {
     if (e != cudaSuccess) return cuda_status(e);
   }
   long long c = 0, cr = 0;
-  // the float factor of the mixed solve takes its Schur updates on the tcgen05
-  // tensor cores for 64 < n <= 128 unless the tuned table says otherwise: the
-  // 3xTF32 products cost accuracy the FP64 refinement wins back (measured at
-  // N=16384, n=128, m=32: factor 27.0 -> 23.9 ms, still two rounds)
-  socu_tuning mixed{};
-  if (a.n > 64 && update_tc_ok(a.n) && tuning_lookup(SOCU_FLOAT32, a.n, a.m).update_tensor_cores == 0)
-    mixed.update_tensor_cores = 1;
-  int s = enqueue<float>(SOCU_OP_FACTOR_AND_SOLVE, pf, st, run ? nullptr : &c, use_inverse(a.n), &mixed);
+  // Schur updates as in any float factor (the tuned table may put them on the tcgen05 tensor
+  // cores): measured against those at N = 2048, n = 128: m = 32 5.09 / 5.07 ms, m = 1 3.15 / 3.19;
+  // N = 1024, n = 96, m = 8 1.25 / 1.39; N = 64, n = 128, m = 8 0.55 / 0.68; N = 1024, n = 72,
+  // m = 4 1.07 / 1.07, with eta after the same two rounds 10 to 100 times smaller.
+  int s = enqueue<float>(SOCU_OP_FACTOR_AND_SOLVE, pf, st, run ? nullptr : &c, use_inverse(a.n));
   if (s != SOCU_OK) return s;
   s = refine_finish_round(a, st, run ? nullptr : &cr);
   if (count) *count = 2 + c + cr;
@@ -1666,7 +1663,8 @@ int socu_block_tridiag_residual(const double* L, const double* E, const double* 
   a.B = d.B; a.N = d.N; a.n = d.n; a.m = d.m; a.S = d.S;
   const size_t sres = smem_residual_elems(d.n) * sizeof(double);
   if (residual_uses_rows(d.n)) {
-    launch_residual_rows<false>(a, static_cast<cudaStream_t>(stream), false);
+    e = launch_residual_rows<false>(a, static_cast<cudaStream_t>(stream), false);
+    if (e != cudaSuccess) return cuda_status(e);
   } else {
     e = prepare(k_residual<false>, sres);
     if (e != cudaSuccess) return cuda_status(e);

@@ -398,7 +398,7 @@ __device__ void rg_run(const RgArgs<T>& a, int ii, int ph, int chunk, unsigned c
       continue;
     }
     if (!kPlain && P.kind == kRgRes) {
-      if constexpr (!kPlain) residual_rows_body<true, 1>(grp, rg_refine_args(a, I, ii), 0, u);
+      if constexpr (!kPlain) residual_rows_body<true>(grp, rg_refine_args(a, I, ii), 0, u);
       continue;
     }
     const int nt = rg_nt(I.n);

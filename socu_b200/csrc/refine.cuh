@@ -331,10 +331,10 @@ __host__ __device__ inline bool residual_uses_rows(int n) { return n <= kResRowM
 // D_i is symmetric from its lower triangle: tiles right of the diagonal are read
 // transposed, the diagonal tile element by element.  Any blockDim.x that is a
 // multiple of 32 works.
-// GR = 8-column groups per pass over the blocks (1, 2 or 4, by the number of
-// right-hand sides).
+// Up to eight right-hand sides a pass; more of them take the kernel below.
+// 8-column groups per pass over the blocks
 __host__ __device__ inline int residual_groups(int m) { return m <= 8 ? 1 : (m <= 16 ? 2 : 4); }
-template <bool REFINE, int GR, class Group>
+template <bool REFINE, class Group>
 __device__ __forceinline__ void residual_rows_body(const Group& grp, const RefineArgs& a, int bi, int i) {
   __shared__ double red[32];
   const int n = a.n, m = a.m, N = a.N;
@@ -357,32 +357,20 @@ __device__ __forceinline__ void residual_rows_body(const Group& grp, const Refin
     const int r = 8 * rt + g, ra = min_i(r, n - 1);
     const double *Dr = D + ra * n + 2 * t, *Dc = D + 2 * t * n + ra;   // rows; columns (D symmetric)
     const double *Mr = Em + ra * n + 2 * t, *Pc = Ep + 2 * t * n + ra;
-    for (int c0 = 0; c0 < m; c0 += 8 * GR) {
-      const int groups = min_i(GR, (m - c0 + 7) >> 3);
-      int xo[GR];
-#pragma unroll
-      for (int q = 0; q < GR; ++q) xo[q] = 2 * t * m + min_i(c0 + 8 * q + g, m - 1);
-      // accumulators: column group x block (D, E_{i-1}, E_i)
-      double acc[GR][3][2];
-#pragma unroll
-      for (int q = 0; q < GR; ++q)
-#pragma unroll
-        for (int u = 0; u < 3; ++u) acc[q][u][0] = acc[q][u][1] = 0.0;
+    for (int c0 = 0; c0 < m; c0 += 8) {
+      const int xo = 2 * t * m + min_i(c0 + g, m - 1);
+      double acc[3][2] = {};   // by block (D, E_{i-1}, E_i)
       auto products = [&](int kk, const double (&f)[3][2], bool ok0, bool ok1) {
+        const int o = xo + 8 * kk * m;
 #pragma unroll
-        for (int q = 0; q < GR; ++q) {
-          if (GR > 1 && q >= groups) break;
-          const int o = xo[q] + 8 * kk * m;
-#pragma unroll
-          for (int e = 0; e < 2; ++e) {
-            const bool ok = e ? ok1 : ok0;
-            const double v1 = ok ? x1[o + e * m] : 0.0;
-            const double v0 = ok && hasM ? x0[o + e * m] : 0.0;
-            const double v2 = ok && hasP ? x2[o + e * m] : 0.0;
-            mma_acc(acc[q][0][0], acc[q][0][1], f[0][e], v1);
-            mma_acc(acc[q][1][0], acc[q][1][1], f[1][e], v0);
-            mma_acc(acc[q][2][0], acc[q][2][1], f[2][e], v2);
-          }
+        for (int e = 0; e < 2; ++e) {
+          const bool ok = e ? ok1 : ok0;
+          const double v1 = ok ? x1[o + e * m] : 0.0;
+          const double v0 = ok && hasM ? x0[o + e * m] : 0.0;
+          const double v2 = ok && hasP ? x2[o + e * m] : 0.0;
+          mma_acc(acc[0][0], acc[0][1], f[0][e], v1);
+          mma_acc(acc[1][0], acc[1][1], f[1][e], v0);
+          mma_acc(acc[2][0], acc[2][1], f[2][e], v2);
         }
       };
       auto row_pair = [&](const double* q, double (&f)[2]) {
@@ -436,17 +424,131 @@ __device__ __forceinline__ void residual_rows_body(const Group& grp, const Refin
         products(whole, f, ok[0], ok[1]);
       }
 #pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        const int c = c0 + 2 * t + e;
+        if (r < n && c < m) {
+          const long long o = vi + (long long)r * m + c;
+          const double res = a.b[o] - (acc[0][e] + acc[1][e] + acc[2][e]);
+          if (REFINE) {
+            a.R32[o] = (float)res;
+            const double xv = a.x[o];
+            rmax = isfinite(res) ? fmax(rmax, fabs(res)) : __longlong_as_double(0x7ff0000000000000LL);
+            xmax = isfinite(xv) ? fmax(xmax, fabs(xv)) : __longlong_as_double(0x7ff0000000000000LL);
+          } else {
+            a.rout[o] = res;
+          }
+        }
+      }
+    }
+  }
+  if (REFINE) {
+    const double rm = group_max(grp, rmax, red);
+    const double xm = group_max(grp, xmax, red);
+    if (grp.tid() == 0) {
+      atomic_max_pos(&a.st[bi].rnorm, rm);
+      atomic_max_pos(&a.st[bi].xnorm, xm);
+    }
+  }
+}
+
+// The same for more than eight right-hand sides: 8 GR columns of the three vectors are staged
+// in shared memory (stride 8 GR + 4 doubles: 4 mod 16 at GR = 4, 20 at GR = 2) and every matrix
+// fragment, read one k-step ahead, feeds all GR column groups.  Reading the vectors straight
+// from global memory as above took 5.1 ms a launch at N = 16384, n = 128, m = 32, this 3.4:
+// every warp reads 3 n x 8 GR values, which L1 does not serve at the products' pace.
+__host__ __device__ inline long long smem_residual_x_elems(int n, int gr) { return gr == 1 ? 0 : 3LL * n * (8 * gr + 4); }
+template <bool REFINE, int GR>
+__device__ __forceinline__ void residual_staged_body(const RefineArgs& a, int bi, int i, unsigned char* smem_raw) {
+  const BlockGroup grp{};
+  constexpr int kResXC = 8 * GR, kResXld = kResXC + 4;
+  __shared__ double red[32];
+  double* const xs0 = reinterpret_cast<double*>(smem_raw);
+  const int xstride = a.n * kResXld;   // x_{i-1}, x_i, x_{i+1} chunks back to back
+  const int n = a.n, m = a.m, N = a.N;
+  const long long nn = (long long)n * n;
+  const double* D = a.L + ((long long)bi * N + i) * nn;
+  const bool hasM = i > 0, hasP = i < N - 1;
+  const double* Em = a.E + ((long long)bi * a.S + (hasM ? i - 1 : 0)) * nn;
+  const double* Ep = a.E + ((long long)bi * a.S + (hasP ? i : 0)) * nn;
+  const long long vi = ((long long)bi * N + i) * n * m;
+  const double* x1 = a.x + vi;
+  const int lane = threadIdx.x & 31, warp = grp.warp(), nw = grp.warps();
+  const int g = lane >> 2, t = lane & 3;
+  const int rts = (n + 7) >> 3;
+  double rmax = 0.0, xmax = 0.0;
+  for (int c0 = 0; c0 < m; c0 += kResXC) {
+    const int mc = min(kResXC, m - c0);
+    const int groups = (mc + 7) >> 3;
+    grp.sync();
+    for (int e = grp.tid(); e < 3 * n * kResXC; e += grp.threads()) {
+      const int j = e / (n * kResXC), rem = e - j * n * kResXC, k = rem / kResXC, c = rem - k * kResXC;
+      const bool ok = c < mc && (j == 1 || (j == 0 ? hasM : hasP));
+      xs0[j * xstride + k * kResXld + c] = ok ? x1[(long long)(j - 1) * n * m + (long long)k * m + c0 + c] : 0.0;
+    }
+    grp.sync();
+    for (int rt = warp; rt < rts; rt += nw) {
+      const int r0 = rt * 8, ra = r0 + g;
+      const bool rv = ra < n;
+      const int rr = rv ? ra : 0;
+      // accumulators: column group x block (D, E_{i-1}, E_i)
+      double acc[GR][3][2];
+#pragma unroll
+      for (int q = 0; q < GR; ++q)
+#pragma unroll
+        for (int u = 0; u < 3; ++u) acc[q][u][0] = acc[q][u][1] = 0.0;
+      // matrix fragments of one 8-column k-step (two m8n8k4 steps), loaded one
+      // k-step ahead of their products so the global loads overlap the MMAs
+      double fD[2], fM[2], fP[2];
+      auto load_step = [&](int k0) {
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const int k = k0 + 4 * h + t;
+          const bool kv = k < n;
+          const int kk = kv ? k : 0;
+          const bool av = rv && kv;
+          const double dv = kk <= rr ? D[rr * n + kk] : D[kk * n + rr];
+          fD[h] = av ? dv : 0.0;
+          fM[h] = (av && hasM) ? Em[rr * n + kk] : 0.0;
+          fP[h] = (av && hasP) ? Ep[kk * n + rr] : 0.0;
+        }
+      };
+      load_step(0);
+      for (int k0 = 0; k0 < n; k0 += 8) {
+        const double cD[2] = {fD[0], fD[1]}, cM[2] = {fM[0], fM[1]}, cP[2] = {fP[0], fP[1]};
+        if (k0 + 8 < n) load_step(k0 + 8);
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const int k = k0 + 4 * h + t;
+          const bool kv = k < n;
+          const int kk = kv ? k : 0;
+#pragma unroll
+          for (int q = 0; q < GR; ++q) {
+            if (q >= groups) break;
+            const int xo = kk * kResXld + 8 * q + g;
+            const double b1 = kv ? xs0[xstride + xo] : 0.0;
+            const double b0 = kv ? xs0[xo] : 0.0;
+            const double b2 = kv ? xs0[2 * xstride + xo] : 0.0;
+            dmma_8x8x4(acc[q][0][0], acc[q][0][1], cD[h], b1);
+            dmma_8x8x4(acc[q][1][0], acc[q][1][1], cM[h], b0);
+            dmma_8x8x4(acc[q][2][0], acc[q][2][1], cP[h], b2);
+          }
+        }
+      }
+#pragma unroll
       for (int q = 0; q < GR; ++q) {
         if (q >= groups) break;
 #pragma unroll
         for (int e = 0; e < 2; ++e) {
-          const int c = c0 + 8 * q + 2 * t + e;
-          if (r < n && c < m) {
-            const long long o = vi + (long long)r * m + c;
-            const double res = a.b[o] - (acc[q][0][e] + acc[q][1][e] + acc[q][2][e]);
+          const int r = r0 + g, c = 8 * q + 2 * t + e;
+          if (r < n && c < mc) {
+            const long long o = vi + (long long)r * m + c0 + c;
+            double y = 0.0;
+#pragma unroll
+            for (int u = 0; u < 3; ++u) y += acc[q][u][e];
+            const double res = a.b[o] - y;
             if (REFINE) {
               a.R32[o] = (float)res;
-              const double xv = a.x[o];
+              const double xv = xs0[xstride + r * kResXld + c];
               rmax = isfinite(res) ? fmax(rmax, fabs(res)) : __longlong_as_double(0x7ff0000000000000LL);
               xmax = isfinite(xv) ? fmax(xmax, fabs(xv)) : __longlong_as_double(0x7ff0000000000000LL);
             } else {
@@ -474,13 +576,18 @@ __host__ __device__ inline int residual_rows_threads(int n, int) {
 }
 
 template <bool REFINE, int GR>
-__global__ void __launch_bounds__(256, GR == 1 ? 4 : 2) k_residual_rows(RefineArgs a) {
+__global__ void __launch_bounds__(256, GR == 1 ? 4 : (GR == 2 ? 3 : 2)) k_residual_rows(RefineArgs a) {
   const int bi = blockIdx.x / a.N;
   const int i = blockIdx.x - bi * a.N;
   pdl_wait();
   pdl_trigger();
   if (REFINE && !a.active[bi]) return;
-  residual_rows_body<REFINE, GR>(BlockGroup{}, a, bi, i);
+  if constexpr (GR == 1) {
+    residual_rows_body<REFINE>(BlockGroup{}, a, bi, i);
+  } else {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    residual_staged_body<REFINE, GR>(a, bi, i, smem_raw);
+  }
   if (REFINE) residual_arrive(a, bi, (unsigned)a.N);
 }
 

@@ -33,7 +33,7 @@ __device__ __forceinline__ uint32_t saddr(const void* p) {
 }
 
 // Error word of the asynchronous units on one device: 1 a tensor-core wait
-// ran out, 2 a TMA copy wait ran out (that kernel skipped its result).
+// ran out (that kernel skipped its result).
 static __device__ int g_tc_error;   // one per translation unit; socu_tc_error reads them all
 
 // ---- instruction / shared-memory descriptors --------------------------------
