@@ -44,20 +44,17 @@ def storage_len(N):
 
 
 RAGGED_COUNT, RAGGED_SEED = 4096, 0
-# DRAM bytes (read + write) per k_bwd<float, resident, inverse> launch, averaged
-# over one backward sweep of this workload, from the ncu capture summarised in
-# profiles/k_bwd_f32_inverse_sweep_N1024_n64_m8.md
-TRAFFIC_BYTES = 5057908
-TRAFFIC_NOTE = "ncu dram__bytes_read.sum + dram__bytes_write.sum, profiles/k_bwd_f32_inverse_sweep_N1024_n64_m8.md"
-# DRAM bytes (read + write) per k_node<float, y, inverse> launch of a float
-# factor_and_solve of this shape, averaged over its 11 levels: ncu capture of
-# `bench.py --ncu-case node` (4 systems, so that the float blocks exceed L2),
-# 254.1 MB over the 11 launches of one pass, per system
-# (profiles/k_node_f32_levels_N1024_n64_m8_B4.md)
-NODE_TRAFFIC_BYTES = 254.13e6 / 4 / 11
-NODE_TRAFFIC_NOTE = ("ncu dram__bytes_read.sum + dram__bytes_write.sum of the 11 k_node<float,1,1,wt> launches of "
-                     "bench.py --ncu-case node (4 systems, inputs > L2), per system and launch; "
-                     "profiles/k_node_f32_levels_N1024_n64_m8_B4.md")
+# DRAM bytes (read + write) per launch of the float level node and of the float
+# backward sweep of a factor_and_solve of this shape, averaged over its 11
+# levels: ncu capture of `bench.py --ncu-case node` (4 systems, so that the
+# float blocks exceed L2), 246.4 and 201.2 MB over the 11 launches, per system
+# (profiles/rows_f32_N1024_n64_m8_B4.md)
+NODE_TRAFFIC_BYTES = 246.40e6 / 4 / 11
+TRAFFIC_BYTES = 201.16e6 / 4 / 11
+TRAFFIC_NOTE = ("ncu dram__bytes_read.sum + dram__bytes_write.sum of the 11 backward launches of "
+                "bench.py --ncu-case node (4 systems, inputs > L2), per system and launch; "
+                "profiles/rows_f32_N1024_n64_m8_B4.md")
+NODE_TRAFFIC_NOTE = TRAFFIC_NOTE.replace("backward", "k_node_rows")
 RAGGED_WORKLOAD = ("4096 independent systems, N ~ U{8..256}, n in {8,16,32,48}, m in {1,4}, shift=10, "
                    "instance i seeded with 0 + i, one persistent launch per solve")
 
@@ -524,7 +521,7 @@ def run_ours(args, rank, world, local_rank):
         "config": dict(workload_config(), parallelism=f"replicas x{world} (one system per GPU)"),
         "fp64_plain": {"value": world / sec_plain, "unit": "solves/s", "ms_per_step": sec_plain * 1e3,
                        "backward_error": eta_plain, "forward_error": fwd_plain,
-                       "roofline": {"kernel": "FP64 factor (k_node<double> + k_update<double>, graph-launched)",
+                       "roofline": {"kernel": "FP64 factor (k_node_rows<double> + k_update_rows<double>, graph-launched)",
                                     "bound": "fp64 tensor (DMMA)", "achieved": fac64_tf, "peak": dmma_tf,
                                     "unit": "TFLOP/s", "frac": fac64_tf / dmma_tf,
                                     "peak_source": "measured in this run: socu_dmma_peak_launch (register-only "
@@ -539,7 +536,7 @@ def run_ours(args, rank, world, local_rank):
         "factor_flops_fp": fac_flops,
         "phases": dict(budget(phases_mixed), note="one eager run with CUDA events around every kernel, "
                        f"{abs(iters)} rounds; events add gaps, so the sum exceeds ms_per_step"),
-        "roofline": {"kernel": f"k_node<float> (level nodes of the mixed solve: potrf + coupling solves + forward "
+        "roofline": {"kernel": f"k_node_rows<float> (level nodes of the mixed solve: potrf + coupling solves + forward "
                                f"step, averaged over its launches; the kernel with the most device time in the "
                                f"mixed solve's ncu launch list; this run's eager profile: node "
                                f"{node_ms:.3f} ms in {node_launches} launches, backward sweeps "
@@ -551,7 +548,7 @@ def run_ours(args, rank, world, local_rank):
                      "traffic": NODE_TRAFFIC_BYTES, "traffic_source": NODE_TRAFFIC_NOTE,
                      "algorithmic_flops_per_launch": nf / node_launches,
                      "ms_per_launch": node_ms / node_launches},
-        "roofline_sweep": {"kernel": "k_bwd<float, resident, inverse> (backward sweep of the mixed solve; "
+        "roofline_sweep": {"kernel": "k_sweep_rows<float, backward, inverse> (backward sweep of the mixed solve; "
                                      f"{sweep_launches} launches per sweep, averaged)", "bound": "hbm",
                            "achieved": bwd_ach, "peak": hbm_peak, "unit": "GB/s", "frac": bwd_ach / hbm_peak,
                            "peak_source": peak_src, "traffic": TRAFFIC_BYTES,

@@ -136,18 +136,18 @@ int socu_launch_run(socu_launch_t launch, void* stream);
 /* ---- launch settings and autotuning (no counterpart in the reference, whose
  * launches take block_dim / block_size per call,
  * socu/block_tridiag_solver.py:739-747, 776-781) ----
- * Every field 0 = not set (built-in heuristic).  node/update/sweep_threads:
- * threads per CTA of the node, Schur-update and sweep kernels (64, 128 or
- * 256).  sweep_tensor_cores: float sweeps on inverse-carrying factors use FP64
- * tensor-core (1) or SIMT (2) products.  update_tile: output tile of the
- * blocked Schur update for n > 64 (16 or 32; the reference's block_size).
+ * Every field 0 = not set (built-in heuristic).  node/update/sweep_threads (64,
+ * 128 or 256), sweep_tensor_cores (1 or 2) and update_tile (16 or 32) are
+ * checked and kept, and choose nothing: the node, Schur-update and sweep kernels
+ * have one warp per 8-row tile and one product path.
  * ragged_units: level nodes per task chunk of a ragged batch (1..64).
  * update_tensor_cores: Schur updates of float factors (n <= 128) on the
  * tcgen05 tensor cores with 3xTF32 operands (1) or on the FP64 tensor pipe
  * (2, the default: exact products of the float operands, FP64 sums).
  * node_tensor_cores: the coupling and forward products of float level nodes
  * (n <= 128) on the tcgen05 tensor cores at every level (1), only on levels
- * with at least 4 nodes per SM (3), or SIMT (2, and the default); 4 keeps a
+ * with at least 4 nodes per SM (3), or on the FP64 tensor pipe (2, and the
+ * default); 4 keeps a
  * float level node with 64 < n <= 128 resident in tensor memory and runs the
  * trailing updates of its blocked Cholesky and coupling solves on the tensor
  * cores (3xTF32), the 32-column panels on SIMT cores. */
@@ -164,7 +164,7 @@ typedef struct socu_tuning {
 
 /* As socu_launch_create, with per-launch settings (NULL: none) applied on top
  * of the tuned table.  The reference's block_dim maps to the three thread
- * counts, its block_size to update_tile. */
+ * counts, its block_size to update_tile (both without effect, see above). */
 int socu_launch_create_tuned(socu_launch_t* out, socu_op op, socu_dtype dtype, void* L, void* E, void* x,
                              const uint8_t* mask, int64_t batch, int64_t horizon, int64_t n, int64_t n_rhs,
                              int use_cuda_graph, const socu_tuning* settings, void* stream);
@@ -382,9 +382,8 @@ int socu_ragged_destroy(socu_ragged_t batch);
 int socu_dmma_peak_launch(int64_t blocks, int threads, int iters, double* sink, void* stream, double* flops);
 
 /* Error word of the asynchronous units on the current device (synchronises):
- * 0 ok, 1 a tensor-core (tcgen05) wait ran out, 2 a TMA copy wait of the
- * resident sweeps ran out (that kernel skipped its result).  reset != 0 clears
- * it afterwards.  No counterpart in the reference. */
+ * 0 ok, 1 a tensor-core (tcgen05) wait ran out (that kernel skipped its
+ * result).  reset != 0 clears it afterwards.  No counterpart in the reference. */
 int socu_tc_error(int* flag, int reset);
 
 /* Self-test of the tensor-core (tcgen05) building block of the float path:

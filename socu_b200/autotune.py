@@ -9,16 +9,16 @@ this module fills that table by measurement and keeps the results in an
 on-disk cache, so a process tunes a shape once and later processes reuse it.
 
 Settings (``socu_tuning``; 0 = built-in heuristic):
-    node_threads, update_threads, sweep_threads   threads per CTA: 64, 128, 256
-    sweep_tensor_cores   float sweeps on inverse-carrying factors: 1 FP64
-                         tensor-core products, 2 SIMT row dots
-    update_tile          output tile of the blocked Schur update (n > 64): 16, 32
+    node_threads, update_threads, sweep_threads, sweep_tensor_cores,
+    update_tile          kept for existing caches and callers; the kernels have
+                         one warp per 8-row tile and one product path, so these
+                         choose nothing
     ragged_units         level nodes per task chunk of a ragged batch: 1..64
     update_tensor_cores  Schur updates of float factors (n <= 128) on the
                          tcgen05 tensor cores, 3xTF32 (1), or not (2)
     node_tensor_cores    products of float level nodes (n <= 128) on the
                          tcgen05 tensor cores at every level (1), on wide
-                         levels only (3), or SIMT (2); 64 < n <= 128: the
+                         levels only (3), or FP64 tensor pipe (2); 64 < n <= 128: the
                          node resident in tensor memory, trailing updates on
                          the tensor cores (4)
 

@@ -167,12 +167,11 @@ def _validate(L, E, x, mask, with_x: bool):
 
 
 def _settings(block_dim, block_size):
-    """Per-launch settings from the reference's tiling arguments: block_dim
-    (threads per tile block) sets the threads per CTA of the node, update and
-    sweep kernels, rounded up to 64, 128 or 256; block_size (tile size of the
-    blocked kernels) sets the output tile of the blocked Schur update, used for
-    n > 64 (16 if block_size <= 16, else 32).  None leaves a setting to the
-    tuned table / heuristics."""
+    """Per-launch settings from the reference's tiling arguments, checked and
+    passed on: block_dim (threads per tile block) as the thread counts, rounded
+    up to 64, 128 or 256, block_size (tile size of the blocked kernels) as the
+    update tile (16 if block_size <= 16, else 32).  The kernels have one warp per
+    8-row tile of a block, so neither changes what runs."""
     out = {}
     if block_dim is not None:
         bd = int(block_dim)
