@@ -119,8 +119,8 @@ __device__ __forceinline__ void solve_frag(const T* L, int n, int i, int kk, boo
   a1 = a[1];
 }
 
-// One vector, its columns col0 .. col0 + cols (a multiple of 8).  ONE: the block has a warp per row tile (else the warps loop over them and the
-// blocks are read as they are used).
+// One vector, its columns col0 .. col0 + cols (a multiple of 8).  ONE: the block has a warp per
+// row tile (else the warps loop over them and the blocks are read as they are used).
 template <typename T, int NT, bool FULL, int MODE, bool INV, bool ONE, class Group>
 __device__ __forceinline__ void sweep_rows_body(const Group& grp, const Problem<T>& p, const Level& lv, int b, int task,
                                                 unsigned char* smem_raw, int wait, int col0 = 0,
@@ -229,8 +229,9 @@ __device__ __forceinline__ void sweep_rows_body(const Group& grp, const Problem<
     // neighbours' vectors, zeros outside (KEEP's products run over all NT tiles: a zero operand
     // does not cancel a NaN that an earlier kernel left in shared memory)
     if (P || Q) {
-      for (int e = grp.tid(); e < 8 * (KEEP ? NT : nta) * 8 * groups; e += grp.threads()) {
-        const int k = e / (8 * groups), c = e - k * (8 * groups);
+      const int w = CG == 1 ? 8 : 8 * groups;   // (a constant up to n = 64: no division)
+      for (int e = grp.tid(); e < 8 * (KEEP ? NT : nta) * w; e += grp.threads()) {
+        const int k = e / w, c = e - k * w;
         const bool in = k < n && c < mc;
         const long long o = (long long)k * m + c0 + c;
         if (P) Zp[k * ldz + c] = in ? (double)__ldcg(p.Xb(b, jp) + o) : 0.0;
