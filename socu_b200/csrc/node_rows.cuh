@@ -74,8 +74,9 @@ __device__ __forceinline__ void bar_wait(int id, int threads) {
 
 // 1 / sqrt(d) without a branch: the approximate instruction, then one step of
 // Householder's third-order iteration y (1 + e/2 + 3 e^2 / 8), e = 1 - d y^2.
-// For normal d; a subnormal one (flushed by the instruction) gives NaN, and the
-// caller starts over with the library function.
+// For normal d.  A subnormal one is flushed by the instruction: infinity comes
+// out, and the caller, whose last pivot is then not finite, starts over with the
+// library function.
 template <typename T, bool FAST>
 __device__ __forceinline__ T pivot_rsqrt(T d) {
   if constexpr (FAST && sizeof(T) == 8) {
@@ -161,8 +162,9 @@ __device__ __forceinline__ void rows_factor_tile(double d0, double d1, T* S, dou
   __syncwarp();
   T c[8][8];
   chol8_tile<T, true>(S, Ivk, c);
-  // a NaN reaches the last pivot from any earlier one
-  const bool redo = sizeof(T) == 8 && c[7][7] != c[7][7];
+  // An infinite factor of column 0 to 6 is a NaN in every later pivot (infinity less infinity, or
+  // infinity times zero); in column 7 it is the last pivot itself.
+  const bool redo = sizeof(T) == 8 && !isfinite(c[7][7]);
   if (redo) chol8_redo<T>(S, Ivk);
   publish();
   if (!redo) chol8_keep(S, c);
