@@ -162,6 +162,7 @@ __device__ __forceinline__ void rows_factor_tile(double d0, double d1, T* S, dou
   __syncwarp();
   T c[8][8];
   chol8_tile<T, true>(S, Ivk, c);
+  __syncwarp();   // every lane has read S and written Ivk: both are written again below
   // An infinite factor of column 0 to 6 is a NaN in every later pivot (infinity less infinity, or
   // infinity times zero); in column 7 it is the last pivot itself.
   const bool redo = sizeof(T) == 8 && !isfinite(c[7][7]);
