@@ -520,7 +520,11 @@ __global__ void __launch_bounds__(rg_threads(BLOCKS), BLOCKS ? 2 : 3) k_ragged(c
   unsigned char* smem = BLOCKS ? smem_raw : smem_raw + (threadIdx.x >> 5) * a.worker_bytes;
   const bool lead = BLOCKS ? threadIdx.x == 0 : (threadIdx.x & 31) == 0;
   auto share = [&](unsigned long long v) {   // the lead's value in every thread of the worker
-    if (!BLOCKS) return __shfl_sync(kFull, v, 0);
+    if (!BLOCKS) {   // (the shuffle orders no memory: what the lead's fence acquired is for every lane)
+      v = __shfl_sync(kFull, v, 0);
+      __syncwarp();
+      return v;
+    }
     if (lead) s_task = v;
     __syncthreads();
     v = s_task;
