@@ -10,11 +10,11 @@
 // tile (8 x n) as FP64 tensor-core accumulators (mma.m8n8k4 .f64, fragment
 // {c0, c1} = C[g][2t + {0, 1}], g = lane / 4, t = lane % 4), read from global
 // memory straight into registers.  Step k:
-//   1. the warp of row k factors its diagonal tile with shuffles
-//      (warp_chol8) and publishes Inv_k = C_kk^{-1} in shared memory;
-//   2. every later row multiplies its tile k by Inv_k^T: the final tile P,
-//      stored to global memory at once and, for rows of L_i, to shared memory;
-//   3. every later row subtracts P P_j^T from its tiles j > k.
+//   1. the warp of row k factors its diagonal tile (every lane the whole tile)
+//      and publishes C_kk and Inv_k = C_kk^{-1} in shared memory;
+//   2. every later row multiplies its tile k by Inv_k^T and corrects the product
+//      against C_kk (rows_panel): the final tile P, as exact as a substitution;
+//   3. every later row adds P P_j^T to the sums that its tiles j > k are less of.
 // The accumulator fragment is the A operand of the next product without any
 // shuffle: the contraction index is enumerated as 2t, 2t + 1 (one MMA each),
 // and the B operand (a row of Inv_k or of P_j) is then one 16-byte load.
@@ -89,16 +89,17 @@ __device__ __forceinline__ T pivot_rsqrt(T d) {
   }
 }
 
-// Cholesky factor of the 8x8 tile in S (lower triangle, left in c) and its
-// inverse, written to Ivk (8 x 8, lane l the column l % 8).  Every lane of the
-// warp factors the whole tile: the chain is 8 times rsqrt -> multiply ->
-// subtract, about 70 cycles each in FP64, with no exchange between lanes.
+// Cholesky factor of the 8x8 tile in S, written over it (lower triangle; the
+// caller clears the rest), and its inverse, written to Ivk (8 x 8, lane l the
+// column l % 8); returns the last pivot's factor.  Every lane of the warp factors
+// the whole tile: the chain is 8 times rsqrt -> multiply -> subtract, about 70
+// cycles each in FP64, with no exchange between lanes; the stores go out beside it.
 // Measured per tile: 770 cycles FP64, 556 float; spread over the lanes instead
 // (16 shuffles a column, which issue every 4.3 cycles) 1500 and 790.
 template <typename T, bool FAST>
-__device__ __forceinline__ void chol8_tile(const T* S, double* Ivk, T (&c)[8][8]) {
-  const int col = threadIdx.x & 7;
-  T y[8];
+__device__ __forceinline__ T chol8_tile(T* S, double* Ivk) {
+  const int lane = threadIdx.x & 31, col = lane & 7;
+  T c[8][8], y[8];
 #pragma unroll
   for (int i = 0; i < 8; ++i)
 #pragma unroll
@@ -113,13 +114,16 @@ __device__ __forceinline__ void chol8_tile(const T* S, double* Ivk, T (&c)[8][8]
         c[i][j + 1] = v.y;
       }
     }
+  __syncwarp();   // every lane has read S
 #pragma unroll
   for (int i = 0; i < 8; ++i) y[i] = T(0);
 #pragma unroll
   for (int j = 0; j < 8; ++j) {
-    const T r = pivot_rsqrt<T, FAST>(c[j][j]);
+    const T d = c[j][j], r = pivot_rsqrt<T, FAST>(d);
 #pragma unroll
     for (int i = j; i < 8; ++i) c[i][j] *= r;
+    // the root itself, off the chain: one Newton step brings d r within half a unit in the last place
+    c[j][j] = fma(T(0.5) * r, fma(-c[j][j], c[j][j], d), c[j][j]);
 #pragma unroll
     for (int l = j + 1; l < 8; ++l)
 #pragma unroll
@@ -128,47 +132,49 @@ __device__ __forceinline__ void chol8_tile(const T* S, double* Ivk, T (&c)[8][8]
 #pragma unroll
     for (int i = j + 1; i < 8; ++i) y[i] = fma(-c[i][j], y[j], y[i]);
     Ivk[8 * j + col] = (double)y[j];
+    if (lane == 0) {
+#pragma unroll
+      for (int i = j; i < 8; ++i) S[8 * i + j] = c[i][j];
+    }
   }
-}
-
-template <typename T>
-__device__ __forceinline__ void chol8_keep(T* S, const T (&c)[8][8]) {
-#pragma unroll
-  for (int i = 0; i < 8; ++i)
-#pragma unroll
-    for (int j = 0; j <= i; ++j) S[8 * i + j] = c[i][j];   // every lane writes the same values
+  return c[7][7];
 }
 
 // the factor with the library's reciprocal square root (subnormal pivots)
 template <typename T>
 __device__ __noinline__ void chol8_redo(T* S, double* Ivk) {
-  T c[8][8];
-  chol8_tile<T, false>(S, Ivk, c);
-  __syncwarp();
-  chol8_keep(S, c);
+  chol8_tile<T, false>(S, Ivk);
 }
 
-// Factor the diagonal tile held as an accumulator fragment (d0, d1): its
-// inverse goes to Ivk, then publish() runs, then lower(C_kk) goes to S (8 x 8,
-// first the tile's scratch).  All lanes of the warp; the caller orders its reads
-// of S and Ivk with __syncwarp.
-template <typename T, class Publish>
-__device__ __forceinline__ void rows_factor_tile(double d0, double d1, T* S, double* Ivk, Publish publish) {
+// an accumulator fragment as an 8 x 8 tile
+template <typename T>
+__device__ __forceinline__ void frag_put(T* S, double d0, double d1) {
   const int lane = threadIdx.x & 31;
   if constexpr (sizeof(T) == 8)
     *reinterpret_cast<double2*>(S + 2 * lane) = make_double2(d0, d1);
   else
     *reinterpret_cast<float2*>(S + 2 * lane) = make_float2((float)d0, (float)d1);
+}
+
+// Factor the diagonal tile held as an accumulator fragment (d0, d1): C_kk goes to
+// S (8 x 8, zeros above the diagonal) and its inverse to Ivk.  All lanes of the
+// warp; the caller orders its reads of S and Ivk with __syncwarp or a barrier.
+template <typename T>
+__device__ __forceinline__ void rows_factor_tile(double d0, double d1, T* S, double* Ivk) {
+  const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  frag_put(S, d0, d1);
   __syncwarp();
-  T c[8][8];
-  chol8_tile<T, true>(S, Ivk, c);
-  __syncwarp();   // every lane has read S and written Ivk: both are written again below
+  const T last = chol8_tile<T, true>(S, Ivk);
   // An infinite factor of column 0 to 6 is a NaN in every later pivot (infinity less infinity, or
   // infinity times zero); in column 7 it is the last pivot itself.
-  const bool redo = sizeof(T) == 8 && !isfinite(c[7][7]);
-  if (redo) chol8_redo<T>(S, Ivk);
-  publish();
-  if (!redo) chol8_keep(S, c);
+  if (sizeof(T) == 8 && !isfinite(last)) {
+    __syncwarp();   // S and Ivk are written again
+    frag_put(S, d0, d1);
+    __syncwarp();
+    chol8_redo<T>(S, Ivk);
+  }
+  if (2 * t > g) S[2 * lane] = T(0);
+  if (2 * t + 1 > g) S[2 * lane + 1] = T(0);
 }
 
 // The warps that work on one node, output block or vector: a whole thread
@@ -214,6 +220,25 @@ __device__ __forceinline__ void load_pair(const T* p, bool vec, bool v0, bool v1
     x1 = v1 ? (double)p[1] : 0.0;
   }
 }
+// two consecutive elements as they are; `vec`: the pair is aligned and inside
+template <typename T>
+__device__ __forceinline__ void load_raw(const T* p, bool vec, bool v0, bool v1, T (&x)[2]) {
+  if (vec) {
+    if constexpr (sizeof(T) == 8) {
+      const double2 v = *reinterpret_cast<const double2*>(p);
+      x[0] = v.x;
+      x[1] = v.y;
+    } else {
+      const float2 v = *reinterpret_cast<const float2*>(p);
+      x[0] = v.x;
+      x[1] = v.y;
+    }
+  } else {
+    x[0] = v0 ? p[0] : T(0);
+    x[1] = v1 ? p[1] : T(0);
+  }
+}
+
 template <typename T>
 __device__ __forceinline__ void store_pair(T* p, bool vec, bool v0, bool v1, double x0, double x1) {
   if (vec) {
@@ -246,23 +271,53 @@ struct RowSrc {
   bool full;    // whole tiles: no bounds to check (n == 8 nta; not the right-hand sides)
 };
 
-// X tile row: P = X_k Inv_k^T
-__device__ __forceinline__ void rows_panel(double& p0, double& p1, double x0, double x1, double2 iv) {
+// What a panel product reads of one diagonal tile: this lane's elements of Inv_k, of C_kk below the
+// diagonal, and the diagonal of its two accumulator columns.
+struct DiagFrag {
+  double2 iv, cv;
+  double d0, d1;
+};
+template <typename T>
+__device__ __forceinline__ DiagFrag diag_frag(const double* Ik, const T* Ck) {
+  const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  DiagFrag f;
+  f.iv = *reinterpret_cast<const double2*>(Ik + 2 * lane);
+  load_pair(Ck + 2 * lane, true, true, true, f.cv.x, f.cv.y);
+  f.d0 = (double)Ck[18 * t];
+  f.d1 = (double)Ck[18 * t + 9];
+  if (2 * t == g) f.cv.x = 0.0;
+  if (2 * t + 1 == g) f.cv.y = 0.0;
+  return f;
+}
+
+// X tile row: P = X_k C_kk^{-T}.  The product with the explicit inverse has a residual that grows
+// with the tile's condition; one correction, P += (X - P C_kk^T) Inv_k^T, brings it down to that of
+// a substitution.  The diagonal's part of the residual is one fused operation, so that what cancels
+// is not rounded before, and the correction is summed by itself and added once.
+__device__ __forceinline__ void rows_panel(double& p0, double& p1, double x0, double x1, const DiagFrag& f) {
+  double s0 = 0.0, s1 = 0.0, q0 = 0.0, q1 = 0.0;
   p0 = p1 = 0.0;
-  mma_acc(p0, p1, x0, iv.x);
-  mma_acc(p0, p1, x1, iv.y);
+  mma_acc(p0, p1, x0, f.iv.x);
+  mma_acc(p0, p1, x1, f.iv.y);
+  mma_acc(s0, s1, p0, f.cv.x);
+  mma_acc(s0, s1, p1, f.cv.y);
+  const double r0 = fma(-p0, f.d0, x0) - s0, r1 = fma(-p1, f.d1, x1) - s1;
+  mma_acc(q0, q1, r0, f.iv.x);
+  mma_acc(q0, q1, r1, f.iv.y);
+  p0 += q0;
+  p1 += q1;
 }
 
 // (identity rows start at their own step: tile k0 is the identity, later tiles zero)
 template <typename T, int NT>
-__device__ __forceinline__ void rows_load(double (&acc)[NT][2], const RowSrc<T>& s, int n, bool vec) {
+__device__ __forceinline__ void rows_load(T (&x)[NT][2], const RowSrc<T>& s, int n, bool vec) {
   const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
   const bool rv = g < s.lim;
   if (s.kind == 0) {
 #pragma unroll
     for (int j = 0; j < NT; ++j) {
       const int c = 8 * j + 2 * t;
-      load_pair(s.base + (g * s.ld + c), vec && 8 * j < n, rv && c < n, rv && c + 1 < n, acc[j][0], acc[j][1]);
+      load_raw(s.base + (g * s.ld + c), vec && 8 * j < n, rv && c < n, rv && c + 1 < n, x[j]);
     }
   } else if (s.kind == 1) {
 #pragma unroll
@@ -271,13 +326,13 @@ __device__ __forceinline__ void rows_load(double (&acc)[NT][2], const RowSrc<T>&
       for (int e = 0; e < 2; ++e) {
         const int c = 8 * j + 2 * t + e;
         const bool in = s.full ? 8 * j < n : rv && c < n;
-        acc[j][e] = in ? (double)s.base[c * s.ld + g] : 0.0;
+        x[j][e] = in ? s.base[c * s.ld + g] : T(0);
       }
   } else {
 #pragma unroll
     for (int j = 0; j < NT; ++j)
 #pragma unroll
-      for (int e = 0; e < 2; ++e) acc[j][e] = (j == s.k0 && g == 2 * t + e) ? 1.0 : 0.0;
+      for (int e = 0; e < 2; ++e) x[j][e] = (j == s.k0 && g == 2 * t + e) ? T(1) : T(0);
   }
 }
 
@@ -305,9 +360,9 @@ __device__ __forceinline__ void rows_store(const double (&acc)[NT][2], const Row
   }
 }
 
-// tiles j0 .. j0 + CH - 1 (below NT) of one row tile -= P P_j^T
+// tiles j0 .. j0 + CH - 1 (below NT) of one row tile += A P_j^T, A = (a0, a1)
 template <int NT, int CH>
-__device__ __forceinline__ void rows_update(double (&acc)[NT][2], int j0, double p0, double p1, const double* Ck,
+__device__ __forceinline__ void rows_update(double (&acc)[NT][2], int j0, double a0, double a1, const double* Ck,
                                             int ld) {
   double2 bv[CH];
 #pragma unroll
@@ -315,28 +370,39 @@ __device__ __forceinline__ void rows_update(double (&acc)[NT][2], int j0, double
     if (j0 + h < NT) bv[h] = *reinterpret_cast<const double2*>(Ck + 8 * (j0 + h) * ld);
 #pragma unroll
   for (int h = 0; h < CH; ++h)
-    if (j0 + h < NT) mma_acc(acc[j0 + h][0], acc[j0 + h][1], -p0, bv[h].x);
+    if (j0 + h < NT) mma_acc(acc[j0 + h][0], acc[j0 + h][1], a0, bv[h].x);
 #pragma unroll
   for (int h = 0; h < CH; ++h)
-    if (j0 + h < NT) mma_acc(acc[j0 + h][0], acc[j0 + h][1], -p1, bv[h].y);
+    if (j0 + h < NT) mma_acc(acc[j0 + h][0], acc[j0 + h][1], a1, bv[h].y);
 }
 
-// All steps of one row tile against the finished factor (FROM0: k0 is 0, and no
+// Sums from zero where the registers hold a row tile twice: X less the sum of the products is rounded
+// once at X's size.  (Larger blocks subtract every product from X, as a substitution does.)
+__host__ __device__ constexpr bool rows_from_zero(int nt) { return nt <= 8; }
+
+// All steps of one row tile x against the finished factor, results in acc (FROM0: k0 is 0, and no
 // branch separates the steps; the tile that the next step starts from comes first).  EXACT: nta is NT.
-template <int NT, bool FROM0, bool EXACT>
-__device__ __forceinline__ void rows_solve(double (&acc)[NT][2], int k0, int nta, const double* Cs, const double* Iv) {
+template <typename T, int NT, bool FROM0, bool EXACT>
+__device__ __forceinline__ void rows_solve(double (&acc)[NT][2], const T (&x)[NT][2], int k0, int nta, const double* Cs,
+                                           const double* Iv, const T* Ct) {
   constexpr int ld = (NT & 1) ? 8 * NT : 8 * NT + 8;
+  constexpr bool ZERO = rows_from_zero(NT);
   const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+#pragma unroll
+  for (int j = 0; j < NT; ++j)
+#pragma unroll
+    for (int e = 0; e < 2; ++e) acc[j][e] = ZERO ? 0.0 : (double)x[j][e];
 #pragma unroll
   for (int k = 0; k < NT; ++k) {
     if ((FROM0 || k >= k0) && (EXACT || k < nta)) {
-      const double2 iv = *reinterpret_cast<const double2*>(Iv + 64 * k + 2 * lane);
       const double* Ck = Cs + g * ld + 8 * k + 2 * t;
       double p0, p1;
-      rows_panel(p0, p1, acc[k][0], acc[k][1], iv);
-      rows_update<NT, 1>(acc, k + 1, p0, p1, Ck, ld);
+      rows_panel(p0, p1, ZERO ? (double)x[k][0] - acc[k][0] : acc[k][0], ZERO ? (double)x[k][1] - acc[k][1] : acc[k][1],
+                 diag_frag(Iv + 64 * k, Ct + 64 * k));
+      const double a0 = ZERO ? p0 : -p0, a1 = ZERO ? p1 : -p1;
+      rows_update<NT, 1>(acc, k + 1, a0, a1, Ck, ld);
 #pragma unroll
-      for (int j = k + 2; j < NT; j += 4) rows_update<NT, 4>(acc, j, p0, p1, Ck, ld);
+      for (int j = k + 2; j < NT; j += 4) rows_update<NT, 4>(acc, j, a0, a1, Ck, ld);
       acc[k][0] = p0;
       acc[k][1] = p1;
     }
@@ -397,18 +463,36 @@ __device__ __forceinline__ void node_rows_body(const Group& grp, const Problem<T
     return o;
   };
 
-  // this warp's row tile of L_i (lower tiles; the padding of the last tile is an identity)
+  // This warp's row tile of L_i (lower tiles; the padding of the last tile is an identity).  Where
+  // the products are summed from zero it waits in its place in shared memory, the diagonal tile in
+  // registers; larger blocks have no registers for both and subtract from the tile.
+  // (FP64 errors at n = 64: 7.9e-17 in C, against 1.6e-16 when every product is rounded at X's size.)
+  constexpr bool ZERO = rows_from_zero(NT);
   const int gr = 8 * row + g;
-  double acc[NT][2];
+  double* Xr = Cs + gr * ld + 2 * tq;
+  double acc[NT][2], dx0 = 0.0, dx1 = 0.0;
+  {
+    double x[NT][2];
 #pragma unroll
-  for (int j = 0; j < NT; ++j) {
-    acc[j][0] = acc[j][1] = 0.0;
-    if (row < nta && j <= row) {
-      const int c = 8 * j + 2 * tq;
-      load_pair(Li + (long long)gr * n + c, vec, gr < n && c < n, gr < n && c + 1 < n, acc[j][0], acc[j][1]);
-      if (!vec && gr >= n) {
-        if (c == gr) acc[j][0] = 1.0;
-        if (c + 1 == gr) acc[j][1] = 1.0;
+    for (int j = 0; j < NT; ++j) {
+      x[j][0] = x[j][1] = 0.0;
+      if (row < nta && j <= row) {
+        const int c = 8 * j + 2 * tq;
+        load_pair(Li + (long long)gr * n + c, vec, gr < n && c < n, gr < n && c + 1 < n, x[j][0], x[j][1]);
+        if (!vec && gr >= n) {
+          if (c == gr) x[j][0] = 1.0;
+          if (c + 1 == gr) x[j][1] = 1.0;
+        }
+      }
+    }
+#pragma unroll
+    for (int j = 0; j < NT; ++j) {
+      acc[j][0] = ZERO ? 0.0 : x[j][0];
+      acc[j][1] = ZERO ? 0.0 : x[j][1];
+      if (ZERO && row < nta && j < row) *reinterpret_cast<double2*>(Xr + 8 * j) = make_double2(x[j][0], x[j][1]);
+      if (ZERO ? j == row : j == 0) {
+        dx0 = x[j][0];
+        dx1 = x[j][1];
       }
     }
   }
@@ -420,33 +504,36 @@ __device__ __forceinline__ void node_rows_body(const Group& grp, const Problem<T
   // its own tile needs nothing else, later rows wait).  Warps past their row
   // leave the steps and meet the others at the end.
   if (row < nta) {
-    double d0 = acc[0][0], d1 = acc[0][1];
+    double d0 = dx0, d1 = dx1;   // the diagonal tile
 #pragma unroll
     for (int k = 0; k < NT - 1; ++k) {
       if (k < row) {
         const int after = nta - 1 - k;   // rows after k
+        double2 x = make_double2(0.0, 0.0);
+        if (ZERO) x = *reinterpret_cast<const double2*>(Xr + 8 * k);
         bar_wait(grp.bar(1), 32 * (after + 1));
-        const double2 iv = *reinterpret_cast<const double2*>(Iv + 64 * k + 2 * lane);
         double p0, p1;
-        rows_panel(p0, p1, acc[k][0], acc[k][1], iv);
-        *reinterpret_cast<double2*>(Cs + gr * ld + 8 * k + 2 * tq) = make_double2(p0, p1);
+        rows_panel(p0, p1, ZERO ? x.x - acc[k][0] : acc[k][0], ZERO ? x.y - acc[k][1] : acc[k][1],
+                   diag_frag(Iv + 64 * k, Ct + 64 * k));
+        *reinterpret_cast<double2*>(Xr + 8 * k) = make_double2(p0, p1);
+        const double a0 = ZERO ? p0 : -p0, a1 = ZERO ? p1 : -p1;
         if (row == k + 1) {
           if (after > 1) bar_arrive(grp.bar(2), 32 * after);
-          d0 = acc[k + 1][0];
-          d1 = acc[k + 1][1];
-          mma_acc(d0, d1, -p0, p0);
-          mma_acc(d0, d1, -p1, p1);
+          double s0 = acc[k + 1][0], s1 = acc[k + 1][1];
+          mma_acc(s0, s1, a0, p0);
+          mma_acc(s0, s1, a1, p1);
+          d0 = ZERO ? dx0 - s0 : s0;
+          d1 = ZERO ? dx1 - s1 : s1;
         } else {
           bar_wait(grp.bar(2), 32 * after);
 #pragma unroll
           for (int j = k + 1; j < NT; j += 4)
-            if (j <= row) rows_update<NT, 4>(acc, j, p0, p1, Cs + g * ld + 8 * k + 2 * tq, ld);
+            if (j <= row) rows_update<NT, 4>(acc, j, a0, a1, Cs + g * ld + 8 * k + 2 * tq, ld);
         }
       }
     }
-    rows_factor_tile<T>(d0, d1, Ct + 64 * row, Iv + 64 * row, [&] {
-      if (row + 1 < nta) bar_arrive(grp.bar(1), 32 * (nta - row));
-    });
+    rows_factor_tile<T>(d0, d1, Ct + 64 * row, Iv + 64 * row);
+    if (row + 1 < nta) bar_arrive(grp.bar(1), 32 * (nta - row));
     if (splits > 1) cluster_wait();   // every block of the cluster has read L_i
     if (q == 0) {
       __syncwarp();
@@ -472,8 +559,8 @@ __device__ __forceinline__ void node_rows_body(const Group& grp, const Problem<T
     cluster_wait();
   }
   // (the first row tile arrives while later rows finish phase 1)
-  double av[NT][2];
-  if (v_first < vtot) rows_load<T, NT>(av, source(v_first), n, vec);
+  T xv[NT][2];
+  if (v_first < vtot) rows_load<T, NT>(xv, source(v_first), n, vec);
   grp.sync();   // the factor is complete in shared memory
 
   // phase 2
@@ -486,11 +573,12 @@ __device__ __forceinline__ void node_rows_body(const Group& grp, const Problem<T
       }
       continue;
     }
-    if (v != v_first) rows_load<T, NT>(av, src, n, vec);
+    if (v != v_first) rows_load<T, NT>(xv, src, n, vec);
+    double av[NT][2];
     if (src.kind == 2)
-      rows_solve<NT, false, EXACT>(av, src.k0, nta, Cs, Iv);
+      rows_solve<T, NT, false, EXACT>(av, xv, src.k0, nta, Cs, Iv, Ct);
     else
-      rows_solve<NT, true, EXACT>(av, 0, nta, Cs, Iv);
+      rows_solve<T, NT, true, EXACT>(av, xv, 0, nta, Cs, Iv, Ct);
     rows_store<T, NT>(av, src, n, vec);
   }
 }

@@ -42,25 +42,6 @@ __host__ __device__ inline int update_rows_warps(int n, int splits) {
   return splits * (((n + 7) / 8 + splits - 1) / splits);
 }
 
-// two consecutive elements as they are; `vec`: the pair is aligned and inside
-template <typename T>
-__device__ __forceinline__ void load_raw(const T* p, bool vec, bool v0, bool v1, T (&x)[2]) {
-  if (vec) {
-    if constexpr (sizeof(T) == 8) {
-      const double2 v = *reinterpret_cast<const double2*>(p);
-      x[0] = v.x;
-      x[1] = v.y;
-    } else {
-      const float2 v = *reinterpret_cast<const float2*>(p);
-      x[0] = v.x;
-      x[1] = v.y;
-    }
-  } else {
-    x[0] = v0 ? p[0] : T(0);
-    x[1] = v1 ? p[1] : T(0);
-  }
-}
-
 // One k-step (8 of the contraction index) of a row's tiles, four at a time.
 // Target: += a F_j^T (+ h G_j); fill-in: += a G_j.  fk, gk: this lane's
 // elements of row tile / column tile 0.  Tiles past jmax repeat the last one

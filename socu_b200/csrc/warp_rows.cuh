@@ -14,9 +14,9 @@ namespace socu {
 
 // Shared memory of one warp (bytes): the lower tiles of C as 8x8 blocks of
 // doubles (off-diagonal tile (i, j) at i (i - 1) / 2 + j, then the inverses of the
-// diagonal tiles) and one tile of scratch.  A fragment is 16 bytes at 2 * lane.
+// diagonal tiles) and the diagonal tiles themselves.  A fragment is 16 bytes at 2 * lane.
 __host__ __device__ constexpr int warp_node_tiles(int nt) { return nt * (nt + 1) / 2; }
-__host__ __device__ inline long long smem_warp_node_bytes(int nt) { return 512LL * (warp_node_tiles(nt) + 1); }
+__host__ __device__ inline long long smem_warp_node_bytes(int nt) { return 512LL * (warp_node_tiles(nt) + nt); }
 
 __device__ __forceinline__ double2 tile_frag(const double* tile) {
   return *reinterpret_cast<const double2*>(tile + 2 * (threadIdx.x & 31));
@@ -34,24 +34,29 @@ __device__ __forceinline__ void warp_prefetch(const T* p, int count) {
 }
 
 // All steps of R row tiles against the finished factor: they share every operand load.
-template <int NT, int R>
-__device__ __forceinline__ void warp_rows_solve(double (&acc)[R][NT][2], int k0, int nta, const double* Ls,
-                                                const double* Iv) {
+template <typename T, int NT, int R>
+__device__ __forceinline__ void warp_rows_solve(double (&acc)[R][NT][2], const T (&x)[R][NT][2], int k0, int nta,
+                                                const double* Ls, const double* Iv, const T* Ct) {
+#pragma unroll
+  for (int r = 0; r < R; ++r)
+#pragma unroll
+    for (int j = 0; j < NT; ++j) acc[r][j][0] = acc[r][j][1] = 0.0;
 #pragma unroll
   for (int k = 0; k < NT; ++k) {
     if (k >= k0 && k < nta) {
-      const double2 iv = tile_frag(Iv + 64 * k);
+      const DiagFrag f = diag_frag(Iv + 64 * k, Ct + 64 * k);
       double p[R][2];
 #pragma unroll
-      for (int r = 0; r < R; ++r) rows_panel(p[r][0], p[r][1], acc[r][k][0], acc[r][k][1], iv);
+      for (int r = 0; r < R; ++r)
+        rows_panel(p[r][0], p[r][1], (double)x[r][k][0] - acc[r][k][0], (double)x[r][k][1] - acc[r][k][1], f);
 #pragma unroll
       for (int j = k + 1; j < NT; ++j) {
         if (j < nta) {
           const double2 bv = tile_frag(Ls + 64 * (j * (j - 1) / 2 + k));
 #pragma unroll
-          for (int r = 0; r < R; ++r) mma_acc(acc[r][j][0], acc[r][j][1], -p[r][0], bv.x);
+          for (int r = 0; r < R; ++r) mma_acc(acc[r][j][0], acc[r][j][1], p[r][0], bv.x);
 #pragma unroll
-          for (int r = 0; r < R; ++r) mma_acc(acc[r][j][0], acc[r][j][1], -p[r][1], bv.y);
+          for (int r = 0; r < R; ++r) mma_acc(acc[r][j][0], acc[r][j][1], p[r][1], bv.y);
         }
       }
 #pragma unroll
@@ -111,14 +116,9 @@ __device__ __forceinline__ void node_warp_body(const Problem<T>& p, const Level&
   // diagonal tiles, factored by the whole warp, need the warp in step)
 #pragma unroll 1
   for (int k = 0; k < nta; ++k) {
-    double acc[NT][2];   // tiles (k + r, k)
+    double acc[NT][2];   // products of tiles (k + r, k), summed from zero (as in node_rows_body)
 #pragma unroll
-    for (int r = 0; r < NT; ++r)
-      if (k + r < nta) {
-        const double2 v = tile_frag(r == 0 ? Iv + 64 * k : Ls + 64 * ((k + r) * (k + r - 1) / 2 + k));
-        acc[r][0] = v.x;
-        acc[r][1] = v.y;
-      }
+    for (int r = 0; r < NT; ++r) acc[r][0] = acc[r][1] = 0.0;
 #pragma unroll 1
     for (int j = 0; j < k; ++j) {
       const double2 bv = tile_frag(Ls + 64 * (k * (k - 1) / 2 + j));
@@ -126,26 +126,33 @@ __device__ __forceinline__ void node_warp_body(const Problem<T>& p, const Level&
       for (int r = 0; r < NT; ++r)
         if (k + r < nta) {
           const double2 av = r == 0 ? bv : tile_frag(Ls + 64 * ((k + r) * (k + r - 1) / 2 + j));
-          mma_acc(acc[r][0], acc[r][1], -av.x, bv.x);
-          mma_acc(acc[r][0], acc[r][1], -av.y, bv.y);
+          mma_acc(acc[r][0], acc[r][1], av.x, bv.x);
+          mma_acc(acc[r][0], acc[r][1], av.y, bv.y);
         }
     }
+#pragma unroll
+    for (int r = 0; r < NT; ++r)
+      if (k + r < nta) {
+        const double2 v = tile_frag(r == 0 ? Iv + 64 * k : Ls + 64 * ((k + r) * (k + r - 1) / 2 + k));
+        acc[r][0] = v.x - acc[r][0];
+        acc[r][1] = v.y - acc[r][1];
+      }
     __syncwarp();
-    rows_factor_tile<T>(acc[0][0], acc[0][1], Ct, Iv + 64 * k, [] {});
+    rows_factor_tile<T>(acc[0][0], acc[0][1], Ct + 64 * k, Iv + 64 * k);
     __syncwarp();
-    const double2 iv = tile_frag(Iv + 64 * k);
+    const DiagFrag f = diag_frag(Iv + 64 * k, Ct + 64 * k);
 #pragma unroll
     for (int r = 1; r < NT; ++r)
       if (k + r < nta) {
         double p0, p1;
-        rows_panel(p0, p1, acc[r][0], acc[r][1], iv);
+        rows_panel(p0, p1, acc[r][0], acc[r][1], f);
         tile_put(Ls + 64 * ((k + r) * (k + r - 1) / 2 + k), p0, p1);
         const int gr = 8 * (k + r) + g, c = 8 * k + 2 * tq;
         store_pair(Li + (long long)gr * n + c, vec, gr < n && c < n, gr < n && c + 1 < n, p0, p1);
       }
     // diagonal tile: C_kk and, above the diagonal, W^T
     const int gr = 8 * k + g, c = 8 * k + 2 * tq;
-    const double c0 = (double)Ct[2 * lane], c1 = (double)Ct[2 * lane + 1];
+    const double c0 = 2 * tq == g ? f.d0 : f.cv.x, c1 = 2 * tq + 1 == g ? f.d1 : f.cv.y;
     store_pair(Li + (long long)gr * n + c, vec, gr < n && c < n, gr < n && c + 1 < n,
                2 * tq <= g ? c0 : Iv[64 * k + 8 * (2 * tq) + g], 2 * tq + 1 <= g ? c1 : Iv[64 * k + 8 * (2 * tq + 1) + g]);
     __syncwarp();
@@ -177,10 +184,11 @@ __device__ __forceinline__ void node_warp_body(const Problem<T>& p, const Level&
 #pragma unroll 1
   for (int v = 0; v < vr + vl + vy; v += 2) {
     const RowSrc<T> s0 = source(v), s1 = source(v + 1);
+    T x[2][NT][2];
     double acc[2][NT][2];
-    rows_load<T, NT>(acc[0], s0, n, vec);
-    rows_load<T, NT>(acc[1], s1, n, vec);
-    warp_rows_solve<NT, 2>(acc, 0, nta, Ls, Iv);
+    rows_load<T, NT>(x[0], s0, n, vec);
+    rows_load<T, NT>(x[1], s1, n, vec);
+    warp_rows_solve<T, NT, 2>(acc, x, 0, nta, Ls, Iv, Ct);
     rows_store<T, NT>(acc[0], s0, n, vec);
     rows_store<T, NT>(acc[1], s1, n, vec);
   }
@@ -194,9 +202,10 @@ __device__ __forceinline__ void node_warp_body(const Problem<T>& p, const Level&
     o.ld = n;
     o.lim = n - 8 * c;
     o.k0 = c;
+    T x[1][NT][2];
     double acc[1][NT][2];
-    rows_load<T, NT>(acc[0], o, n, vec);
-    warp_rows_solve<NT, 1>(acc, c, nta, Ls, Iv);
+    rows_load<T, NT>(x[0], o, n, vec);
+    warp_rows_solve<T, NT, 1>(acc, x, c, nta, Ls, Iv, Ct);
     rows_store<T, NT>(acc[0], o, n, vec);
   }
 }
