@@ -17,8 +17,8 @@
 // of the previous level are needed.  Only the vectors go through shared memory.
 //
 // On a factor that carries W = C^{-1} (INV) the solve is one more product.
-// Otherwise it is a substitution by 8-row tiles: each warp inverts its diagonal
-// tile ahead of the vectors, the warps take turns.
+// Otherwise it is a substitution by 8-row tiles: the warps take turns; in FP64 a
+// lane solves a column against the tile, for floats the tile's FP64 inverse is an operand.
 #pragma once
 
 #include "node_rows.cuh"
@@ -93,8 +93,9 @@ __device__ __forceinline__ void block_frag(const T* M, int n, int i, int kk, boo
   }
 }
 
-// Operand of the solve, row tile i, column tile kk (0 outside its triangle).
-//   INV forward: W (strictly upper L transposed), backward: W^T; the diagonal is 1 / C[r][r].
+// Operand of the solve, row tile i, column tile kk (0 outside its strict triangle).
+//   INV forward: W (strictly upper L transposed), backward: W^T; their diagonal, 1 / C[r][r], is
+//   a factor of its own (solve_diag).
 //   Else forward: C left of the diagonal tile, backward: C^T right of it.
 template <typename T, bool BWD, bool INV>
 __device__ __forceinline__ void solve_frag(const T* L, int n, int i, int kk, bool vec, T& a0, T& a1) {
@@ -110,13 +111,16 @@ __device__ __forceinline__ void solve_frag(const T* L, int n, int i, int kk, boo
 #pragma unroll
   for (int e = 0; e < 2; ++e) {
     const int k = c + e;
-    const bool in = r < n && k < n;
-    const bool off = BWD ? k > r : k < r;
-    const T v = in && (off || k == r) ? (BWD ? L[(long long)r * n + k] : L[(long long)k * n + r]) : T(0);
-    a[e] = in && k == r ? T(1) / v : (off ? v : T(0));
+    a[e] = r < n && k < n && (BWD ? k > r : k < r) ? (BWD ? L[r * n + k] : L[k * n + r]) : T(0);
   }
   a0 = a[0];
   a1 = a[1];
+}
+// diagonal of C in this lane's row of row tile i
+template <typename T>
+__device__ __forceinline__ T solve_diag(const T* L, int n, int i) {
+  const int r = 8 * i + ((threadIdx.x & 31) >> 2);
+  return r < n ? L[r * n + r] : T(1);
 }
 
 // One vector, its columns col0 .. col0 + cols (a multiple of 8).  ONE: the block has a warp per
@@ -168,7 +172,7 @@ __device__ __forceinline__ void sweep_rows_body(const Group& grp, const Problem<
   }
   // fs: the solve's operands, by column tile (INV) or by step of the substitution; larger
   // blocks read them four steps at a time as they are used
-  T fp[NK][2], fq[NK][2], fs[KEEP ? NT : 4][2];
+  T fp[NK][2], fq[NK][2], fs[KEEP ? NT : 4][2], dc = T(1);
   auto load_solve = [&](int e0) {
 #pragma unroll
     for (int e = 0; e < (KEEP ? NT : 4); ++e) {
@@ -185,39 +189,51 @@ __device__ __forceinline__ void sweep_rows_body(const Group& grp, const Problem<
       if (P) block_frag<T, false>(P, n, warp, kk, vec && kk < nta, fp[KEEP ? kk : 0][0], fp[KEEP ? kk : 0][1]);
       if (Q) block_frag<T, true>(Q, n, warp, kk, vec && kk < nta, fq[KEEP ? kk : 0][0], fq[KEEP ? kk : 0][1]);
     }
-    if (solve) load_solve(0);
+    if (solve) {
+      load_solve(0);
+      if (INV) dc = solve_diag(L, n, warp);
+    }
   }
   if (!KEEP && solve)   // the solve's block is read after the products: into L2 meanwhile
     for (int e = grp.tid() * (128 / (int)sizeof(T)); e < n * n; e += grp.threads() * (128 / (int)sizeof(T)))
       asm volatile("prefetch.global.L2 [%0];\n" ::"l"(L + e));
-  double i0 = 0.0, i1 = 0.0;   // inverse of the diagonal tile (transposed for the backward sweep)
+  // The diagonal tile, for its own warp.  FP64: the tile with its pivots' reciprocals (forward: its
+  // transpose; padding: an identity), against which a lane solves a column.  Float: its inverse in
+  // FP64, exact beyond float's rounding, as an operand (i0, i1; transposed for the backward sweep).
+  constexpr bool SUBST = sizeof(T) == 8;
+  double* D = Iv + 64 * warp;
+  double i0 = 0.0, i1 = 0.0;
   if (!INV && solve && warp < nta) {
-    // every lane: column lane % 8 of C_kk^{-1}, from the tile in shared memory
-    double* D = Iv + 64 * warp;
-    {
-      T d0, d1;
-      block_frag<T, false>(L, n, warp, warp, vec, d0, d1);
-      const int r = 8 * warp + g, c = 8 * warp + 2 * t;   // padding: an identity
-      D[2 * lane] = r >= n && r == c ? 1.0 : (double)d0;
-      D[2 * lane + 1] = r >= n && r == c + 1 ? 1.0 : (double)d1;
+    T d0, d1;
+    block_frag<T, false>(L, n, warp, warp, vec, d0, d1);
+    const int r = 8 * warp + g, c = 8 * warp + 2 * t;
+    const double v0 = r >= n && r == c ? 1.0 : (double)d0, v1 = r >= n && r == c + 1 ? 1.0 : (double)d1;
+    if (SUBST) {
+      D[BWD ? 8 * g + 2 * t : 16 * t + g] = r == c ? 1.0 / v0 : v0;
+      D[BWD ? 8 * g + 2 * t + 1 : 16 * t + 8 + g] = r == c + 1 ? 1.0 / v1 : v1;
+    } else {
+      // every lane: column lane % 8 of C_kk^{-1}
+      D[2 * lane] = v0;
+      D[2 * lane + 1] = v1;
+      __syncwarp();
+      double y[8], rd[8];
+#pragma unroll
+      for (int a = 0; a < 8; ++a) rd[a] = 1.0 / D[9 * a];
+#pragma unroll
+      for (int a = 0; a < 8; ++a) {
+        double v = a == (lane & 7) ? 1.0 : 0.0;
+#pragma unroll
+        for (int c = 0; c < a; ++c) v = fma(-D[8 * a + c], y[c], v);
+        y[a] = v * rd[a];
+      }
+      __syncwarp();
+#pragma unroll
+      for (int a = 0; a < 8; ++a) D[8 * a + (lane & 7)] = y[a];
+      __syncwarp();
+      i0 = BWD ? D[8 * (2 * t) + g] : D[8 * g + 2 * t];
+      i1 = BWD ? D[8 * (2 * t + 1) + g] : D[8 * g + 2 * t + 1];
     }
     __syncwarp();
-    double y[8], rd[8];
-#pragma unroll
-    for (int a = 0; a < 8; ++a) rd[a] = 1.0 / D[9 * a];
-#pragma unroll
-    for (int a = 0; a < 8; ++a) {
-      double v = a == (lane & 7) ? 1.0 : 0.0;
-#pragma unroll
-      for (int c = 0; c < a; ++c) v = fma(-D[8 * a + c], y[c], v);
-      y[a] = v * rd[a];
-    }
-    __syncwarp();
-#pragma unroll
-    for (int a = 0; a < 8; ++a) D[8 * a + (lane & 7)] = y[a];
-    __syncwarp();
-    i0 = BWD ? D[8 * (2 * t) + g] : D[8 * g + 2 * t];
-    i1 = BWD ? D[8 * (2 * t + 1) + g] : D[8 * g + 2 * t + 1];
   }
   if (wait == kWaitVectors) pdl_wait();
   if (wait == kWaitFirst || wait == kWaitVectors) pdl_trigger();
@@ -312,6 +328,7 @@ __device__ __forceinline__ void sweep_rows_body(const Group& grp, const Problem<
         }
         y0 -= ap[q][0] + (CG == 1 ? aq[0][0] : 0.0);
         y1 -= ap[q][1] + (CG == 1 ? aq[0][1] : 0.0);
+        if (!FULL && r >= n) y0 = y1 = 0.0;   // (padding: zero times an infinity is not)
         if (!solve) {
           store_pair(yj + (long long)r * m + c, vecx && ok0, ok0, ok1, y0, y1);
         } else {
@@ -334,6 +351,7 @@ __device__ __forceinline__ void sweep_rows_body(const Group& grp, const Problem<
 #pragma unroll
         for (int q = 0; q < CG; ++q) ax[q][0] = ax[q][1] = ay[q][0] = ay[q][1] = 0.0;
         T fr[ONE ? 1 : NT][2];   // (all requested before the first is used)
+        if (!ONE) dc = solve_diag(L, n, i);
         if (!ONE)
 #pragma unroll
           for (int kk = 0; kk < NT; ++kk) {
@@ -360,8 +378,10 @@ __device__ __forceinline__ void sweep_rows_body(const Group& grp, const Problem<
         for (int q = 0; q < CG; ++q) {
           if (CG > 1 && q >= groups) break;
           const int r = 8 * i + g, c = c0 + 8 * q + 2 * t;
+          const double* Rr = Rs + r * ldz + 8 * q + 2 * t;   // (this lane's own)
+          const double rd = 1.0 / (double)dc;
           store_pair(yj + (long long)r * m + c, vecx && r < n && c < m, r < n && c < m, r < n && c + 1 < m,
-                     ax[q][0] + ay[q][0], ax[q][1] + ay[q][1]);
+                     fma(rd, Rr[0], ax[q][0] + ay[q][0]), fma(rd, Rr[1], ax[q][1] + ay[q][1]));
         }
       }
     } else {
@@ -369,6 +389,9 @@ __device__ __forceinline__ void sweep_rows_body(const Group& grp, const Problem<
       // unrolled at a time, the next four's operands requested before them (all steps unrolled
       // did not fit the instruction cache at n = 128: 3 us a step).
       constexpr int U = KEEP ? NT : 4;
+      double sum[ONE ? CG : 1][2];   // products with the rows solved so far, summed from zero
+#pragma unroll
+      for (int q = 0; q < (ONE ? CG : 1); ++q) sum[q][0] = sum[q][1] = 0.0;
       if (!KEEP && warp < nta) load_solve(0);
 #pragma unroll 1
       for (int s0 = 0; s0 < nta; s0 += U) {
@@ -384,29 +407,49 @@ __device__ __forceinline__ void sweep_rows_body(const Group& grp, const Problem<
           const int st = s0 + h, kk = BWD ? nta - 1 - st : st;
           if (st < nta) {
             if (warp == kk) {
+              double* Rk = Rs + 8 * kk * ldz;
 #pragma unroll
               for (int q = 0; q < CG; ++q) {
                 if (CG > 1 && q >= groups) break;
-                Rs[(8 * kk + g) * ldz + 8 * q + 2 * t] = ys[ONE ? q : 0][0];
-                Rs[(8 * kk + g) * ldz + 8 * q + 2 * t + 1] = ys[ONE ? q : 0][1];
+                Rk[g * ldz + 8 * q + 2 * t] = ys[ONE ? q : 0][0] - sum[ONE ? q : 0][0];
+                Rk[g * ldz + 8 * q + 2 * t + 1] = ys[ONE ? q : 0][1] - sum[ONE ? q : 0][1];
               }
               __syncwarp();
+              if (SUBST) {
+                if (lane < 8 * groups) {
+                  double z[8];
 #pragma unroll
-              for (int q = 0; q < CG; ++q) {
-                if (CG > 1 && q >= groups) break;
-                double x0 = 0.0, x1 = 0.0;
-                const int zo = (8 * kk + 2 * t) * ldz + 8 * q + g;
-                mma_acc(x0, x1, i0, Rs[zo]);
-                mma_acc(x0, x1, i1, Rs[zo + ldz]);
-                ys[ONE ? q : 0][0] = x0;
-                ys[ONE ? q : 0][1] = x1;
-              }
-              __syncwarp();
+                  for (int a = 0; a < 8; ++a) z[a] = Rk[a * ldz + lane];
 #pragma unroll
-              for (int q = 0; q < CG; ++q) {
-                if (CG > 1 && q >= groups) break;
-                Rs[(8 * kk + g) * ldz + 8 * q + 2 * t] = ys[ONE ? q : 0][0];
-                Rs[(8 * kk + g) * ldz + 8 * q + 2 * t + 1] = ys[ONE ? q : 0][1];
+                  for (int e = 0; e < 8; ++e) {
+                    const int a = BWD ? 7 - e : e;
+                    z[a] *= D[9 * a];
+                    Rk[a * ldz + lane] = z[a];
+#pragma unroll
+                    for (int h = 0; h < 8; h += 2) {
+                      const double2 c = *reinterpret_cast<const double2*>(D + 8 * a + h);
+                      if (BWD ? h < a : h > a) z[h] = fma(-c.x, z[a], z[h]);
+                      if (BWD ? h + 1 < a : h + 1 > a) z[h + 1] = fma(-c.y, z[a], z[h + 1]);
+                    }
+                  }
+                }
+              } else {
+                double x[ONE ? CG : 1][2];
+#pragma unroll
+                for (int q = 0; q < CG; ++q) {
+                  if (CG > 1 && q >= groups) break;
+                  double(&xq)[2] = x[ONE ? q : 0];
+                  xq[0] = xq[1] = 0.0;
+                  mma_acc(xq[0], xq[1], i0, Rk[2 * t * ldz + 8 * q + g]);
+                  mma_acc(xq[0], xq[1], i1, Rk[(2 * t + 1) * ldz + 8 * q + g]);
+                }
+                __syncwarp();
+#pragma unroll
+                for (int q = 0; q < CG; ++q) {
+                  if (CG > 1 && q >= groups) break;
+                  Rk[g * ldz + 8 * q + 2 * t] = x[ONE ? q : 0][0];
+                  Rk[g * ldz + 8 * q + 2 * t + 1] = x[ONE ? q : 0][1];
+                }
               }
             }
             grp.sync();
@@ -415,8 +458,8 @@ __device__ __forceinline__ void sweep_rows_body(const Group& grp, const Problem<
               for (int q = 0; q < CG; ++q) {
                 if (CG > 1 && q >= groups) break;
                 const int zo = (8 * kk + 2 * t) * ldz + 8 * q + g;
-                mma_acc(ys[ONE ? q : 0][0], ys[ONE ? q : 0][1], -(double)cur[h][0], Rs[zo]);
-                mma_acc(ys[ONE ? q : 0][0], ys[ONE ? q : 0][1], -(double)cur[h][1], Rs[zo + ldz]);
+                mma_acc(sum[ONE ? q : 0][0], sum[ONE ? q : 0][1], (double)cur[h][0], Rs[zo]);
+                mma_acc(sum[ONE ? q : 0][0], sum[ONE ? q : 0][1], (double)cur[h][1], Rs[zo + ldz]);
               }
             }
           }
@@ -428,7 +471,7 @@ __device__ __forceinline__ void sweep_rows_body(const Group& grp, const Problem<
           if (CG > 1 && q >= groups) break;
           const int r = 8 * warp + g, c = c0 + 8 * q + 2 * t;
           store_pair(yj + (long long)r * m + c, vecx && r < n && c < m, r < n && c < m, r < n && c + 1 < m,
-                     ys[ONE ? q : 0][0], ys[ONE ? q : 0][1]);
+                     Rs[r * ldz + 8 * q + 2 * t], Rs[r * ldz + 8 * q + 2 * t + 1]);
         }
       }
     }

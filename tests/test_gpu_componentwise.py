@@ -16,7 +16,11 @@ import numpy as np
 import pytest
 import torch
 
-from socu_b200.block_tridiag_solver import create_cholesky_factor_launch
+from socu_b200.block_tridiag_solver import (
+    create_cholesky_backward_substitution_launch,
+    create_cholesky_factor_launch,
+    create_cholesky_forward_substitution_launch,
+)
 from socu_b200.ragged import RaggedBatch, create_ragged_factor_and_solve_launch
 
 pytestmark = pytest.mark.gpu
@@ -35,6 +39,28 @@ def _tile(n, a):
 def _ok(got, want, scale, bound):
     r = np.abs(got - want)
     assert (r <= bound * scale).all(), float((r[scale > 0] / scale[scale > 0]).max() / bound)
+
+
+@pytest.mark.parametrize("dtype", [torch.float64, torch.float32])
+@pytest.mark.parametrize("m", [1, 8, 19])
+@pytest.mark.parametrize("n", [5, 8, 29, 32, 64, 65, 100, 128])
+def test_sweeps_on_a_plain_factor(dtype, n, m):
+    rng = np.random.default_rng(n)
+    C = np.tril(rng.standard_normal((n, n)) * 0.5 / np.sqrt(n), -1)
+    for k in range(0, n, 8):
+        e = min(n, k + 8)
+        C[k:e, k:e] = _tile(e - k, 4.3)
+    C = C.astype(NP[dtype])
+    x0 = rng.standard_normal((n, m))
+    E = torch.zeros(0, n, n, dtype=dtype, device="cuda")
+    Cl = C.astype(np.longdouble)
+    for make, M in ((create_cholesky_forward_substitution_launch, Cl), (create_cholesky_backward_substitution_launch, Cl.T)):
+        b = (M @ x0).astype(NP[dtype])
+        L, x = torch.tensor(C[None], device="cuda"), torch.tensor(b[None], device="cuda")
+        make(L, E, x, dtype=dtype)()
+        torch.cuda.synchronize()
+        xl = x[0].cpu().numpy().astype(np.longdouble)
+        _ok(M @ xl, b, np.abs(M) @ np.abs(xl), _bound(dtype, n))
 
 
 def _spd(n, a, seed, np_dtype):
