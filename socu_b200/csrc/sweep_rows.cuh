@@ -362,7 +362,7 @@ __device__ __forceinline__ void sweep_rows_body(const Group& grp, const Problem<
           }
 #pragma unroll
         for (int kk = 0; kk < NT; ++kk) {
-          if (ONE ? kk < nta : (BWD ? kk >= i && kk < nta : kk <= i)) {
+          if (BWD ? kk >= i && kk < nta : kk <= i) {   // (the triangle only: zero times an infinity is not zero)
             const T f0 = ONE ? fs[KEEP ? kk : 0][0] : fr[ONE ? 0 : kk][0];
             const T f1 = ONE ? fs[KEEP ? kk : 0][1] : fr[ONE ? 0 : kk][1];
             const int zo = (8 * kk + 2 * t) * ldz + g;
