@@ -489,9 +489,18 @@ __host__ __device__ inline int sweep_tasks(int N, const Level& lv) {
 #endif
 }
 
+// Blocks per SM that the registers are cut for.  Blocks of up to 24 rows hold few operands, and wide
+// levels want warps: 28 an SM (21 at three tiles, where 75 registers spilt) against 16.  FP64 solve on
+// factors with inverses, 33 x (N = 882, n = 10, m = 1): 211 -> 145 us, 100 x (N = 512, m = 1) at n = 12
+// 324 -> 233, at n = 20 583 -> 502.  At three tiles the substitution needs more registers (24 x (N = 63,
+// n = 17, m = 3): 51 us with 16 warps, 58 with 21).
+__host__ __device__ constexpr int sweep_blocks(int nt, bool inv) {
+  return nt <= 2 ? 28 / nt : (inv && nt == 3 ? 7 : (nt <= 8 ? 16 / nt : 1));
+}
+
 // cols: columns per block; on narrow levels several blocks (along y) share a vector's right-hand sides
 template <typename T, int NT, bool FULL, int MODE, bool INV>
-__global__ void __launch_bounds__(32 * NT, NT <= 8 ? 16 / NT : 1)
+__global__ void __launch_bounds__(32 * NT, sweep_blocks(NT, INV))
     k_sweep_rows(Problem<T> p, Level lv, int wait, int cols) {
   const int per_b = sweep_tasks<MODE>(p.N, lv);
   const int b = blockIdx.x / per_b;
