@@ -115,8 +115,10 @@ cudaError_t prepare(K kernel, size_t smem) {
 
 int sm_count() {
   int dev = 0, sms = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+  if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) {
+    (void)cudaGetLastError();   // (no device: kernels are only counted)
     return 0;
+  }
   return sms;
 }
 
@@ -413,6 +415,13 @@ cudaError_t launch_residual_rows(const RefineArgs& a, cudaStream_t st, bool pdl)
   return e;
 }
 
+// Right-hand sides per block of a sweep over `vecs` vectors: halved while all blocks fit `room` SMs.
+int sweep_columns(int m, long long vecs, long long room) {
+  int cols = 8 * std::max(1, ceil_div(m, 8));
+  while (cols > 8 && vecs * ceil_div(m, 8 * ceil_div(cols, 16)) <= room) cols = 8 * ceil_div(cols, 16);
+  return cols;
+}
+
 // Enqueue (or count, when st == nullptr and count != nullptr) the kernels of one op.
 // inv: the factor carries (FACTOR, FACTOR_AND_SOLVE) or has (SOLVE) its
 // diagonal inverses; only for internal factors or within factor_and_solve.
@@ -465,13 +474,13 @@ int enqueue(socu_op op, const Problem<T>& p, cudaStream_t st, long long* count, 
   const NodeRowsFn<T> rows_kernel = node_rows_kernel<T>(n, full);
   long long launches = 0;
   const bool run = count == nullptr;
-  const int sms = run ? sm_count() : 0;
+  const int sms = sm_count();
 
   if (run) {
     cudaError_t e = cudaSuccess;
     if (op == SOCU_OP_FACTOR || op == SOCU_OP_FACTOR_AND_SOLVE) {
       e = prepare(rows_kernel, sd_rows);
-      if (e == cudaSuccess) e = prepare(update_kernel, su);
+      if (e == cudaSuccess) e = prepare(update_kernel, withY ? std::max(su, ss_pull) : su);
       if (e == cudaSuccess && upd_tc) e = prepare(k_update_tc, su_tc);
       if (e == cudaSuccess && node_tc_any) e = prepare(node_tc_kernel, sd_tc);
       if (e == cudaSuccess && node_tm) e = prepare(node_tm_kernel, sd_tm);
@@ -500,9 +509,8 @@ int enqueue(socu_op op, const Problem<T>& p, cudaStream_t st, long long* count, 
   // 8, 16, ... right-hand sides share a vector (each reads the vector's blocks,
   // from L2; the products, which bound the block, are shared out).
   auto go_sweep = [&](SweepFn<T> kernel, int kind, long long vecs, size_t smem, const Level& L, SweepWait wait) {
-    int cols = 8 * ceil_div(p.m, 8);
-    while (cols > 8 && vecs * ceil_div(p.m, 8 * ceil_div(cols, 16)) <= sms) cols = 8 * ceil_div(cols, 16);
     if (vecs <= 0) return;
+    const int cols = sweep_columns(p.m, vecs, sms);
     ++launches;
     if (!run) return;
     const bool pdl = !first && g_prof == nullptr;
@@ -611,25 +619,28 @@ int enqueue(socu_op op, const Problem<T>& p, cudaStream_t st, long long* count, 
         go_rows(node_blocks, L);
       }
       if (l + 1 < K) {
+        // Schur update, and in factor_and_solve the forward pull of this level's
+        // nodes on every target vector.  Neither needs the other, but a kernel
+        // may read the nodes only behind its own wait for all before it: where
+        // both fit the SMs at once, one launch does both (N = 100, n = 32: 96 -> 88 us,
+        // N = 1024, n = 64, m = 8: 425 -> 412); wide levels take two.
         const long long upd_blocks = (long long)p.B * update_blocks(p.N, L);
-        bool tc_done = false;
-        if constexpr (sizeof(T) == 4) {
-          if (upd_tc) {
-            go_on(st, k_update_tc, SOCU_KIND_UPDATE, upd_blocks, su_tc, L, 256);
-            tc_done = true;
-          }
-        }
-        if (!tc_done) {
+        const long long pull_vecs = withY ? (long long)p.B * (p.N / lv[l + 1].s) : 0;
+        bool pulled = false;
+        if (upd_tc) {
+          if constexpr (sizeof(T) == 4) go_on(st, k_update_tc, SOCU_KIND_UPDATE, upd_blocks, su_tc, L, 256);
+        } else {
           // narrow levels: several blocks per output block (k_update_rows)
           int splits = 1;
           while (splits < 8 && splits * 2 <= ceil_div(n, 8) && upd_blocks * splits * 2 <= sms) splits *= 2;
-          go_on(st, update_kernel, SOCU_KIND_UPDATE, upd_blocks * splits, su, L, 32 * update_rows_warps(n, splits),
-                splits);
+          const long long upd = upd_blocks * splits;
+          const int cols = sweep_columns(p.m, pull_vecs, sms - upd), chunks = ceil_div(p.m, cols);
+          pulled = pull_vecs > 0 && upd + pull_vecs * chunks <= sms;
+          go_on(st, update_kernel, SOCU_KIND_UPDATE, upd + (pulled ? pull_vecs * chunks : 0),
+                pulled ? std::max(su, ss_pull) : su, L, 32 * update_rows_warps(n, splits), splits, (int)upd, lv[l + 1],
+                chunks, cols);
         }
-        // Fused forward: apply this level's updates to every target vector.  It
-        // only depends on the node, as the update does, and runs beside it.
-        const long long pull_blocks = withY ? (long long)p.B * (p.N / lv[l + 1].s) : 0;
-        go_sweep(pull_kernel, SOCU_KIND_PULL, pull_blocks, ss_pull, lv[l + 1], kWaitEnd);
+        if (!pulled) go_sweep(pull_kernel, SOCU_KIND_PULL, pull_vecs, ss_pull, lv[l + 1], kWaitFirst);
       }
     }
   }

@@ -30,15 +30,8 @@ enum SweepMode { kModeForward = 0, kModeBackward = 1, kModePull = 2 };
 enum SweepWait {
   kWaitNone = 0,    // called inside another kernel
   kWaitFirst = 1,   // the blocks themselves come from the previous kernel
-  kWaitVectors = 2, // the blocks were complete before: only the vectors are waited for
-  kWaitEnd = 3      // nothing comes from the previous kernel, see below
+  kWaitVectors = 2  // the blocks were complete before: only the vectors are waited for
 };
-// kWaitEnd: the pull of factor_and_solve needs a level's nodes and is launched
-// behind their Schur update, which gives it nothing.  The update's blocks let
-// their successor start only after their own wait for the nodes, so the nodes'
-// results are complete when the pull runs: it works beside the update and waits
-// for it at its end, so that whatever waits for the pull has waited for both.
-
 // columns per pass: 8 up to n = 64, where the blocks stay in registers between passes, else 32
 __host__ __device__ constexpr int sweep_cols(int nt) { return nt <= 8 ? 8 : 32; }
 // stride of a staged vector row: 2 (mod 8) doubles, so the two rows of an operand pair and the
@@ -166,10 +159,6 @@ __device__ __forceinline__ void sweep_rows_body(const Group& grp, const Problem<
   double* Iv = Rs + 8 * NT * ldz;
 
   if (wait == kWaitFirst) pdl_wait();
-  if (wait == kWaitEnd) {
-    __threadfence();
-    pdl_trigger();
-  }
   // fs: the solve's operands, by column tile (INV) or by step of the substitution; larger
   // blocks read them four steps at a time as they are used
   T fp[NK][2], fq[NK][2], fs[KEEP ? NT : 4][2], dc = T(1);
@@ -476,7 +465,6 @@ __device__ __forceinline__ void sweep_rows_body(const Group& grp, const Problem<
       }
     }
   }
-  if (wait == kWaitEnd) pdl_wait();
 }
 
 // vectors of one level per instance

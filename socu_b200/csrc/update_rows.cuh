@@ -22,7 +22,7 @@
 // tile keeps its contraction order, so the bits do not depend on the split.
 #pragma once
 
-#include "node_rows.cuh"
+#include "sweep_rows.cuh"
 
 namespace socu {
 
@@ -216,16 +216,26 @@ __device__ __forceinline__ void update_rows_body(const Group& grp, const Problem
   }
 }
 
+// The first `upd` blocks update; any others are the forward pull that factor_and_solve needs of the
+// same nodes, `chunks` blocks of `cols` right-hand sides to a vector of level `next`.
 template <typename T, int NT, bool FULL>
 __global__ void __launch_bounds__(NT <= 8 ? 256 : 512, NT <= 8 ? 2 : 1)
-    k_update_rows(Problem<T> p, Level lv, int splits) {
+    k_update_rows(Problem<T> p, Level lv, int splits, int upd, Level next, int chunks, int cols) {
+  pdl_wait();
+  pdl_trigger();
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  if ((int)blockIdx.x >= upd) {
+    const int v = (blockIdx.x - upd) / chunks, q = blockIdx.x - upd - v * chunks;
+    const int per_b = sweep_tasks<kModePull>(p.N, next), b = v / per_b;
+    if (p.active(b))
+      sweep_rows_body<T, NT, FULL, kModePull, true, true>(BlockGroup{}, p, next, b, v - b * per_b, smem_raw, kWaitNone,
+                                                          q * cols, cols);
+    return;
+  }
   const int block = blockIdx.x / splits, q = blockIdx.x - block * splits;
   const int per_b = update_blocks(p.N, lv);
   const int b = block / per_b, task = block - b * per_b;
-  pdl_wait();
-  pdl_trigger();
   if (!p.active(b)) return;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
   if (splits > 1)
     update_rows_body<T, NT, FULL, true>(BlockGroup{}, p, lv, b, task, smem_raw, q, splits);
   else
@@ -233,7 +243,7 @@ __global__ void __launch_bounds__(NT <= 8 ? 256 : 512, NT <= 8 ? 2 : 1)
 }
 
 template <typename T>
-using UpdateRowsFn = void (*)(Problem<T>, Level, int);
+using UpdateRowsFn = void (*)(Problem<T>, Level, int, int, Level, int, int);
 
 template <typename T>
 UpdateRowsFn<T> update_rows_kernel(int n, bool full);
