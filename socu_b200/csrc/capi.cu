@@ -1189,11 +1189,16 @@ int rg_create(socu_ragged_s* r, const int64_t* horizon, const int64_t* n, const 
     const int c = rg_chunks(rg_phase(r->inst[i], mode, 0));
     for (int j = 0; j < c; ++j) init.push_back(rg_encode(i, 0, j));
   }
-  // Few nodes per warp worker: block workers (rg_use_blocks).
   const int es = r->refine ? 4 : (r->dtype == SOCU_FLOAT64 ? 8 : 4);
-  long long nodes = 0;
-  for (const RgInst& I : r->inst) nodes += I.N;
-  r->blocks = rg_use_blocks(nodes, sm_count());
+  double load = 0.0;
+  unsigned bodies = 0;
+  for (const RgInst& I : r->inst) {
+    load += I.N / rg_warp_nodes(I.n);
+    bodies |= 1u << (2 * (rg_nt(I.n) - 1) + (I.n % 8 != 0));
+  }
+  int sizes = 0;
+  for (; bodies != 0; bodies &= bodies - 1) ++sizes;
+  r->blocks = rg_use_blocks(load, sizes, sm_count());
   size_t smem = 0;
   for (const RgInst& I : r->inst) {
     smem = std::max(smem, (size_t)rg_block_bytes(I.n, es, r->refine, r->blocks));

@@ -202,10 +202,14 @@ struct WarpGroup {
   }
 };
 
-// two consecutive elements, widened; `vec`: the pair is aligned and inside
+// two consecutive elements, widened; `vec`: the pair is aligned and inside; `pair`: it is aligned
+// and, where its first element is inside, all of it
 template <typename T>
-__device__ __forceinline__ void load_pair(const T* p, bool vec, bool v0, bool v1, double& x0, double& x1) {
-  if (vec) {
+__device__ __forceinline__ void load_pair(const T* p, bool vec, bool v0, bool v1, double& x0, double& x1,
+                                          bool pair = false) {
+  if (pair && !vec && !v0) {
+    x0 = x1 = 0.0;
+  } else if (vec || pair) {
     if constexpr (sizeof(T) == 8) {
       const double2 v = *reinterpret_cast<const double2*>(p);
       x0 = v.x;
@@ -220,10 +224,12 @@ __device__ __forceinline__ void load_pair(const T* p, bool vec, bool v0, bool v1
     x1 = v1 ? (double)p[1] : 0.0;
   }
 }
-// two consecutive elements as they are; `vec`: the pair is aligned and inside
+// two consecutive elements as they are
 template <typename T>
-__device__ __forceinline__ void load_raw(const T* p, bool vec, bool v0, bool v1, T (&x)[2]) {
-  if (vec) {
+__device__ __forceinline__ void load_raw(const T* p, bool vec, bool v0, bool v1, T (&x)[2], bool pair = false) {
+  if (pair && !vec && !v0) {
+    x[0] = x[1] = T(0);
+  } else if (vec || pair) {
     if constexpr (sizeof(T) == 8) {
       const double2 v = *reinterpret_cast<const double2*>(p);
       x[0] = v.x;
@@ -240,22 +246,26 @@ __device__ __forceinline__ void load_raw(const T* p, bool vec, bool v0, bool v1,
 }
 
 template <typename T>
-__device__ __forceinline__ void store_pair(T* p, bool vec, bool v0, bool v1, double x0, double x1) {
-  if (vec) {
+__device__ __forceinline__ void store_pair(T* p, bool vec, bool v0, bool v1, double x0, double x1, bool pair = false) {
+  if (vec || (pair && v0)) {
     if constexpr (sizeof(T) == 8)
       *reinterpret_cast<double2*>(p) = make_double2(x0, x1);
     else
       *reinterpret_cast<float2*>(p) = make_float2((float)x0, (float)x1);
-  } else {
+  } else if (!pair) {
     if (v0) p[0] = (T)x0;
     if (v1) p[1] = (T)x1;
   }
 }
 
-// Whole 8x8 tiles, and every row of a block on a pair boundary.
+// Every row of a block on a pair boundary; and whole 8x8 tiles besides.
+template <typename T>
+__host__ __device__ __forceinline__ bool rows_paired(const Problem<T>& p, int n) {
+  return (n & 1) == 0 && ((reinterpret_cast<uintptr_t>(p.L) | reinterpret_cast<uintptr_t>(p.E)) & (2 * sizeof(T) - 1)) == 0;
+}
 template <typename T>
 __host__ __device__ __forceinline__ bool pairs_ok(const Problem<T>& p, int n) {
-  return (n & 7) == 0 && ((reinterpret_cast<uintptr_t>(p.L) | reinterpret_cast<uintptr_t>(p.E)) & (2 * sizeof(T) - 1)) == 0;
+  return (n & 7) == 0 && rows_paired(p, n);
 }
 
 // A row tile outside L_i: element (r, c) of X, r < lim, at base[r * rs + c * cs].
@@ -309,7 +319,7 @@ __device__ __forceinline__ void rows_panel(double& p0, double& p1, double x0, do
 }
 
 // (identity rows start at their own step: tile k0 is the identity, later tiles zero)
-template <typename T, int NT>
+template <typename T, int NT, bool PAIR = false>
 __device__ __forceinline__ void rows_load(T (&x)[NT][2], const RowSrc<T>& s, int n, bool vec) {
   const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
   const bool rv = g < s.lim;
@@ -317,7 +327,7 @@ __device__ __forceinline__ void rows_load(T (&x)[NT][2], const RowSrc<T>& s, int
 #pragma unroll
     for (int j = 0; j < NT; ++j) {
       const int c = 8 * j + 2 * t;
-      load_raw(s.base + (g * s.ld + c), vec && 8 * j < n, rv && c < n, rv && c + 1 < n, x[j]);
+      load_raw(s.base + (g * s.ld + c), vec && 8 * j < n, rv && c < n, rv && c + 1 < n, x[j], PAIR);
     }
   } else if (s.kind == 1) {
 #pragma unroll
@@ -336,7 +346,7 @@ __device__ __forceinline__ void rows_load(T (&x)[NT][2], const RowSrc<T>& s, int
   }
 }
 
-template <typename T, int NT>
+template <typename T, int NT, bool PAIR = false>
 __device__ __forceinline__ void rows_store(const double (&acc)[NT][2], const RowSrc<T>& s, int n, bool vec) {
   const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
   const bool rv = g < s.lim;
@@ -355,7 +365,7 @@ __device__ __forceinline__ void rows_store(const double (&acc)[NT][2], const Row
     for (int j = 0; j < NT; ++j) {
       const int c = 8 * j + 2 * t;
       if (j >= j0)
-        store_pair(s.base + (g * s.ld + c), vec && 8 * j < n, rv && c < n, rv && c + 1 < n, acc[j][0], acc[j][1]);
+        store_pair(s.base + (g * s.ld + c), vec && 8 * j < n, rv && c < n, rv && c + 1 < n, acc[j][0], acc[j][1], PAIR);
     }
   }
 }
@@ -411,8 +421,8 @@ __device__ __forceinline__ void rows_solve(double (&acc)[NT][2], const T (&x)[NT
 
 // One node.  q, splits: this block's share of the row tiles outside L_i (every
 // block of a cluster runs phase 1).  Warp w < n / 8 of the group owns row tile w of L_i.
-// FULL: n is 8 NT and pairs are aligned, so sizes and offsets are constants.
-template <typename T, int NT, bool FULL, bool EXACT, class Group>
+// FULL: n is 8 NT and pairs are aligned, so sizes and offsets are constants.  PAIR: rows_paired holds.
+template <typename T, int NT, bool FULL, bool EXACT, bool PAIR = false, class Group>
 __device__ __forceinline__ void node_rows_body(const Group& grp, const Problem<T>& p, const Level& lv, int b, int t,
                                                unsigned char* smem_raw, int q, int splits, bool with_y, bool inv) {
   constexpr int ld = (NT & 1) ? 8 * NT : 8 * NT + 8;
@@ -429,7 +439,7 @@ __device__ __forceinline__ void node_rows_body(const Group& grp, const Problem<T
   T* Lf = left ? p.Eb(b, lv.oc + 2 * t - 1) : nullptr;
   T* yi = with_y ? p.Xb(b, i) : nullptr;
   // paired accesses: whole tiles, and every row of a block on a pair boundary
-  const bool vec = FULL || pairs_ok(p, n);
+  const bool vec = FULL || (NT > 8 && pairs_ok(p, n));   // (up to 64: NT is exact, whole tiles are FULL)
   const int vr = right ? nta : 0, vl = left ? nta : 0, vy = with_y ? (p.m + 7) >> 3 : 0;
   const int vtot = vr + vl + vy + nta;
   auto source = [&](int v) {
@@ -478,7 +488,7 @@ __device__ __forceinline__ void node_rows_body(const Group& grp, const Problem<T
       x[j][0] = x[j][1] = 0.0;
       if (row < nta && j <= row) {
         const int c = 8 * j + 2 * tq;
-        load_pair(Li + (long long)gr * n + c, vec, gr < n && c < n, gr < n && c + 1 < n, x[j][0], x[j][1]);
+        load_pair(Li + (long long)gr * n + c, vec, gr < n && c < n, gr < n && c + 1 < n, x[j][0], x[j][1], PAIR);
         if (!vec && gr >= n) {
           if (c == gr) x[j][0] = 1.0;
           if (c + 1 == gr) x[j][1] = 1.0;
@@ -540,7 +550,7 @@ __device__ __forceinline__ void node_rows_body(const Group& grp, const Problem<T
       for (int j = 0; j < row; ++j) {
         const double2 v = *reinterpret_cast<const double2*>(Cs + gr * ld + 8 * j + 2 * tq);
         const int c = 8 * j + 2 * tq;
-        store_pair(Li + (long long)gr * n + c, vec, gr < n && c < n, gr < n && c + 1 < n, v.x, v.y);
+        store_pair(Li + (long long)gr * n + c, vec, gr < n && c < n, gr < n && c + 1 < n, v.x, v.y, PAIR);
       }
       // diagonal tile: C_kk and, above the diagonal, W^T (or zeros)
       const double* Ik = Iv + 64 * row;
@@ -548,7 +558,7 @@ __device__ __forceinline__ void node_rows_body(const Group& grp, const Problem<T
       const int c = 8 * row + 2 * tq;
       const double u0 = inv ? Ik[8 * (2 * tq) + g] : 0.0, u1 = inv ? Ik[8 * (2 * tq + 1) + g] : 0.0;
       store_pair(Li + (long long)gr * n + c, vec, gr < n && c < n, gr < n && c + 1 < n, 2 * tq <= g ? c0 : u0,
-                 2 * tq + 1 <= g ? c1 : u1);
+                 2 * tq + 1 <= g ? c1 : u1, PAIR);
       if (p.info != nullptr) {
         const double dg = (g & 1) ? c1 : c0;   // lanes with t = g / 2 hold the diagonal
         const bool bad = (g >> 1) == tq && gr < n && (!(dg > 0.0) || isinf(dg));
@@ -560,7 +570,7 @@ __device__ __forceinline__ void node_rows_body(const Group& grp, const Problem<T
   }
   // (the first row tile arrives while later rows finish phase 1)
   T xv[NT][2];
-  if (v_first < vtot) rows_load<T, NT>(xv, source(v_first), n, vec);
+  if (v_first < vtot) rows_load<T, NT, PAIR>(xv, source(v_first), n, vec);
   grp.sync();   // the factor is complete in shared memory
 
   // phase 2
@@ -569,17 +579,17 @@ __device__ __forceinline__ void node_rows_body(const Group& grp, const Problem<T
     if (src.kind == 3) {   // no inverse kept: zeros right of the diagonal tile
       for (int k = src.k0 + 1; k < nta; ++k) {
         const int c = 8 * k + 2 * tq;
-        store_pair(src.base + (long long)g * n + c, vec, g < src.lim && c < n, g < src.lim && c + 1 < n, 0.0, 0.0);
+        store_pair(src.base + (long long)g * n + c, vec, g < src.lim && c < n, g < src.lim && c + 1 < n, 0.0, 0.0, PAIR);
       }
       continue;
     }
-    if (v != v_first) rows_load<T, NT>(xv, src, n, vec);
+    if (v != v_first) rows_load<T, NT, PAIR>(xv, src, n, vec);
     double av[NT][2];
     if (src.kind == 2)
       rows_solve<T, NT, false, EXACT>(av, xv, src.k0, nta, Cs, Iv, Ct);
     else
       rows_solve<T, NT, true, EXACT>(av, xv, 0, nta, Cs, Iv, Ct);
-    rows_store<T, NT>(av, src, n, vec);
+    rows_store<T, NT, PAIR>(av, src, n, vec);
   }
 }
 

@@ -26,7 +26,7 @@
 // In a small batch the levels of its largest systems, one after another, are
 // the time: there a thread block of eight warps is the worker, and a unit gets a
 // warp per 8-row tile (smaller blocks run side by side, rg_group_warps).  The
-// host chooses by the nodes per warp worker (rg_use_blocks).  UPD of the plain
+// host chooses (rg_use_blocks).  UPD of the plain
 // path also applies the fused forward pull of the next level (the uniform
 // factor_and_solve launches it separately).
 //
@@ -152,7 +152,7 @@ __host__ __device__ inline RgPhase rg_phase(const RgInst& I, int mode, int ph) {
   } else {
     r.kind = kRgRes;
     r.level = 0;
-    r.units = I.N;   // block rows (n <= 64: one CTA pass per row)
+    r.units = I.N;   // block rows
   }
   return r;
 }
@@ -293,8 +293,9 @@ __device__ __forceinline__ RefineArgs rg_refine_args(const RgArgs<T>& a, const R
   return r;
 }
 
-// Tile counts the bodies are built for.
-__host__ __device__ inline int rg_nt(int n) { return n <= 8 ? 1 : (n <= 16 ? 2 : (n <= 32 ? 4 : (n <= 48 ? 6 : 8))); }
+// Tile counts the bodies are built for: every one, as a body for more tiles than the block has tests
+// every step, which keeps the steps from overlapping.
+__host__ __device__ inline int rg_nt(int n) { return (n + 7) / 8; }
 // Block workers: warps per unit, one per 8-row tile, as a power of two.
 __host__ __device__ inline int rg_group_warps(int n) { return n <= 8 ? 1 : (n <= 16 ? 2 : (n <= 32 ? 4 : 8)); }
 // Shared memory of one unit (bytes) for blocks of size n.
@@ -316,54 +317,67 @@ __host__ __device__ inline long long rg_block_bytes(int n, int es, bool refine, 
   const long long v = rg_unit_bytes(n, es, refine, blocks);
   return v * (blocks ? kRgBlockWarps / rg_group_warps(n) : kRgWorkers);
 }
-// Block workers for batches with few nodes per warp worker (12 of those per SM).  Measured in
-// FP64 on N ~ U{8..256}, n in {8, 16, 32, 48}, m in {1, 4} (132 nodes a system), warp against
-// block workers, ms: 16 systems 1.28 / 0.55, 64 1.51 / 0.95, 128 2.07 / 1.82, 512 4.56 / 6.54,
-// 1024 7.6 / 11.8; on either side of the line (240 such systems) 190 take 2.54 on blocks and 256
-// 2.88 on warps.
-__host__ __device__ inline bool rg_use_blocks(long long nodes, int sms) { return nodes < 18LL * 12 * sms; }
+// Block or warp workers.  Blocks of size n alone want this many nodes per SM before single warps beat
+// thread blocks (measured at 32 to 512 systems of N ~ U{8..256}, FP64, float and refined, the crossings
+// of the three within a third of each other): many where a power of two of warps has no idle one (one,
+// two and four tiles; eight never), few where it has (three, five and six tiles); half as many more where
+// the last tile is not whole.
+__host__ inline double rg_warp_nodes(int n) {
+  constexpr double kNodes[] = {360, 180, 80, 110, 50, 55, 150, 1e9};
+  return kNodes[rg_nt(n) - 1] * (n % 8 == 0 ? 1.0 : 1.4);
+}
+// `load` sums nodes / rg_warp_nodes over the batch; `sizes` counts its different bodies (tile count, whole
+// or not): the warps of an SM run different ones at a time, which the instruction cache does not hold.
+// Crossings in systems, measured and by this rule: {24, 40} 55, 116; {12, 36} 150 to 300, 207;
+// {8, 16, 32, 48} 220 to 450, 356; {8, 16, ..., 64} 512 and more, 566.
+// Times at 256 systems, warp / block workers: n = 40 3.1 / 6.2 ms FP64, 5.8 / 11.5 refined; n = 64
+// 9.0 / 8.4 ms float; n ~ U{4..64} 14.7 / 5.6 ms float.
+__host__ inline bool rg_use_blocks(double load, int sizes, int sms) {
+  return load < sms * sqrt(sizes * sqrt((double)sizes));
+}
 
-// One unit of a level phase (one copy of each per tile count: the kernel calls them).
-template <typename T, int NT, bool FULL, bool BLOCKS>
+// One unit of a level phase (one copy of each per tile count and kind of rows:
+// whole tiles, rows on pair boundaries (warps only: blocks gained nothing), neither; the kernel calls them).
+template <typename T, int NT, bool FULL, bool PAIR, bool BLOCKS>
 __device__ __noinline__ void rg_node_unit(const Problem<T>& p, const Level& lv, int u, unsigned char* smem,
                                           WarpGroup grp) {
   if constexpr (BLOCKS)
-    node_rows_body<T, NT, FULL, FULL>(grp, p, lv, 0, u, smem, 0, 1, true, true);
+    node_rows_body<T, NT, FULL, true, PAIR>(grp, p, lv, 0, u, smem, 0, 1, true, true);
   else
-    node_warp_body<T, NT, FULL>(p, lv, 0, u, smem);
+    node_warp_body<T, NT, FULL, PAIR>(p, lv, 0, u, smem);
 }
-template <typename T, int NT, bool FULL, bool BLOCKS>
+template <typename T, int NT, bool FULL, bool PAIR, bool BLOCKS>
 __device__ __noinline__ void rg_update_unit(const Problem<T>& p, const Level& lv, int task, unsigned char* smem,
                                             WarpGroup grp) {
   if constexpr (BLOCKS)
-    update_rows_body<T, NT, FULL, false>(grp, p, lv, 0, task, smem, 0, 1);
+    update_rows_body<T, NT, FULL, false, PAIR>(grp, p, lv, 0, task, smem, 0, 1);
   else
-    update_warp_body<T, NT, FULL>(p, lv, 0, task);
+    update_warp_body<T, NT, FULL, PAIR>(p, lv, 0, task);
 }
-template <typename T, int NT, bool FULL, bool BLOCKS, int MODE>
+template <typename T, int NT, bool FULL, bool PAIR, bool BLOCKS, int MODE>
 __device__ __noinline__ void rg_sweep_unit(const Problem<T>& p, const Level& lv, int u, unsigned char* smem,
                                            WarpGroup grp) {
-  sweep_rows_body<T, NT, FULL, MODE, true, BLOCKS>(grp, p, lv, 0, u, smem, kWaitNone);
+  sweep_rows_body<T, NT, FULL, MODE, true, BLOCKS, true, PAIR>(grp, p, lv, 0, u, smem, kWaitNone);
 }
 
-template <typename T, int MODE, int NT, bool FULL, bool BLOCKS>
+template <typename T, int MODE, int NT, bool FULL, bool PAIR, bool BLOCKS>
 __device__ __forceinline__ void rg_level_unit(const Problem<T>& p, int kind, int level, const Level& lv, int u,
                                               unsigned char* smem, const WarpGroup& grp) {
   if (kind == kRgNode) {
-    rg_node_unit<T, NT, FULL, BLOCKS>(p, lv, u, smem, grp);
+    rg_node_unit<T, NT, FULL, PAIR, BLOCKS>(p, lv, u, smem, grp);
   } else if (kind == kRgUpd) {
-    rg_update_unit<T, NT, FULL, BLOCKS>(p, lv, u, smem, grp);
+    rg_update_unit<T, NT, FULL, PAIR, BLOCKS>(p, lv, u, smem, grp);
     if (u + 1 <= lv.d - 1) {   // fill-in block of node t = u + 1
       grp.sync();
-      rg_update_unit<T, NT, FULL, BLOCKS>(p, lv, update_targets(p.N, lv) + u, smem, grp);
+      rg_update_unit<T, NT, FULL, PAIR, BLOCKS>(p, lv, update_targets(p.N, lv) + u, smem, grp);
     }
     // y_j -= F y_{j-s} + G^T y_{j+s} for target j = 2s(u+1) - 1
     grp.sync();
-    rg_sweep_unit<T, NT, FULL, BLOCKS, kModePull>(p, rg_level(p.N, level + 1), u, smem, grp);
+    rg_sweep_unit<T, NT, FULL, PAIR, BLOCKS, kModePull>(p, rg_level(p.N, level + 1), u, smem, grp);
   } else if (kind == kRgBwd) {
-    rg_sweep_unit<T, NT, FULL, BLOCKS, kModeBackward>(p, lv, u, smem, grp);
+    rg_sweep_unit<T, NT, FULL, PAIR, BLOCKS, kModeBackward>(p, lv, u, smem, grp);
   } else {
-    if constexpr (MODE != kRgPlain) rg_sweep_unit<T, NT, FULL, BLOCKS, kModeForward>(p, lv, u, smem, grp);
+    if constexpr (MODE != kRgPlain) rg_sweep_unit<T, NT, FULL, PAIR, BLOCKS, kModeForward>(p, lv, u, smem, grp);
   }
 }
 
@@ -402,21 +416,24 @@ __device__ void rg_run(const RgArgs<T>& a, int ii, int ph, int chunk, unsigned c
       continue;
     }
     const int nt = rg_nt(I.n);
-    const bool full = I.n == 8 * nt && pairs_ok(p, I.n);
-#define SOCU_RG_UNIT(NT)                                                                    \
-  if (full)                                                                                 \
-    rg_level_unit<T, MODE, NT, true, BLOCKS>(p, P.kind, P.level, lv, u, smem, grp);         \
-  else                                                                                      \
-    rg_level_unit<T, MODE, NT, false, BLOCKS>(p, P.kind, P.level, lv, u, smem, grp);
-    if (nt == 1) {
+    const bool pair = rows_paired(p, I.n);
+#define SOCU_RG_UNIT(NT)                                                                      \
+  case NT:                                                                                    \
+    if (pair && I.n == 8 * NT)                                                                \
+      rg_level_unit<T, MODE, NT, true, false, BLOCKS>(p, P.kind, P.level, lv, u, smem, grp);  \
+    else if (!BLOCKS && pair)                                                                 \
+      rg_level_unit<T, MODE, NT, false, !BLOCKS, BLOCKS>(p, P.kind, P.level, lv, u, smem, grp);  \
+    else                                                                                      \
+      rg_level_unit<T, MODE, NT, false, false, BLOCKS>(p, P.kind, P.level, lv, u, smem, grp); \
+    break;
+    switch (nt) {
       SOCU_RG_UNIT(1)
-    } else if (nt == 2) {
       SOCU_RG_UNIT(2)
-    } else if (nt == 4) {
+      SOCU_RG_UNIT(3)
       SOCU_RG_UNIT(4)
-    } else if (nt == 6) {
+      SOCU_RG_UNIT(5)
       SOCU_RG_UNIT(6)
-    } else {
+      SOCU_RG_UNIT(7)
       SOCU_RG_UNIT(8)
     }
 #undef SOCU_RG_UNIT

@@ -62,15 +62,19 @@ __device__ __forceinline__ void ldcg_pair(const T* p, bool vec, bool v0, bool v1
 }
 
 // MMA operand of an n x n block, row tile i, column tile kk: elements (r, c), (r, c + 1) with
-// r = 8i + g, c = 8kk + 2t; TR: of the block's transpose.  vec: the tile is whole (and pairs are aligned).
+// r = 8i + g, c = 8kk + 2t; TR: of the block's transpose.  vec: the tile is whole (and pairs are aligned);
+// pair: rows_paired.
 template <typename T, bool TR>
-__device__ __forceinline__ void block_frag(const T* M, int n, int i, int kk, bool vec, T& a0, T& a1) {
+__device__ __forceinline__ void block_frag(const T* M, int n, int i, int kk, bool vec, T& a0, T& a1,
+                                           bool pair = false) {
   const int lane = threadIdx.x & 31, r = 8 * i + (lane >> 2), c = 8 * kk + 2 * (lane & 3);
   if (TR) {
     const T* q = M + (c * n + r);   // (n <= 128: offsets inside a block fit 32 bits)
     a0 = vec || (r < n && c < n) ? q[0] : T(0);
     a1 = vec || (r < n && c + 1 < n) ? q[n] : T(0);
-  } else if (vec) {
+  } else if (pair && !vec && !(r < n && c < n)) {
+    a0 = a1 = T(0);
+  } else if (vec || pair) {
     if constexpr (sizeof(T) == 8) {
       const double2 v = *reinterpret_cast<const double2*>(M + (r * n + c));
       a0 = v.x;
@@ -91,11 +95,11 @@ __device__ __forceinline__ void block_frag(const T* M, int n, int i, int kk, boo
 //   a factor of its own (solve_diag).
 //   Else forward: C left of the diagonal tile, backward: C^T right of it.
 template <typename T, bool BWD, bool INV>
-__device__ __forceinline__ void solve_frag(const T* L, int n, int i, int kk, bool vec, T& a0, T& a1) {
+__device__ __forceinline__ void solve_frag(const T* L, int n, int i, int kk, bool vec, T& a0, T& a1, bool pair) {
   a0 = a1 = T(0);
   if (BWD ? kk < i : kk > i) return;
   if (kk != i) {
-    block_frag<T, INV != BWD>(L, n, i, kk, vec, a0, a1);
+    block_frag<T, INV != BWD>(L, n, i, kk, vec, a0, a1, pair);
     return;
   }
   if (!INV) return;
@@ -118,7 +122,8 @@ __device__ __forceinline__ T solve_diag(const T* L, int n, int i) {
 
 // One vector, its columns col0 .. col0 + cols (a multiple of 8).  ONE: the block has a warp per
 // row tile (else the warps loop over them and the blocks are read as they are used).
-template <typename T, int NT, bool FULL, int MODE, bool INV, bool ONE, class Group>
+template <typename T, int NT, bool FULL, int MODE, bool INV, bool ONE, bool EXACT = (NT <= 8), bool PAIR = false,
+          class Group>
 __device__ __forceinline__ void sweep_rows_body(const Group& grp, const Problem<T>& p, const Level& lv, int b, int task,
                                                 unsigned char* smem_raw, int wait, int col0 = 0,
                                                 int cols = 1 << 30) {
@@ -151,7 +156,7 @@ __device__ __forceinline__ void sweep_rows_body(const Group& grp, const Problem<
   }
   const T* L = p.Lb(b, j);
   T* yj = p.Xb(b, j);
-  const bool vec = FULL || pairs_ok(p, n);
+  const bool vec = FULL || (!EXACT && pairs_ok(p, n));
   const bool vecx = (m & 1) == 0 && (reinterpret_cast<uintptr_t>(p.X) & (2 * sizeof(T) - 1)) == 0;
   double* Zp = reinterpret_cast<double*>(smem_raw);
   double* Zq = Zp + 8 * NT * ldz;
@@ -167,7 +172,7 @@ __device__ __forceinline__ void sweep_rows_body(const Group& grp, const Problem<
     for (int e = 0; e < (KEEP ? NT : 4); ++e) {
       const int kk = INV || !BWD ? e0 + e : nta - 1 - e0 - e;
       T f0 = T(0), f1 = T(0);
-      if (kk >= 0 && kk < nta) solve_frag<T, BWD, INV>(L, n, warp, kk, vec, f0, f1);
+      if (kk >= 0 && kk < nta) solve_frag<T, BWD, INV>(L, n, warp, kk, vec, f0, f1, PAIR);
       fs[e][0] = f0;
       fs[e][1] = f1;
     }
@@ -175,7 +180,7 @@ __device__ __forceinline__ void sweep_rows_body(const Group& grp, const Problem<
   if (KEEP && warp < nta) {
 #pragma unroll
     for (int kk = 0; kk < NT; ++kk) {
-      if (P) block_frag<T, false>(P, n, warp, kk, vec && kk < nta, fp[KEEP ? kk : 0][0], fp[KEEP ? kk : 0][1]);
+      if (P) block_frag<T, false>(P, n, warp, kk, vec && kk < nta, fp[KEEP ? kk : 0][0], fp[KEEP ? kk : 0][1], PAIR);
       if (Q) block_frag<T, true>(Q, n, warp, kk, vec && kk < nta, fq[KEEP ? kk : 0][0], fq[KEEP ? kk : 0][1]);
     }
     if (solve) {
@@ -194,7 +199,7 @@ __device__ __forceinline__ void sweep_rows_body(const Group& grp, const Problem<
   double i0 = 0.0, i1 = 0.0;
   if (!INV && solve && warp < nta) {
     T d0, d1;
-    block_frag<T, false>(L, n, warp, warp, vec, d0, d1);
+    block_frag<T, false>(L, n, warp, warp, vec, d0, d1, PAIR);
     const int r = 8 * warp + g, c = 8 * warp + 2 * t;
     const double v0 = r >= n && r == c ? 1.0 : (double)d0, v1 = r >= n && r == c + 1 ? 1.0 : (double)d1;
     if (SUBST) {
@@ -285,7 +290,7 @@ __device__ __forceinline__ void sweep_rows_body(const Group& grp, const Problem<
           for (int h = 0; h < BK; ++h) {
             f[h][0] = f[h][1] = f[h][2] = f[h][3] = T(0);
             if (k0 + h < nta) {
-              if (P) block_frag<T, false>(P, n, i, k0 + h, vec, f[h][0], f[h][1]);
+              if (P) block_frag<T, false>(P, n, i, k0 + h, vec, f[h][0], f[h][1], PAIR);
               if (Q) block_frag<T, true>(Q, n, i, k0 + h, vec, f[h][2], f[h][3]);
             }
           }
@@ -345,7 +350,7 @@ __device__ __forceinline__ void sweep_rows_body(const Group& grp, const Problem<
 #pragma unroll
           for (int kk = 0; kk < NT; ++kk) {
             T f0 = T(0), f1 = T(0);
-            if (kk < nta) solve_frag<T, BWD, INV>(L, n, i, kk, vec, f0, f1);
+            if (kk < nta) solve_frag<T, BWD, INV>(L, n, i, kk, vec, f0, f1, PAIR);
             fr[ONE ? 0 : kk][0] = f0;
             fr[ONE ? 0 : kk][1] = f1;
           }

@@ -55,7 +55,7 @@ __global__ void __launch_bounds__(32 * NT) k_top(Problem<T> p, const __grid_cons
     const Level& L = tl.fl[li];
     for (int t = rank; t < sweep_tasks<kModeForward>(p.N, L); t += C) {
       __syncthreads();
-      sweep_rows_body<T, NT, false, kModeForward, INV, true>(BlockGroup{}, p, L, b, t, smem_raw, kWaitNone);
+      sweep_rows_body<T, NT, false, kModeForward, INV, true, false>(BlockGroup{}, p, L, b, t, smem_raw, kWaitNone);
     }
     if (li + 1 < tl.fwd_n || tl.bwd_n > 0) {
       cluster_arrive();
@@ -66,7 +66,7 @@ __global__ void __launch_bounds__(32 * NT) k_top(Problem<T> p, const __grid_cons
     const Level& L = tl.bl[li];
     for (int t = rank; t < L.d; t += C) {
       __syncthreads();
-      sweep_rows_body<T, NT, false, kModeBackward, INV, true>(BlockGroup{}, p, L, b, t, smem_raw, kWaitNone);
+      sweep_rows_body<T, NT, false, kModeBackward, INV, true, false>(BlockGroup{}, p, L, b, t, smem_raw, kWaitNone);
     }
     if (li > 0) {
       cluster_arrive();

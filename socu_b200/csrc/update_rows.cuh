@@ -88,7 +88,7 @@ __device__ __forceinline__ void upd_step(double (&acc)[NT][2], const T* fk, cons
 }
 
 // One output block, `task` in [0, update_blocks).
-template <typename T, int NT, bool FULL, bool SPLIT, class Group>
+template <typename T, int NT, bool FULL, bool SPLIT, bool PAIR = false, class Group>
 __device__ __forceinline__ void update_rows_body(const Group& grp, const Problem<T>& p, const Level& lv, int b, int task,
                                                  unsigned char* smem_raw, int q, int splits) {
   constexpr int es = sizeof(T), ldg = upd_ldg(NT, es);
@@ -112,7 +112,7 @@ __device__ __forceinline__ void update_rows_body(const Group& grp, const Problem
     G = p.Eb(b, lv.oc + 2 * f - 1);
     Out = p.Eb(b, lv.on + f - 1);
   }
-  const bool vec = FULL || pairs_ok(p, n);
+  const bool vec = FULL || (NT > 8 && pairs_ok(p, n));
   const int part = warp % splits, step = splits * (W / splits);
   const int first = q + splits * (warp / splits);       // this warp's first row tile
   const int last = q + splits * ((nta - 1 - q) / splits);  // the block's last row tile
@@ -154,7 +154,7 @@ __device__ __forceinline__ void update_rows_body(const Group& grp, const Problem
       acc[jj][0] = acc[jj][1] = 0.0;
       const int j = part + splits * jj, c = 8 * j + 2 * t;
       if (kAhead && on && j <= jmax)
-        load_raw(Out + (long long)gr * n + c, vec, gr < n && c < n, gr < n && c + 1 < n, out[kAhead ? jj : 0]);
+        load_raw(Out + (long long)gr * n + c, vec, gr < n && c < n, gr < n && c + 1 < n, out[kAhead ? jj : 0], PAIR);
     }
     for (int c = 0; c < chunks; ++c) {
       if (!staged) {
@@ -209,7 +209,7 @@ __device__ __forceinline__ void update_rows_body(const Group& grp, const Problem
           }
           store_pair(Out + (long long)gr * n + c, vec && !diag, gr < n && c < n && (!diag || c <= gr),
                      gr < n && c + 1 < n && (!diag || c + 1 <= gr), (double)o[0] - acc[jj][0],
-                     (double)o[1] - acc[jj][1]);
+                     (double)o[1] - acc[jj][1], PAIR && !diag);
         }
       }
     }

@@ -71,7 +71,7 @@ __device__ __forceinline__ void warp_rows_solve(double (&acc)[R][NT][2], const T
 // One node (with its right-hand sides, keeping the inverse): as node_rows_body.
 // The factor is left-looking: column k of tiles is L_i's column less the products
 // of the columns before it, so only one column is in registers at a time.
-template <typename T, int NT, bool FULL>
+template <typename T, int NT, bool FULL, bool PAIR>
 __device__ __forceinline__ void node_warp_body(const Problem<T>& p, const Level& lv, int b, int t,
                                                unsigned char* smem_raw) {
   const int lane = threadIdx.x & 31, g = lane >> 2, tq = lane & 3;
@@ -81,7 +81,7 @@ __device__ __forceinline__ void node_warp_body(const Problem<T>& p, const Level&
   double* Iv = Ls + 64 * (NT * (NT - 1) / 2);
   T* Ct = reinterpret_cast<T*>(Iv + 64 * NT);
   T* Li = p.Lb(b, i);
-  const bool vec = FULL || pairs_ok(p, n);
+  constexpr bool vec = FULL;
   // the coupling blocks, needed after the factor: into L2 meanwhile
   T* R = right ? p.Eb(b, lv.oc + 2 * t) : nullptr;
   T* Lf = left ? p.Eb(b, lv.oc + 2 * t - 1) : nullptr;
@@ -97,7 +97,7 @@ __device__ __forceinline__ void node_warp_body(const Problem<T>& p, const Level&
       for (int j = 0; j <= r; ++j) {
         const int gr = 8 * r + g, c = 8 * j + 2 * tq, e = r * (r + 1) / 2 + j;
         x[e][0] = x[e][1] = T(0);
-        if (r < nta) load_raw(Li + (gr * n + c), vec, gr < n && c < n, gr < n && c + 1 < n, x[e]);
+        if (r < nta) load_raw(Li + (gr * n + c), vec, gr < n && c < n, gr < n && c + 1 < n, x[e], PAIR);
         if (!FULL && gr >= n) {
           if (c == gr) x[e][0] = T(1);
           if (c + 1 == gr) x[e][1] = T(1);
@@ -148,13 +148,14 @@ __device__ __forceinline__ void node_warp_body(const Problem<T>& p, const Level&
         rows_panel(p0, p1, acc[r][0], acc[r][1], f);
         tile_put(Ls + 64 * ((k + r) * (k + r - 1) / 2 + k), p0, p1);
         const int gr = 8 * (k + r) + g, c = 8 * k + 2 * tq;
-        store_pair(Li + (long long)gr * n + c, vec, gr < n && c < n, gr < n && c + 1 < n, p0, p1);
+        store_pair(Li + (long long)gr * n + c, vec, gr < n && c < n, gr < n && c + 1 < n, p0, p1, PAIR);
       }
     // diagonal tile: C_kk and, above the diagonal, W^T
     const int gr = 8 * k + g, c = 8 * k + 2 * tq;
     const double c0 = 2 * tq == g ? f.d0 : f.cv.x, c1 = 2 * tq + 1 == g ? f.d1 : f.cv.y;
     store_pair(Li + (long long)gr * n + c, vec, gr < n && c < n, gr < n && c + 1 < n,
-               2 * tq <= g ? c0 : Iv[64 * k + 8 * (2 * tq) + g], 2 * tq + 1 <= g ? c1 : Iv[64 * k + 8 * (2 * tq + 1) + g]);
+               2 * tq <= g ? c0 : Iv[64 * k + 8 * (2 * tq) + g], 2 * tq + 1 <= g ? c1 : Iv[64 * k + 8 * (2 * tq + 1) + g],
+               PAIR);
     __syncwarp();
   }
   // rows of the right slot, columns of the left slot and of y, two tiles at a time
@@ -186,11 +187,11 @@ __device__ __forceinline__ void node_warp_body(const Problem<T>& p, const Level&
     const RowSrc<T> s0 = source(v), s1 = source(v + 1);
     T x[2][NT][2];
     double acc[2][NT][2];
-    rows_load<T, NT>(x[0], s0, n, vec);
-    rows_load<T, NT>(x[1], s1, n, vec);
+    rows_load<T, NT, PAIR>(x[0], s0, n, vec);
+    rows_load<T, NT, PAIR>(x[1], s1, n, vec);
     warp_rows_solve<T, NT, 2>(acc, x, 0, nta, Ls, Iv, Ct);
-    rows_store<T, NT>(acc[0], s0, n, vec);
-    rows_store<T, NT>(acc[1], s1, n, vec);
+    rows_store<T, NT, PAIR>(acc[0], s0, n, vec);
+    rows_store<T, NT, PAIR>(acc[1], s1, n, vec);
   }
   // rows of the identity: W^T right of the diagonal tiles (the last row tile has none)
 #pragma unroll 1
@@ -204,15 +205,15 @@ __device__ __forceinline__ void node_warp_body(const Problem<T>& p, const Level&
     o.k0 = c;
     T x[1][NT][2];
     double acc[1][NT][2];
-    rows_load<T, NT>(x[0], o, n, vec);
+    rows_load<T, NT, PAIR>(x[0], o, n, vec);
     warp_rows_solve<T, NT, 1>(acc, x, c, nta, Ls, Iv, Ct);
-    rows_store<T, NT>(acc[0], o, n, vec);
+    rows_store<T, NT, PAIR>(acc[0], o, n, vec);
   }
 }
 
 // One output block: as update_rows_body, operands straight from global memory,
 // two row tiles of the output at a time (each operand feeds both).
-template <typename T, int NT, bool FULL>
+template <typename T, int NT, bool FULL, bool PAIR>
 __device__ __forceinline__ void update_warp_body(const Problem<T>& p, const Level& lv, int b, int task) {
   const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
   const int n = FULL ? 8 * NT : p.n, N = p.N, s = lv.s, nta = (n + 7) >> 3, U = update_targets(N, lv);
@@ -231,7 +232,7 @@ __device__ __forceinline__ void update_warp_body(const Problem<T>& p, const Leve
     G = p.Eb(b, lv.oc + 2 * f - 1);
     Out = p.Eb(b, lv.on + f - 1);
   }
-  const bool vec = FULL || pairs_ok(p, n);
+  constexpr bool vec = FULL;
   warp_prefetch(Out, n * n);
 #pragma unroll 1
   for (int i = 0; i < nta; i += 2) {
@@ -250,17 +251,17 @@ __device__ __forceinline__ void update_warp_body(const Problem<T>& p, const Leve
 #pragma unroll
       for (int r = 0; r < 2; ++r) {
         if (tr)
-          block_frag<T, true>(G, n, i + r, kk, vec && i + r < nta, a[r][0], a[r][1]);
+          block_frag<T, true>(G, n, i + r, kk, vec && i + r < nta, a[r][0], a[r][1], PAIR);
         else
-          block_frag<T, false>(F, n, i + r, kk, vec && i + r < nta, a[r][0], a[r][1]);
+          block_frag<T, false>(F, n, i + r, kk, vec && i + r < nta, a[r][0], a[r][1], PAIR);
       }
 #pragma unroll
       for (int j = 0; j < NT; ++j)
         if (j <= jmax) {
           if (part == 1)
-            block_frag<T, true>(G, n, j, kk, vec, x[j][0], x[j][1]);
+            block_frag<T, true>(G, n, j, kk, vec, x[j][0], x[j][1], PAIR);
           else
-            block_frag<T, false>(F, n, j, kk, vec, x[j][0], x[j][1]);
+            block_frag<T, false>(F, n, j, kk, vec, x[j][0], x[j][1], PAIR);
         }
 #pragma unroll
       for (int e = 0; e < 2; ++e)
@@ -279,7 +280,7 @@ __device__ __forceinline__ void update_warp_body(const Problem<T>& p, const Leve
       for (int j = 0; j < NT; ++j)
         if (j <= jmax) {
           const int c = 8 * j + 2 * t;
-          load_raw(Out + (long long)gr * n + c, vec && i + r < nta, gr < n && c < n, gr < n && c + 1 < n, o[j]);
+          load_raw(Out + (long long)gr * n + c, vec && i + r < nta, gr < n && c < n, gr < n && c + 1 < n, o[j], PAIR);
         }
 #pragma unroll
       for (int j = 0; j < NT; ++j)
@@ -288,7 +289,7 @@ __device__ __forceinline__ void update_warp_body(const Problem<T>& p, const Leve
           const bool diag = target && j == i + r;   // only the lower triangle of a target is written
           store_pair(Out + (long long)gr * n + c, vec && i + r < nta && !diag, gr < n && c < n && (!diag || c <= gr),
                      gr < n && c + 1 < n && (!diag || c + 1 <= gr), (double)o[j][0] - acc[r][j][0],
-                     (double)o[j][1] - acc[r][j][1]);
+                     (double)o[j][1] - acc[r][j][1], PAIR && !diag);
         }
     }
   }
