@@ -28,7 +28,8 @@ is timed as the median of graph-launched runs of the tuned operation on a
 synthetic system of the requested shape (README construction, inputs restored
 by a device copy outside the timed region).  A candidate replaces the
 incumbent only when it is faster by more than ``min_gain`` (default 2 %), so
-noise does not churn the table.
+noise does not churn the table.  A knob that chooses nothing is run once per
+value, for its result, and never wins.
 
 Cache: JSON at ``$SOCU_TUNE_CACHE`` (default ``~/.cache/socu_b200/tune.json``),
 entries keyed by device name, dtype, n and n_rhs.  ``load_cache()`` installs
@@ -63,6 +64,8 @@ _VALUES = {
     "update_tensor_cores": (0, 1, 2),
     "node_tensor_cores": (0, 1, 3),
 }
+# knobs that some kernel reads (float, n <= 128)
+EFFECTIVE = ("update_tensor_cores", "node_tensor_cores")
 _loaded = set()
 _tuned = set()
 _lock = threading.Lock()
@@ -153,9 +156,9 @@ def save_entry(device_name: str, dtype, n: int, n_rhs: int, settings: dict, ms: 
 
 
 def candidates(n: int, n_rhs: int, dtype) -> dict:
-    """Values worth trying per knob for this shape (knobs that cannot matter are
-    left out: the blocked update tile exists only for n > 64, and the sweep
-    product switch only for float factors with n <= 64)."""
+    """Values of every knob that a shape takes (the update tile for n > 64, the
+    sweep product switch for float with n <= 64, the tensor-core switches for
+    float with n <= 128).  Only those of EFFECTIVE can change what runs."""
     out = {}
     for k in KNOBS:
         vals = list(_VALUES[k])
@@ -226,13 +229,14 @@ def tune(n: int, n_rhs: int, dtype=torch.float64, horizon: int = 256, batch: int
                 continue
             trial = dict(best)
             trial[knob] = v
-            ms, x = _time_op(op, tdt, trial, L0, E0, b0, reps, warmup)
+            live = knob in EFFECTIVE
+            ms, x = _time_op(op, tdt, trial, L0, E0, b0, reps if live else 1, warmup if live else 0)
             if check:
                 err = float((x - x_ref).abs().max()) / scale
                 if not err <= tol:
                     raise RuntimeError(f"autotune: settings {trial} changed the result by {err:.3e}")
             trials.append((trial, ms))
-            if ms < best_ms * (1.0 - min_gain):
+            if live and ms < best_ms * (1.0 - min_gain):
                 best, best_ms = trial, ms
     install(tdt, n, n_rhs, best)
     if save:
