@@ -408,7 +408,7 @@ template <bool REFINE>
 cudaError_t launch_residual_rows(const RefineArgs& a, cudaStream_t st, bool pdl) {
   const int gr = residual_groups(a.m);
   const size_t smem = smem_residual_x_elems(a.n, gr) * sizeof(double);
-  const unsigned blocks = (unsigned)((long long)a.B * a.N), threads = (unsigned)residual_rows_threads(a.n, a.m);
+  const unsigned blocks = (unsigned)((long long)a.B * a.N), threads = (unsigned)residual_rows_threads(a.n);
   void (*k)(RefineArgs) = gr == 1 ? k_residual_rows<REFINE, 1> : (gr == 2 ? k_residual_rows<REFINE, 2> : k_residual_rows<REFINE, 4>);
   const cudaError_t e = prepare(k, smem);
   if (e == cudaSuccess) launch(k, blocks, threads, smem, st, pdl, a);
@@ -704,7 +704,8 @@ int validate(socu_op op, socu_dtype dtype, const void* L, const void* E, const v
   d->n = (int)n;
   d->m = needs_x ? (int)n_rhs : 0;
   d->S = (int)S;
-  // grid sizes of the widest launches must fit (smallest update tile: 16)
+  // grid sizes of the widest launches must fit (with room: the bound of 16-row output tiles, which
+  // callers have met so far)
   const int nt = ceil_div(d->n, 16);
   const long long per_node = 2LL * nt * nt + 1;
   const long long widest = (long long)d->B * ((d->N + 1) / 2) * per_node + 1;

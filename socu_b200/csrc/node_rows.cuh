@@ -38,8 +38,6 @@
 
 namespace socu {
 
-constexpr int kRowsMaxN = 128;
-__host__ __device__ inline bool node_uses_rows(int n) { return n <= kRowsMaxN; }
 // 8-column tiles: exact up to 64, then even counts (fewer instantiations)
 __host__ __device__ inline int rows_nt(int n) {
   const int t = (n + 7) / 8;

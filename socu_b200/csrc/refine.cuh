@@ -570,7 +570,7 @@ __device__ __forceinline__ void residual_staged_body(const RefineArgs& a, int bi
 }
 
 // (at most 256: warps loop over the 8-row tiles of larger blocks)
-__host__ __device__ inline int residual_rows_threads(int n, int) {
+__host__ __device__ inline int residual_rows_threads(int n) {
   const int t = 32 * ((n + 7) / 8);
   return t < 256 ? t : 256;
 }

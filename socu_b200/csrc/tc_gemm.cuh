@@ -34,7 +34,8 @@ __device__ __forceinline__ uint32_t saddr(const void* p) {
 
 // Error word of the asynchronous units on one device: 1 a tensor-core wait
 // ran out (that kernel skipped its result).
-static __device__ int g_tc_error;   // one per translation unit; socu_tc_error reads them all
+static __device__ int g_tc_error;   // one per translation unit; the solver's tensor-core kernels are all in
+                                    // capi.cu's, which socu_tc_error reads
 
 // ---- instruction / shared-memory descriptors --------------------------------
 // kind::tf32 instruction descriptor: D F32 (bits 4-5 = 1), A and B TF32
