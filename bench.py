@@ -47,10 +47,10 @@ RAGGED_COUNT, RAGGED_SEED = 4096, 0
 # DRAM bytes (read + write) per launch of the float level node and of the float
 # backward sweep of a factor_and_solve of this shape, averaged over its 11
 # levels: ncu capture of `bench.py --ncu-case node` (4 systems, so that the
-# float blocks exceed L2), 246.4 and 201.2 MB over the 11 launches, per system
+# float blocks exceed L2), 245.5 and 201.4 MB over the 11 launches, per system
 # (profiles/rows_f32_N1024_n64_m8_B4.md)
-NODE_TRAFFIC_BYTES = 246.40e6 / 4 / 11
-TRAFFIC_BYTES = 201.16e6 / 4 / 11
+NODE_TRAFFIC_BYTES = 245.49e6 / 4 / 11
+TRAFFIC_BYTES = 201.42e6 / 4 / 11
 TRAFFIC_NOTE = ("ncu dram__bytes_read.sum + dram__bytes_write.sum of the 11 backward launches of "
                 "bench.py --ncu-case node (4 systems, inputs > L2), per system and launch; "
                 "profiles/rows_f32_N1024_n64_m8_B4.md")

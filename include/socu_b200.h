@@ -192,7 +192,7 @@ int socu_tuning_clear(void);
 typedef enum socu_kernel_kind {
   SOCU_KIND_NODE = 0,          /* level node: potrf + coupling solves (+ forward step) */
   SOCU_KIND_UPDATE = 1,        /* Schur updates and fill-in */
-  SOCU_KIND_PULL = 2,          /* forward coupling updates fused into factor_and_solve */
+  SOCU_KIND_PULL = 2,          /* forward coupling updates fused into factor_and_solve (where not in the update's launch) */
   SOCU_KIND_FORWARD = 3,       /* forward sweep */
   SOCU_KIND_BACKWARD = 4,      /* backward sweep */
   SOCU_KIND_REFINE_SETUP = 5,  /* refinement: state reset, float copies, norms */

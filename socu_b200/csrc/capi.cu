@@ -347,8 +347,8 @@ int cluster_capacity(K kernel, int cluster, int threads, size_t smem) {
 // k_top instead of one launch per level.  Off by default: measured on B200,
 // the per-level launches of a graph (programmatic dependent launch, blocks
 // loaded before the dependency wait) are faster at every shape tried -- a
-// float solve on an inverse-carrying factor at N=1024, n=64, m=8 takes 132 us
-// with a launch per level vs 153 us with k_top, at N=20, n=16, m=1 29 vs 35 us
+// float solve on an inverse-carrying factor at N=1024, n=64, m=8 takes 96 us
+// with a launch per level vs 114 us with k_top, at N=20, n=16, m=1 26 vs 34 us
 // (one k_top launch instead of ten): the cluster barrier and the L2 reads of
 // the vectors after it cost more per level than a kernel boundary.
 bool top_sweep_enabled() {
@@ -449,13 +449,12 @@ int enqueue(socu_op op, const Problem<T>& p, cudaStream_t st, long long* count, 
   // Schur updates of float factors on the tcgen05 tensor cores (3xTF32), on
   // request: the FP64-pipe updates (exact products of the float operands,
   // FP64 sums) keep the float factor accurate enough for the reference's
-  // float tolerances and for three refinement rounds instead of five
+  // float tolerances and for two refinement rounds
   const bool upd_tc = sizeof(T) == 4 && update_tc_ok(n) && cfg.update_tensor_cores == 1;
   const size_t su_tc = (size_t)smem_update_tc_bytes(n);
   // products of float level nodes on the tcgen05 tensor cores: on request
   // (node_tensor_cores = 1) at every level, or with node_tensor_cores = 3 only
-  // on levels wide enough to be throughput-bound (at least 4 nodes per SM),
-  // where the SIMT products cost more issue slots than the MMA round trips
+  // on levels wide enough to be throughput-bound (at least 4 nodes per SM)
   const bool node_tc_any = sizeof(T) == 4 && node_tc_ok(n, withY ? p.m : 0) &&
                            (cfg.node_tensor_cores == 1 || cfg.node_tensor_cores == 3) &&
                            (long long)smem_node_tc_bytes(n, withY ? p.m : 0) <= (long long)max_smem_optin();

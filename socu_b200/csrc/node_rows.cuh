@@ -26,12 +26,14 @@
 // no barrier (phase 2); the first one is loaded when the warp leaves phase 1.
 //
 // Bound by the latency of phase 1: per step one tile factor (770 cycles FP64,
-// 556 float) and two dependent MMA pairs, about 1200 / 950 cycles.  The blocks
+// 556 float), the panel's three dependent MMA pairs (26 cycles each half) and the
+// next diagonal tile's.  The blocks
 // of a cluster repeat phase 1 and share out phase 2; the cluster barrier keeps
 // one block from overwriting L_i before the others have read it.  Measured,
 // all level nodes of one factor_and_solve (event-timed launches), against the
 // blocked solve in shared memory that it replaces: N=1024, n=64, m=8 FP64
-// 409 -> 214 us, float 373 -> 212 us; N=2048, n=128, m=32 FP64 3308 -> 995 us.
+// 409 -> 231 us, float 373 -> 208 us; N=2048, n=128, m=32 FP64 3308 -> 1203 us
+// (201, 178 and 917 us with the inverse's product alone, see rows_panel).
 #pragma once
 
 #include "nd_kernels.cuh"
@@ -92,8 +94,8 @@ __device__ __forceinline__ T pivot_rsqrt(T d) {
 // column l % 8); returns the last pivot's factor.  Every lane of the warp factors
 // the whole tile: the chain is 8 times rsqrt -> multiply -> subtract, about 70
 // cycles each in FP64, with no exchange between lanes; the stores go out beside it.
-// Measured per tile: 770 cycles FP64, 556 float; spread over the lanes instead
-// (16 shuffles a column, which issue every 4.3 cycles) 1500 and 790.
+// Measured per tile, without the stores: 770 cycles FP64, 556 float; spread over
+// the lanes instead (16 shuffles a column, which issue every 4.3 cycles) 1500 and 790.
 template <typename T, bool FAST>
 __device__ __forceinline__ T chol8_tile(T* S, double* Ivk) {
   const int lane = threadIdx.x & 31, col = lane & 7;
@@ -301,7 +303,10 @@ __device__ __forceinline__ DiagFrag diag_frag(const double* Ik, const T* Ck) {
 // X tile row: P = X_k C_kk^{-T}.  The product with the explicit inverse has a residual that grows
 // with the tile's condition; one correction, P += (X - P C_kk^T) Inv_k^T, brings it down to that of
 // a substitution.  The diagonal's part of the residual is one fused operation, so that what cancels
-// is not rounded before, and the correction is summed by itself and added once.
+// is not rounded before, and the correction is summed by itself and added once.  Componentwise
+// backward error of C and F at a tile of condition 1e4: over 1000 u without it, a few u with it; true
+// error of F at n = 16: 1.5e-16 without, 1.3e-16 corrected in the product's own accumulators, 1.0e-16
+// so.  N = 1024, n = 64, m = 8 FP64 368, 396 and 404 us.
 __device__ __forceinline__ void rows_panel(double& p0, double& p1, double x0, double x1, const DiagFrag& f) {
   double s0 = 0.0, s1 = 0.0, q0 = 0.0, q1 = 0.0;
   p0 = p1 = 0.0;
@@ -385,7 +390,8 @@ __device__ __forceinline__ void rows_update(double (&acc)[NT][2], int j0, double
 }
 
 // Sums from zero where the registers hold a row tile twice: X less the sum of the products is rounded
-// once at X's size.  (Larger blocks subtract every product from X, as a substitution does.)
+// once at X's size (true error of F at n = 64: 3.0e-16 -> 1.5e-16).  Larger blocks subtract every
+// product from X, as a substitution does: at n = 128 the second copy spilt.
 __host__ __device__ constexpr bool rows_from_zero(int nt) { return nt <= 8; }
 
 // All steps of one row tile x against the finished factor, results in acc (FROM0: k0 is 0, and no
